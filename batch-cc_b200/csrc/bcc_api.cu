@@ -134,7 +134,80 @@ Rec rec_cuboid(const float* b, bool z_aligned) {
     return make_rec(c, A, h, 0.0);
 }
 
+// Does the record's distance function bound how distances change (1-Lipschitz,
+// all values finite, no negative radius)?  The caller's axes are taken as given;
+// only near-orthonormal ones, or shorter, do.  By Gershgorin the largest
+// eigenvalue of A A^T is at most the largest absolute row sum.
+bool regular_rec(const Rec& r) {
+    for (int k = 0; k < 16; ++k)
+        if (!std::isfinite(r.v[k])) return false;
+    if (r.v[3] < 0.0f) return false;
+    for (int i = 0; i < 3; ++i) {
+        double row = 0.0;
+        for (int j = 0; j < 3; ++j) {
+            double d = 0.0;
+            for (int k = 0; k < 3; ++k) d += (double)r.v[4 + 4 * i + k] * r.v[4 + 4 * j + k];
+            row += std::fabs(d);
+        }
+        if (!(row <= 1.0001)) return false;
+    }
+    return true;
+}
+
 int clamp_tile(int v, int lo, int hi) { return std::max(lo, std::min(hi, v)); }
+
+// Probe grids of the uploaded set for a robot's reach, built on the first check
+// that uses them after an upload (or after a check of another robot): cubic
+// voxels, as many as kMaxVoxels allow.  Stream-ordered on st; the caller
+// synchronises st before any other stream can use the grids.  Without the
+// memory for them checks run unprobed.
+bcc::ProbeGrid probe_grid(bcc_ctx* ctx, const bcc::RobotOps* ops, cudaStream_t st) {
+    bcc::ProbeGrid& g = ctx->probe;
+    if (ctx->probe_robot == ops->robot && ctx->probe_version == ctx->env_version) return g;
+    float lo[3], hi[3];
+    ops->reach(lo, hi);
+    double ext[3], h = 0.0;
+    for (int a = 0; a < 3; ++a) ext[a] = std::max(1e-3, (double)hi[a] - lo[a]);
+    int n[3];
+    for (h = std::cbrt(ext[0] * ext[1] * ext[2] / bcc::kMaxVoxels);; h *= 1.01) {
+        for (int a = 0; a < 3; ++a) n[a] = std::max(1, (int)std::ceil(ext[a] / h));
+        if ((long long)n[0] * n[1] * n[2] <= bcc::kMaxVoxels) break;
+    }
+    g = bcc::ProbeGrid{};
+    g.nx = n[0];
+    g.ny = n[1];
+    g.nz = n[2];
+    g.h = (float)h;
+    g.inv_h = (float)(1.0 / h);
+    g.ox = (float)(0.5 * (lo[0] + hi[0]) - 0.5 * (n[0] - 1) * h);
+    g.oy = (float)(0.5 * (lo[1] + hi[1]) - 0.5 * (n[1] - 1) * h);
+    g.oz = (float)(0.5 * (lo[2] + hi[2]) - 0.5 * (n[2] - 1) * h);
+    g.stride = (uint32_t)((n[0] * n[1] * n[2] * 2 + 15) & ~15);
+    ctx->probe_robot = ops->robot;
+    ctx->probe_version = ctx->env_version;
+    if (ctx->vox.ensure((size_t)g.stride * ctx->num_envs) != cudaSuccess ||
+        bcc::launch_probe_grid(ctx->blobs.as<float4>(), ctx->env_hdr.as<float4>(), ctx->num_envs, g,
+                               ctx->vox.as<uint16_t>(), st) != cudaSuccess) {
+        cudaGetLastError();  // not an error of the check
+        return g;            // vox stays null
+    }
+    g.vox = ctx->vox.as<uint16_t>();
+    return g;
+}
+
+// The launch shape of a check of E edges: the context's once it was set or
+// tuned, else by size.  Below kProbeMinPairs pairs the probe's extra kernels cost
+// as much as the walks they save.
+constexpr long long kProbeMinPairs = 1 << 14;
+
+bcc::Tune launch_shape(const bcc_ctx* ctx, int E) {
+    bcc::Tune t = ctx->tune;
+    if (t.tuned) return t;
+    t.persistent = (long long)ctx->num_envs * E >= kProbeMinPairs ? 1 : 0;
+    // Large records leave room for fewer CTAs an SM: eight warps share one copy.
+    t.warps = t.persistent && ctx->blob_smem <= 8192 ? 4 : 8;
+    return t;
+}
 
 // Discretisation, sample offsets and every per-call buffer of a check; fills
 // `a` up to (not including) the FK / self / swept / check launches.
@@ -147,6 +220,7 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
         return fail(ctx, BCC_ERR_LIMIT, "an environment has more primitives than this robot's checker supports");
     if (!ctx->tables[r]) {
         BCC_CUDA(ctx, ops->upload_tables());
+        BCC_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));  // (see bcc_upload_envs)
         ctx->tables[r] = true;
     }
     a = bcc::PipelineArgs{};
@@ -160,6 +234,32 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     BCC_CUDA(ctx, ctx->swept.ensure(sizeof(float4) * 2 * (size_t)G * E));
     BCC_CUDA(ctx, ctx->edge_tri.ensure(sizeof(int) * (size_t)G * E));
     BCC_CUDA(ctx, ctx->error_flag.ensure(sizeof(int)));
+    // Probed checks: grids, middle spheres and the queue, all or none.
+    const bcc::Tune tune = launch_shape(ctx, E);
+    if (d_results && tune.persistent && (long long)E <= bcc::kQueuePairs &&
+        ctx->blob_smem + bcc::kProbeBatch * sizeof(uint2) + 2 * bcc::kMaxVoxels <= 200 * 1024) {
+        const long long cap = std::min<long long>((long long)ctx->num_envs * E, bcc::kQueuePairs);
+        const long long slab = cap / E;
+        // Pairs per work item: few where there are few pairs, so that the undecided
+        // ones spread over the CTAs (12 .. 24 against 96 pairs: plain 0.14 against 0.23
+        // ms, Fetch 0.43 against 0.54, Baxter 0.30 against 0.45), many where an item's
+        // barriers and staging count (uneven Panda 1.39 ms at 96 against 1.64 at 12).
+        const int chunk = (int)std::max<long long>(12, std::min<long long>(96, (long long)ctx->num_envs * E / 100000 / 12 * 12));
+        // items: every full chunk, and one part chunk per probe CTA
+        const size_t items = (size_t)(cap / chunk + slab * ((E + bcc::kProbeBatch - 1) / bcc::kProbeBatch));
+        a.probe = probe_grid(ctx, ops, st);
+        if (a.probe.vox && ctx->mid.ensure(sizeof(float4) * (size_t)G * E) == cudaSuccess &&
+            ctx->pq_entries.ensure(sizeof(uint2) * (size_t)cap) == cudaSuccess &&
+            ctx->pq_items.ensure(sizeof(int4) * items) == cudaSuccess &&
+            ctx->pq_head.ensure(16 * (size_t)((ctx->num_envs + slab - 1) / slab)) == cudaSuccess) {
+            a.mid = ctx->mid.as<float4>();
+            a.queue = bcc::ProbeQueue{ctx->pq_entries.as<uint2>(), ctx->pq_items.as<int4>(), ctx->pq_head.as<int>(),
+                                      cap, chunk};
+        } else {
+            cudaGetLastError();  // no memory for it: one pass over all pairs
+            a.probe = bcc::ProbeGrid{};
+        }
+    }
     a.steps = ctx->steps.as<int>();
     a.offs = ctx->offs.as<int>();
     a.edge_self = ctx->edge_self.as<int>();
@@ -188,6 +288,8 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     BCC_CUDA(ctx, ctx->table.ensure(sizeof(float4) * (size_t)NS * tiles * bcc::kMaxTableTile));
     BCC_CUDA(ctx, ctx->row_edge.ensure(sizeof(int) * (size_t)std::max(total, 1)));
     a.total_rows = total;
+    BCC_CUDA(ctx, ctx->seg.ensure(sizeof(float2) * (size_t)G * (std::max(total, bcc::kSegment) / bcc::kSegment)));
+    a.seg = ctx->seg.as<float2>();
     a.table = ctx->table.as<float4>();
     a.row_edge = ctx->row_edge.as<int>();
     a.blobs = ctx->blobs.as<float4>();
@@ -197,19 +299,18 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     a.blob_smem = ctx->blob_smem;
     a.d_results = d_results;
     // Tile: warps per CTA (tuned, limited by shared memory); edges per CTA.
-    int warps = ctx->tune.warps;
+    int warps = tune.warps;
     while (warps > 1 && bcc::check_smem_bytes(a.max_prims, G, a.blob_smem, warps) > 200 * 1024) warps >>= 1;
     if (bcc::check_smem_bytes(a.max_prims, G, a.blob_smem, warps) > 220 * 1024)
         return fail(ctx, BCC_ERR_LIMIT, "an environment has too many primitives for shared-memory staging");
     a.warps = warps;
-    a.edges_per_cta = clamp_tile(opts && opts->tile_override > 0 ? opts->tile_override : ctx->tune.edges_per_cta, 1,
+    a.edges_per_cta = clamp_tile(opts && opts->tile_override > 0 ? opts->tile_override : tune.edges_per_cta, 1,
                                  1 << 20);
     if ((E + a.edges_per_cta - 1) / a.edges_per_cta > 65535)
         a.edges_per_cta = (E + 65534) / 65535;
-    a.persistent = ctx->tune.persistent;
     a.queue_min_items = ctx->tune.queue_min_items;
     a.finish_split = ctx->tune.finish_split;
-    a.mode = ctx->tune.lanes == 16 ? 5 : 0;  // the plain walk: whole warp or half-warp per pair
+    a.mode = 0;
     BCC_CUDA(ctx, ctx->work_counter.ensure(64));
     a.work_counter = ctx->work_counter.as<int>();
     return BCC_OK;
@@ -285,6 +386,7 @@ bcc_status ensure_env_clusters(bcc_ctx* ctx, cudaStream_t st) {
     BCC_CUDA(ctx, ctx->centroids.ensure(sizeof(float) * cen.size()));
     BCC_CUDA(ctx, cudaMemcpy(ctx->env_cluster.p, id.data(), sizeof(int) * (size_t)N, cudaMemcpyHostToDevice));
     BCC_CUDA(ctx, cudaMemcpy(ctx->centroids.p, cen.data(), sizeof(float) * cen.size(), cudaMemcpyHostToDevice));
+    BCC_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));  // (see bcc_upload_envs)
     ctx->cluster_k = K;
     return BCC_OK;
 }
@@ -314,6 +416,7 @@ bcc_status prepare_learned(bcc_ctx* ctx, bcc::PipelineArgs& a, int row_cap) {
     a.q_cap = q_cap;
     a.row_cap = cap;
     a.logits = ctx->mlp.logits.as<float>();
+    a.features = ctx->mlp.x.p;
     a.queue_min_items = ctx->tune.queue_min_items;
     a.finish_counter = a.work_counter + 1;
     ctx->learned_rows_dev = reinterpret_cast<int*>(a.q_head);  // the low word counts rows
@@ -345,7 +448,7 @@ bcc_status run_learned(bcc_ctx* ctx, const bcc::RobotOps* ops, bcc::PipelineArgs
 }
 
 // Inline learned order: buffers for K x segments MLP rows and the
-// per-(cluster, edge) 32-block permutations, sized outside any stream capture.
+// per-(cluster, edge) segment orders, sized outside any stream capture.
 bcc_status prepare_inline(bcc_ctx* ctx, bcc::PipelineArgs& a) {
     bcc_status s = ensure_env_clusters(ctx, ctx->stream);
     if (s != BCC_OK) return s;
@@ -356,8 +459,9 @@ bcc_status prepare_inline(bcc_ctx* ctx, bcc::PipelineArgs& a) {
         return fail(ctx, BCC_ERR_LIMIT, "too many (cluster, segment) rows for the inline learned order");
     BCC_CUDA(ctx, ctx->mlp.x.ensure(sizeof(uint16_t) * bcc::kMlpIn * rows));
     BCC_CUDA(ctx, ctx->mlp.logits.ensure(sizeof(float) * rows));
-    BCC_CUDA(ctx, ctx->perms.ensure((size_t)K * std::max(a.num_edges, 1) * bcc::kLanes));
+    BCC_CUDA(ctx, ctx->perms.ensure((size_t)K * std::max(a.num_edges, 1) * bcc::kMaxSegments));
     a.logits = ctx->mlp.logits.as<float>();
+    a.features = ctx->mlp.x.p;
     a.env_cluster = ctx->env_cluster.as<int>();
     a.perms = ctx->perms.as<uint8_t>();
     a.row_cap = (int)rows;
@@ -367,15 +471,9 @@ bcc_status prepare_inline(bcc_ctx* ctx, bcc::PipelineArgs& a) {
 }
 
 // Inline learned order: FK / self / swept, features of every (cluster,
-// segment) row, tcgen05 MLP scores, per-(cluster, edge) permutations, then one
-// check in which every pair walks rank 0 (sample 0) and then its other samples
-// in its cluster's learned order (mode 4): no queue, no second pass.
-// With one cluster the permutation depends on the edge alone, so the FK
-// kernel writes each edge's table rows in learned order (lane block pi(t) at
-// block position t) and the plain check kernel (mode 0) walks them: the order
-// costs the check kernel nothing.  With several clusters the table stays in
-// sample order and the check kernel (mode 4) maps ranks through each pair's
-// cluster permutation.
+// segment) row, tcgen05 MLP scores, per-(cluster, edge) segment orders, then one
+// check in which every pair walks its segments in its cluster's order (mode 4):
+// no queue, no second pass.
 bcc_status run_learned_inline(bcc_ctx* ctx, const bcc::RobotOps* ops, bcc::PipelineArgs& a, cudaStream_t st) {
     cudaEvent_t* ev = a.stage_events;
     const int K = ctx->cluster_k;
@@ -386,9 +484,8 @@ bcc_status run_learned_inline(bcc_ctx* ctx, const bcc::RobotOps* ops, bcc::Pipel
                                    ctx->mlp.params.as<float>(), ctx->mlp.logits.as<float>(), a.error_flag,
                                    std::max(sms, 1), st));
     BCC_CUDA(ctx, ops->cluster_perms(a, K, ctx->perms.as<uint8_t>(), st));
-    a.fk_perm = K == 1 ? ctx->perms.as<uint8_t>() : nullptr;
     BCC_CUDA(ctx, ops->prep(a, st));  // records stage events 1-4
-    a.mode = K == 1 ? a.mode : 4;  // one cluster: the plain walk (whole or half warp) over the permuted table
+    a.mode = 4;
     BCC_CUDA(ctx, ops->check_mode(a, st));
     if (ev) cudaEventRecord(ev[5], st);
     return BCC_OK;
@@ -406,6 +503,19 @@ bool same_tune(const bcc::Tune& x, const bcc::Tune& y) {
     return x.edges_per_cta == y.edges_per_cta && x.warps == y.warps && x.persistent == y.persistent &&
            x.queue_min_items == y.queue_min_items && x.finish_split == y.finish_split &&
            x.learned_mode == y.learned_mode && x.clusters == y.clusters && x.lanes == y.lanes;
+}
+
+// A captured graph holds the addresses of the context's buffers: calls of other
+// sizes, orders or robots in between may have replaced some.
+bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
+    return x.steps == y.steps && x.offs == y.offs && x.table == y.table && x.row_edge == y.row_edge && x.seg == y.seg &&
+           x.edge_self == y.edge_self && x.swept == y.swept && x.edge_tri == y.edge_tri &&
+           x.grid_bounds == y.grid_bounds && x.blobs == y.blobs && x.env_hdr == y.env_hdr && x.mid == y.mid &&
+           x.probe.vox == y.probe.vox && x.queue.entries == y.queue.entries && x.queue.items == y.queue.items &&
+           x.queue.head == y.queue.head && x.queue.chunk == y.queue.chunk && x.warps == y.warps &&
+           x.edges_per_cta == y.edges_per_cta && x.q_head == y.q_head && x.q_pairs == y.q_pairs &&
+           x.q_rows == y.q_rows && x.logits == y.logits && x.perms == y.perms && x.env_cluster == y.env_cluster &&
+           x.features == y.features && x.work_counter == y.work_counter && x.error_flag == y.error_flag;
 }
 
 bcc_status run_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution,
@@ -432,13 +542,14 @@ bcc_status run_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E,
     const bool hit = G.exec && G.edges == d_edges && G.results == d_results && G.num_edges == E &&
                      G.resolution == resolution && G.total_rows == a.total_rows && G.robot == (int)robot &&
                      G.row_cap == a.row_cap &&
-                     G.env_version == ctx->env_version && same_tune(G.tune, ctx->tune);
+                     G.env_version == ctx->env_version && same_tune(G.tune, ctx->tune) && same_buffers(G.args, a);
     if (!hit) {
         if (G.exec) {
             cudaGraphExecDestroy(G.exec);
             G.exec = nullptr;
         }
         a.stage_events = nullptr;
+        const bcc::PipelineArgs key = a;
         cudaGraph_t g = nullptr;
         // Captured on the context's private stream (the caller's may be the legacy
         // default stream, which cannot be captured); launched on the caller's.
@@ -461,6 +572,7 @@ bcc_status run_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E,
         G.resolution = resolution;
         G.total_rows = a.total_rows;
         G.row_cap = a.row_cap;
+        G.args = key;
         G.robot = (int)robot;
         G.env_version = ctx->env_version;
         G.tune = ctx->tune;
@@ -709,6 +821,10 @@ void build_arena(const std::vector<Rec>& recs, const std::vector<int>& off, Aren
         const uint32_t shape = (uint32_t)np | ((uint32_t)W << 16);
         float* h = &A.hdr[(size_t)i * 8];
         std::memcpy(&h[3], &off16, 4);
+        uint32_t flags = 0;
+        for (int p = 0; p < np; ++p)
+            if (!regular_rec(recs[p0 + p])) flags = bcc::kEnvIrregular;
+        std::memcpy(&h[6], &flags, 4);
         std::memcpy(&h[7], &shape, 4);
     }
     if (A.blob.empty()) A.blob.assign(4, 0.0f);
@@ -757,6 +873,9 @@ bcc_status bcc_upload_envs(bcc_ctx* ctx, const bcc_env_soa* envs) {
     ctx->blob_smem = blob_smem;
     BCC_CUDA(ctx, ctx->grid_bounds.ensure(sizeof(A.bnd)));
     BCC_CUDA(ctx, cudaMemcpy(ctx->grid_bounds.p, A.bnd, sizeof(A.bnd), cudaMemcpyHostToDevice));
+    // A copy from pageable memory may return with its DMA still in flight on the
+    // legacy stream, which a check's (non-blocking) stream is not ordered after.
+    BCC_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
     ctx->env_code_ready = false;
     ctx->cluster_k = 0;
     ctx->env_version += 1;
@@ -1187,6 +1306,7 @@ bcc_status bcc_set_launch_config(bcc_ctx* ctx, const int32_t* cfg) {
     ctx->tune.learned_mode = cfg[5];
     ctx->tune.clusters = cfg[6];
     ctx->tune.lanes = cfg[7];
+    ctx->tune.tuned = true;
     return BCC_OK;
 }
 
@@ -1225,6 +1345,7 @@ bcc_status bcc_autotune(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32
     ctx->profiling = false;
     auto time_cfg = [&](const bcc::Tune& t, float& ms) -> bcc_status {
         ctx->tune = t;
+        ctx->tune.tuned = true;
         bcc_status s = run_check(ctx, robot, ctx->edges.as<float>(), num_edges, resolution, ctx->results.as<uint8_t>(),
                                  &opts, st);
         if (s != BCC_OK) return s;
@@ -1272,23 +1393,16 @@ bcc_status bcc_autotune(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32
     // Launch shape first (for the learned order at a middle threshold with
     // one-warp finishes), then the learned order's threshold x finish mode at
     // that shape, then the shape once more at the chosen threshold and mode.
-    // Lanes per walking pair: 16 only where the robot has the half-warp walk
-    // (elsewhere it would time the 32-lane walk twice and could report 16).
-    const int lanes[2] = {32, 16};
-    const bcc::RobotOps* tops = bcc::robot_ops((int)robot);
-    const int n_lanes = tops && tops->half_warp_walk ? 2 : 1;
     auto sweep_shape = [&](const bcc::Tune& from) {
         for (int ti = 0; ti < 4 && s == BCC_OK; ++ti)
             for (int wi = 0; wi < 2 && s == BCC_OK; ++wi)
-                for (int pe = 0; pe < 2 && s == BCC_OK; ++pe)
-                    for (int li = 0; li < n_lanes && s == BCC_OK; ++li) {
-                        bcc::Tune t = from;
-                        t.edges_per_cta = tiles[ti];
-                        t.warps = warps[wi];
-                        t.persistent = pe;
-                        t.lanes = lanes[li];
-                        keep(t);
-                    }
+                for (int pe = 0; pe < 2 && s == BCC_OK; ++pe) {
+                    bcc::Tune t = from;
+                    t.edges_per_cta = tiles[ti];
+                    t.warps = warps[wi];
+                    t.persistent = pe;
+                    keep(t);
+                }
     };
     bcc::Tune start = base;
     if (learned) {  // the inline order at one cluster while the shape is swept

@@ -7,6 +7,8 @@
 
 #include <cuda_runtime.h>
 
+#include "bcc_kernels.h"
+
 namespace bcc {
 
 // Device buffer grown on demand and reused across calls.
@@ -47,14 +49,14 @@ struct MlpState {
 // Launch configuration of the environment check (set by bcc_autotune).
 struct Tune {
     int edges_per_cta = 128;
-    int warps = 8;
+    int warps = 4;
     int persistent = 1;
     int queue_min_items = 128;
     int finish_split = 0;    // learned order, queued: 1 = split each queued pair over a CTA's warps
     int learned_mode = 0;    // learned order: 0 = inline (per-cluster scores), 1 = queued (per-pair scores)
     int clusters = 1;        // learned order, inline: environment clusters scored per edge
-    int lanes = 32;          // lanes per walking pair in the plain-order walk: 32 or 16 (half-warps)
-    bool tuned = false;
+    int lanes = 32;          // accepted and reported; every walk takes a whole warp
+    bool tuned = false;      // set or tuned: taken as it is, else the shape is chosen by size
 };
 
 // A captured launch sequence (everything after the discretisation) and the
@@ -67,6 +69,7 @@ struct GraphCache {
     int num_edges = -1, resolution = -1, total_rows = -1, order = -1, robot = -1, row_cap = -1;
     long long env_version = -1;
     Tune tune;
+    PipelineArgs args{};     // the buffers it was captured with
     ~GraphCache() {
         if (exec) cudaGraphExecDestroy(exec);
     }
@@ -97,13 +100,20 @@ struct bcc_ctx {
     bcc::MlpState mlp;
     bcc::DevBuf edge_tri;    // [E][groups] packed slab ranges of each group's swept box
     bcc::DevBuf grid_bounds; // [3][kGridSlabs + 1] slab boundaries of the uploaded set's cull grid
+    bcc::DevBuf mid;         // [groups][E] probe spheres around the edges' middle samples
+    bcc::DevBuf pq_entries, pq_items, pq_head;  // queue of the pairs a probe leaves undecided
+    bcc::DevBuf vox;         // probe grids of the uploaded set
+    bcc::ProbeGrid probe{};  // ... their shape (vox null: none)
+    int probe_robot = -1;    // ... the robot and upload they were built for
+    long long probe_version = -1;
     bcc::DevBuf env_code;    // [num_envs][32] environment encodings
     bool env_code_ready = false;
     // inline learned order: environment clusters (k-means over the codes)
     bcc::DevBuf env_cluster; // [num_envs] cluster id
     bcc::DevBuf centroids;   // [K][32] cluster centroid codes
     int cluster_k = 0;       // K of the current clustering, 0 = none
-    bcc::DevBuf perms;       // [K][edges][32] per-check lane-block permutations
+    bcc::DevBuf perms;       // [K][edges][kMaxSegments] per-check segment orders
+    bcc::DevBuf seg;         // [rows / kSegment][groups] segment spheres
     bcc::DevBuf q_head, q_pairs, q_rows;   // learned-order queue of undecided pairs
     const int* learned_rows_dev = nullptr; // queue head of the last learned check (entries << 32 | rows)
     int learned_row_cap = 0;

@@ -246,17 +246,27 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(addr), "r"(count) : "memory");
 }
 
-// One thread: expect `bytes` on the barrier and start a 1-D bulk copy
-// global -> shared (no multicast).  src/dst 16-byte aligned, bytes % 16 == 0.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+// One thread: expect `bytes` in all on the barrier's phase (its one arrival).
+__device__ __forceinline__ void bulk_expect(uint64_t* bar, uint32_t bytes) {
     const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
+}
+
+// One thread: start a 1-D bulk copy global -> shared (no multicast) that counts
+// towards the expected bytes.  src/dst 16-byte aligned, bytes % 16 == 0.
+__device__ __forceinline__ void bulk_copy_part(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const uint32_t b = (uint32_t)__cvta_generic_to_shared(bar);
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
         "l"(src), "r"(bytes), "r"(b)
         : "memory");
+}
+
+__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    bulk_expect(bar, bytes);
+    bulk_copy_part(dst, src, bytes, bar);
 }
 
 }  // namespace bcc

@@ -18,10 +18,44 @@ __host__ __device__ __forceinline__ int tri_index(int i0, int i1) {
     return i0 * kGridSlabs - (i0 * (i0 - 1)) / 2 + (i1 - i0);
 }
 
+// Probe grid of an environment: for every voxel centre of a box around the
+// robot's reach the nearest primitive and a quantised signed distance to it.
+// One 16-bit word a voxel: bits 0-7 the distance code (the distance lies in
+// [kVoxMin + code * kVoxStep, + kVoxStep), clamped to the code range), bits
+// 8-15 the primitive (kVoxUnknown: not representable, nothing is claimed).
+// Signed distance is 1-Lipschitz, so at a point q the distance differs from the
+// stored one by at most |q - voxel centre|, inside the box or outside it.
+constexpr int kMaxVoxels = 14336;      // 28 KB a grid: with an environment's records it leaves 6 CTAs an SM
+constexpr float kVoxMin = -0.128f;
+constexpr float kVoxStep = 0.003f;     // codes reach 0.637 m
+constexpr float kVoxSlack = 1e-4f;     // FP32 rounding of distances and positions (~1e-6 m), generously
+constexpr unsigned kVoxUnknown = 255u;
+// Environment header flag (second float4, z): some record's axes stretch
+// distances or hold non-finite values, so no distance bound holds and the
+// check makes every test on the primitives themselves.
+constexpr unsigned kEnvIrregular = 1u;
+
+struct ProbeGrid {
+    const uint16_t* vox;     // [num_envs][stride / 2] voxel words, null = no grid
+    uint32_t stride;         // bytes per environment (16-byte multiple)
+    int nx, ny, nz;
+    float h, inv_h;          // voxel edge
+    float ox, oy, oz;        // centre of voxel (0, 0, 0)
+};
+
+// Queue between the probe and the walk of a probed check.
+struct ProbeQueue {
+    uint2* entries;          // [cap] undecided pairs of one environment after another: edge, alive groups
+    int4* items;             // work items: environment, first entry, entries
+    int* head;               // per slab: entries used, items, next item, -
+    long long cap;
+    int chunk;               // entries per work item
+};
+
 struct CheckParams {
     const float4* blobs;     // per env: [np][5] rounded-box records, then 3 x kGridTri x W masks
-    const float4* env_hdr;   // [num_envs][2]: (grid origin xyz, blob offset in float4s),
-                             //                 (1/slab width xyz, np | W << 16)
+    const float4* env_hdr;   // [num_envs][2]: (0, 0, 0, blob offset in float4s),
+                             //                 (0, 0, flags, np | W << 16)
     int num_envs;
     int num_edges;
     int max_prims;           // max primitives of one env (pair-list sizing)
@@ -32,8 +66,12 @@ struct CheckParams {
     const int* offs;         // [E + 1] first sample row of each edge
     const float4* table;     // [rows][num_spheres] sphere centres + radius
     const float4* swept;     // [E][groups][2] cull AABB centre / half-size
+    const float2* seg;       // [rows / kSegment][groups] segment spheres (plain and inline learned walks)
     const int* edge_tri;     // [E][groups] slab ranges on the set's grid (tx | ty << 10 | tz << 20), -1 = none
     const int* edge_self;    // [E] 1 when some sample self-collides
+    ProbeGrid probe;         // probed checks (vox null: one pass over all pairs)
+    const float4* mid;       // [groups][E] each group's sphere around the edge's middle sample
+    ProbeQueue queue;
     uint8_t* results;        // [E][num_envs]
     int* error_flag;         // set when a bounded wait gives up
     unsigned long long* counters;  // null, or kNumCounters work counters (diagnostics)
@@ -47,11 +85,9 @@ struct CheckParams {
     int queue_min_items;     // probe: queue only pairs with at least this many items left
     int* finish_counter;     // next queue entry for the finish kernel
     int finish_split;        // 1: each queued pair split over a CTA's warps, 0: one warp per pair
-    int persistent;          // 1: persistent kernel pulling work items from work_counter
-    int* work_counter;
     // Inline learned order (mode 4): per (cluster, edge) segment permutations.
     const int* env_cluster;  // [num_envs] cluster of each environment
-    const uint8_t* perms;    // [K][num_edges][32] lane block at each rank of a round
+    const uint8_t* perms;    // [K][num_edges][kMaxSegments] segment at each rank
     int total_segs;          // offs[E] / kSegment
 };
 
@@ -75,10 +111,13 @@ struct PipelineArgs {
     int total_rows;          // offs[E], read back after the scan
     float4* table;           // [total_rows][num_spheres]
     int* row_edge;           // [total_rows]
-    const uint8_t* fk_perm;  // null, or [E][32] lane-block permutation the FK table is written in
+    float2* seg;             // [total_rows / kSegment][groups] segment spheres, null = not needed
     int* edge_self;          // [E]
     float4* swept;           // [E][groups][2]
     int* edge_tri;           // [E][groups], null = not needed (records check)
+    ProbeGrid probe;
+    ProbeQueue queue;
+    float4* mid;             // [groups][E] spheres around the middle sample, null = not needed
     const float* grid_bounds;  // [3][kGridSlabs + 1] cull-grid slab boundaries of the environment set
     const float4* blobs;
     const float4* env_hdr;
@@ -102,10 +141,10 @@ struct PipelineArgs {
     int queue_min_items;
     int* finish_counter;
     int finish_split;
-    int persistent;
     int* work_counter;
     const int* env_cluster;
     const uint8_t* perms;
+    const void* features;    // the MLP feature rows of a learned check
     int total_segs;
 };
 
@@ -137,6 +176,11 @@ constexpr int kRecordsWarps = 4;  // warps per CTA of the records check kernel
 // Entries of a warp's (primitive, link) pair list in shared memory; a pair with
 // more candidates is walked in segments of this many.
 constexpr int kPairCap = 1024;
+// Edges a probe CTA takes (their undecided ones are listed in shared memory).
+constexpr int kProbeBatch = 1024;
+// Pairs a probed check takes at a time: bounds the queue (8 bytes a pair) to
+// 512 MB however many environments and edges a call has.
+constexpr long long kQueuePairs = 64ll << 20;
 
 // One robot's pipeline, instantiated in its own translation unit
 // (bcc_robot_<name>.cu) from the templates of bcc_pipeline.cuh.
@@ -146,7 +190,8 @@ struct RobotOps {
     int num_spheres;         // sample-table row width (float4 per sample)
     int num_env_groups;
     int max_prims;           // primitives per environment the pair packing allows
-    bool half_warp_walk;     // the 16-lane walk exists (no overhang, grouped cull); else lanes 16 walks as 32
+    // Box around the group bounds' centres over the joint limits (probe grid domain).
+    void (*reach)(float lo[3], float hi[3]);
     cudaError_t (*upload_tables)();  // robot tables -> __constant__ of the current device
     // Stage 1: steps + sample offsets (total rows land in offs[E]).
     cudaError_t (*steps)(const PipelineArgs& a, cudaStream_t st);
@@ -165,7 +210,7 @@ struct RobotOps {
     // pairs (lab, 8 per MLP row) and of each segment's scored sample (y).
     cudaError_t (*queue_labels)(const PipelineArgs& a, uint8_t* lab, uint8_t* y, int grid, cudaStream_t st);
     // Inline learned order: MLP feature rows of every (cluster, segment) and,
-    // from their scores (a.logits), the per-(cluster, edge) 32-block permutations.
+    // from their scores (a.logits), the per-(cluster, edge) segment orders.
     cudaError_t (*cluster_features)(const PipelineArgs& a, const float* centroids, int K, uint16_t* x,
                                     cudaStream_t st);
     cudaError_t (*cluster_perms)(const PipelineArgs& a, int K, uint8_t* perms, cudaStream_t st);
@@ -180,6 +225,9 @@ cudaError_t launch_env_encode(const float4* blobs, const float4* env_hdr, int nu
 // Row gather for training: x2[i] = x[perm[i]] (kMlpIn BF16 values), y2[i] = y[perm[i]].
 cudaError_t launch_gather_rows(const uint16_t* x, const uint8_t* y, const int* perm, int rows, uint16_t* x2,
                                uint8_t* y2, cudaStream_t st);
+// Probe grids of every environment (p.vox is written).
+cudaError_t launch_probe_grid(const float4* blobs, const float4* env_hdr, int num_envs, const ProbeGrid& p,
+                              uint16_t* vox, cudaStream_t st);
 size_t check_smem_bytes(int max_prims, int groups, size_t blob_smem, int warps);
 size_t records_smem_bytes(int max_prims, int groups, int warps);
 
@@ -196,8 +244,12 @@ inline CheckParams params_of(const PipelineArgs& a) {
     P.offs = a.offs;
     P.table = a.table;
     P.swept = a.swept;
+    P.seg = a.seg;
     P.edge_tri = a.edge_tri;
     P.edge_self = a.edge_self;
+    P.probe = a.probe;
+    P.mid = a.mid;
+    P.queue = a.queue;
     P.results = a.d_results;
     P.error_flag = a.error_flag;
     P.counters = a.counters;
@@ -210,8 +262,6 @@ inline CheckParams params_of(const PipelineArgs& a) {
     P.queue_min_items = a.queue_min_items;
     P.finish_counter = a.finish_counter;
     P.finish_split = a.finish_split;
-    P.persistent = a.persistent;
-    P.work_counter = a.work_counter;
     P.env_cluster = a.env_cluster;
     P.perms = a.perms;
     P.total_segs = a.total_segs;

@@ -16,17 +16,21 @@
 //                          for Panda), OR-reduced per edge; env-independent
 //   5. swept_kernel        per (edge, link) AABB of the link's cull sphere over
 //                          all the edge's samples
-//   6. check_kernel        CTA = one environment x a tile of edges.  The
-//                          environment's primitive records are staged into shared
-//                          memory once by a cp.async.bulk copy and reused by every
-//                          edge of the tile.  Each warp takes one edge at a time:
-//                          lane g turns link g's swept AABB into three slab ranges
-//                          and ANDs three 64-bit primitive masks of the
-//                          environment's interval-mask tables (the cull, read
-//                          through L1), the surviving (primitive, link) pairs are
-//                          compacted (lane g writes link g's), and the warp walks
-//                          (sample, pair) items 32 at a time in check order with a
-//                          warp-ballot exit on the first hit.
+//   6. probe_kernel        one lane per (environment, edge) pair: decides most pairs
+//                          from the environment's probe grid (a voxel grid of
+//                          nearest primitives and distances) and queues the rest
+//   7. walk_kernel         persistent CTAs pull queued pairs, one environment at a
+//                          time, its primitive records staged into shared memory by
+//                          a cp.async.bulk copy.  Per pair, lane g turns link g's
+//                          swept AABB into three slab ranges and ANDs three 64-bit
+//                          primitive masks of the environment's interval-mask tables
+//                          (the cull, read through L1), the surviving (primitive,
+//                          link) pairs are compacted (lane g writes link g's), and
+//                          the warp walks (sample, pair) items 32 at a time in check
+//                          order with a warp-ballot exit on the first hit.
+// or, for both, check_kernel: CTA = one environment x a tile of edges, every pair
+// walked as above (the queued learned order's probe, and launch configurations
+// without the first pass).
 //
 // Gate semantics.  The reference tests a link's leaves only after the link's
 // bounding sphere hit SOME primitive (fkcc: `if (bound in collision) { if
@@ -65,6 +69,8 @@ struct DevTables {
     // Certain-hit radius of env group g (0: none): a primitive whose core lies
     // within rho + cert_r[g] of the bound's centre is hit by a leaf of g.
     float cert_r[M::num_env_groups];
+    // Groups by descending certain-hit radius (the probe's order).
+    int probe_group[M::num_env_groups];
     int self_bound[M::num_self_groups][2];
     int self_pair_begin[M::num_self_groups + 1];
     unsigned char self_pairs[M::num_self_pairs][2];
@@ -185,6 +191,9 @@ DevTables<M> host_tables() {
         t.cull_pad[g] = M::env_cull_pad[g];
         t.cert_r[g] = cert_radius<M>(g);
     }
+    for (int g = 0; g < M::num_env_groups; ++g) t.probe_group[g] = g;
+    std::stable_sort(t.probe_group, t.probe_group + M::num_env_groups,
+                     [&](int a, int b) { return t.cert_r[a] > t.cert_r[b]; });
     for (int g = 0; g <= M::num_env_groups; ++g) t.leaf_begin[g] = M::env_leaf_begin[g];
     // Self tables hold sample-table row positions, not sphere indices.
     for (int g = 0; g < M::num_self_groups; ++g) {
@@ -203,6 +212,62 @@ DevTables<M> host_tables() {
         t.s_a[j] = M::s_a[j];
     }
     return t;
+}
+
+// Box around the group bounds' centres over the joint limits: the domain of the
+// probe grid.  Sampled (a seeded sequence of 2048 configurations, 2 cm added):
+// a centre outside it costs the probe precision there, never correctness.
+template <class M>
+void sample_reach(float lo[3], float hi[3]) {
+    double l[3] = {1e30, 1e30, 1e30}, h[3] = {-1e30, -1e30, -1e30};
+    uint64_t rng = 0x9E3779B97F4A7C15ull;
+    for (int it = 0; it < 2048; ++it) {
+        double R[M::dof + 1][9] = {{1, 0, 0, 0, 1, 0, 0, 0, 1}}, p[M::dof + 1][3] = {};
+        for (int k = 0; k < M::dof; ++k) {
+            rng = rng * 6364136223846793005ull + 1442695040888963407ull;
+            const double q = (double)(rng >> 11) / 9007199254740992.0 * (double)M::s_m[k] + (double)M::s_a[k];
+            const double* f = M::joint_tf[k];
+            const double* P = R[M::joint_parent[k]];
+            double A[9];
+            for (int a = 0; a < 3; ++a) {
+                for (int b = 0; b < 3; ++b)
+                    A[a * 3 + b] = P[a * 3] * f[b] + P[a * 3 + 1] * f[4 + b] + P[a * 3 + 2] * f[8 + b];
+                p[k + 1][a] = P[a * 3] * f[3] + P[a * 3 + 1] * f[7] + P[a * 3 + 2] * f[11] + p[M::joint_parent[k]][a];
+            }
+            const bool rev = M::joint_type[k] == 0;
+            const double s = rev ? std::sin(q) : 0.0, c = rev ? std::cos(q) : 1.0;
+            for (int a = 0; a < 3; ++a) {
+                R[k + 1][a * 3 + 0] = A[a * 3] * c + A[a * 3 + 1] * s;
+                R[k + 1][a * 3 + 1] = A[a * 3 + 1] * c - A[a * 3] * s;
+                R[k + 1][a * 3 + 2] = A[a * 3 + 2];
+                if (!rev) p[k + 1][a] += A[a * 3 + 2] * q;
+            }
+        }
+        for (int g = 0; g < M::num_env_groups; ++g) {
+            const int b = M::env_bound[g], fr = M::sphere_frame[b];
+            const double* o = M::sphere_local[b];
+            for (int a = 0; a < 3; ++a) {
+                const double c = R[fr][a * 3] * o[0] + R[fr][a * 3 + 1] * o[1] + R[fr][a * 3 + 2] * o[2] + p[fr][a];
+                l[a] = std::min(l[a], c);
+                h[a] = std::max(h[a], c);
+            }
+        }
+    }
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = (float)(l[a] - 0.02);
+        hi[a] = (float)(h[a] + 0.02);
+    }
+}
+
+template <class M>
+void reach_box(float lo[3], float hi[3]) {
+    struct Box {
+        float lo[3], hi[3];
+        Box() { sample_reach<M>(lo, hi); }
+    };
+    static const Box box;  // once per process
+    std::copy(box.lo, box.lo + 3, lo);
+    std::copy(box.hi, box.hi + 3, hi);
 }
 
 // Bits of the link-group index in a packed (primitive, group) pair.
@@ -247,22 +312,12 @@ __global__ void edge_steps_kernel(const float* __restrict__ edges, int E, int re
 // (env-group bounds, then env leaves, then the rest), one row per (edge,
 // sample) in edge order then sample index order; stored in tiles of
 // M::table_tile rows (table_index).
-// Sample at table position k of edge e: k itself, or with a block
-// permutation (inline learned order, one cluster) lane block perm[e][k / n]'s
-// sample of the same round, so the reference walk over the table visits the
-// samples in learned order.
-__device__ __forceinline__ int table_sample(const uint8_t* __restrict__ perm, int e, int n, int k) {
-    if (!perm) return k;
-    const int blk = k / n;
-    return (int)perm[(size_t)e * kLanes + blk] * n + (k - blk * n);
-}
-
 template <class M>
 __global__ void __launch_bounds__(128) fk_kernel(const float* __restrict__ edges, int E,
                                                  const int* __restrict__ steps,
                                                  const int* __restrict__ offs,
                                                  float4* __restrict__ table,
-                                                 int* __restrict__ row_edge, const uint8_t* __restrict__ perm) {
+                                                 int* __restrict__ row_edge) {
     const int total = offs[E];
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= total) return;
@@ -280,7 +335,7 @@ __global__ void __launch_bounds__(128) fk_kernel(const float* __restrict__ edges
         s[j] = edges[(size_t)e * 2 * M::dof + j];
         t[j] = edges[(size_t)e * 2 * M::dof + M::dof + j];
     }
-    edge_sample<M::dof>(s, t, steps[e], table_sample(perm, e, steps[e], k), q);
+    edge_sample<M::dof>(s, t, steps[e], k, q);
     fk_spheres<M>(q, table + table_index<M>(row, 0));
     row_edge[row] = e;
 }
@@ -348,6 +403,45 @@ __device__ __forceinline__ bool self_rows_hit(const float4* my, bool live) {
     return false;
 }
 
+__device__ __forceinline__ float dist2(float4 a, float4 b) {
+    const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
+    return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
+
+// A segment's (kSegment consecutive samples of an edge) spheres are centred at
+// its middle sample, row kSegMid.  Group g's entry (R, rho) of segment s: the
+// sphere of radius R around the bound's centre there holds all that group g can
+// hit with at any of the samples (bound, overhang, inflation, margin); a leaf's
+// centre stays within rho of where it is at the middle sample.
+constexpr int kSegMid = kSegment / 2;
+constexpr float kSegMargin = 1e-4f;  // FP32 rounding of centres and distances (~1e-6 m), generously
+
+// The four segments of a warp's 32 staged rows (row base + lane at srow +
+// lane * (num_spheres | 1)): every lane measures its row against its segment's
+// middle one, eight lanes reduce.  The group's leaves one after another.
+template <class M>
+__device__ __forceinline__ void segment_spheres(const float4* srow, int base, float2* __restrict__ seg) {
+    constexpr int G = M::num_env_groups;
+    constexpr int STRIDE = M::num_spheres | 1;
+    const DevTables<M>& T = tab<M>();
+    const int lane = threadIdx.x & 31;
+    const float4* mine = srow + lane * STRIDE;
+    const float4* mid = srow + ((lane & ~(kSegment - 1)) + kSegMid) * STRIDE;
+    for (int g = 0; g < G; ++g) {
+        float b = dist2(mine[g], mid[g]), l = 0.0f;
+        for (int i = T.leaf_begin[g]; i < T.leaf_begin[g + 1]; ++i) l = fmaxf(l, dist2(mine[G + i], mid[G + i]));
+#pragma unroll
+        for (int o = 1; o < kSegment; o <<= 1) {
+            b = fmaxf(b, __shfl_xor_sync(kFull, b, o));
+            l = fmaxf(l, __shfl_xor_sync(kFull, l, o));
+        }
+        if ((lane & (kSegment - 1)) == 0)
+            seg[((size_t)base / kSegment + lane / kSegment) * G + g] =
+                make_float2(sqrtf(b) * 1.00001f + T.sphere_radius[g] + kEnvInflate + T.cull_pad[g] + kSegMargin,
+                            sqrtf(l) * 1.00001f + kSegMargin);
+    }
+}
+
 // Row-major tables (tile 1): a thread's row is 16 * num_spheres contiguous
 // bytes, so per-thread stores would touch 32 rows per warp instruction.  One
 // warp per CTA computes 32 rows into shared memory (odd float4 row stride,
@@ -362,8 +456,8 @@ __global__ void __launch_bounds__(32) fk_staged_kernel(const float* __restrict__
                                                        const int* __restrict__ steps,
                                                        const int* __restrict__ offs,
                                                        float4* __restrict__ table,
-                                                       int* __restrict__ row_edge, const uint8_t* __restrict__ perm,
-                                                       int* __restrict__ edge_self) {
+                                                       int* __restrict__ row_edge, int* __restrict__ edge_self,
+                                                       float2* __restrict__ seg) {
     static_assert(M::table_tile == 1, "row-major tables only");
     constexpr int NS = M::num_spheres;
     constexpr int STRIDE = NS | 1;
@@ -387,7 +481,7 @@ __global__ void __launch_bounds__(32) fk_staged_kernel(const float* __restrict__
                 s[j] = edges[(size_t)e * 2 * M::dof + j];
                 t[j] = edges[(size_t)e * 2 * M::dof + M::dof + j];
             }
-            edge_sample<M::dof>(s, t, n, table_sample(perm, e, n, row - offs[e]), q);
+            edge_sample<M::dof>(s, t, n, row - offs[e], q);
             fk_spheres<M>(q, srow + lane * STRIDE);
             row_edge[row] = e;
         }
@@ -399,6 +493,7 @@ __global__ void __launch_bounds__(32) fk_staged_kernel(const float* __restrict__
             const int r = i / NS;
             dst[i] = srow[r * STRIDE + (i - r * NS)];
         }
+        if (seg) segment_spheres<M>(srow, base, seg);
         // self-collision of the block's rows (any hit marks the edge); skipped
         // when another block of the edge has already marked it
         int decided = lane == 0 ? *(volatile const int*)(edge_self + e) : 0;
@@ -498,7 +593,10 @@ __device__ __forceinline__ int slab_tri(float lo, float hi, const float* __restr
 // One warp per edge: AABB (lo, hi) of every link group's bounding sphere over
 // the edge's samples, inflated by radius + 0.005 + the group's leaf overhang +
 // cull margin; and (edge_tri non-null) its slab ranges on the set's cull grid,
-// packed tx | ty << 10 | tz << 20 (-1 when some axis misses every primitive).
+// packed tx | ty << 10 | tz << 20 (-1 when some axis misses every primitive);
+// and (mid non-null) the bound's centre at the edge's middle sample with the
+// radius, inflated likewise, of the sphere around it that holds them all; and
+// (seg non-null, tiled tables) the segments' spheres (see segment_spheres).
 // Lane g ends up holding group g's box.  Row-major tables: lane g scans group
 // g's bound down the rows (a row's bounds are contiguous).  Tiled tables: the
 // lanes scan 32 rows of one group at a time (contiguous in a tile) and a
@@ -506,7 +604,7 @@ __device__ __forceinline__ int slab_tri(float lo, float hi, const float* __restr
 template <class M>
 __global__ void swept_kernel(const float4* __restrict__ table, const int* __restrict__ offs, int E,
                              float4* __restrict__ swept, int* __restrict__ edge_tri,
-                             const float* __restrict__ bounds) {
+                             const float* __restrict__ bounds, float4* __restrict__ mid, float2* __restrict__ seg) {
     constexpr int G = M::num_env_groups;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -514,6 +612,8 @@ __global__ void swept_kernel(const float4* __restrict__ table, const int* __rest
     const int r0 = offs[warp], r1 = offs[warp + 1];
     const DevTables<M>& T = tab<M>();
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    float far2 = 0.0f;  // largest squared distance of the bound's centre from its middle one
+    const int rm = r0 + ((r1 - r0) >> 1);
     if constexpr (M::table_tile == 1) {
         // 32 / G row streams: lane s G + g scans group g's bound on rows
         // r0 + s, r0 + s + 32 / G, ... (bounds lead every table row); lane g then
@@ -521,8 +621,10 @@ __global__ void swept_kernel(const float4* __restrict__ table, const int* __rest
         constexpr int RS = kLanes / G;
         const int rs = lane / G, gl = lane - rs * G;
         if (rs < RS) {
+            const float4 m = table[table_index<M>(rm, gl)];
             for (int r = r0 + rs; r < r1; r += RS) {
                 const float4 c = table[table_index<M>(r, gl)];
+                far2 = fmaxf(far2, dist2(c, m));
                 lo[0] = fminf(lo[0], c.x); lo[1] = fminf(lo[1], c.y); lo[2] = fminf(lo[2], c.z);
                 hi[0] = fmaxf(hi[0], c.x); hi[1] = fmaxf(hi[1], c.y); hi[2] = fmaxf(hi[2], c.z);
             }
@@ -530,6 +632,7 @@ __global__ void swept_kernel(const float4* __restrict__ table, const int* __rest
 #pragma unroll
         for (int t = 1; t < RS; ++t) {
             const int src = min(lane + t * G, kLanes - 1);  // lanes >= G read a valid lane and discard it
+            far2 = fmaxf(far2, __shfl_sync(kFull, far2, src));
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 lo[a] = fminf(lo[a], __shfl_sync(kFull, lo[a], src));
@@ -539,13 +642,31 @@ __global__ void swept_kernel(const float4* __restrict__ table, const int* __rest
     } else {
         for (int g = 0; g < G; ++g) {
             float l3[3] = {INFINITY, INFINITY, INFINITY}, h3[3] = {-INFINITY, -INFINITY, -INFINITY};
+            const float4 m = table[table_index<M>(rm, g)];
+            float f2 = 0.0f;
             for (int r = r0 + lane; r < r1; r += 32) {
                 const float4 c = table[table_index<M>(r, g)];
+                f2 = fmaxf(f2, dist2(c, m));
+                if (seg) {  // rows r0 + 32 i: eight lanes hold a segment
+                    const int src = (lane & ~(kSegment - 1)) + kSegMid;
+                    float4 s;
+                    s.x = __shfl_sync(kFull, c.x, src);
+                    s.y = __shfl_sync(kFull, c.y, src);
+                    s.z = __shfl_sync(kFull, c.z, src);
+                    float d = dist2(c, s);
+#pragma unroll
+                    for (int o = 1; o < kSegment; o <<= 1) d = fmaxf(d, __shfl_xor_sync(kFull, d, o));
+                    if ((lane & (kSegment - 1)) == 0)
+                        seg[(size_t)(r / kSegment) * G + g] =
+                            make_float2(sqrtf(d) * 1.00001f + T.sphere_radius[g] + kEnvInflate + T.cull_pad[g] +
+                                            kSegMargin, 0.0f);
+                }
                 l3[0] = fminf(l3[0], c.x); l3[1] = fminf(l3[1], c.y); l3[2] = fminf(l3[2], c.z);
                 h3[0] = fmaxf(h3[0], c.x); h3[1] = fmaxf(h3[1], c.y); h3[2] = fmaxf(h3[2], c.z);
             }
 #pragma unroll
             for (int o = 16; o; o >>= 1) {
+                f2 = fmaxf(f2, __shfl_xor_sync(kFull, f2, o));
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     l3[a] = fminf(l3[a], __shfl_xor_sync(kFull, l3[a], o));
@@ -553,6 +674,7 @@ __global__ void swept_kernel(const float4* __restrict__ table, const int* __rest
                 }
             }
             if (lane == g) {
+                far2 = f2;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     lo[a] = l3[a];
@@ -564,6 +686,11 @@ __global__ void swept_kernel(const float4* __restrict__ table, const int* __rest
     if (lane >= G) return;
     const int g = lane;
     const float pad = T.sphere_radius[g] + kEnvInflate + T.cull_pad[g] + kCullMargin;
+    if (mid) {  // group-major: the probe's lanes read consecutive edges
+        float4 c = table[table_index<M>(rm, g)];
+        c.w = sqrtf(far2) * 1.00001f + pad;
+        mid[(size_t)g * E + warp] = c;
+    }
     const float4 l = make_float4(lo[0] - pad, lo[1] - pad, lo[2] - pad, 0.0f);
     const float4 h = make_float4(hi[0] + pad, hi[1] + pad, hi[2] + pad, 0.0f);
     swept[((size_t)warp * G + g) * 2 + 0] = l;
@@ -600,13 +727,6 @@ __device__ __forceinline__ int learned_rank_to_sample(const uint8_t* perm, int r
     return (int)perm[r >> 3] * kSegment + (kSegment - 1 - (r & (kSegment - 1)));
 }
 
-// Inline learned order: a permutation pi of the 32 lane blocks (block t =
-// samples t n .. t n + n - 1, the samples the reference's lane t checks) with
-// pi[0] = 0; rank r -> sample pi[r % 32] n + r / 32, so every round visits the
-// blocks in learned order, round 0 first (the reference's coarse sweep,
-// re-prioritised), starting with sample 0 (where most colliding pairs collide).
-// Each lane holds pi[lane]; the walk fetches pi[r % 32] by shuffle.
-
 // Per-pair walk counts (32 bits: a pair walks at most 32 n C items, far below
 // 2^32; the registers and adds are paid on every walk, counting or not).
 struct WalkStats {
@@ -642,6 +762,141 @@ __device__ __forceinline__ GroupLanes group_lanes() {
     return r;
 }
 
+// Whole warp, one step of 32 (sample, candidate) items: lane's item is sample k
+// of the edge (rows from row0) and the packed (primitive, group) pair pr, if
+// live.  The bounds are tested (one per item); a bound centre deep enough proves
+// a leaf hit (cert_radius); else the leaf work of the items whose bound hit is
+// flattened over the warp (item j owns leaf slots [incl_j - cnt_j, incl_j)).
+// Returns whether some item collides.
+template <class M>
+__device__ __forceinline__ bool walk_items(const float4* __restrict__ table, size_t row0, int k, uint32_t pr, bool live,
+                                           const float4* prim, int np, const GroupLanes& GL, WalkStats& st) {
+    constexpr int G = M::num_env_groups;
+    constexpr int GB = group_bits<M>();
+    constexpr bool kOver = has_overhang<M>();
+    const int lane = threadIdx.x & 31;
+    const int g = (int)(pr & ((1u << GB) - 1u)), p = (int)(pr >> GB);
+    bool gate = false, cert = false;
+    int cnt = 0, first = 0;
+    if constexpr (!kOver) {
+        // the group's leaf range by shuffle (measured faster for Panda than
+        // lane-indexed constant memory)
+        const int fc = __shfl_sync(kFull, GL.fc, g);
+        const float cr = __shfl_sync(kFull, GL.cert, g);
+        first = fc & 0xffff;
+        if (live) {
+            float4 bs = table[table_index<M>(row0 + (size_t)k, g)];
+            bs.w += kEnvInflate;
+            float rho;
+            const float d2 = prim_core_d2(bs, prim + p * kPrimF4, &rho);
+            const float rr = bs.w + rho, rc = rho + cr;
+            gate = d2 - rr * rr < 0.0f;
+            cert = cr > 0.0f && d2 - rc * rc < 0.0f;
+            cnt = gate ? fc >> 16 : 0;
+        }
+    } else {
+        // The overhang-aware walk reads its group fields from constant memory,
+        // which leaves its longer body the registers it needs (measured faster
+        // for Fetch and Baxter).
+        const DevTables<M>& T = tab<M>();
+        if (live) {
+            float4 bs = table[table_index<M>(row0 + (size_t)k, g)];
+            bs.w += kEnvInflate;
+            float rho;
+            const float d2 = prim_core_d2(bs, prim + p * kPrimF4, &rho);
+            const float rr = bs.w + rho;
+            gate = d2 - rr * rr < 0.0f;
+            const float rc = rho + T.cert_r[g];
+            cert = T.cert_r[g] > 0.0f && d2 - rc * rc < 0.0f;
+            cnt = gate ? T.leaf_begin[g + 1] - T.leaf_begin[g] : 0;
+            // overhanging leaves (listed first) near a primitive the bound misses
+            if (!gate && T.over_count[g] > 0) {
+                const float rp = rr + T.cull_pad[g];
+                if (d2 - rp * rp < 0.0f) cnt = T.over_count[g];
+            }
+        }
+        first = T.leaf_begin[g];
+    }
+    ++st.chunks;
+    if (__any_sync(kFull, cert)) return true;  // a leaf hit is certain: no leaf step
+    if (__any_sync(kFull, cnt > 0)) {
+        ++st.gates;
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int L = __shfl_sync(kFull, incl, 31);
+        // Without overhang a slot needs only its item's sample, primitive
+        // and leaf offset: p | (first - exclusive count) << 12, one shuffle.
+        int dp = 0;
+        if constexpr (!kOver) {
+            static_assert(max_prims_of<M>() < 4096, "primitive index packs into 12 bits");
+            dp = (int)(((unsigned)(first - (incl - cnt)) << 12) | (unsigned)p);
+        } else if constexpr (pack_overhang_leaf<M>()) {
+            // the 16-bit pair code (p << GB | g), the gate bit, the leaf offset
+            dp = (int)(((unsigned)(first - (incl - cnt)) << 17) | ((unsigned)gate << 16) |
+                       ((unsigned)p << GB) | (unsigned)g);
+        }
+        for (int t0 = 0; t0 < L; t0 += 32) {
+            const int t = t0 + lane;
+            // owner j: the first lane whose inclusive count exceeds t
+            int j = 0;
+#pragma unroll
+            for (int step = 16; step; step >>= 1) {
+                const int v = __shfl_sync(kFull, incl, j + step - 1);
+                if (v <= t) j += step;
+            }
+            int j_k, j_p, leaf, jd = 0;
+            if constexpr (!kOver) {
+                jd = __shfl_sync(kFull, dp, j);
+                j_k = __shfl_sync(kFull, k, j);
+                j_p = jd & 4095;
+                leaf = t + (jd >> 12);
+            } else if constexpr (pack_overhang_leaf<M>()) {
+                jd = __shfl_sync(kFull, dp, j);
+                j_k = __shfl_sync(kFull, k, j);
+                j_p = (jd & 0xffff) >> GB;
+                leaf = t + (jd >> 17);
+            } else {
+                const int j_incl = __shfl_sync(kFull, incl, j);
+                const int j_cnt = __shfl_sync(kFull, cnt, j);
+                const int j_first = __shfl_sync(kFull, first, j);
+                j_k = __shfl_sync(kFull, k, j);
+                j_p = __shfl_sync(kFull, p, j);
+                leaf = j_first + (t - (j_incl - j_cnt));
+            }
+            bool hit = false;
+            if (t < L) {
+                float4 ls = table[table_index<M>(row0 + (size_t)j_k, G + leaf)];
+                ls.w += kEnvInflate;
+                hit = sphere_hits_prim(ls, prim + j_p * kPrimF4);
+            }
+            ++st.leaf;
+            if constexpr (kOver) {
+                const bool j_gate = pack_overhang_leaf<M>() ? ((jd >> 16) & 1) != 0
+                                                            : __shfl_sync(kFull, (int)gate, j) != 0;
+                if (__any_sync(kFull, hit && j_gate)) return true;
+                // Hits of overhanging leaves whose bound missed this primitive:
+                // they count once the bound hits some primitive at that sample.
+                const int j_g = pack_overhang_leaf<M>() ? (jd & ((1 << GB) - 1)) : __shfl_sync(kFull, g, j);
+                uint32_t pend = __ballot_sync(kFull, hit);
+                while (pend) {
+                    const int u = __ffs(pend) - 1;
+                    const int uk = __shfl_sync(kFull, j_k, u);
+                    const int ug = __shfl_sync(kFull, j_g, u);
+                    if (bound_hits_any<M>(table, row0, uk, ug, prim, np)) return true;
+                    pend &= ~__ballot_sync(kFull, j_k == uk && j_g == ug);
+                }
+            } else {
+                if (__any_sync(kFull, hit)) return true;
+            }
+        }
+    }
+    return false;
+}
+
 // Whole warp: walk (sample rank, pair) items 32 at a time in check order --
 // plain reference order, or with `perm` the edge's segments in learned order --
 // and return whether some item collides.  Items [w_begin, w_end) are walked
@@ -650,9 +905,7 @@ __device__ __forceinline__ GroupLanes group_lanes() {
 // queue(); if that queues the pair, the walk stops with `undecided` set,
 // otherwise it goes on in plain order (robots without overhang make that
 // decision in check_pair, between two walks).
-// Each chunk tests the bounds (one per item); the leaf work of the items whose
-// bound hit is then flattened over the warp (item j owns leaf slots
-// [incl_j - cnt_j, incl_j)) and the warp stops at the first step with a hit.
+// Each chunk is a walk_items step and the first one with a hit ends the walk.
 // MODE 2 (finish): the CTA's warps split the pair -- this warp walks the
 // chunks at w_begin, w_begin + 32 stride, ... and all stop once one of them
 // sets *stop.
@@ -662,20 +915,11 @@ __device__ __forceinline__ bool walk_pairs(const float4* __restrict__ table, siz
                                            int queue_min_items, const GroupLanes& GL, bool& undecided,
                                            WalkStats& st, Queue&& queue, int w_begin = 0, int w_end = -1,
                                            int stride = 1, volatile int* stop = nullptr) {
-    constexpr int G = M::num_env_groups;
-    constexpr int GB = group_bits<M>();
     constexpr bool kOver = has_overhang<M>();
-    // rank -> sample: reference order (MODE 0, 1, or no perm), learned order
-    // (MODE 2, 3), inline learned order (MODE 4: perm = the pair's 32-block
-    // permutation, block fetched by a shuffle every lane executes).
-    const int pi = MODE == 4 && perm ? (int)perm[threadIdx.x & 31] : (int)(threadIdx.x & 31);
-    auto block_of = [&](int rr) {
-        if constexpr (MODE == 4) return __shfl_sync(kFull, pi, rr & (kLanes - 1));
-        return rr & (kLanes - 1);
-    };
-    auto sample_of = [&](int rr, int blk) {
-        if constexpr (MODE == 0 || MODE == 1 || MODE == 4) {
-            return blk * n + (rr >> 5);
+    // rank -> sample: reference order (MODE 0, 1, or no perm), learned order (MODE 2, 3)
+    auto sample_of = [&](int rr) {
+        if constexpr (MODE == 0 || MODE == 1) {
+            return reference_rank_to_sample(rr, n);
         } else {
             return perm ? learned_rank_to_sample(perm, rr) : reference_rank_to_sample(rr, n);
         }
@@ -708,152 +952,11 @@ __device__ __forceinline__ bool walk_pairs(const float4* __restrict__ table, siz
                 if (lane == 0) s = *stop;
                 if (__shfl_sync(kFull, s, 0)) break;
             }
-            bool gate = false, cert = false;
-            int g = 0, p = 0, k = 0, cnt = 0, first = 0;
-            if constexpr (!kOver) {
-                // c < C on every lane, also past the last item: the pair is decoded and
-                // its group's leaf range fetched by shuffle on every lane (measured
-                // faster for Panda than lane-indexed constant memory), the table and
-                // the primitive read only for live items.
-                const uint32_t pr = pairs[c];
-                g = (int)(pr & ((1u << GB) - 1u));
-                p = (int)(pr >> GB);
-                const int fc = __shfl_sync(kFull, GL.fc, g);
-                const float cr = __shfl_sync(kFull, GL.cert, g);
-                first = fc & 0xffff;
-                const int gcnt = fc >> 16;
-                const int blk = block_of(r);
-                if (w0 + lane < total) {
-                    k = sample_of(r, blk);
-                    float4 bs = table[table_index<M>(row0 + (size_t)k, g)];
-                    bs.w += kEnvInflate;
-                    float rho;
-                    const float d2 = prim_core_d2(bs, prim + p * kPrimF4, &rho);
-                    const float rr = bs.w + rho;
-                    gate = d2 - rr * rr < 0.0f;
-                    // the bound's centre close enough to the core proves a leaf hit
-                    const float rc = rho + cr;
-                    cert = cr > 0.0f && d2 - rc * rc < 0.0f;
-                    cnt = gate ? gcnt : 0;
-                }
-            } else {
-                // The overhang-aware walk reads its group fields from constant memory,
-                // which leaves its longer body the registers it needs (measured faster
-                // for Fetch and Baxter).
-                const DevTables<M>& T = tab<M>();
-                const int blk = block_of(r);
-                if (w0 + lane < total) {
-                    k = sample_of(r, blk);
-                    const uint32_t pr = pairs[c];
-                    g = (int)(pr & ((1u << GB) - 1u));
-                    p = (int)(pr >> GB);
-                    float4 bs = table[table_index<M>(row0 + (size_t)k, g)];
-                    bs.w += kEnvInflate;
-                    float rho;
-                    const float d2 = prim_core_d2(bs, prim + p * kPrimF4, &rho);
-                    const float rr = bs.w + rho;
-                    gate = d2 - rr * rr < 0.0f;
-                    const float rc = rho + T.cert_r[g];
-                    cert = T.cert_r[g] > 0.0f && d2 - rc * rc < 0.0f;
-                    cnt = gate ? T.leaf_begin[g + 1] - T.leaf_begin[g] : 0;
-                    // overhanging leaves (listed first) near a primitive the bound misses
-                    if (!gate && T.over_count[g] > 0) {
-                        const float rp = rr + T.cull_pad[g];
-                        if (d2 - rp * rp < 0.0f) cnt = T.over_count[g];
-                    }
-                }
-                first = T.leaf_begin[g];
-            }
-            ++st.chunks;
-            if (__any_sync(kFull, cert)) {  // a leaf hit is certain: no leaf step
+            const bool live = w0 + lane < total;
+            // c < C on every lane, also past the last item
+            if (walk_items<M>(table, row0, live ? sample_of(r) : 0, pairs[c], live, prim, np, GL, st)) {
                 collide = true;
                 break;
-            }
-            if (__any_sync(kFull, cnt > 0)) {
-                ++st.gates;
-                int incl = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(kFull, incl, o);
-                    if (lane >= o) incl += y;
-                }
-                const int L = __shfl_sync(kFull, incl, 31);
-                // Without overhang a slot needs only its item's sample, primitive
-                // and leaf offset: p | (first - exclusive count) << 12, one shuffle.
-                int dp = 0;
-                if constexpr (!kOver) {
-                    static_assert(max_prims_of<M>() < 4096, "primitive index packs into 12 bits");
-                    dp = (int)(((unsigned)(first - (incl - cnt)) << 12) | (unsigned)p);
-                } else if constexpr (pack_overhang_leaf<M>()) {
-                    // the 16-bit pair code (p << GB | g), the gate bit, the leaf offset
-                    dp = (int)(((unsigned)(first - (incl - cnt)) << 17) | ((unsigned)gate << 16) |
-                               ((unsigned)p << GB) | (unsigned)g);
-                }
-                for (int t0 = 0; t0 < L; t0 += 32) {
-                    const int t = t0 + lane;
-                    // owner j: the first lane whose inclusive count exceeds t
-                    int j = 0;
-#pragma unroll
-                    for (int step = 16; step; step >>= 1) {
-                        const int v = __shfl_sync(kFull, incl, j + step - 1);
-                        if (v <= t) j += step;
-                    }
-                    int j_k, j_p, leaf, jd = 0;
-                    if constexpr (!kOver) {
-                        jd = __shfl_sync(kFull, dp, j);
-                        j_k = __shfl_sync(kFull, k, j);
-                        j_p = jd & 4095;
-                        leaf = t + (jd >> 12);
-                    } else if constexpr (pack_overhang_leaf<M>()) {
-                        jd = __shfl_sync(kFull, dp, j);
-                        j_k = __shfl_sync(kFull, k, j);
-                        j_p = (jd & 0xffff) >> GB;
-                        leaf = t + (jd >> 17);
-                    } else {
-                        const int j_incl = __shfl_sync(kFull, incl, j);
-                        const int j_cnt = __shfl_sync(kFull, cnt, j);
-                        const int j_first = __shfl_sync(kFull, first, j);
-                        j_k = __shfl_sync(kFull, k, j);
-                        j_p = __shfl_sync(kFull, p, j);
-                        leaf = j_first + (t - (j_incl - j_cnt));
-                    }
-                    bool hit = false;
-                    if (t < L) {
-                        float4 ls = table[table_index<M>(row0 + (size_t)j_k, G + leaf)];
-                        ls.w += kEnvInflate;
-                        hit = sphere_hits_prim(ls, prim + j_p * kPrimF4);
-                    }
-                    ++st.leaf;
-                    if constexpr (kOver) {
-                        const bool j_gate = pack_overhang_leaf<M>() ? ((jd >> 16) & 1) != 0
-                                                                    : __shfl_sync(kFull, (int)gate, j) != 0;
-                        if (__any_sync(kFull, hit && j_gate)) {
-                            collide = true;
-                            break;
-                        }
-                        // Hits of overhanging leaves whose bound missed this primitive:
-                        // they count once the bound hits some primitive at that sample.
-                        const int j_g = pack_overhang_leaf<M>() ? (jd & ((1 << GB) - 1)) : __shfl_sync(kFull, g, j);
-                        uint32_t pend = __ballot_sync(kFull, hit);
-                        while (pend) {
-                            const int u = __ffs(pend) - 1;
-                            const int uk = __shfl_sync(kFull, j_k, u);
-                            const int ug = __shfl_sync(kFull, j_g, u);
-                            if (bound_hits_any<M>(table, row0, uk, ug, prim, np)) {
-                                collide = true;
-                                break;
-                            }
-                            pend &= ~__ballot_sync(kFull, j_k == uk && j_g == ug);
-                        }
-                        if (collide) break;
-                    } else {
-                        if (__any_sync(kFull, hit)) {
-                            collide = true;
-                            break;
-                        }
-                    }
-                }
-                if (collide) break;
             }
             // Probe (overhang-aware walk): the queue decision stays inside the
             // loop, measured 5 % faster for Baxter than a separate first walk.
@@ -877,15 +980,156 @@ __device__ __forceinline__ bool walk_pairs(const float4* __restrict__ table, siz
     return collide;
 }
 
+// Whole warp: the walk of plain and inline learned checks.  Items are
+// (segment rank, candidate) pairs, 32 a step, segments in order (ascending, or
+// as `order` ranks them).
+//   1. Per item the segment's sphere of the candidate's group against its
+//      primitive: a miss rules out all of the segment's samples.  At the middle
+//      sample the test is exact where it matters: a bound centre deep enough
+//      proves a leaf hit (cert_radius).
+//   2. Items that survive, robots whose leaves lie inside their bounds: every
+//      leaf of the group at the middle sample, flattened over the warp -- an
+//      exact hit test, and with the leaf's reach over the segment a test that
+//      rules out its other samples.
+//   3. What survives that: the leaf at each of the segment's samples.
+// Robots with overhanging leaves take the per-sample bound, certain-hit and leaf
+// tests (walk_items) on the segments that survive 1.
+// A collision-free pair then costs a test per segment and near-miss instead of
+// one per sample: the walk is bound by instruction issue, and on the uneven
+// Panda workload most of it went to pairs that never collide.
+template <class M>
+__device__ __forceinline__ bool walk_segments(const CheckParams& P, size_t row0, int n, int C, const uint16_t* pairs,
+                                              const float4* prim, int np, const uint8_t* order, const GroupLanes& GL,
+                                              uint2* scratch, WalkStats& st) {
+    constexpr int G = M::num_env_groups;
+    constexpr int GB = group_bits<M>();
+    constexpr bool kOver = has_overhang<M>();
+    static_assert(kSegment == 8, "segments are expanded eight lanes an item");
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const int S = kLanes / kSegment * n;
+    const float4* __restrict__ rows = P.table + table_index<M>(row0, 0);  // row0 starts a tile
+    const float2* __restrict__ segs = P.seg + row0 / kSegment * G;
+    // a / C in FP32, exact (walk_pairs)
+    const float inv_c = __frcp_rn((float)C);
+    const int dr = (int)(32.5f * inv_c), dc = 32 - dr * C;
+    int r = (int)(((float)lane + 0.5f) * inv_c);
+    int c = lane - r * C;
+    const unsigned steps = (unsigned)(((long long)S * C + 31) / 32);
+    for (unsigned w = 0; w < steps; ++w) {
+        const uint32_t pr = pairs[c];  // c < C on every lane
+        const int g = (int)(pr & ((1u << GB) - 1u)), p = (int)(pr >> GB);
+        const float cr = __shfl_sync(kFull, GL.cert, g);
+        const int fc = __shfl_sync(kFull, GL.fc, g);
+        bool near = false, cert = false;
+        int k = 0;
+        float reach = 0.0f;
+        if (r < S) {
+            const int sg = order ? (int)order[r] : r;
+            k = sg * kSegment + kSegMid;
+            const float4 bs = rows[table_index<M>((size_t)k, g)];
+            const float2 sr = segs[(size_t)sg * G + g];
+            float rho;
+            const float d2 = prim_core_d2(bs, prim + p * kPrimF4, &rho);
+            const float rs = sr.x + rho, rc = rho + cr;
+            near = d2 - rs * rs < 0.0f;
+            cert = cr > 0.0f && d2 - rc * rc < 0.0f;
+            reach = sr.y;
+        }
+        ++st.chunks;
+        if (__any_sync(kFull, cert)) return true;
+        const unsigned nm = __ballot_sync(kFull, near);
+        if (nm) {
+            ++st.gates;
+            if constexpr (!kOver) {
+                const int cnt = near ? fc >> 16 : 0;
+                int incl = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const int L = __shfl_sync(kFull, incl, 31);
+                static_assert(max_prims_of<M>() < 4096, "primitive index packs into 12 bits");
+                const int dp = (int)(((unsigned)((fc & 0xffff) - (incl - cnt)) << 12) | (unsigned)p);
+                for (int t0 = 0; t0 < L; t0 += 32) {
+                    const int t = t0 + lane;
+                    int j = 0;  // owner: the first lane whose inclusive count exceeds t
+#pragma unroll
+                    for (int step = 16; step; step >>= 1) {
+                        const int v = __shfl_sync(kFull, incl, j + step - 1);
+                        if (v <= t) j += step;
+                    }
+                    const int jd = __shfl_sync(kFull, dp, j);
+                    const int jk = __shfl_sync(kFull, k, j);
+                    const float jr = __shfl_sync(kFull, reach, j);
+                    const int jp = jd & 4095, leaf = G + t + (jd >> 12);
+                    bool hit = false, open = false;
+                    if (t < L) {
+                        float4 ls = rows[table_index<M>((size_t)jk, leaf)];
+                        ls.w += kEnvInflate;
+                        float rho;
+                        const float d2 = prim_core_d2(ls, prim + jp * kPrimF4, &rho);
+                        const float rr = ls.w + rho, ro = rr + jr;
+                        hit = d2 - rr * rr < 0.0f;
+                        open = d2 - ro * ro < 0.0f;
+                    }
+                    ++st.leaf;
+                    if (__any_sync(kFull, hit)) return true;
+                    const unsigned om = __ballot_sync(kFull, open);
+                    if (om) {
+                        if (open) scratch[__popc(om & lt)] = make_uint2((unsigned)(jk - kSegMid), (unsigned)(leaf << 12 | jp));
+                        __syncwarp();
+                        const int m = __popc(om) * kSegment;
+                        for (int q = lane; q - lane < m; q += 32) {
+                            bool h = false;
+                            if (q < m) {
+                                const uint2 x = scratch[q / kSegment];
+                                float4 ls = rows[table_index<M>((size_t)(x.x + (unsigned)(q & (kSegment - 1))),
+                                                                (int)(x.y >> 12))];
+                                ls.w += kEnvInflate;
+                                h = sphere_hits_prim(ls, prim + (x.y & 4095u) * kPrimF4);
+                            }
+                            ++st.leaf;
+                            if (__any_sync(kFull, h)) return true;
+                        }
+                        __syncwarp();  // scratch is read before the next step's writes
+                    }
+                }
+            } else {
+                if (near) scratch[__popc(nm & lt)] = make_uint2((unsigned)(k - kSegMid), pr);
+                __syncwarp();
+                const int m = __popc(nm) * kSegment;
+                for (int q = lane; q - lane < m; q += 32) {
+                    const uint2 x = scratch[min(q, m - 1) / kSegment];
+                    if (walk_items<M>(P.table, row0, (int)x.x + (q & (kSegment - 1)), x.y, q < m, prim, np,
+                                      GL, st))
+                        return true;
+                }
+                __syncwarp();
+            }
+        }
+        c += dc;
+        r += dr;
+        if (c >= C) {
+            c -= C;
+            ++r;
+        }
+    }
+    return false;
+}
+
 // Learned order, whole warp: perm_buf[rank] = segment, the edge's nseg <= 64
 // segments in descending MLP score (scores[0 .. nseg)), ties by index, NaN
-// last; returns segment 0's rank.
-__device__ __forceinline__ int rank_segments(const float* scores, int nseg, uint8_t* perm_buf) {
+// last, with first_ahead segment 0 before all others; returns segment 0's rank.
+__device__ __forceinline__ int rank_segments(const float* scores, int nseg, uint8_t* perm_buf,
+                                             bool first_ahead = false) {
     const int lane = threadIdx.x & 31;
     float v0 = lane < nseg ? scores[lane] : -INFINITY;
     float v1 = lane + 32 < nseg ? scores[lane + 32] : -INFINITY;
     v0 = isnan(v0) ? -INFINITY : v0;
     v1 = isnan(v1) ? -INFINITY : v1;
+    if (first_ahead && lane == 0) v0 = INFINITY;
     int rank0 = 0, rank1 = 0;
     for (int i = 0; i < nseg; ++i) {
         const float vi = __shfl_sync(kFull, i < 32 ? v0 : v1, i & 31);
@@ -922,10 +1166,16 @@ __device__ __forceinline__ int queue_pair(const CheckParams& P, int e, int env, 
     return r;
 }
 
-// Inline learned order of pair (env, e): the 32-block permutation scored for
-// the environment's cluster.
-__device__ __forceinline__ const uint8_t* inline_perm(const CheckParams& P, int env, int e) {
-    return P.perms + ((size_t)P.env_cluster[env] * P.num_edges + e) * kLanes;
+// The calling warp's 32 scratch entries (walk_segments); at most 8 warps a CTA.
+__device__ __forceinline__ uint2* warp_scratch() {
+    __shared__ uint2 scratch[8][32];
+    return scratch[threadIdx.x >> 5];
+}
+
+// Inline learned order of pair (env, e): the segment order scored for the
+// environment's cluster; null for edges of too many segments (plain order).
+__device__ __forceinline__ const uint8_t* inline_perm(const CheckParams& P, int env, int e, int n) {
+    return 4 * n <= kMaxSegments ? P.perms + ((size_t)P.env_cluster[env] * P.num_edges + e) * kMaxSegments : nullptr;
 }
 
 // One (environment, edge) pair, whole warp: cull, pair-list compaction and the
@@ -936,12 +1186,13 @@ __device__ __forceinline__ const uint8_t* inline_perm(const CheckParams& P, int 
 // segment score, its chunks split over the CTA's warps; MODE 3 (phase 3, one
 // warp per pair): the same walk by this warp alone, which writes the verdict.
 // `prim` holds the environment's records (shared or global memory), `masks`
-// its cull masks, W 64-bit words per mask.
+// its cull masks, W 64-bit words per mask; `alive` the groups that can hit at
+// all (bit g; the others are left out of the cull).
 template <class M, int MODE>
 __device__ __forceinline__ void check_pair(const CheckParams& P, int env, int e, int seg_row, const float4* prim,
                                            const uint64_t* __restrict__ masks, int np, int W, uint16_t* pairs,
                                            uint8_t* perm_buf, const GroupLanes& GL, int chunk0 = 0, int stride = 1,
-                                           volatile int* stop = nullptr) {
+                                           volatile int* stop = nullptr, unsigned alive = kFull) {
     constexpr int G = M::num_env_groups;
     constexpr int GB = group_bits<M>();
     const int lane = threadIdx.x & 31;
@@ -957,7 +1208,7 @@ __device__ __forceinline__ void check_pair(const CheckParams& P, int env, int e,
     }
     // Cull: lane g < G takes link g's slab ranges on the set's grid (computed
     // once per edge) and ANDs the environment's three masks over them.
-    const int code = lane < G ? P.edge_tri[(size_t)e * G + lane] : -1;
+    const int code = lane < G && ((alive >> lane) & 1u) ? P.edge_tri[(size_t)e * G + lane] : -1;
     // Word w of link g's candidate mask (only the packed code stays live
     // across the walk; the three offsets are re-derived where needed).
     auto mask_word = [&](int w) {
@@ -1037,9 +1288,9 @@ __device__ __forceinline__ void check_pair(const CheckParams& P, int env, int e,
                 collide = walk_pairs<M, 0>(P.table, row0, n, Cs, pairs, prim, np, nullptr, 0, GL, undecided, st,
                                            queue);
             }
-        } else if constexpr (MODE == 4) {
-            collide = walk_pairs<M, 4>(P.table, row0, n, Cs, pairs, prim, np, inline_perm(P, env, e), 0, GL,
-                                       undecided, st, queue);
+        } else if constexpr (MODE == 0 || MODE == 4) {
+            collide = walk_segments<M>(P, row0, n, Cs, pairs, prim, np, MODE == 4 ? inline_perm(P, env, e, n) : nullptr,
+                                       GL, warp_scratch(), st);
         } else {
             collide = walk_pairs<M, MODE>(P.table, row0, n, Cs, pairs, prim, np, learned ? perm_buf : nullptr,
                                           P.queue_min_items, GL, undecided, st, queue, 32 * chunk0, -1, stride,
@@ -1148,9 +1399,9 @@ __device__ __forceinline__ void walk_listed_pair(const CheckParams& P, int env, 
         } else {
             collide = walk_pairs<M, 0>(P.table, row0, n, C, pairs, prim, np, nullptr, 0, GL, undecided, st, queue);
         }
-    } else if constexpr (MODE == 4) {
-        collide = walk_pairs<M, 4>(P.table, row0, n, C, pairs, prim, np, inline_perm(P, env, e), 0, GL, undecided,
-                                   st, queue);
+    } else if constexpr (MODE == 0 || MODE == 4) {
+        collide = walk_segments<M>(P, row0, n, C, pairs, prim, np, MODE == 4 ? inline_perm(P, env, e, n) : nullptr, GL,
+                                   warp_scratch(), st);
     } else {
         collide = walk_pairs<M, MODE>(P.table, row0, n, C, pairs, prim, np, nullptr, P.queue_min_items, GL, undecided,
                                       st, queue);
@@ -1169,164 +1420,16 @@ __device__ __forceinline__ void walk_listed_pair(const CheckParams& P, int env, 
     }
 }
 
-// Plain order with 16 lanes per walking pair (MODE 5; robots whose leaves lie
-// inside their bounds): the warp's two halves walk two listed pairs at once,
-// 16 (sample rank, candidate) items a step each, in the reference's order.
-// The leaf work of a step is flattened inside each half; a half whose pair is
-// decided (a hit, or every item walked) writes the verdict and takes the next
-// pair of the walk list wt[0 .. nwalk).  A pair that collides in its first 16
-// items -- most of them -- then costs half a warp step instead of a whole one.
-template <class M, int SUB>
-__device__ __forceinline__ void walk_halves(const CheckParams& P, int env, int e0, int nwalk, const int (&wt)[SUB],
-                                            const int (&Cs)[SUB], const int (&base)[SUB], const uint16_t* pairs,
-                                            const float4* prim, const GroupLanes& GL) {
-    static_assert(!has_overhang<M>(), "the half-warp walk covers robots whose leaves lie inside their bounds");
-    constexpr int G = M::num_env_groups;
-    constexpr int GB = group_bits<M>();
-    constexpr int H = 16;
-    const int lane = threadIdx.x & 31, h = lane >> 4, hl = lane & (H - 1);
-    const unsigned hmask = h ? 0xffff0000u : 0x0000ffffu;
-    int t = -1, C = 1, bse = 0, n = 1, total = 0, w0 = 0, r = 0, c = 0, dr = 0, dc = 0, e = e0, row0 = 0;
-    WalkStats st;
-    auto take = [&](int idx) {
-        int tt = -1;
-#pragma unroll
-        for (int u = 0; u < SUB; ++u)
-            if (u == idx && u < nwalk) tt = wt[u];
-        t = tt;
-        if (t >= 0) {
-            int cc = 1, bb = 0;
-#pragma unroll
-            for (int u = 0; u < SUB; ++u)
-                if (u == t) {
-                    cc = Cs[u];
-                    bb = base[u];
-                }
-            C = cc;
-            bse = bb;
-            e = e0 + t;
-            n = P.steps[e];
-            row0 = P.offs[e];
-            total = kLanes * n * C;
-            w0 = 0;
-            // a / C for a <= 16 in FP32, exact as in walk_pairs
-            const float inv_c = __frcp_rn((float)C);
-            dr = (int)(16.5f * inv_c);
-            dc = H - dr * C;
-            r = (int)(((float)hl + 0.5f) * inv_c);
-            c = hl - r * C;
-            st = WalkStats();
-        }
-    };
-    take(h);
-    int nxt = 2;
-    // Bound on the loop (the warp-uniform step count): every step walks 16
-    // items of each live pair or ends one, so a group of pairs needs far fewer;
-    // past it the warp flags the error and leaves.
-    unsigned steps_left = 1u << 24;
-    for (;;) {
-        const bool act = t >= 0;
-        if (!__any_sync(kFull, act)) break;
-        if (--steps_left == 0) {
-            if (lane == 0) atomicOr(P.error_flag, 4);
-            break;
-        }
-        const uint32_t pr = act ? (uint32_t)pairs[bse + c] : 0u;
-        const int g = (int)(pr & ((1u << GB) - 1u));
-        const int p = (int)(pr >> GB);
-        const int fc = __shfl_sync(kFull, GL.fc, g);
-        const int first = fc & 0xffff, gcnt = fc >> 16;
-        int k = 0, cnt = 0;
-        if (act && w0 + hl < total) {
-            k = reference_rank_to_sample(r, n);
-            float4 bs = P.table[table_index<M>((size_t)(row0 + k), g)];
-            bs.w += kEnvInflate;
-            cnt = sphere_hits_prim(bs, prim + p * kPrimF4) ? gcnt : 0;
-        }
-        if (act) ++st.chunks;
-        bool hitp = false;
-        const unsigned gates = __ballot_sync(kFull, cnt > 0);
-        if (gates) {
-            if (gates & hmask) ++st.gates;
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < H; o <<= 1) {
-                const int y = __shfl_up_sync(kFull, incl, o, H);
-                if (hl >= o) incl += y;
-            }
-            const int L = __shfl_sync(kFull, incl, H - 1, H);
-            const int Lw = max(L, __shfl_xor_sync(kFull, L, 16));
-            // a slot's item: its sample, primitive and leaf offset (first - exclusive count)
-            static_assert(max_prims_of<M>() < 4096, "primitive index packs into 12 bits");
-            const int dp = (int)(((unsigned)(first - (incl - cnt)) << 12) | (unsigned)p);
-            for (int t0 = 0; t0 < Lw; t0 += H) {
-                const int tt = t0 + hl;
-                int j = 0;  // owner: the first lane of the half whose inclusive count exceeds tt
-#pragma unroll
-                for (int step = H / 2; step; step >>= 1) {
-                    const int v = __shfl_sync(kFull, incl, j + step - 1, H);
-                    if (v <= tt) j += step;
-                }
-                const int jd = __shfl_sync(kFull, dp, j, H);
-                const int jk = __shfl_sync(kFull, k, j, H);
-                bool hit = false;
-                if (tt < L) {
-                    float4 ls = P.table[table_index<M>((size_t)(row0 + jk), G + tt + (jd >> 12))];
-                    ls.w += kEnvInflate;
-                    hit = sphere_hits_prim(ls, prim + (jd & 4095) * kPrimF4);
-                }
-                if (t0 < L) ++st.leaf;
-                // the ballot on its own statement: every lane must reach it, so it
-                // must not sit behind a short-circuiting ||
-                const unsigned hb = __ballot_sync(kFull, hit);
-                hitp = hitp || (hb & hmask) != 0;
-                if (__all_sync(kFull, hitp || t0 + H >= L)) break;  // every half hit or out of slots
-            }
-        }
-        bool fin = false;
-        if (act) {
-            if (hitp) {
-                fin = true;
-            } else {
-                w0 += H;
-                c += dc;
-                r += dr;
-                if (c >= C) {
-                    c -= C;
-                    ++r;
-                }
-                fin = w0 >= total;
-            }
-        }
-        if (fin && hl == 0) {
-            P.results[(size_t)e * P.num_envs + env] = hitp ? 1 : 0;
-            if (P.counters) {
-                atomicAdd(P.counters + 0, 1ull);
-                atomicAdd(P.counters + 1, (unsigned long long)C);
-                atomicAdd(P.counters + 2, (unsigned long long)st.chunks);
-                atomicAdd(P.counters + 3, (unsigned long long)st.gates);
-                atomicAdd(P.counters + 4, (unsigned long long)st.leaf);
-                atomicAdd(P.counters + 5, hitp ? 1ull : 0ull);
-            }
-        }
-        // next pairs, in half order, the same on every lane
-        const unsigned fb = __ballot_sync(kFull, fin && hl == 0);
-        const int f0 = (int)(fb & 1u), f1 = (int)((fb >> 16) & 1u);
-        const int i0 = nxt, i1 = nxt + f0;
-        nxt += f0 + f1;
-        if (fin) take(h ? i1 : i0);
-    }
-}
-
-// Pairs (env, e0 .. e0 + count - 1), count <= pairs_per_setup<M>(), whole
-// warp: lane group s = lane / G culls pair s (lane g of the group ANDs link
+// Pairs (env, e0 .. e0 + count - 1), or with a list (env, list[0 .. count).x)
+// and their alive groups (.y), count <= pairs_per_setup<M>(), whole warp: lane group s = lane / G culls pair s (lane g of the group ANDs link
 // g's three masks), a scan inside each group gives every link its offset,
 // the groups' lists are laid out one after another in `pairs` and written in
 // one pass; then the warp walks the pairs one at a time.  When the lists do
 // not fit the warp's buffer together, each pair goes through check_pair
 // (segments).
 template <class M, int MODE>
-__device__ __forceinline__ void check_pair_group(const CheckParams& P, int env, int e0, int count, const float4* prim,
+__device__ __forceinline__ void check_pair_group(const CheckParams& P, int env, int e0, int count,
+                                                 const uint2* list, const float4* prim,
                                                  const uint64_t* __restrict__ masks, int np, int W, uint16_t* pairs,
                                                  const GroupLanes& GL) {
     constexpr int G = M::num_env_groups;
@@ -1336,9 +1439,10 @@ __device__ __forceinline__ void check_pair_group(const CheckParams& P, int env, 
     const int sub = lane / G;
     const int g = lane - sub * G;
     const bool live = sub < count;
-    const int e = e0 + (live ? sub : 0);
+    const uint2 entry = list ? list[live ? sub : 0] : make_uint2((unsigned)(e0 + (live ? sub : 0)), kFull);
+    const int e = (int)entry.x;
     const int self = live ? P.edge_self[e] : 1;
-    const int code = (live && !self && np > 0) ? P.edge_tri[(size_t)e * G + g] : -1;
+    const int code = (live && !self && np > 0 && ((entry.y >> g) & 1u)) ? P.edge_tri[(size_t)e * G + g] : -1;
     auto mask_word = [&](int w) {
         const int tx = code & 1023, ty = (code >> 10) & 1023, tz = code >> 20;
         return __ldg(masks + tx * W + w) & __ldg(masks + (kGridTri + ty) * W + w) &
@@ -1371,10 +1475,10 @@ __device__ __forceinline__ void check_pair_group(const CheckParams& P, int env, 
         base[t] = total;
         total += t < count ? Cs[t] : 0;
     }
-    constexpr int PAIR_MODE = MODE == 5 ? 0 : MODE;
     if (total > P.pairs_per_warp) {
         for (int t = 0; t < count; ++t)
-            check_pair<M, PAIR_MODE>(P, env, e0 + t, -1, prim, masks, np, W, pairs, nullptr, GL);
+            check_pair<M, MODE>(P, env, list ? (int)list[t].x : e0 + t, -1, prim, masks, np, W, pairs, nullptr, GL, 0,
+                                1, nullptr, list ? list[t].y : kFull);
         return;
     }
     if (cnt > 0) {
@@ -1404,38 +1508,9 @@ __device__ __forceinline__ void check_pair_group(const CheckParams& P, int env, 
         }
     }
     __syncwarp();
-    if constexpr (MODE == 5) {
-        // the pairs decided without a walk first, the rest walked by half-warps
-        int wt[SUB];
-        int nwalk = 0;
-#pragma unroll
-        for (int t = 0; t < SUB; ++t) wt[t] = -1;
-#pragma unroll
-        for (int t = 0; t < SUB; ++t) {
-            if (t >= count) continue;  // warp-uniform
-            const int et = e0 + t;
-            const int self_t = __shfl_sync(kFull, self, t * G);
-            if (np == 0 || self_t) {
-                if (lane == 0) P.results[(size_t)et * P.num_envs + env] = self_t ? 1 : 0;
-                continue;
-            }
-            if (Cs[t] == 0) {
-                if (lane == 0) {
-                    P.results[(size_t)et * P.num_envs + env] = 0;
-                    if (P.counters) atomicAdd(P.counters + 0, 1ull);
-                }
-                continue;
-            }
-#pragma unroll
-            for (int u = 0; u < SUB; ++u)
-                if (u == nwalk) wt[u] = t;
-            ++nwalk;
-        }
-        walk_halves<M, SUB>(P, env, e0, nwalk, wt, Cs, base, pairs, prim, GL);
-    } else {
 #pragma unroll 1
     for (int t = 0; t < count; ++t) {
-        const int et = e0 + t;
+        const int et = __shfl_sync(kFull, e, t * G);
         const int self_t = __shfl_sync(kFull, self, t * G);
         if (np == 0 || self_t) {  // decided without a walk (not counted as walked, as in check_pair)
             if (lane == 0) P.results[(size_t)et * P.num_envs + env] = self_t ? 1 : 0;
@@ -1454,21 +1529,246 @@ __device__ __forceinline__ void check_pair_group(const CheckParams& P, int env, 
             if (u == t) bt = base[u];
         walk_listed_pair<M, MODE>(P, env, et, Cs[t], pairs + bt, prim, np, GL);
     }
-    }
     __syncwarp();  // every lane is done with the lists before the next group's writes
 }
 
+// Bytes of an environment's primitive records (what a CTA stages).
+__device__ __forceinline__ uint32_t record_bytes_of(float4 h1) {
+    return (__float_as_uint(h1.w) & 0xffffu) * kPrimF4 * 16u;
+}
+
+// Check CTAs are compiled for M::check_warps_per_sm resident warps per SM (a
+// register budget of 65536 / (32 x that) per thread), at most 32 CTAs per SM.
+template <class M, int WARPS>
+constexpr int check_min_ctas() {
+    return M::check_warps_per_sm / WARPS < 32 ? M::check_warps_per_sm / WARPS : 32;
+}
+
+// Probe of pair (env, e), one lane per pair (decided: the lane has none).  Per
+// group P.mid holds the bound's centre at the edge's middle sample and the
+// radius R of the sphere around it that holds the group's leaves, inflated,
+// over all of the edge's samples.  The voxel of the centre gives the signed
+// distance to the nearest primitive, good to the offset from the voxel's
+// centre.  Well inside the certain-hit radius (cert_radius) it proves a leaf
+// hit at the middle sample; above R it proves the group free along the whole
+// edge; between the two the exact certain-hit test on the voxel's nearest
+// primitive finds most of the other hits.  Returns 1 for a hit, else 0; `alive`
+// gets the groups not proved free (none: the pair is free).  Groups in
+// descending certain-hit radius; the warp leaves once all its lanes are decided.
+template <class M>
+__device__ __forceinline__ bool probe_pair(const CheckParams& P, int e, bool decided, const uint16_t* vox,
+                                           const float4* prim, unsigned& alive) {
+    const DevTables<M>& T = tab<M>();
+    const ProbeGrid& V = P.probe;
+    const float bx = -V.ox * V.inv_h, by = -V.oy * V.inv_h, bz = -V.oz * V.inv_h;
+    const float mx = (float)(V.nx - 1), my = (float)(V.ny - 1), mz = (float)(V.nz - 1);
+    const float sy = (float)V.nx, sz = (float)(V.nx * V.ny);
+    const float h2 = V.h * V.h * 1.0002f;
+    constexpr float kRound = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
+    bool hit = false;
+    alive = 0u;
+    for (int i = 0; i < M::num_env_groups; ++i) {
+        if (__all_sync(kFull, decided)) break;
+        const int g = T.probe_group[i];
+        if (!decided) {
+            const float4 c = P.mid[(size_t)g * P.num_edges + e];
+            const float kappa = T.cert_r[g];
+            // position in voxels from the centre of voxel 0, the nearest voxel, the offset from it
+            const float fx = fmaf(c.x, V.inv_h, bx), fy = fmaf(c.y, V.inv_h, by), fz = fmaf(c.z, V.inv_h, bz);
+            const float ix = (fminf(fmaxf(fx, 0.0f), mx) + kRound) - kRound;
+            const float iy = (fminf(fmaxf(fy, 0.0f), my) + kRound) - kRound;
+            const float iz = (fminf(fmaxf(fz, 0.0f), mz) + kRound) - kRound;
+            const float rx = fx - ix, ry = fy - iy, rz = fz - iz;
+            const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz)) * h2;  // squared offset (m^2)
+            const unsigned w = vox[(int)fmaf(iz, sz, fmaf(iy, sy, ix))];
+            // the voxel's distance lies in [lo, lo + step + 2 slack)
+            const float lo = fmaf((float)(w & 255u), kVoxStep, kVoxMin - kVoxSlack);
+            const float miss = lo - c.w, up = kappa - (lo + kVoxStep + 2.0f * kVoxSlack), dn = lo - kappa;
+            if (miss > 0.0f && miss * miss > r2) continue;
+            alive |= 1u << g;
+            if (kappa > 0.0f) {
+                if (up > 0.0f && up * up > r2) {
+                    hit = decided = true;
+                } else if (!(dn > 0.0f && dn * dn > r2) && r2 < 1e30f && (w >> 8) != kVoxUnknown) {
+                    // the voxel leaves it open (a non-finite centre is left to the walk)
+                    float rho;
+                    const float d2 = prim_core_d2(c, prim + (w >> 8) * kPrimF4, &rho);
+                    const float rc = rho + kappa;
+                    hit = decided = d2 - rc * rc < 0.0f;
+                }
+            }
+        }
+    }
+    return hit;
+}
+
+// First pass of a check with probe grids: CTA = one environment x kProbeBatch
+// edges, one lane per pair.  Decided pairs get their verdict; the others go to
+// the queue (Q) as (edge, alive groups), contiguous per CTA, with one work item
+// per Q.chunk of them.  On the uneven Panda workload (1000 x 10000) it decides
+// 84 % of the pairs in 0.33 ms, 29 warp instructions a pair, bound by issue;
+// walking every pair took 390 instructions a pair and 4.2 ms, probe and walk
+// take 1.4 ms.
+constexpr int kProbeThreads = 256;
+
+template <class M>
+__global__ void __launch_bounds__(kProbeThreads, 6) probe_kernel(CheckParams P, ProbeQueue Q, int env0) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t bar;
+    __shared__ int s_cnt, s_base, s_item;
+    const int env = env0 + blockIdx.x, e0 = blockIdx.y * kProbeBatch;
+    const int nb = min(kProbeBatch, P.num_edges - e0);
+    const int lane = threadIdx.x & 31;
+    const float4 h0 = P.env_hdr[2 * env + 0];
+    const float4 h1 = P.env_hdr[2 * env + 1];
+    const uint32_t bytes = record_bytes_of(h1);
+    const int np = (int)(__float_as_uint(h1.w) & 0xffffu);
+    const bool probe = np > 0 && !(__float_as_uint(h1.z) & kEnvIrregular);
+    const float4* prim = reinterpret_cast<const float4*>(smem);
+    const uint16_t* vox = reinterpret_cast<const uint16_t*>(smem + P.blob_smem);
+    uint2* list = reinterpret_cast<uint2*>(smem + P.blob_smem + P.probe.stride);
+    if (threadIdx.x == 0) {
+        s_cnt = 0;
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (probe) {
+        if (threadIdx.x == 0) {
+            bulk_expect(&bar, bytes + P.probe.stride);
+            bulk_copy_part(smem, P.blobs + (size_t)__float_as_uint(h0.w), bytes, &bar);
+            bulk_copy_part(smem + P.blob_smem, P.probe.vox + (size_t)env * (P.probe.stride / 2), P.probe.stride, &bar);
+        }
+        // One path for the whole CTA (see check_kernel).
+        const bool ok = mbar_wait_bounded(&bar, 0u, 1u << 22);
+        if (__syncthreads_or(!ok)) {
+            if (threadIdx.x == 0) atomicOr(P.error_flag, 1);
+            mbar_wait_bounded(&bar, 0u, 1u << 22);
+            return;
+        }
+    }
+    for (int i0 = threadIdx.x & ~31; i0 < nb; i0 += kProbeThreads) {
+        const int i = i0 + lane, e = e0 + min(i, nb - 1);
+        const int self = i < nb ? P.edge_self[e] : 1;
+        unsigned alive = np > 0 ? kFull : 0u;
+        bool hit = self != 0;
+        if (probe) hit = probe_pair<M>(P, e, hit, vox, prim, alive) || hit;
+        const bool open = !hit && alive != 0u;
+        if (i < nb && !open) P.results[(size_t)e * P.num_envs + env] = hit ? 1 : 0;
+        const unsigned m = __ballot_sync(kFull, open);
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(&s_cnt, __popc(m));
+        at = __shfl_sync(kFull, at, 0);
+        if (open) list[at + __popc(m & ((1u << lane) - 1u))] = make_uint2((unsigned)e, alive);
+        if (P.counters && np > 0) {
+            const unsigned dec = __ballot_sync(kFull, !open && !self), col = __ballot_sync(kFull, hit && !self);
+            if (lane == 0) {
+                atomicAdd(P.counters + 0, (unsigned long long)__popc(dec));
+                atomicAdd(P.counters + 5, (unsigned long long)__popc(col));
+            }
+        }
+    }
+    __syncthreads();
+    const int u = s_cnt;
+    if (u == 0) return;
+    const int items = (u + Q.chunk - 1) / Q.chunk;
+    if (threadIdx.x == 0) {
+        s_base = atomicAdd(Q.head + 0, u);
+        s_item = atomicAdd(Q.head + 1, items);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < u; i += kProbeThreads) Q.entries[s_base + i] = list[i];
+    for (int i = threadIdx.x; i < items; i += kProbeThreads)
+        Q.items[s_item + i] = make_int4(env, s_base + i * Q.chunk, min(Q.chunk, u - i * Q.chunk), 0);
+}
+
+// Resident warps per SM the walk is compiled for: 48 registers a thread.  Swept
+// on 1000 x 20000 stress pairs: 5.97 ms at 48 warps, 5.16 at 40, 5.73 at 32,
+// 6.34 at 24 (probe 0.77 ms included).
+constexpr int kWalkWarps = 40;
+
+template <class M, int WARPS>
+constexpr int walk_min_ctas() {
+    return kWalkWarps / WARPS < 32 ? kWalkWarps / WARPS : 32;
+}
+
+// Second pass: persistent CTAs pull work items (an environment and up to
+// Q.chunk of its undecided pairs), stage the environment's records when it
+// changes, and their warps take pairs_per_setup pairs at a time from a shared
+// counter.  Items of a few dozen pairs even out what a tile of edges could not:
+// the undecided pairs of a set cluster in its sparse environments.
+template <class M, int WARPS, int MODE>
+__global__ void __launch_bounds__(WARPS * 32, walk_min_ctas<M, WARPS>()) walk_kernel(CheckParams P, ProbeQueue Q) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t bar;
+    __shared__ int4 s_work;
+    __shared__ int s_next;
+    constexpr int SUB = pairs_per_setup<M>();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int total = Q.head[1];
+    const float4* prim = reinterpret_cast<const float4*>(smem);
+    uint16_t* pairs = reinterpret_cast<uint16_t*>(smem + P.blob_smem) + (size_t)warp * P.pairs_per_warp;
+    const GroupLanes GL = group_lanes<M>();
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    int staged = -1;
+    uint32_t phase = 0;
+    for (;;) {
+        __syncthreads();  // every warp is done with the previous item
+        if (threadIdx.x == 0) {
+            const int i = atomicAdd(Q.head + 2, 1);
+            s_work = i < total ? Q.items[i] : make_int4(-1, 0, 0, 0);
+            s_next = 0;
+        }
+        __syncthreads();
+        const int4 work = s_work;
+        const int env = work.x;
+        if (env < 0) break;
+        const float4 h0 = P.env_hdr[2 * env + 0];
+        const float4 h1 = P.env_hdr[2 * env + 1];
+        if (env != staged) {  // an item's environment has primitives
+            if (threadIdx.x == 0)
+                bulk_copy_g2s(smem, P.blobs + (size_t)__float_as_uint(h0.w), record_bytes_of(h1), &bar);
+            const bool ok = mbar_wait_bounded(&bar, phase, 1u << 22);
+            if (__syncthreads_or(!ok)) {  // one path for the whole CTA (see check_kernel)
+                if (threadIdx.x == 0) atomicOr(P.error_flag, 1);
+                mbar_wait_bounded(&bar, phase, 1u << 22);
+                break;
+            }
+            phase ^= 1u;
+            staged = env;
+        }
+        const uint32_t shape = __float_as_uint(h1.w);
+        const int np = (int)(shape & 0xffffu), W = (int)(shape >> 16);
+        const uint64_t* __restrict__ masks =
+            reinterpret_cast<const uint64_t*>(P.blobs + (size_t)__float_as_uint(h0.w) + (size_t)np * kPrimF4);
+        const uint2* list = Q.entries + work.y;
+        for (;;) {
+            int slot = 0;
+            if (lane == 0) slot = atomicAdd(&s_next, SUB);
+            slot = __shfl_sync(kFull, slot, 0);
+            if (slot >= work.z) break;
+            if constexpr (SUB > 1)
+                check_pair_group<M, MODE>(P, env, 0, min(SUB, work.z - slot), list + slot, prim, masks, np, W, pairs,
+                                          GL);
+            else
+                check_pair<M, MODE>(P, env, (int)list[slot].x, -1, prim, masks, np, W, pairs, nullptr, GL, 0, 1,
+                                    nullptr, list[slot].y);
+        }
+    }
+}
+
 // check_tile processes the edges of one (environment, edge tile) work item
-// (modes 0 and 1) with the environment's records already staged in shared
-// memory; it is shared by the one-CTA-per-item grid kernel and the persistent
-// kernel.  Each warp takes pairs_per_setup consecutive edges at a time.
+// (modes 0, 1 and 4) with the environment's records already staged in shared
+// memory.  Each warp takes pairs_per_setup consecutive edges at a time.
 template <class M, int WARPS, int MODE>
 __device__ __forceinline__ void check_tile(const CheckParams& P, int env, int tile, int n_slots,
-                                           const unsigned char* smem, float4 h0, float4 h1,
-                                           int* s_next = nullptr) {
+                                           const unsigned char* smem, float4 h0, float4 h1, int* s_next) {
     constexpr int SUB = pairs_per_setup<M>();
     const int e_begin = tile * P.edges_per_cta;
-    const int warp = threadIdx.x >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t shape = __float_as_uint(h1.w);
     const int np = (int)(shape & 0xffffu);
     const int W = (int)(shape >> 16);  // 64-bit words per primitive mask
@@ -1480,29 +1780,19 @@ __device__ __forceinline__ void check_tile(const CheckParams& P, int env, int ti
     uint16_t* pairs =
         reinterpret_cast<uint16_t*>(const_cast<unsigned char*>(smem) + P.blob_smem) + (size_t)warp * P.pairs_per_warp;
     const GroupLanes GL = group_lanes<M>();
-    if (s_next) {
-        // Warps take the tile's next pass from a shared counter: a pass costs
-        // from one chunk (a pair colliding at its first sample) to dozens (a
-        // collision-free pair), so a fixed stride leaves warps idle while the
-        // CTA's last one finishes.
-        const int lane = threadIdx.x & 31;
-        for (;;) {
-            int slot = 0;
-            if (lane == 0) slot = atomicAdd(s_next, SUB);
-            slot = __shfl_sync(kFull, slot, 0);
-            if (slot >= n_slots) break;
-            if constexpr (SUB > 1)
-                check_pair_group<M, MODE>(P, env, e_begin + slot, min(SUB, n_slots - slot), prim, masks, np, W,
-                                          pairs, GL);
-            else
-                check_pair<M, MODE>(P, env, e_begin + slot, -1, prim, masks, np, W, pairs, nullptr, GL);
-        }
-    } else if constexpr (SUB > 1) {
-        for (int slot = warp * SUB; slot < n_slots; slot += WARPS * SUB)
-            check_pair_group<M, MODE>(P, env, e_begin + slot, min(SUB, n_slots - slot), prim, masks, np, W, pairs,
-                                      GL);
-    } else {
-        for (int slot = warp; slot < n_slots; slot += WARPS)
+    // Warps take the tile's next pass from a shared counter: a pass costs
+    // from one chunk (a pair colliding at its first sample) to dozens (a
+    // collision-free pair), so a fixed stride leaves warps idle while the
+    // CTA's last one finishes.
+    for (;;) {
+        int slot = 0;
+        if (lane == 0) slot = atomicAdd(s_next, SUB);
+        slot = __shfl_sync(kFull, slot, 0);
+        if (slot >= n_slots) break;
+        if constexpr (SUB > 1)
+            check_pair_group<M, MODE>(P, env, e_begin + slot, min(SUB, n_slots - slot), nullptr, prim, masks, np, W,
+                                      pairs, GL);
+        else
             check_pair<M, MODE>(P, env, e_begin + slot, -1, prim, masks, np, W, pairs, nullptr, GL);
     }
 }
@@ -1512,19 +1802,7 @@ __device__ __forceinline__ int tile_slots(const CheckParams& P, int tile) {
     return min(P.edges_per_cta, P.num_edges - e_begin);
 }
 
-// Bytes of an environment's primitive records (what a CTA stages).
-__device__ __forceinline__ uint32_t record_bytes_of(float4 h1) {
-    return (__float_as_uint(h1.w) & 0xffffu) * kPrimF4 * 16u;
-}
-
 // One CTA per (environment, edge tile): blockIdx.x = environment, blockIdx.y = tile.
-// Check CTAs are compiled for M::check_warps_per_sm resident warps per SM (a
-// register budget of 65536 / (32 x that) per thread), at most 32 CTAs per SM.
-template <class M, int WARPS>
-constexpr int check_min_ctas() {
-    return M::check_warps_per_sm / WARPS < 32 ? M::check_warps_per_sm / WARPS : 32;
-}
-
 template <class M, int WARPS, int MODE>
 __global__ void __launch_bounds__(WARPS * 32, check_min_ctas<M, WARPS>()) check_kernel(CheckParams P) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1556,65 +1834,6 @@ __global__ void __launch_bounds__(WARPS * 32, check_min_ctas<M, WARPS>()) check_
         __syncthreads();  // s_next is set before any warp takes a pass
     }
     check_tile<M, WARPS, MODE>(P, env, tile, n_slots, smem, h0, h1, &s_next);
-}
-
-// Persistent: a grid sized to the resident capacity pulls environment-major
-// work items (environment, edge tile) from an atomic counter, two at a time so
-// that consecutive items usually share the environment and its staged blob.
-constexpr int kItemsPerGrab = 2;
-
-template <class M, int WARPS, int MODE>
-__global__ void __launch_bounds__(WARPS * 32, check_min_ctas<M, WARPS>()) check_persistent_kernel(CheckParams P) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ uint64_t bar;
-    __shared__ int s_item;
-    __shared__ int s_next[kItemsPerGrab];  // per grabbed item: the next pass a warp takes
-    const int tiles = (P.num_edges + P.edges_per_cta - 1) / P.edges_per_cta;
-    const long long items = (long long)P.num_envs * tiles;
-    if (threadIdx.x == 0) {
-        mbar_init(&bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    int staged = -1;
-    uint32_t phase = 0;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            s_item = atomicAdd(P.work_counter, kItemsPerGrab);
-            for (int i = 0; i < kItemsPerGrab; ++i) s_next[i] = 0;
-        }
-        __syncthreads();
-        const int first = s_item;
-        __syncthreads();
-        if (first >= items) break;
-        bool failed = false;
-        for (int item = first; item < first + kItemsPerGrab && item < items; ++item) {
-            const int env = item / tiles, tile = item - (item / tiles) * tiles;
-            const int n_slots = tile_slots(P, tile);
-            if (n_slots <= 0) continue;
-            const float4 h0 = P.env_hdr[2 * env + 0];
-            const float4 h1 = P.env_hdr[2 * env + 1];
-            if (env != staged) {
-                const uint32_t bytes = record_bytes_of(h1);
-                __syncthreads();  // every warp is done with the previous blob
-                if (bytes) {
-                    if (threadIdx.x == 0) bulk_copy_g2s(smem, P.blobs + (size_t)__float_as_uint(h0.w), bytes, &bar);
-                    const bool ok = mbar_wait_bounded(&bar, phase, 1u << 22);
-                    if (__syncthreads_or(!ok)) {
-                        if (threadIdx.x == 0) atomicOr(P.error_flag, 1);
-                        mbar_wait_bounded(&bar, phase, 1u << 22);
-                        failed = true;
-                        break;
-                    }
-                    phase ^= 1u;
-                }
-                staged = env;
-            }
-            check_tile<M, WARPS, MODE>(P, env, tile, n_slots, smem, h0, h1, &s_next[item - first]);
-        }
-        if (failed) break;
-        __syncthreads();
-    }
 }
 
 // Learned order, phase 3: each CTA pulls queued pairs from finish_counter, one
@@ -1873,30 +2092,21 @@ __global__ void cluster_features_kernel(CheckParams P, const float* __restrict__
     write_features<M>(q, centroids + (size_t)c * kEnvCode, sample_position(k, P.steps[e]), x + (size_t)i * kMlpIn);
 }
 
-// Inline learned order, permutations: one warp per (cluster c, edge e).
-// Lane block t is scored by the segment holding its last sample t n + n - 1
-// (row c * S + offs[e] / 8 + segment); blocks are ranked by descending score,
-// ties (blocks of one segment) by descending index, so a segment is walked
-// from its end back, and block 0 is ranked first.  perms[(c * E + e) * 32 +
-// rank] = block.
+// Inline learned order, one warp per (cluster c, edge e): perms[(c * E + e) *
+// kMaxSegments + rank] = segment, segment 0 first (the scores tell where an edge
+// with a free start collides), the others by descending score (row c * S +
+// offs[e] / 8 + segment).  Edges of more segments keep the plain order.
 template <class M>
 __global__ void cluster_perm_kernel(CheckParams P, int K, uint8_t* __restrict__ perms) {
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
     const int E = P.num_edges;
     if (warp >= (long long)K * E) return;
     const int c = (int)(warp / E);
     const int e = (int)(warp - (long long)c * E);
-    const int n = P.steps[e];
-    float v = P.logits[(size_t)c * P.total_segs + P.offs[e] / kSegment + (lane * n + n - 1) / kSegment];
-    v = isnan(v) ? -INFINITY : v;
-    if (lane == 0) v = INFINITY;
-    int rank = 0;
-    for (int u = 0; u < kLanes; ++u) {
-        const float vu = __shfl_sync(kFull, v, u);
-        rank += (vu > v || (vu == v && u > lane)) ? 1 : 0;
-    }
-    perms[((size_t)c * E + e) * kLanes + rank] = (uint8_t)lane;
+    const int nseg = 4 * P.steps[e];
+    if (nseg > kMaxSegments) return;
+    rank_segments(P.logits + (size_t)c * P.total_segs + P.offs[e] / kSegment, nseg,
+                  perms + (size_t)warp * kMaxSegments, true);
 }
 
 // Training rows: row i draws (environment, edge, sample) from a hash of
@@ -2090,27 +2300,41 @@ cudaError_t run_steps(const PipelineArgs& a, cudaStream_t st) {
     return launch_scan(a.steps, E, a.offs, st);
 }
 
+// Probe and walk, in slabs of environments whose pairs fit the queue.
+template <class M, int W, int MODE>
+cudaError_t launch_probed(const CheckParams& P, int E, cudaStream_t st) {
+    const size_t smem = P.blob_smem + P.probe.stride + kProbeBatch * sizeof(uint2);
+    const size_t walk_smem = check_smem_bytes(P.max_prims, M::num_env_groups, P.blob_smem, W);
+    cudaError_t err = cudaFuncSetAttribute(probe_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    err = cudaFuncSetAttribute(walk_kernel<M, W, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem);
+    if (err != cudaSuccess) return err;
+    int per_sm = 0, dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk_kernel<M, W, MODE>, W * 32, walk_smem);
+    if (err != cudaSuccess) return err;
+    const int slots = std::max(per_sm, 1) * std::max(sms, 1);
+    ProbeQueue Q = P.queue;
+    const int slab = (int)std::min<long long>(P.num_envs, Q.cap / E);
+    err = cudaMemsetAsync(Q.head, 0, (size_t)((P.num_envs + slab - 1) / slab) * 16, st);
+    if (err != cudaSuccess) return err;
+    for (int env0 = 0; env0 < P.num_envs; env0 += slab, Q.head += 4) {
+        const int n = std::min(slab, P.num_envs - env0);
+        probe_kernel<M><<<dim3(n, (E + kProbeBatch - 1) / kProbeBatch), kProbeThreads, smem, st>>>(P, Q, env0);
+        const long long most = (long long)n * E;  // every pair undecided
+        const int grid = (int)std::min<long long>(slots, (most + Q.chunk - 1) / Q.chunk);
+        walk_kernel<M, W, MODE><<<grid, W * 32, walk_smem, st>>>(P, Q);
+    }
+    return cudaGetLastError();
+}
+
 template <class M, int W, int MODE>
 cudaError_t launch_check_wm(CheckParams P, int E, cudaStream_t st) {
     P.pairs_per_warp = std::min((P.max_prims * M::num_env_groups + 7) & ~7, kPairCap);
-    const size_t smem = P.blob_smem + (size_t)W * P.pairs_per_warp * sizeof(uint16_t);
-    if (P.persistent) {
-        cudaError_t err = cudaFuncSetAttribute(check_persistent_kernel<M, W, MODE>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (err != cudaSuccess) return err;
-        int per_sm = 0, dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, check_persistent_kernel<M, W, MODE>, W * 32, smem);
-        if (err != cudaSuccess) return err;
-        const long long items = (long long)P.num_envs * ((E + P.edges_per_cta - 1) / P.edges_per_cta);
-        long long grid = (long long)std::max(per_sm, 1) * std::max(sms, 1);
-        grid = std::min(grid, (items + kItemsPerGrab - 1) / kItemsPerGrab);
-        err = cudaMemsetAsync(P.work_counter, 0, sizeof(int), st);
-        if (err != cudaSuccess) return err;
-        check_persistent_kernel<M, W, MODE><<<(unsigned)std::max(grid, 1ll), W * 32, smem, st>>>(P);
-        return cudaGetLastError();
-    }
+    const size_t smem = check_smem_bytes(P.max_prims, M::num_env_groups, P.blob_smem, W);
+    if constexpr (MODE != 1)
+        if (P.probe.vox) return launch_probed<M, W, MODE>(P, E, st);
     cudaError_t err = cudaFuncSetAttribute(check_kernel<M, W, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem);
     if (err != cudaSuccess) return err;
@@ -2145,9 +2369,6 @@ cudaError_t launch_check_w(CheckParams P, int E, cudaStream_t st, int mode) {
         case 1: return launch_check_wm<M, W, 1>(P, E, st);
         case 2: return launch_finish_w<M, W>(P, st);
         case 4: return launch_check_wm<M, W, 4>(P, E, st);
-        case 5:  // 16 lanes per walking pair, where the robot has a grouped cull and no overhang
-            if constexpr (!has_overhang<M>() && pairs_per_setup<M>() > 1) return launch_check_wm<M, W, 5>(P, E, st);
-            return launch_check_wm<M, W, 0>(P, E, st);
         default: return launch_check_wm<M, W, 0>(P, E, st);
     }
 }
@@ -2187,11 +2408,10 @@ cudaError_t run_prep(const PipelineArgs& a, cudaStream_t st) {
             if (err != cudaSuccess) return err;
             const int blocks = (R + 31) / 32;
             const int grid = std::min(blocks, std::max(per_sm, 1) * std::max(sms, 1));
-            fk_staged_kernel<M><<<grid, 32, smem, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.row_edge, a.fk_perm,
-                                                        a.edge_self);
+            fk_staged_kernel<M><<<grid, 32, smem, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.row_edge,
+                                                        a.edge_self, a.seg);
         } else {
-            fk_kernel<M><<<(R + 127) / 128, 128, 0, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.row_edge,
-                                                           a.fk_perm);
+            fk_kernel<M><<<(R + 127) / 128, 128, 0, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.row_edge);
         }
     }
     if (ev) cudaEventRecord(ev[2], st);
@@ -2208,7 +2428,8 @@ cudaError_t run_prep(const PipelineArgs& a, cudaStream_t st) {
     }
     if (ev) cudaEventRecord(ev[3], st);
     swept_kernel<M><<<(E * 32 + 255) / 256, 256, 0, st>>>(a.table, a.offs, E, a.swept,
-                                                           a.grid_bounds ? a.edge_tri : nullptr, a.grid_bounds);
+                                                           a.grid_bounds ? a.edge_tri : nullptr, a.grid_bounds, a.mid,
+                                                           M::table_tile == 1 ? nullptr : a.seg);
     if (ev) cudaEventRecord(ev[4], st);
     return cudaGetLastError();
 }
@@ -2293,7 +2514,7 @@ RobotOps robot_ops_of(int robot, cudaError_t (*upload)()) {
     o.num_spheres = M::num_spheres;
     o.num_env_groups = M::num_env_groups;
     o.max_prims = max_prims_of<M>();
-    o.half_warp_walk = !has_overhang<M>() && pairs_per_setup<M>() > 1;
+    o.reach = reach_box<M>;
     o.upload_tables = upload;
     o.steps = run_steps<M>;
     o.check = run_check<M>;

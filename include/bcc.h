@@ -145,9 +145,9 @@ int32_t bcc_stage_times(bcc_ctx* ctx, float* ms, int32_t max_stages);
 
 /*
  * Work counters of the last check, when profiling was switched on with bit 1
- * set (bcc_set_profiling(ctx, 3)): [0] pairs walked, [1] candidate
- * (primitive, link) pairs after the cull, [2] walk steps (32 items, or 16
- * with 16 lanes per walking pair), [3] steps with a gate hit, [4] leaf steps,
+ * set (bcc_set_profiling(ctx, 3)): [0] pairs decided by the probe or the walk,
+ * [1] candidate (primitive, link) pairs of the walked pairs after the cull, [2]
+ * walk steps (32 items), [3] steps with a gate hit, [4] leaf steps,
  * [5] colliding pairs.  Diagnostics only: counting
  * adds atomics to the check kernel.  Returns the number written, or -1.
  */
@@ -275,10 +275,12 @@ bcc_status bcc_measure_fp32_peak(int32_t device, double* tflops);
 
 /*
  * Launch configuration of the environment check, BCC_LAUNCH_CONFIG_LEN values:
- * cfg[0] edges per CTA, cfg[1] warps per CTA (1, 2, 4, 8; lowered
- * automatically when an environment's shared-memory footprint needs it),
- * cfg[2] 1 = persistent kernel pulling (environment, edge tile) work items
- * from an atomic queue, 0 = one CTA per item, cfg[3] learned order: a pair is
+ * cfg[0] edges per CTA of the one-pass check, cfg[1] warps per CTA (1, 2, 4, 8;
+ * lowered automatically when an environment's shared-memory footprint needs
+ * it), cfg[2] 1 = a first pass decides most pairs from a voxel grid of each
+ * environment (built by the first such check after an upload) and a persistent
+ * kernel pulls the rest from a queue, 0 = one pass, one CTA per (environment,
+ * edge tile), cfg[3] learned order: a pair is
  * scored by the MLP only when at least this many (sample, pair) items remain
  * once its rank 0 (first sample) is walked, cfg[4] learned order: 1 = each
  * queued pair's walk split over a CTA's warps, 0 = one warp per queued pair,
@@ -288,17 +290,15 @@ bcc_status bcc_measure_fp32_peak(int32_t device, double* tflops);
  * their first sample are scored per pair and finished in a second pass),
  * cfg[6] inline order: environment clusters, 1..64 (k-means over the
  * environment codes; the MLP scores each edge's segments once per cluster),
- * cfg[7] lanes per walking pair in the plain-order walk: 32 (a whole warp) or
- * 16 (the warp's halves walk two pairs at once, 16 items a step each; robots
- * whose leaves lie inside their bounds, otherwise 32 is used).
+ * cfg[7] lanes per walking pair: 32, or 16 for builds with a half-warp walk (this
+ * one has none: 32 are used).
  */
 #define BCC_LAUNCH_CONFIG_LEN 8
 bcc_status bcc_get_launch_config(const bcc_ctx* ctx, int32_t* cfg);
 bcc_status bcc_set_launch_config(bcc_ctx* ctx, const int32_t* cfg);
 /*
  * Autotuner: times candidate configurations (edges per CTA 32..256, 4 or 8
- * warps, persistent or not, 32 or 16 lanes per walking pair; for the learned
- * order also the inline order's
+ * warps, probed or one pass; for the learned order also the inline order's
  * cluster count and the queued order's threshold 64..4096 items and finish
  * mode) on the given host edges against the
  * uploaded environments, timing graph replays, and keeps the fastest in the

@@ -1,0 +1,78 @@
+"""GPU tests of the probed check (a first pass over a voxel grid of each
+environment, the undecided pairs walked from a queue): bit for bit the verdicts
+of the one-pass check, at the edges of its batches, lists, grids and queue."""
+import numpy as np
+import pytest
+
+from bcc import EnvSet, workload
+from bcc.workload import make_cuboids, make_spheres
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def both(checker, envs, edges, robot, resolution=32):
+    checker.upload(envs)
+    cfg = checker.launch_config()
+    out = {}
+    try:
+        for persistent in (0, 1):
+            checker.set_launch_config(edges_per_cta=64, warps=4, persistent=persistent)
+            out[persistent] = checker.check(edges, robot=robot, resolution=resolution)
+    finally:
+        checker.set_launch_config(**cfg)
+    assert np.array_equal(out[0], out[1])
+    return out[1]
+
+
+# 1023 .. 1025 edges: a probe CTA's batch; 255 .. 257 primitives: the ids a voxel
+# holds; resolution 1 / 200: one sample block and long edges.
+@pytest.mark.parametrize("name,nenv,nedge,resolution", [
+    ("uneven", 1, 1, 32), ("uneven", 33, 31, 32), ("uneven", 20, 1023, 32), ("stress", 20, 1024, 32),
+    ("stress", 9, 1025, 200), ("plain", 40, 333, 32), ("uneven", 40, 500, 1), ("multi_fetch", 60, 1025, 32),
+    ("multi_baxter", 40, 400, 32)])
+def test_probed_check_is_the_one_pass_check(checker, name, nenv, nedge, resolution):
+    robot = workload.robot_of(name)
+    envs = workload.gen_envs(name, nenv, seed=71)
+    edges = workload.gen_edges(name, nedge, seed=71)
+    got = both(checker, envs, edges, robot, resolution)
+    part = slice(0, min(nedge, 60))
+    want = orc.check(envs, edges[part], resolution=resolution, robot=robot)
+    assert len(orc.adjudicate(envs, edges[part], got[part], want, resolution=resolution, robot=robot)[2]) == 0
+
+
+@pytest.mark.parametrize("prims", [255, 256, 257, 600])
+def test_more_primitives_than_voxel_ids(checker, prims):
+    rng = np.random.default_rng(prims)
+    c = rng.uniform(-1.0, 1.0, (prims, 3))
+    far = {"spheres": make_spheres(c + np.sign(c) * 0.35, rng.uniform(0.02, 0.06, prims))}
+    near = {"spheres": make_spheres(c, rng.uniform(0.02, 0.06, prims))}
+    both(checker, EnvSet.from_lists([far, near, {}]), workload.gen_edges("uneven", 300, seed=5), "panda")
+
+
+def test_records_without_a_distance_bound(checker):
+    """Axes that stretch distances, a negative radius, non-finite values, and an
+    edge that is not a number: the walk decides all of them, as without the probe."""
+    rng = np.random.default_rng(3)
+    n = 6
+    box = make_cuboids(rng.uniform(-0.6, 0.6, (n, 3)), rng.uniform(-3, 3, (n, 3)), rng.uniform(0.02, 0.2, (n, 3)))
+    wide, skew, inf = box.copy(), box.copy(), box.copy()
+    wide[:, 3:12] *= 2.0
+    skew[:, 6:9] = skew[:, 3:6]
+    inf[2, 12:15] = np.inf
+    neg = make_spheres(rng.uniform(-0.6, 0.6, (n, 3)), np.full(n, -0.3))
+    nan = make_spheres(rng.uniform(-0.6, 0.6, (n, 3)), np.full(n, np.nan))
+    envs = EnvSet.from_lists([{"cuboids": wide}, {"cuboids": skew}, {"cuboids": inf}, {"spheres": neg},
+                              {"spheres": nan}, {"cuboids": box}])
+    edges = workload.gen_edges("uneven", 200, seed=6)
+    edges[7, :, 3] = np.nan
+    both(checker, envs, edges, "panda")
+
+
+def test_more_pairs_than_the_queue_holds(checker):
+    """70 000 environments x 1000 edges: two slabs."""
+    n = 70000
+    rng = np.random.default_rng(8)
+    r = make_spheres(rng.uniform(-0.8, 0.8, (n, 3)) + [0, 0, 0.5], rng.uniform(0.05, 0.15, n))
+    envs = EnvSet({"spheres": np.ones(n, np.uint32)}, {"spheres": r})
+    both(checker, envs, workload.gen_edges("uneven", 1000, seed=9), "panda")
