@@ -701,6 +701,11 @@ bcc_status pack(bcc_ctx* ctx, const bcc_env_soa* envs, std::vector<Rec>& recs, s
                         std::string("positive ") + names[k] + " count with null records");
     }
     recs.clear();
+    size_t total = 0;
+    for (int k = 0; k < 5; ++k)
+        for (int i = 0; cnt[k] && i < N; ++i) total += cnt[k][i];
+    if (total > (size_t)0x7fffffff) return fail(ctx, BCC_ERR_LIMIT, "too many primitives");
+    recs.reserve(total);
     off.assign(N + 1, 0);
     size_t pos[6] = {0, 0, 0, 0, 0, 0};
     max_prims = 0;
@@ -722,31 +727,35 @@ bcc_status pack(bcc_ctx* ctx, const bcc_env_soa* envs, std::vector<Rec>& recs, s
         if (cnt[5]) pos[5] += cnt[5][i];  // cylinders: never tested (src/utils.cuh:213-245)
         off[i + 1] = (int)recs.size();
         max_prims = std::max(max_prims, off[i + 1] - off[i]);
-        if (recs.size() > (size_t)0x7fffffff) return fail(ctx, BCC_ERR_LIMIT, "too many primitives");
     }
     if (max_prims > 4095) return fail(ctx, BCC_ERR_LIMIT, "more than 4095 primitives in one environment");
     return BCC_OK;
 }
 
-// Device arena: per environment a blob of its rounded-box records followed by
-// its interval-mask cull tables, and a 2 x float4 header.  The check kernel
-// stages the records into shared memory and reads the mask tables through L1.
+// What an upload derives on the host: per environment a 2 x float4 header
+// (first record, blob offset, flags, shape; see CheckParams::env_hdr) and the
+// boundaries of the cull grid.  The blobs themselves -- records, then
+// interval-mask tables -- are laid out by launch_build_arena.
 struct Arena {
-    std::vector<float> blob;     // concatenated blobs (float words, 16-byte granules)
     std::vector<float> hdr;      // [N][8]
+    size_t float4s = 0;          // of all blobs
     size_t max_record_bytes = 0;
     // Cull grid shared by every environment of the set: slab s of axis a is
     // [bnd[a][s], bnd[a][s + 1]).
     float bnd[3][bcc::kGridSlabs + 1] = {};
 };
 
-// Largest slab s in [0, K) with bnd[s] <= x (0 below the first boundary);
-// the device lookup (swept_kernel) compares against the same floats.
-int slab_of(const float* bnd, double x) {
-    int s = 0;
-    for (int i = 1; i < bcc::kGridSlabs; ++i)
-        if ((double)bnd[i] <= x) s = i;
-    return s;
+// Order statistics k0 .. k1 - 1 of the sorted ranks want[k] of c[lo, hi), placed
+// at those ranks by selection, halving the ranks: O(n log K) instead of a sort.
+void select_ranks(std::vector<float>& c, size_t lo, size_t hi, const size_t* want, int k0, int k1) {
+    if (k0 >= k1 || hi - lo < 2) return;
+    const int k = (k0 + k1) / 2;
+    std::nth_element(c.begin() + lo, c.begin() + want[k], c.begin() + hi);
+    int a = k, b = k + 1;
+    while (a > k0 && want[a - 1] == want[k]) --a;
+    while (b < k1 && want[b] == want[k]) ++b;
+    select_ranks(c, lo, want[k], want, k0, a);
+    select_ranks(c, want[k] + 1, hi, want, b, k1);
 }
 
 // One cull grid serves all environments of the set, so an edge's slab ranges
@@ -754,18 +763,19 @@ int slab_of(const float* bnd, double x) {
 // kGridSlabs slabs of an axis run from below every primitive AABB to above
 // them, split at quantiles of the primitives' centres: slabs are narrow where
 // primitives are dense.
-void build_arena(const std::vector<Rec>& recs, const std::vector<int>& off, Arena& A) {
+void describe_arena(const std::vector<Rec>& recs, const std::vector<int>& off, Arena& A) {
     const int N = (int)off.size() - 1;
     constexpr int K = bcc::kGridSlabs;
-    constexpr int TRI = bcc::kGridTri;
-    A.blob.clear();
     A.hdr.assign((size_t)N * 8, 0.0f);
+    std::vector<float> c(recs.size());
+    size_t want[K];
+    for (int i = 1; i < K; ++i)
+        want[i] = recs.empty() ? 0 : std::min(recs.size() - 1, (size_t)((double)i * recs.size() / K));
     for (int a = 0; a < 3; ++a) {
-        std::vector<double> c;
         double lo = 1e30, hi = -1e30;
-        c.reserve(recs.size());
-        for (const Rec& r : recs) {
-            c.push_back(r.v[a]);
+        for (size_t k = 0; k < recs.size(); ++k) {
+            const Rec& r = recs[k];
+            c[k] = std::isnan(r.v[a]) ? INFINITY : r.v[a];  // an order exists
             lo = std::min(lo, (double)r.v[a] - r.v[16 + a]);
             hi = std::max(hi, (double)r.v[a] + r.v[16 + a]);
         }
@@ -774,60 +784,30 @@ void build_arena(const std::vector<Rec>& recs, const std::vector<int>& off, Aren
             for (int i = 0; i <= K; ++i) b[i] = (float)i;
             continue;
         }
-        std::sort(c.begin(), c.end());
+        select_ranks(c, 0, c.size(), want, 1, K);
         b[0] = std::nextafter((float)(lo - 1e-4), -INFINITY);
         b[K] = std::nextafter((float)(hi + 1e-4), INFINITY);
-        for (int i = 1; i < K; ++i) {
-            const double q = c[std::min(c.size() - 1, (size_t)((double)i * c.size() / K))];
-            b[i] = std::min(std::max((float)q, std::nextafter(b[i - 1], INFINITY)), b[K]);
-        }
+        for (int i = 1; i < K; ++i) b[i] = std::min(std::max(c[want[i]], std::nextafter(b[i - 1], INFINITY)), b[K]);
         for (int i = K - 1; i >= 1; --i)  // strictly increasing up to b[K]
             if (b[i] >= b[i + 1]) b[i] = std::nextafter(b[i + 1], -INFINITY);
     }
     for (int i = 0; i < N; ++i) {
         const int p0 = off[i], np = off[i + 1] - off[i];
-        const int W = np > 0 ? (np + 63) / 64 : 0;
-        const size_t start = A.blob.size();  // in floats, multiple of 4
-        for (int p = 0; p < np; ++p) {
-            const Rec& r = recs[p0 + p];
-            for (int k = 0; k < 20; ++k) A.blob.push_back(r.v[k]);
-        }
-        if (np > 0) {
-            // Slab range of each primitive's AABB, widened by 1e-5 m so that the
-            // FP32 swept boxes on the device can only over-include.
-            std::vector<int> s0(3 * (size_t)np), s1(3 * (size_t)np);
-            for (int p = 0; p < np; ++p) {
-                const Rec& r = recs[p0 + p];
-                for (int a = 0; a < 3; ++a) {
-                    s0[3 * p + a] = slab_of(A.bnd[a], (double)r.v[a] - r.v[16 + a] - 1e-5);
-                    s1[3 * p + a] = slab_of(A.bnd[a], (double)r.v[a] + r.v[16 + a] + 1e-5);
-                }
-            }
-            std::vector<uint64_t> m((size_t)3 * TRI * W, 0);
-            for (int a = 0; a < 3; ++a)
-                for (int i0 = 0; i0 < K; ++i0)
-                    for (int i1 = i0; i1 < K; ++i1) {
-                        uint64_t* dst = &m[((size_t)a * TRI + bcc::tri_index(i0, i1)) * W];
-                        for (int p = 0; p < np; ++p)
-                            if (s0[3 * p + a] <= i1 && s1[3 * p + a] >= i0) dst[p >> 6] |= 1ull << (p & 63);
-                    }
-            const size_t words = m.size() * 2;
-            const size_t at = A.blob.size();
-            A.blob.resize(at + words);
-            std::memcpy(&A.blob[at], m.data(), m.size() * sizeof(uint64_t));
-        }
-        A.max_record_bytes = std::max(A.max_record_bytes, (size_t)np * sizeof(Rec));
-        const uint32_t off16 = (uint32_t)(start / 4);  // float4 units
+        const int W = (np + 63) / 64;
+        const uint32_t off16 = (uint32_t)A.float4s;  // float4 units
         const uint32_t shape = (uint32_t)np | ((uint32_t)W << 16);
-        float* h = &A.hdr[(size_t)i * 8];
-        std::memcpy(&h[3], &off16, 4);
+        const uint32_t first = (uint32_t)p0;
         uint32_t flags = 0;
         for (int p = 0; p < np; ++p)
             if (!regular_rec(recs[p0 + p])) flags = bcc::kEnvIrregular;
+        float* h = &A.hdr[(size_t)i * 8];
+        std::memcpy(&h[3], &off16, 4);
+        std::memcpy(&h[4], &first, 4);
         std::memcpy(&h[6], &flags, 4);
         std::memcpy(&h[7], &shape, 4);
+        A.float4s += (size_t)np * bcc::kPrimF4 + (size_t)3 * bcc::kGridTri * W / 2;  // two mask words a float4
+        A.max_record_bytes = std::max(A.max_record_bytes, (size_t)np * sizeof(Rec));
     }
-    if (A.blob.empty()) A.blob.assign(4, 0.0f);
 }
 
 }  // namespace
@@ -857,25 +837,31 @@ bcc_status bcc_upload_envs(bcc_ctx* ctx, const bcc_env_soa* envs) {
     if (s != BCC_OK) return s;
     const int N = envs->num_envs;
     Arena A;
-    build_arena(recs, off, A);
+    describe_arena(recs, off, A);
     const size_t blob_smem = (A.max_record_bytes + 15) & ~(size_t)15;
     if (blob_smem > 160 * 1024)
         return fail(ctx, BCC_ERR_LIMIT, "an environment's primitives do not fit shared-memory staging (max 2048)");
-    if (A.blob.size() / 4 > 0xffffffffull) return fail(ctx, BCC_ERR_LIMIT, "environment arena too large");
+    if (A.float4s > 0xffffffffull) return fail(ctx, BCC_ERR_LIMIT, "environment arena too large");
     BCC_CUDA(ctx, cudaSetDevice(ctx->device));
-    BCC_CUDA(ctx, ctx->blobs.ensure(A.blob.size() * sizeof(float)));
+    const size_t rec_bytes = recs.size() * sizeof(Rec);
+    BCC_CUDA(ctx, ctx->blobs.ensure(std::max<size_t>(1, A.float4s) * sizeof(float4)));
     BCC_CUDA(ctx, ctx->env_hdr.ensure(std::max<size_t>(1, A.hdr.size()) * sizeof(float)));
-    BCC_CUDA(ctx, cudaMemcpy(ctx->blobs.p, A.blob.data(), A.blob.size() * sizeof(float), cudaMemcpyHostToDevice));
-    if (N > 0)
-        BCC_CUDA(ctx, cudaMemcpy(ctx->env_hdr.p, A.hdr.data(), A.hdr.size() * sizeof(float), cudaMemcpyHostToDevice));
-    ctx->num_envs = N;
-    ctx->max_prims = max_prims;
-    ctx->blob_smem = blob_smem;
     BCC_CUDA(ctx, ctx->grid_bounds.ensure(sizeof(A.bnd)));
+    BCC_CUDA(ctx, ctx->records.ensure(std::max<size_t>(16, rec_bytes)));
     BCC_CUDA(ctx, cudaMemcpy(ctx->grid_bounds.p, A.bnd, sizeof(A.bnd), cudaMemcpyHostToDevice));
+    if (rec_bytes) BCC_CUDA(ctx, cudaMemcpy(ctx->records.p, recs.data(), rec_bytes, cudaMemcpyHostToDevice));
+    if (N > 0) {
+        BCC_CUDA(ctx, cudaMemcpy(ctx->env_hdr.p, A.hdr.data(), A.hdr.size() * sizeof(float), cudaMemcpyHostToDevice));
+        BCC_CUDA(ctx, bcc::launch_build_arena(ctx->records.as<float4>(), ctx->env_hdr.as<float4>(),
+                                              ctx->grid_bounds.as<float>(), N, ctx->blobs.as<float4>(),
+                                              cudaStreamLegacy));
+    }
     // A copy from pageable memory may return with its DMA still in flight on the
     // legacy stream, which a check's (non-blocking) stream is not ordered after.
     BCC_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));
+    ctx->num_envs = N;
+    ctx->max_prims = max_prims;
+    ctx->blob_smem = blob_smem;
     ctx->env_code_ready = false;
     ctx->cluster_k = 0;
     ctx->env_version += 1;

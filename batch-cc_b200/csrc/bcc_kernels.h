@@ -55,7 +55,7 @@ struct ProbeQueue {
 struct CheckParams {
     const float4* blobs;     // per env: [np][5] rounded-box records, then 3 x kGridTri x W masks
     const float4* env_hdr;   // [num_envs][2]: (0, 0, 0, blob offset in float4s),
-                             //                 (0, 0, flags, np | W << 16)
+                             //                 (first record, 0, flags, np | W << 16)
     int num_envs;
     int num_edges;
     int max_prims;           // max primitives of one env (pair-list sizing)
@@ -225,6 +225,10 @@ cudaError_t launch_env_encode(const float4* blobs, const float4* env_hdr, int nu
 // Row gather for training: x2[i] = x[perm[i]] (kMlpIn BF16 values), y2[i] = y[perm[i]].
 cudaError_t launch_gather_rows(const uint16_t* x, const uint8_t* y, const int* perm, int rows, uint16_t* x2,
                                uint8_t* y2, cudaStream_t st);
+// Blobs of an upload: every environment's records (copied from the packed ones)
+// and its interval-mask tables on the cull grid (bounds: 3 x (kGridSlabs + 1)).
+cudaError_t launch_build_arena(const float4* records, const float4* env_hdr, const float* bounds, int num_envs,
+                               float4* blobs, cudaStream_t st);
 // Probe grids of every environment (p.vox is written).
 cudaError_t launch_probe_grid(const float4* blobs, const float4* env_hdr, int num_envs, const ProbeGrid& p,
                               uint16_t* vox, cudaStream_t st);

@@ -76,3 +76,28 @@ def test_more_pairs_than_the_queue_holds(checker):
     r = make_spheres(rng.uniform(-0.8, 0.8, (n, 3)) + [0, 0, 0.5], rng.uniform(0.05, 0.15, n))
     envs = EnvSet({"spheres": np.ones(n, np.uint32)}, {"spheres": r})
     both(checker, envs, workload.gen_edges("uneven", 1000, seed=9), "panda")
+
+
+@pytest.mark.parametrize("prims", [1, 63, 64, 65, 127, 129, 700])
+@pytest.mark.parametrize("persistent", [0, 1])
+def test_mask_words_hold_every_primitive(checker, prims, persistent):
+    """Environments at the edges of the cull's 64-primitive words, between an empty
+    one and one of a single primitive: the oracle's verdicts (a primitive missing
+    from a mask shows as a collision not found)."""
+    rng = np.random.default_rng(prims)
+    c = rng.uniform(-0.7, 0.7, (prims, 3)) + [0, 0, 0.4]
+    half = prims // 2
+    many = {"spheres": make_spheres(c[:half], rng.uniform(0.01, 0.05, half)),
+            "cuboids": make_cuboids(c[half:], rng.uniform(-3, 3, (prims - half, 3)),
+                                    rng.uniform(0.01, 0.05, (prims - half, 3)))}
+    envs = EnvSet.from_lists([{}, many, {"spheres": make_spheres(c[:1], [0.2])}, many])
+    edges = workload.gen_edges("uneven", 80, seed=prims)
+    cfg = checker.launch_config()
+    checker.upload(envs)
+    try:
+        checker.set_launch_config(persistent=persistent)
+        got = checker.check(edges)
+    finally:
+        checker.set_launch_config(**cfg)
+    assert len(orc.adjudicate(envs, edges, got, orc.check(envs, edges))[2]) == 0
+    assert np.array_equal(got[:, 1], got[:, 3])
