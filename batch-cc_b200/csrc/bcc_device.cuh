@@ -95,6 +95,15 @@ __device__ __forceinline__ void edge_sample(const float* s, const float* e, int 
     }
 }
 
+// One joint of edge_sample (the joints are independent).
+__device__ __forceinline__ float edge_sample_joint(float s, float e, int n, int k) {
+    const int lane = k / n, round = k - lane * n;
+    const float delta = __fdiv_rn(__fsub_rn(e, s), (float)(kBdim * n));
+    float c = __fmaf_rn(delta, (float)(lane * n), s);
+    for (int i = 0; i < round; ++i) c = __fadd_rn(c, delta);
+    return c;
+}
+
 // Rank r of the reference's check order -> sample index k: round r / 32,
 // lane r % 32 checks sample k = lane * n + round (src/batch_cc.cu:113-129).
 __device__ __forceinline__ int reference_rank_to_sample(int r, int n) {
@@ -163,45 +172,57 @@ __device__ __forceinline__ void emit_frame(const Frames<M, T>& F, float4* __rest
 __device__ __forceinline__ void sin_cos(float q, float* s, float* c) { sincosf(q, s, c); }
 __device__ __forceinline__ void sin_cos(double q, double* s, double* c) { sincos(q, s, c); }
 
-// One joint: compile-time constants of F_K are folded into the multiply-adds.
+// One joint: frame K + 1 from its parent's, compile-time constants of F_K folded
+// into the multiply-adds.  sq, cq: sine and cosine of a revolute joint's value.
 template <class M, int K, class T>
-struct FkJoint {
-    __device__ __forceinline__ static void run(const float* q, Frames<M, T>& F, float4* __restrict__ out) {
-        constexpr int P = M::joint_parent[K];
-        static_assert(P <= K, "joints must follow their parents");
-        constexpr T f[12] = {
-            (T)M::joint_tf[K][0], (T)M::joint_tf[K][1], (T)M::joint_tf[K][2],
-            (T)M::joint_tf[K][3], (T)M::joint_tf[K][4], (T)M::joint_tf[K][5],
-            (T)M::joint_tf[K][6], (T)M::joint_tf[K][7], (T)M::joint_tf[K][8],
-            (T)M::joint_tf[K][9], (T)M::joint_tf[K][10], (T)M::joint_tf[K][11]};
-        T A[9];
+__device__ __forceinline__ void fk_advance(T qk, T sq, T cq, Frames<M, T>& F) {
+    constexpr int P = M::joint_parent[K];
+    static_assert(P <= K, "joints must follow their parents");
+    constexpr T f[12] = {
+        (T)M::joint_tf[K][0], (T)M::joint_tf[K][1], (T)M::joint_tf[K][2],
+        (T)M::joint_tf[K][3], (T)M::joint_tf[K][4], (T)M::joint_tf[K][5],
+        (T)M::joint_tf[K][6], (T)M::joint_tf[K][7], (T)M::joint_tf[K][8],
+        (T)M::joint_tf[K][9], (T)M::joint_tf[K][10], (T)M::joint_tf[K][11]};
+    T A[9];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+            A[a * 3 + b] = F.R[P][a * 3 + 0] * f[0 * 4 + b] + F.R[P][a * 3 + 1] * f[1 * 4 + b] +
+                           F.R[P][a * 3 + 2] * f[2 * 4 + b];
+        F.p[K + 1][a] = F.R[P][a * 3 + 0] * f[3] + F.R[P][a * 3 + 1] * f[7] +
+                        F.R[P][a * 3 + 2] * f[11] + F.p[P][a];
+    }
+    if constexpr (M::joint_type[K] == 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            F.R[K + 1][a * 3 + 0] = A[a * 3 + 0] * cq + A[a * 3 + 1] * sq;
+            F.R[K + 1][a * 3 + 1] = A[a * 3 + 1] * cq - A[a * 3 + 0] * sq;
+            F.R[K + 1][a * 3 + 2] = A[a * 3 + 2];
+        }
+    } else {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
 #pragma unroll
-            for (int b = 0; b < 3; ++b)
-                A[a * 3 + b] = F.R[P][a * 3 + 0] * f[0 * 4 + b] + F.R[P][a * 3 + 1] * f[1 * 4 + b] +
-                               F.R[P][a * 3 + 2] * f[2 * 4 + b];
-            F.p[K + 1][a] = F.R[P][a * 3 + 0] * f[3] + F.R[P][a * 3 + 1] * f[7] +
-                            F.R[P][a * 3 + 2] * f[11] + F.p[P][a];
+            for (int b = 0; b < 3; ++b) F.R[K + 1][a * 3 + b] = A[a * 3 + b];
+            F.p[K + 1][a] += A[a * 3 + 2] * qk;
         }
-        const T qk = (T)q[K];
-        if constexpr (M::joint_type[K] == 0) {
-            T sq, cq;
-            sin_cos(qk, &sq, &cq);
+    }
+}
+
+template <class M, class T>
+__device__ __forceinline__ void fk_base(Frames<M, T>& F) {
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                F.R[K + 1][a * 3 + 0] = A[a * 3 + 0] * cq + A[a * 3 + 1] * sq;
-                F.R[K + 1][a * 3 + 1] = A[a * 3 + 1] * cq - A[a * 3 + 0] * sq;
-                F.R[K + 1][a * 3 + 2] = A[a * 3 + 2];
-            }
-        } else {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-#pragma unroll
-                for (int b = 0; b < 3; ++b) F.R[K + 1][a * 3 + b] = A[a * 3 + b];
-                F.p[K + 1][a] += A[a * 3 + 2] * qk;
-            }
-        }
+    for (int i = 0; i < 9; ++i) F.R[0][i] = (i % 4 == 0) ? T(1) : T(0);
+    F.p[0][0] = F.p[0][1] = F.p[0][2] = T(0);
+}
+
+template <class M, int K, class T>
+struct FkJoint {
+    __device__ __forceinline__ static void run(const float* q, Frames<M, T>& F, float4* __restrict__ out) {
+        T sq = T(0), cq = T(1);
+        if constexpr (M::joint_type[K] == 0) sin_cos((T)q[K], &sq, &cq);
+        fk_advance<M, K, T>((T)q[K], sq, cq, F);
         emit_frame<M, K + 1, T>(F, out, std::make_integer_sequence<int, M::num_spheres>{});
         FkJoint<M, K + 1, T>::run(q, F, out);
     }
@@ -217,9 +238,7 @@ template <class M>
 __device__ __forceinline__ void fk_spheres(const float* q, float4* __restrict__ out) {
     using T = typename std::conditional<M::fk_precision == 64, double, float>::type;
     Frames<M, T> F;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) F.R[0][i] = (i % 4 == 0) ? T(1) : T(0);
-    F.p[0][0] = F.p[0][1] = F.p[0][2] = T(0);
+    fk_base<M, T>(F);
     emit_frame<M, 0, T>(F, out, std::make_integer_sequence<int, M::num_spheres>{});
     FkJoint<M, 0, T>::run(q, F, out);
 }
@@ -263,6 +282,19 @@ __device__ __forceinline__ void bulk_copy_part(void* dst, const void* src, uint3
         "l"(src), "r"(bytes), "r"(b)
         : "memory");
 }
+
+// One thread: start a 1-D bulk copy shared -> global as a bulk group of its own
+// (the writers of src have fenced to the async proxy); 16-byte alignment.
+__device__ __forceinline__ void bulk_copy_s2g(void* dst, const void* src, uint32_t bytes) {
+    const uint32_t s = (uint32_t)__cvta_generic_to_shared(src);
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(s), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// The same thread: its bulk groups have read their sources / completed.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     bulk_expect(bar, bytes);

@@ -84,6 +84,14 @@ struct DevTables {
     int self_la_begin[M::num_self_groups + 1], self_lb_begin[M::num_self_groups + 1];
     unsigned char self_la[M::num_self_pairs], self_lb[M::num_self_pairs];
     float self_pad[M::num_self_groups][2];
+    unsigned char self_frame[M::num_self_groups][2];  // frames of a group's bounds
+    unsigned char frame_at[M::num_spheres];           // frame by sample-table position
+    // Spheres by frame (frame f: entries fk_begin[f] .. fk_begin[f + 1], the first up
+    // to fk_x_end[f] with their x product rounded first, see fk_x_first): offset in the
+    // frame and radius, row position.
+    int fk_begin[M::dof + 2], fk_x_end[M::dof + 1];
+    float4 fk_local[M::num_spheres];
+    int fk_pos[M::num_spheres];
     float sphere_radius[M::num_spheres];  // by sample-table position
     float s_m[M::dof], s_a[M::dof];       // joint-limit scale q = u * s_m + s_a
 };
@@ -91,6 +99,10 @@ struct DevTables {
 // Specialised by the robot's translation unit to return its __constant__ tables.
 template <class M>
 __device__ __forceinline__ const DevTables<M>& tab();
+// ... and its copy in global memory, for reads whose index differs by lane:
+// constant memory serialises those, one pass per distinct address.
+template <class M>
+__device__ __forceinline__ const DevTables<M>& lane_tab();
 
 // Margin (m) added to a side's containment excess in the self groups' leaf
 // filter: far above the FP32 rounding of FK-computed centres (~1e-6 m).
@@ -130,6 +142,15 @@ float cert_radius(int g) {
     return f;
 }
 
+// A sphere's centre is R0 x + R1 y + R2 z + p in fused multiply-adds, and which
+// product is rounded by itself decides its last bit: R1 y, or R0 x for the row
+// positions a robot's specialisation names.  Verdicts at contact follow those
+// bits, so a robot's spheres keep the order they have always been computed in.
+template <class M>
+constexpr bool fk_x_first(int pos) {
+    return false;
+}
+
 template <class M>
 void self_products(DevTables<M>& t) {
     int na_tot = 0, nb_tot = 0;
@@ -165,6 +186,8 @@ void self_products(DevTables<M>& t) {
             t.self_pad[g][side] = (float)(excess + kSelfFilterMargin);
         }
         t.self_prod[g] = prod ? 1 : 0;
+        for (int side = 0; side < 2; ++side)
+            t.self_frame[g][side] = (unsigned char)M::sphere_frame[M::self_bound[g][side]];
         t.self_la_begin[g] = na_tot;
         t.self_lb_begin[g] = nb_tot;
         if (prod) {
@@ -206,7 +229,24 @@ DevTables<M> host_tables() {
         t.self_pairs[i][1] = (unsigned char)M::table_pos[M::self_pairs[i][1]];
     }
     self_products<M>(t);
-    for (int s = 0; s < M::num_spheres; ++s) t.sphere_radius[M::table_pos[s]] = M::sphere_radius[s];
+    for (int s = 0; s < M::num_spheres; ++s) {
+        t.sphere_radius[M::table_pos[s]] = M::sphere_radius[s];
+        t.frame_at[M::table_pos[s]] = (unsigned char)M::sphere_frame[s];
+    }
+    int at = 0;
+    for (int f = 0; f <= M::dof; ++f) {
+        t.fk_begin[f] = at;
+        for (int y_first = 0; y_first < 2; ++y_first) {
+            for (int s = 0; s < M::num_spheres; ++s)
+                if (M::sphere_frame[s] == f && fk_x_first<M>(M::table_pos[s]) == !y_first) {
+                    t.fk_local[at] = make_float4((float)M::sphere_local[s][0], (float)M::sphere_local[s][1],
+                                                 (float)M::sphere_local[s][2], M::sphere_radius[s]);
+                    t.fk_pos[at++] = M::table_pos[s];
+                }
+            if (!y_first) t.fk_x_end[f] = at;
+        }
+    }
+    t.fk_begin[M::dof + 1] = at;
     for (int j = 0; j < M::dof; ++j) {
         t.s_m[j] = M::s_m[j];
         t.s_a[j] = M::s_a[j];
@@ -352,57 +392,6 @@ __device__ __forceinline__ bool self_hit_pad(float4 a, float4 b, float pad) {
     return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - rs * rs < 0.0f;
 }
 
-// Self-collision of a warp's rows, one lane per row (sphere s at my[s]; live:
-// the lane holds a row), all rows of one edge: group g gates on its bound pair
-// and its leaf pairs count only where the gate hit (the reference's
-// gate-then-leaves).  The warp walks the groups together, so every table index
-// is warp-uniform (constant-cache broadcasts), skips a group's leaves when no
-// lane's gate hit, and stops at the first hit in any lane.  A group whose
-// leaf pairs are a product of two leaf sets (self_prod) first drops the leaves
-// of either side that miss the other side's padded bound -- a leaf of side A
-// that misses bound B (grown by B's containment pad) misses every leaf inside
-// B -- and tests only the pairs of surviving leaves, skipping those no lane
-// keeps; the verdict is the one the full pair list gives.  Warp-uniform.
-template <class M>
-__device__ __forceinline__ bool self_rows_hit(const float4* my, bool live) {
-    const DevTables<M>& T = tab<M>();
-    for (int g = 0; g < M::num_self_groups; ++g) {
-        const float4 ba = my[T.self_bound[g][0]], bb = my[T.self_bound[g][1]];
-        const bool gate = live && self_hit(ba, bb);
-        if (!__any_sync(kFull, gate)) continue;
-        bool h = false;
-        if (T.self_prod[g]) {
-            const int a0 = T.self_la_begin[g], na = T.self_la_begin[g + 1] - a0;
-            const int b0 = T.self_lb_begin[g], nb = T.self_lb_begin[g + 1] - b0;
-            const float pa = T.self_pad[g][0], pb = T.self_pad[g][1];
-            uint32_t ma = 0u, mb = 0u;
-            for (int i = 0; i < na; ++i) ma |= (uint32_t)self_hit_pad(my[T.self_la[a0 + i]], bb, pb) << i;
-            for (int j = 0; j < nb; ++j) mb |= (uint32_t)self_hit_pad(my[T.self_lb[b0 + j]], ba, pa) << j;
-            if (!gate || !mb) ma = 0u;
-            uint32_t ia = __reduce_or_sync(kFull, ma);
-            while (ia) {
-                const int i = __ffs(ia) - 1;
-                ia &= ia - 1u;
-                const uint32_t mj = ((ma >> i) & 1u) ? mb : 0u;
-                uint32_t jb = __reduce_or_sync(kFull, mj);
-                const float4 la = my[T.self_la[a0 + i]];
-                while (jb) {
-                    const int j = __ffs(jb) - 1;
-                    jb &= jb - 1u;
-                    h |= ((mj >> j) & 1u) && self_hit(la, my[T.self_lb[b0 + j]]);
-                }
-            }
-        } else {
-            const int k1 = T.self_pair_begin[g + 1];
-#pragma unroll 4
-            for (int k = T.self_pair_begin[g]; k < k1; ++k)
-                h |= self_hit(my[T.self_pairs[k][0]], my[T.self_pairs[k][1]]);
-        }
-        if (__any_sync(kFull, gate && h)) return true;
-    }
-    return false;
-}
-
 __device__ __forceinline__ float dist2(float4 a, float4 b) {
     const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
     return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
@@ -416,91 +405,274 @@ __device__ __forceinline__ float dist2(float4 a, float4 b) {
 constexpr int kSegMid = kSegment / 2;
 constexpr float kSegMargin = 1e-4f;  // FP32 rounding of centres and distances (~1e-6 m), generously
 
-// The four segments of a warp's 32 staged rows (row base + lane at srow +
-// lane * (num_spheres | 1)): every lane measures its row against its segment's
-// middle one, eight lanes reduce.  The group's leaves one after another.
+// Shared state of a staged block of 32 rows: how far any sphere of a frame moves
+// from its place at its segment's middle row (squared, as bits: they order like
+// the values), and the (self group, segment) items still in question.
+constexpr int kBlockSegs = 32 / kSegment;
 template <class M>
-__device__ __forceinline__ void segment_spheres(const float4* srow, int base, float2* __restrict__ seg) {
+struct BlockState {
+    int move2[M::dof + 1][kBlockSegs];
+    int num_items;
+    unsigned short items[M::num_self_groups * kBlockSegs];
+};
+
+// Is every group's leaf in its bound's frame?
+template <class M>
+constexpr bool groups_are_rigid() {
+    for (int g = 0; g < M::num_env_groups; ++g)
+        for (int k = M::env_leaf_begin[g]; k < M::env_leaf_begin[g + 1]; ++k)
+            if (M::sphere_frame[M::env_leaves[k]] != M::sphere_frame[M::env_bound[g]]) return false;
+    return true;
+}
+
+// The four segments of the CTA's 32 staged rows (row base + l at srow + l *
+// num_spheres): every lane measures its row against its segment's middle one,
+// eight lanes reduce.  The warps share out the groups (a group's leaves one
+// after another), then the spheres outside any.
+template <class M>
+__device__ __forceinline__ void segment_spheres(const float4* srow, int base, int warp, int warps, BlockState<M>& B,
+                                                float2* __restrict__ seg) {
     constexpr int G = M::num_env_groups;
-    constexpr int STRIDE = M::num_spheres | 1;
+    constexpr int NS = M::num_spheres;
+    static_assert(groups_are_rigid<M>(), "a group's movement is its frame's");
     const DevTables<M>& T = tab<M>();
-    const int lane = threadIdx.x & 31;
-    const float4* mine = srow + lane * STRIDE;
-    const float4* mid = srow + ((lane & ~(kSegment - 1)) + kSegMid) * STRIDE;
-    for (int g = 0; g < G; ++g) {
+    const int lane = threadIdx.x & 31, sg = lane / kSegment;
+    const float4* mine = srow + lane * NS;
+    const float4* mid = srow + ((lane & ~(kSegment - 1)) + kSegMid) * NS;
+    for (int g = warp; g < G; g += warps) {
         float b = dist2(mine[g], mid[g]), l = 0.0f;
-        for (int i = T.leaf_begin[g]; i < T.leaf_begin[g + 1]; ++i) l = fmaxf(l, dist2(mine[G + i], mid[G + i]));
+        const int end = T.leaf_begin[g + 1];
+#pragma unroll 4
+        for (int i = T.leaf_begin[g]; i < end; ++i) l = fmaxf(l, dist2(mine[G + i], mid[G + i]));
 #pragma unroll
         for (int o = 1; o < kSegment; o <<= 1) {
             b = fmaxf(b, __shfl_xor_sync(kFull, b, o));
             l = fmaxf(l, __shfl_xor_sync(kFull, l, o));
         }
-        if ((lane & (kSegment - 1)) == 0)
-            seg[((size_t)base / kSegment + lane / kSegment) * G + g] =
-                make_float2(sqrtf(b) * 1.00001f + T.sphere_radius[g] + kEnvInflate + T.cull_pad[g] + kSegMargin,
-                            sqrtf(l) * 1.00001f + kSegMargin);
+        if ((lane & (kSegment - 1)) == 0) {
+            if (seg)
+                seg[((size_t)base / kSegment + sg) * G + g] =
+                    make_float2(sqrtf(b) * 1.00001f + T.sphere_radius[g] + kEnvInflate + T.cull_pad[g] + kSegMargin,
+                                sqrtf(l) * 1.00001f + kSegMargin);
+            atomicMax(&B.move2[T.frame_at[g]][sg], __float_as_int(fmaxf(b, l)));
+        }
+    }
+    for (int p = G + M::num_env_leaves + warp; p < NS; p += warps) {
+        float d = dist2(mine[p], mid[p]);
+#pragma unroll
+        for (int o = 1; o < kSegment; o <<= 1) d = fmaxf(d, __shfl_xor_sync(kFull, d, o));
+        if ((lane & (kSegment - 1)) == 0) atomicMax(&B.move2[T.frame_at[p]][sg], __float_as_int(d));
     }
 }
 
-// Row-major tables (tile 1): a thread's row is 16 * num_spheres contiguous
-// bytes, so per-thread stores would touch 32 rows per warp instruction.  One
-// warp per CTA computes 32 rows into shared memory (odd float4 row stride,
-// conflict-free) and then copies the 32 consecutive rows out as one contiguous
-// block, 512 bytes per warp store.  While the rows are still in shared memory
-// the warp also runs their self-collision check, one lane per row, so the rows
-// are never read back from global memory for it.  A block's 32 rows belong to
-// one edge (every edge has 32 n rows and starts on a multiple of 32), so the
-// first hit in any lane decides the block.  The CTA strides over 32-row blocks.
+// Does (self group, segment) item `item` hold a hit: a sample whose bound pair
+// overlaps and one of whose leaf pairs does (the reference's gate-then-leaves,
+// src/utils.cuh:1192-5440)?  Whole warp.  A product group first drops, at the
+// middle sample, the leaves of either side that stay clear of the other side's
+// bound over the whole segment (that bound grown by its containment pad and by
+// what both frames move), then the pairs that stay clear of each other; the
+// surviving pairs are tested at the segment's eight samples.  Other groups test
+// their whole pair list at each sample.
 template <class M>
-__global__ void __launch_bounds__(32) fk_staged_kernel(const float* __restrict__ edges, int E,
-                                                       const int* __restrict__ steps,
-                                                       const int* __restrict__ offs,
-                                                       float4* __restrict__ table,
-                                                       int* __restrict__ row_edge, int* __restrict__ edge_self,
-                                                       float2* __restrict__ seg) {
-    static_assert(M::table_tile == 1, "row-major tables only");
+__device__ __forceinline__ bool self_item_hit(const float4* srow, int item, const BlockState<M>& B, uint8_t (*list)[32],
+                                              uint8_t (*pair)[2]) {
     constexpr int NS = M::num_spheres;
-    constexpr int STRIDE = NS | 1;
-    extern __shared__ float4 srow[];  // [32][STRIDE]
-    const int lane = threadIdx.x;
-    const int total = offs[E];
-    for (int base = blockIdx.x * 32; base < total; base += gridDim.x * 32) {
-        const int row = base + lane;
-        // the block's edge: the last e with offs[e] <= base (one search per block)
-        int lo = 0, hi = E - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (offs[mid] <= base) lo = mid; else hi = mid - 1;
+    const DevTables<M>& T = tab<M>();
+    const DevTables<M>& L = lane_tab<M>();
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const int g = item / kBlockSegs, sg = item - g * kBlockSegs;
+    const float4* rows = srow + sg * kSegment * NS;
+    const float4* mid = rows + kSegMid * NS;
+    const int b0 = T.self_bound[g][0], b1 = T.self_bound[g][1];
+    // leaf pair (x, y) at sample k of the segment, counted where the bounds overlap
+    auto hit_at = [&](int k, int x, int y) {
+        const float4* r = rows + k * NS;
+        return self_hit(r[x], r[y]) && self_hit(r[b0], r[b1]);
+    };
+    if (!T.self_prod[g]) {
+        const int k0 = T.self_pair_begin[g], m = (T.self_pair_begin[g + 1] - k0) * kSegment;
+        for (int t = lane; t - lane < m; t += 32) {
+            const int k = k0 + min(t, m - 1) / kSegment;
+            if (__any_sync(kFull, t < m && hit_at(t & (kSegment - 1), L.self_pairs[k][0], L.self_pairs[k][1]))) return true;
         }
-        const int e = lo;
-        const int n = steps[e];
-        if (row < total) {
-            float s[M::dof], t[M::dof], q[M::dof];
-#pragma unroll
-            for (int j = 0; j < M::dof; ++j) {
-                s[j] = edges[(size_t)e * 2 * M::dof + j];
-                t[j] = edges[(size_t)e * 2 * M::dof + M::dof + j];
-            }
-            edge_sample<M::dof>(s, t, n, row - offs[e], q);
-            fk_spheres<M>(q, srow + lane * STRIDE);
-            row_edge[row] = e;
+        return false;
+    }
+    const float move = sqrtf(__int_as_float(B.move2[T.self_frame[g][0]][sg])) * 1.00001f +
+                       sqrtf(__int_as_float(B.move2[T.self_frame[g][1]][sg])) * 1.00001f;
+    const int a0 = T.self_la_begin[g], na = T.self_la_begin[g + 1] - a0;
+    const int c0 = T.self_lb_begin[g], nb = T.self_lb_begin[g + 1] - c0;
+    const float4 ba = mid[b0], bb = mid[b1];
+    const int la = lane < na ? L.self_la[a0 + lane] : 0, lb = lane < nb ? L.self_lb[c0 + lane] : 0;
+    const bool ka = lane < na && self_hit_pad(mid[la], bb, T.self_pad[g][1] + move);
+    const bool kb = lane < nb && self_hit_pad(mid[lb], ba, T.self_pad[g][0] + move);
+    const unsigned ma = __ballot_sync(kFull, ka), mb = __ballot_sync(kFull, kb);
+    if (!ma || !mb) return false;
+    if (ka) list[0][__popc(ma & lt)] = (uint8_t)la;
+    if (kb) list[1][__popc(mb & lt)] = (uint8_t)lb;
+    __syncwarp();
+    const int cb = __popc(mb), m = __popc(ma) * cb;
+    const float inv = __frcp_rn((float)cb);
+    bool hit = false;
+    for (int t0 = 0; t0 < m && !hit; t0 += 32) {
+        const int t = min(t0 + lane, m - 1);
+        const int i = (int)(((float)t + 0.5f) * inv);  // t / cb, exact: t < 1024, cb <= 32
+        const int x = list[0][i], y = list[1][t - i * cb];
+        const bool near = t0 + lane < m && self_hit_pad(mid[x], mid[y], move + kSegMargin);
+        const unsigned nm = __ballot_sync(kFull, near);
+        if (near) {
+            uint8_t* d = pair[__popc(nm & lt)];
+            d[0] = (uint8_t)x;
+            d[1] = (uint8_t)y;
         }
         __syncwarp();
-        const int rows = min(32, total - base);
-        const int cnt = rows * NS;
-        float4* __restrict__ dst = table + (size_t)base * NS;
-        for (int i = lane; i < cnt; i += 32) {
-            const int r = i / NS;
-            dst[i] = srow[r * STRIDE + (i - r * NS)];
+        const int n = __popc(nm) * kSegment;
+        for (int q = lane; q - lane < n && !hit; q += 32) {
+            const uint8_t* d = pair[min(q, n - 1) / kSegment];
+            hit = __any_sync(kFull, q < n && hit_at(q & (kSegment - 1), d[0], d[1]));
         }
-        if (seg) segment_spheres<M>(srow, base, seg);
-        // self-collision of the block's rows (any hit marks the edge); skipped
-        // when another block of the edge has already marked it
-        int decided = lane == 0 ? *(volatile const int*)(edge_self + e) : 0;
-        if (!__shfl_sync(kFull, decided, 0) && self_rows_hit<M>(srow + lane * STRIDE, row < total) && lane == 0)
-            atomicOr(edge_self + e, 1);
-        __syncwarp();  // the next block overwrites srow
+        __syncwarp();
     }
+    return hit;
+}
+
+// Edge of table row `row` (the last e with offs[e] <= row), whole warp: each
+// round probes 32 offsets at once, three dependent loads for 10 000 edges where a
+// binary search makes fourteen.
+__device__ __forceinline__ int edge_of_row(const int* __restrict__ offs, int E, int row) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = E;
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) >> 5, i = lo + lane * step;
+        const unsigned m = __ballot_sync(kFull, i < hi && offs[i] <= row);  // lane 0 holds
+        lo += (__popc(m) - 1) * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
+// Row-major tables (tile 1): a CTA of four warps computes 32 consecutive rows
+// (one edge's: every edge has 32 n rows and starts on a multiple of 32) into
+// shared memory, lane l row l.  Each warp evaluates the joints it needs and a
+// quarter of the spheres; the 32 rows leave as one bulk copy, the shared layout
+// being the table's.  While it runs the warps share out the segments' spheres
+// and the self-collision check: one thread per (self group, segment) tests the
+// bounds at the segment's middle sample, grown by what their frames move within
+// it, and the warps take the items that leaves (self_item_hit).  The CTA strides
+// over 32-row blocks.  Shared memory (39 KB for Panda) holds five CTAs an SM, and
+// a block's instruction chain bounds it.  One warp a block, straight-line code for
+// every sphere and one lane per row walking the self groups took 0.252 ms for the
+// uneven workload's 11 300 blocks (0.315 with the segments' spheres); four warps
+// alone gave 0.352 (the code, several times the instruction cache, was read once
+// per warp), sphere and joint tables read in loops and the self check by segments
+// 0.194 ms: 9 650 instructions a block, half of the issue slots.
+constexpr int kFkWarps = 4;
+
+// Frame FR's spheres, every kFkWarps-th from `warp`, into the row at out (fk_x_first).
+template <class M, int FR>
+__device__ __forceinline__ void emit_listed(const Frames<M, float>& F, int warp, float4* out) {
+    const DevTables<M>& T = tab<M>();
+    const float* R = F.R[FR];
+    const float* p = F.p[FR];
+    const int begin = T.fk_begin[FR], mid = T.fk_x_end[FR], end = T.fk_begin[FR + 1];
+#pragma unroll 2
+    for (int i = begin + warp; i < mid; i += kFkWarps) {
+        const float4 l = T.fk_local[i];
+        float4 c;
+        c.x = __fadd_rn(__fmaf_rn(R[2], l.z, __fmaf_rn(R[1], l.y, __fmul_rn(R[0], l.x))), p[0]);
+        c.y = __fadd_rn(__fmaf_rn(R[5], l.z, __fmaf_rn(R[4], l.y, __fmul_rn(R[3], l.x))), p[1]);
+        c.z = __fadd_rn(__fmaf_rn(R[8], l.z, __fmaf_rn(R[7], l.y, __fmul_rn(R[6], l.x))), p[2]);
+        c.w = l.w;
+        out[T.fk_pos[i]] = c;
+    }
+#pragma unroll 2
+    for (int i = mid + warp; i < end; i += kFkWarps) {
+        const float4 l = T.fk_local[i];
+        float4 c;
+        c.x = __fadd_rn(__fmaf_rn(R[2], l.z, __fmaf_rn(R[0], l.x, __fmul_rn(R[1], l.y))), p[0]);
+        c.y = __fadd_rn(__fmaf_rn(R[5], l.z, __fmaf_rn(R[3], l.x, __fmul_rn(R[4], l.y))), p[1]);
+        c.z = __fadd_rn(__fmaf_rn(R[8], l.z, __fmaf_rn(R[6], l.x, __fmul_rn(R[7], l.y))), p[2]);
+        c.w = l.w;
+        out[T.fk_pos[i]] = c;
+    }
+}
+
+// Joints K, K + 1, ... of one row from their values and sines and cosines (sc[k]
+// at [k * 32]), the warp's share of every frame's spheres.
+template <class M, int K>
+__device__ __forceinline__ void fk_rows(const float* q, const float2* sc, Frames<M, float>& F, int warp, float4* out) {
+    if constexpr (K == 0) {
+        fk_base<M, float>(F);
+        emit_listed<M, 0>(F, warp, out);
+    }
+    if constexpr (K < M::dof) {
+        fk_advance<M, K, float>(q[K * 32], sc[K * 32].x, sc[K * 32].y, F);
+        emit_listed<M, K + 1>(F, warp, out);
+        fk_rows<M, K + 1>(q, sc, F, warp, out);
+    }
+}
+
+template <class M>
+__global__ void __launch_bounds__(32 * kFkWarps) fk_staged_kernel(const float* __restrict__ edges, int E,
+                                                                  const int* __restrict__ steps,
+                                                                  const int* __restrict__ offs,
+                                                                  float4* __restrict__ table,
+                                                                  int* __restrict__ edge_self,
+                                                                  float2* __restrict__ seg) {
+    static_assert(M::table_tile == 1 && M::num_spheres % 2 == 1,
+                  "row-major table whose odd row length is a conflict-free stride");
+    constexpr int NS = M::num_spheres;
+    extern __shared__ __align__(128) float4 srow[];  // [32][NS]
+    __shared__ BlockState<M> B;
+    __shared__ uint8_t s_list[kFkWarps][2][32], s_pair[kFkWarps][32][2];
+    __shared__ float s_q[M::dof][32];
+    __shared__ float2 s_sc[M::dof][32];
+    const DevTables<M>& L = lane_tab<M>();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int total = offs[E];
+    for (int base = blockIdx.x * 32; base < total; base += gridDim.x * 32) {
+        const int e = edge_of_row(offs, E, base);
+        {
+            const int n = steps[e], k = base + lane - offs[e];
+            const float* ends = edges + (size_t)e * 2 * M::dof;
+#pragma unroll 1
+            for (int j = warp; j < M::dof; j += kFkWarps) {
+                const float v = edge_sample_joint(ends[j], ends[M::dof + j], n, k);
+                s_q[j][lane] = v;
+                sin_cos(v, &s_sc[j][lane].x, &s_sc[j][lane].y);
+            }
+            __syncthreads();
+            Frames<M, float> F;
+            fk_rows<M, 0>(&s_q[0][lane], &s_sc[0][lane], F, warp, srow + lane * NS);
+        }
+        if (threadIdx.x < (M::dof + 1) * kBlockSegs) (&B.move2[0][0])[threadIdx.x] = 0;
+        if (threadIdx.x == 0) B.num_items = 0;
+        fence_async_shared();
+        __syncthreads();
+        if (threadIdx.x == 0) bulk_copy_s2g(table + (size_t)base * NS, srow, 32 * NS * sizeof(float4));
+        segment_spheres<M>(srow, base, warp, kFkWarps, B, seg);
+        __syncthreads();
+        // any hit marks the edge; skipped when another block or warp already has
+        if (*(volatile const int*)(edge_self + e) == 0) {
+            for (int i = threadIdx.x; i < M::num_self_groups * kBlockSegs; i += 32 * kFkWarps) {
+                const int g = i / kBlockSegs, sg = i - g * kBlockSegs;
+                const float4* mid = srow + (sg * kSegment + kSegMid) * NS;
+                const float move = sqrtf(__int_as_float(B.move2[L.self_frame[g][0]][sg])) +
+                                   sqrtf(__int_as_float(B.move2[L.self_frame[g][1]][sg]));
+                if (self_hit_pad(mid[L.self_bound[g][0]], mid[L.self_bound[g][1]], move * 1.00001f + kSegMargin))
+                    B.items[atomicAdd(&B.num_items, 1)] = (unsigned short)i;
+            }
+        }
+        __syncthreads();
+        for (int i = warp; i < B.num_items; i += kFkWarps)
+            if (self_item_hit<M>(srow, B.items[i], B, s_list[warp], s_pair[warp])) {
+                if (lane == 0) atomicOr(edge_self + e, 1);
+                break;
+            }
+        if (threadIdx.x == 0) bulk_wait_read();
+        __syncthreads();  // the next block overwrites srow
+    }
+    if (threadIdx.x == 0) bulk_wait();
 }
 
 // ------------------------------------------------------------------ 4. self
@@ -2398,18 +2570,18 @@ cudaError_t run_prep(const PipelineArgs& a, cudaStream_t st) {
         if constexpr (M::table_tile == 1) {
             // FK and self-collision in one kernel; a grid of the resident CTAs
             // strides over the 32-row blocks
-            const size_t smem = 32 * (size_t)(M::num_spheres | 1) * sizeof(float4);
+            const size_t smem = 32 * (size_t)M::num_spheres * sizeof(float4);
             err = cudaFuncSetAttribute(fk_staged_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (err != cudaSuccess) return err;
             int dev = 0, sms = 0, per_sm = 0;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk_staged_kernel<M>, 32, smem);
+            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk_staged_kernel<M>, 32 * kFkWarps, smem);
             if (err != cudaSuccess) return err;
             const int blocks = (R + 31) / 32;
             const int grid = std::min(blocks, std::max(per_sm, 1) * std::max(sms, 1));
-            fk_staged_kernel<M><<<grid, 32, smem, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.row_edge,
-                                                        a.edge_self, a.seg);
+            fk_staged_kernel<M><<<grid, 32 * kFkWarps, smem, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.edge_self,
+                                                                   a.seg);
         } else {
             fk_kernel<M><<<(R + 127) / 128, 128, 0, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.row_edge);
         }

@@ -6,15 +6,22 @@
 namespace bcc {
 
 __constant__ DevTables<BaxterModel> c_tab_baxter;
+__device__ DevTables<BaxterModel> g_tab_baxter;  // the same tables for lane-indexed reads
 
 template <>
 __device__ __forceinline__ const DevTables<BaxterModel>& tab<BaxterModel>() {
     return c_tab_baxter;
 }
 
+template <>
+__device__ __forceinline__ const DevTables<BaxterModel>& lane_tab<BaxterModel>() {
+    return g_tab_baxter;
+}
+
 static cudaError_t upload_baxter_tables() {
     const DevTables<BaxterModel> t = host_tables<BaxterModel>();
-    return cudaMemcpyToSymbol(c_tab_baxter, &t, sizeof(t));
+    const cudaError_t err = cudaMemcpyToSymbol(g_tab_baxter, &t, sizeof(t));
+    return err != cudaSuccess ? err : cudaMemcpyToSymbol(c_tab_baxter, &t, sizeof(t));
 }
 
 extern const RobotOps kBaxterOps = robot_ops_of<BaxterModel>(BCC_ROBOT_BAXTER, upload_baxter_tables);

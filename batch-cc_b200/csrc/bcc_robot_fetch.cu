@@ -6,15 +6,22 @@
 namespace bcc {
 
 __constant__ DevTables<FetchModel> c_tab_fetch;
+__device__ DevTables<FetchModel> g_tab_fetch;  // the same tables for lane-indexed reads
 
 template <>
 __device__ __forceinline__ const DevTables<FetchModel>& tab<FetchModel>() {
     return c_tab_fetch;
 }
 
+template <>
+__device__ __forceinline__ const DevTables<FetchModel>& lane_tab<FetchModel>() {
+    return g_tab_fetch;
+}
+
 static cudaError_t upload_fetch_tables() {
     const DevTables<FetchModel> t = host_tables<FetchModel>();
-    return cudaMemcpyToSymbol(c_tab_fetch, &t, sizeof(t));
+    const cudaError_t err = cudaMemcpyToSymbol(g_tab_fetch, &t, sizeof(t));
+    return err != cudaSuccess ? err : cudaMemcpyToSymbol(c_tab_fetch, &t, sizeof(t));
 }
 
 extern const RobotOps kFetchOps = robot_ops_of<FetchModel>(BCC_ROBOT_FETCH, upload_fetch_tables);

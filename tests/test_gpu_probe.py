@@ -101,3 +101,17 @@ def test_mask_words_hold_every_primitive(checker, prims, persistent):
         checker.set_launch_config(**cfg)
     assert len(orc.adjudicate(envs, edges, got, orc.check(envs, edges))[2]) == 0
     assert np.array_equal(got[:, 1], got[:, 3])
+
+
+@pytest.mark.parametrize("name,nedge,resolution", [("uneven", 700, 32), ("plain", 150, 32), ("uneven", 200, 1),
+                                                   ("plain", 40, 200)])
+def test_self_collision_by_segments(checker, name, nedge, resolution):
+    """Without primitives a verdict is the edge's self-collision: the oracle's, on
+    edges of one block of samples and of many."""
+    envs = EnvSet.from_lists([{}])
+    edges = workload.gen_edges(name, nedge, seed=77)
+    checker.upload(envs)
+    got = checker.check(edges, resolution=resolution)
+    want = orc.check(envs, edges, resolution=resolution)
+    assert 0 < int(got.sum()) < nedge
+    assert len(orc.adjudicate(envs, edges, got, want, resolution=resolution)[2]) == 0
