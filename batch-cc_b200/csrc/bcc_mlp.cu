@@ -140,35 +140,6 @@ __device__ __forceinline__ void epilogue_relu_only(uint32_t taddr, uint8_t* himg
     }
 }
 
-// Bias + ReLU of one 128-column accumulator row (this thread's row), written as
-// BF16 into the H image; `taddr` = TMEM address of column 0 of this warp's lanes.
-// One warp group's epilogue of a hidden layer: TMEM accumulator row + bias, ReLU,
-// BF16 into the H image.  Two 16-column loads are in flight before each wait.
-__device__ __forceinline__ void epilogue_relu_to_smem(uint32_t taddr, const float* bias, uint8_t* himg, int row) {
-#pragma unroll 1
-    for (int c0 = 0; c0 < kMlpHidden; c0 += 32) {
-        float v[32];
-        tc::tmem_ld16(taddr + c0, v);
-        tc::tmem_ld16(taddr + c0 + 16, v + 16);
-        tc::wait_ld();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint32_t packed[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float a = fmaxf(v[16 * h + 2 * i] + bias[c0 + 16 * h + 2 * i], 0.0f);
-                const float b = fmaxf(v[16 * h + 2 * i + 1] + bias[c0 + 16 * h + 2 * i + 1], 0.0f);
-                __nv_bfloat162 hh = __floats2bfloat162_rn(a, b);
-                packed[i] = *reinterpret_cast<uint32_t*>(&hh);
-            }
-            *reinterpret_cast<uint4*>(himg + tc::cm_offset(row, c0 + 16 * h, kMlpHidden)) =
-                make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            *reinterpret_cast<uint4*>(himg + tc::cm_offset(row, c0 + 16 * h + 8, kMlpHidden)) =
-                make_uint4(packed[4], packed[5], packed[6], packed[7]);
-        }
-    }
-}
-
 // Barrier of one 128-thread warp group (named barrier 1 + group).
 __device__ __forceinline__ void group_sync(int grp) {
     asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
@@ -311,8 +282,7 @@ __global__ void __launch_bounds__(128 * kFwdGroups, 1)
 }
 
 // ---------------------------------------------------------------- training
-// One CTA (128 threads, one row per thread) runs forward and backward over its
-// 128-row tiles.  Activations stay in shared memory as BF16 images; the three
+// One CTA runs forward and backward over its 128-row tiles.  Activations stay in shared memory as BF16 images; the three
 // weight-gradient accumulators stay in tensor memory across tiles and are
 // added to the global FP32 gradient once at the end.  Loss: mean binary
 // cross-entropy of the logit against the 0/1 label (scale = 1 / total rows).
@@ -332,9 +302,11 @@ constexpr uint32_t kTrH2 = kTrH1 + kImgW;
 constexpr uint32_t kTrD = kTrH2 + kImgW;
 constexpr uint32_t kTrVec = kTrD + kImgW;                 // b1 b2 b3 w4 b4 (params)
 constexpr uint32_t kTrGrad = kTrVec + 5 * kMlpHidden * 4;  // db1 db2 db3 dw4 db4 loss
-constexpr uint32_t kTrBar = kTrGrad + 5 * kMlpHidden * 4 + 16;
-constexpr uint32_t kTrTmem = kTrBar + 8;
+constexpr uint32_t kTrPart = kTrGrad + 5 * kMlpHidden * 4 + 16;
+constexpr uint32_t kTrBar = kTrPart + 128 * 4;             // MMAs, weights
+constexpr uint32_t kTrTmem = kTrBar + 16;
 constexpr uint32_t kTrainSmem = kTrTmem + 8;
+static_assert(kOffW2 % 4 == 0 && kOffW3 % 4 == 0 && kTrBar % 8 == 0 && kTrainSmem <= 227 * 1024, "training kernel layout");
 // TMEM columns: forward / backward-data accumulator, dW3, dW2, dW1^T.
 constexpr uint32_t kColAcc = 0, kColW3 = 128, kColW2 = 256, kColW1 = 384;
 
@@ -346,60 +318,119 @@ __device__ __forceinline__ void gemm_issue(uint32_t d, uint32_t a0, uint32_t a_l
                      idesc, (accumulate || s > 0) ? 1u : 0u);
 }
 
-// Column sums over the CTA's 128 rows of per-row values v[0..15] (columns
-// c0..c0+15), added into acc[c0 + i] in shared memory.
-__device__ __forceinline__ void colsum16(const float* v, float* acc, int c0) {
+// Sum over the warp's 32 lanes of each of 32 per-lane values: lane i returns the
+// sum of v[i].  Halves the values with the lanes: 31 shuffles where a butterfly
+// per value takes 160.
+__device__ __forceinline__ float warp_colsum32(float (&v)[32]) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        float x = v[i];
+    for (int o = 16; o; o >>= 1) {
+        const bool up = (lane & o) != 0;
 #pragma unroll
-        for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if ((threadIdx.x & 31) == i) atomicAdd(acc + c0 + i, x);
+        for (int i = 0; i < o; ++i) {
+            const float send = up ? v[i] : v[i + o];
+            const float keep = up ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0];
+}
+
+// 32 values as BF16 into columns c0 .. c0 + 31 of row r of a 128-column image.
+__device__ __forceinline__ void store_bf16x32(uint8_t* img, int r, int c0, const float* v) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]);
+            w[i] = *reinterpret_cast<uint32_t*>(&h);
+        }
+        *reinterpret_cast<uint4*>(img + tc::cm_offset(r, c0 + 8 * q, kMlpHidden)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
-__device__ __forceinline__ float bf16_at(const uint8_t* img, int r, int c, int K) {
-    return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(img + tc::cm_offset(r, c, K)));
+// Zero the values whose activation (BF16 image, >= 0) is zero.
+__device__ __forceinline__ void mask_by_activation(const uint8_t* img, int r, int c0, float* v) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint4 h = *reinterpret_cast<const uint4*>(img + tc::cm_offset(r, c0 + 8 * q, kMlpHidden));
+        const uint32_t w[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if ((int16_t)(w[i] & 0xffffu) <= 0) v[8 * q + 2 * i] = 0.0f;
+            if ((int16_t)(w[i] >> 16) <= 0) v[8 * q + 2 * i + 1] = 0.0f;
+        }
+    }
 }
 
-__global__ void __launch_bounds__(128, 1)
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
+    tc::tmem_ld16(taddr, v);
+    tc::tmem_ld16(taddr + 16, v + 16);
+    tc::wait_ld();
+}
+
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+                 : "memory");
+}
+
+// Two threads per row: thread t holds row t % 128 and column half t / 128, so
+// each of the six epilogues is 64 columns of one row deep.  A batch of up to
+// 148 x 128 rows is one tile per CTA and the kernel is that tile's serial chain:
+// with one thread a row, a butterfly of five shuffles per column sum, 2-byte
+// reads of the activations, word-by-word weight loads and scalar atomics it took
+// 150 us for 16 384 rows; 27 us now.
+constexpr int kTrainThreads = 256;
+
+__global__ void __launch_bounds__(kTrainThreads, 1)
     mlp_train_kernel(const uint16_t* __restrict__ x, const uint8_t* __restrict__ y, int rows,
                      const uint4* __restrict__ images, const float* __restrict__ params, float* __restrict__ grads,
                      float* __restrict__ loss_sum, int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    const int t = threadIdx.x, warp = t >> 5;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int r = t & 127, half = t >> 7, col0 = half * (kMlpHidden / 2);
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kTrBar);
+    uint64_t* bar_w = bar + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kTrTmem);
     float* vec = reinterpret_cast<float*>(sm + kTrVec);    // b1 | b2 | b3 | w4 | b4
     float* gv = reinterpret_cast<float*>(sm + kTrGrad);    // db1 | db2 | db3 | dw4 | db4, loss
+    float* part = reinterpret_cast<float*>(sm + kTrPart);  // [128] logits half way, then whole
     const float inv_rows = 1.0f / (float)rows;
 
-    for (uint32_t i = t; i < kImagesW / 16; i += blockDim.x) reinterpret_cast<uint4*>(sm)[i] = images[i];
-    for (int i = t; i < kMlpHidden; i += blockDim.x) {
+    if (t == 0) {
+        mbar_init(bar, 1);
+        mbar_init(bar_w, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        bulk_copy_g2s(sm + kTrW1, images, kImagesW, bar_w);
+    }
+    for (int i = t; i < kMlpHidden; i += kTrainThreads) {
         vec[i] = params[kOffB1 + i];
         vec[kMlpHidden + i] = params[kOffB2 + i];
         vec[2 * kMlpHidden + i] = params[kOffB3 + i];
         vec[3 * kMlpHidden + i] = params[kOffW4 + i];
     }
-    for (int i = t; i < 5 * kMlpHidden + 4; i += blockDim.x) gv[i] = 0.0f;
-    if (t == 0) {
-        vec[4 * kMlpHidden] = params[kOffB4];
-        mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+    for (int i = t; i < 5 * kMlpHidden + 4; i += kTrainThreads) gv[i] = 0.0f;
+    if (t == 0) vec[4 * kMlpHidden] = params[kOffB4];
     if (warp == 0) tc::tmem_alloc(tmem_slot, 512);
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t lane_off = (uint32_t)(32 * warp) << 16;
+    const uint32_t lane_off = (uint32_t)(32 * (warp & 3)) << 16;
+    const uint32_t acc = tmem + lane_off + kColAcc + (uint32_t)col0;  // this thread's half row of the accumulator
     const uint32_t sb = tc::smem_addr(sm);
     const uint32_t id_fwd = tc::make_idesc_bf16(128, 128, 0, 0);   // A K-major, B K-major
     const uint32_t id_dw = tc::make_idesc_bf16(128, 128, 1, 1);    // A MN, B MN
     const uint32_t id_dh = tc::make_idesc_bf16(128, 128, 0, 1);    // A K, B MN
     const uint32_t id_dw1 = tc::make_idesc_bf16(128, 48, 1, 1);    // dW1^T: N = 48
     uint32_t phase = 0;
-    bool bad = false, first = true;
+    bool first = true;
+    // The weights' copy; waited for again (bounded) before the CTA may leave.
+    const bool ok_w = mbar_wait_bounded(bar_w, 0u, 1u << 22);
+    bool bad = __syncthreads_or(!ok_w) != 0;
+    if (bad) mbar_wait_bounded(bar_w, 0u, 1u << 22);
+    const bool issued_any = !bad;
     float* db1 = gv;
     float* db2 = gv + kMlpHidden;
     float* db3 = gv + 2 * kMlpHidden;
@@ -421,70 +452,99 @@ __global__ void __launch_bounds__(128, 1)
         tc::fence_after();
         return true;
     };
+    // Hidden layer's epilogue: accumulator + bias, ReLU, BF16 into an H image.
+    auto relu_to = [&](const float* bias, uint8_t* himg) {
+#pragma unroll 1
+        for (int c = 0; c < kMlpHidden / 2; c += 32) {
+            float v[32];
+            tmem_ld32(acc + c, v);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i] + bias[col0 + c + i], 0.0f);
+            store_bf16x32(himg, r, col0 + c, v);
+        }
+    };
+    // A hidden layer's dZ: the accumulator where the activation is positive, its
+    // column sums added to db and its BF16 image written.
+    auto dz_to = [&](const uint8_t* himg, float* db) {
+#pragma unroll 1
+        for (int c = 0; c < kMlpHidden / 2; c += 32) {
+            float v[32];
+            tmem_ld32(acc + c, v);
+            mask_by_activation(himg, r, col0 + c, v);
+            store_bf16x32(sm + kTrD, r, col0 + c, v);
+            const float s = warp_colsum32(v);
+            atomicAdd(db + col0 + c + lane, s);
+        }
+    };
 
     const int tiles = (rows + 127) / 128;
     for (int tile = blockIdx.x; tile < tiles && !bad; tile += gridDim.x) {
-        const int row = tile * 128 + t;
+        const int row = tile * 128 + r;
         const bool live = row < rows;
         const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * kMlpIn);
 #pragma unroll
-        for (int j = 0; j < kMlpIn / 8; ++j)
-            *reinterpret_cast<uint4*>(sm + kTrX + tc::cm_offset(t, 8 * j, kMlpIn)) = live ? src[j] : make_uint4(0, 0, 0, 0);
+        for (int j = 0; j < kMlpIn / 16; ++j) {
+            const int c = half * (kMlpIn / 16) + j;
+            *reinterpret_cast<uint4*>(sm + kTrX + tc::cm_offset(r, 8 * c, kMlpIn)) = live ? src[c] : make_uint4(0, 0, 0, 0);
+        }
         const float label = live ? (float)y[row] : 0.0f;
 
         // ---- forward
         if (!sync_issue([&] { gemm_issue(tmem + kColAcc, sb + kTrX, 128, 768, 256, sb + kTrW1, 128, 768, 256, 3, id_fwd, false); })) { bad = true; break; }
-        epilogue_relu_to_smem(tmem + lane_off + kColAcc, vec, sm + kTrH1, t);
+        relu_to(vec, sm + kTrH1);
         if (!sync_issue([&] { gemm_issue(tmem + kColAcc, sb + kTrH1, 128, 2048, 256, sb + kTrW2, 128, 2048, 256, 8, id_fwd, false); })) { bad = true; break; }
-        epilogue_relu_to_smem(tmem + lane_off + kColAcc, vec + kMlpHidden, sm + kTrH2, t);
+        relu_to(vec + kMlpHidden, sm + kTrH2);
         if (!sync_issue([&] { gemm_issue(tmem + kColAcc, sb + kTrH2, 128, 2048, 256, sb + kTrW3, 128, 2048, 256, 8, id_fwd, false); })) { bad = true; break; }
+        // The logit is one chain over the 128 columns in order (its last bits decide
+        // roundings of every gradient): the lower half's threads, then the upper's.
         float logit = vec[4 * kMlpHidden];
+        for (int h = 0; h < 2; ++h) {
+            if (half == h) {
+                if (h) logit = part[r];
 #pragma unroll 1
-        for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(tmem + lane_off + kColAcc + c0, v);
-            tc::wait_ld();
+                for (int c = 0; c < kMlpHidden / 2; c += 32) {
+                    float v[32];
+                    tmem_ld32(acc + c, v);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) logit = fmaf(fmaxf(v[i] + vec[2 * kMlpHidden + c0 + i], 0.0f), vec[3 * kMlpHidden + c0 + i], logit);
+                    for (int i = 0; i < 32; ++i)
+                        logit = fmaf(fmaxf(v[i] + vec[2 * kMlpHidden + col0 + c + i], 0.0f), vec[3 * kMlpHidden + col0 + c + i], logit);
+                }
+                part[r] = logit;
+            }
+            __syncthreads();
         }
+        logit = part[r];
         // ---- loss and dlogit (mean BCE)
         const float prob = 1.0f / (1.0f + __expf(-logit));
         const float dlogit = live ? (prob - label) * inv_rows : 0.0f;
-        const float l = live ? (fmaxf(logit, 0.0f) - logit * label + log1pf(__expf(-fabsf(logit)))) : 0.0f;
-        {
+        if (half == 0) {
+            const float l = live ? (fmaxf(logit, 0.0f) - logit * label + log1pf(__expf(-fabsf(logit)))) : 0.0f;
             float s1 = l, s2 = dlogit;
 #pragma unroll
             for (int o = 16; o; o >>= 1) {
                 s1 += __shfl_xor_sync(0xffffffffu, s1, o);
                 s2 += __shfl_xor_sync(0xffffffffu, s2, o);
             }
-            if ((t & 31) == 0) {
+            if (lane == 0) {
                 atomicAdd(gv + 5 * kMlpHidden + 1, s1);
                 atomicAdd(gv + 4 * kMlpHidden, s2);
             }
         }
         // dz3 = dlogit * w4 * (h3 > 0); dw4 += dlogit * h3; db3 += dz3
 #pragma unroll 1
-        for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
-            float v[16], g3[16], gw[16];
-            tc::tmem_ld16(tmem + lane_off + kColAcc + c0, v);
-            tc::wait_ld();
-            uint32_t packed[8];
+        for (int c = 0; c < kMlpHidden / 2; c += 32) {
+            float v[32], g3[32];
+            tmem_ld32(acc + c, v);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float h3 = fmaxf(v[i] + vec[2 * kMlpHidden + c0 + i], 0.0f);
-                gw[i] = dlogit * h3;
-                g3[i] = h3 > 0.0f ? dlogit * vec[3 * kMlpHidden + c0 + i] : 0.0f;
+            for (int i = 0; i < 32; ++i) {
+                const float h3 = fmaxf(v[i] + vec[2 * kMlpHidden + col0 + c + i], 0.0f);
+                g3[i] = h3 > 0.0f ? dlogit * vec[3 * kMlpHidden + col0 + c + i] : 0.0f;
+                v[i] = dlogit * h3;
             }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(g3[2 * i], g3[2 * i + 1]);
-                packed[i] = *reinterpret_cast<uint32_t*>(&h);
-            }
-            *reinterpret_cast<uint4*>(sm + kTrD + tc::cm_offset(t, c0, kMlpHidden)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            *reinterpret_cast<uint4*>(sm + kTrD + tc::cm_offset(t, c0 + 8, kMlpHidden)) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-            colsum16(gw, dw4, c0);
-            colsum16(g3, db3, c0);
+            store_bf16x32(sm + kTrD, r, col0 + c, g3);
+            const float s3 = warp_colsum32(g3), s4 = warp_colsum32(v);
+            atomicAdd(db3 + col0 + c + lane, s3);
+            atomicAdd(dw4 + col0 + c + lane, s4);
         }
         // ---- dW3 += H2^T dZ3 ; dH2 = dZ3 W3^T
         const bool acc_w = !first;
@@ -492,46 +552,13 @@ __global__ void __launch_bounds__(128, 1)
                 gemm_issue(tmem + kColW3, sb + kTrH2, 2048, 128, 4096, sb + kTrD, 2048, 128, 4096, 8, id_dw, acc_w);
                 gemm_issue(tmem + kColAcc, sb + kTrD, 128, 2048, 256, sb + kTrW3, 2048, 128, 4096, 8, id_dh, false);
             })) { bad = true; break; }
-        // dz2 = dh2 * (h2 > 0) -> D ; db2 += dz2
-#pragma unroll 1
-        for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(tmem + lane_off + kColAcc + c0, v);
-            tc::wait_ld();
-            uint32_t packed[8];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = bf16_at(sm + kTrH2, t, c0 + i, kMlpHidden) > 0.0f ? v[i] : 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                packed[i] = *reinterpret_cast<uint32_t*>(&h);
-            }
-            *reinterpret_cast<uint4*>(sm + kTrD + tc::cm_offset(t, c0, kMlpHidden)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            *reinterpret_cast<uint4*>(sm + kTrD + tc::cm_offset(t, c0 + 8, kMlpHidden)) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-            colsum16(v, db2, c0);
-        }
+        dz_to(sm + kTrH2, db2);
         // ---- dW2 += H1^T dZ2 ; dH1 = dZ2 W2^T
         if (!sync_issue([&] {
                 gemm_issue(tmem + kColW2, sb + kTrH1, 2048, 128, 4096, sb + kTrD, 2048, 128, 4096, 8, id_dw, acc_w);
                 gemm_issue(tmem + kColAcc, sb + kTrD, 128, 2048, 256, sb + kTrW2, 2048, 128, 4096, 8, id_dh, false);
             })) { bad = true; break; }
-#pragma unroll 1
-        for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(tmem + lane_off + kColAcc + c0, v);
-            tc::wait_ld();
-            uint32_t packed[8];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = bf16_at(sm + kTrH1, t, c0 + i, kMlpHidden) > 0.0f ? v[i] : 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                packed[i] = *reinterpret_cast<uint32_t*>(&h);
-            }
-            *reinterpret_cast<uint4*>(sm + kTrD + tc::cm_offset(t, c0, kMlpHidden)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            *reinterpret_cast<uint4*>(sm + kTrD + tc::cm_offset(t, c0 + 8, kMlpHidden)) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-            colsum16(v, db1, c0);
-        }
+        dz_to(sm + kTrH1, db1);
         // ---- dW1^T += dZ1^T X
         if (!sync_issue([&] {
                 gemm_issue(tmem + kColW1, sb + kTrD, 2048, 128, 4096, sb + kTrX, 768, 128, 1536, 8, id_dw1, acc_w);
@@ -540,32 +567,34 @@ __global__ void __launch_bounds__(128, 1)
     }
     if (bad) {
         if (t == 0) atomicOr(err, 1);
-        mbar_wait_bounded(bar, phase, 1u << 22);
+        if (issued_any) mbar_wait_bounded(bar, phase, 1u << 22);
     }
-    // ---- write gradients: thread t owns TMEM lane t of each accumulator.
+    // ---- write gradients: a thread owns its row's half of each accumulator.
     if (!bad && !first) {
+        const uint32_t lanes = tmem + lane_off;
 #pragma unroll 1
-        for (int c0 = 0; c0 < kMlpHidden; c0 += 16) {
-            float v[16];
-            tc::tmem_ld16(tmem + lane_off + kColW3 + c0, v);
-            tc::wait_ld();
-            for (int i = 0; i < 16; ++i) atomicAdd(grads + kOffW3 + t * kMlpHidden + c0 + i, v[i]);
-            tc::tmem_ld16(tmem + lane_off + kColW2 + c0, v);
-            tc::wait_ld();
-            for (int i = 0; i < 16; ++i) atomicAdd(grads + kOffW2 + t * kMlpHidden + c0 + i, v[i]);
+        for (int c = col0; c < col0 + kMlpHidden / 2; c += 32) {
+            float v[32];
+            tmem_ld32(lanes + kColW3 + c, v);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) red_add4(grads + kOffW3 + r * kMlpHidden + c + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
+            tmem_ld32(lanes + kColW2 + c, v);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) red_add4(grads + kOffW2 + r * kMlpHidden + c + i, v[i], v[i + 1], v[i + 2], v[i + 3]);
         }
 #pragma unroll 1
-        for (int c0 = 0; c0 < kMlpIn; c0 += 16) {
+        for (int c = half * 32; c < (half ? kMlpIn : 32); c += 16) {
             float v[16];
-            tc::tmem_ld16(tmem + lane_off + kColW1 + c0, v);
+            tc::tmem_ld16(lanes + kColW1 + c, v);
             tc::wait_ld();
-            for (int i = 0; i < 16; ++i) atomicAdd(grads + kOffW1 + (c0 + i) * kMlpHidden + t, v[i]);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) atomicAdd(grads + kOffW1 + (c + i) * kMlpHidden + r, v[i]);
         }
     }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    if (!bad) {
+    if (!bad && t < 128) {
         atomicAdd(grads + kOffB1 + t, db1[t]);
         atomicAdd(grads + kOffB2 + t, db2[t]);
         atomicAdd(grads + kOffB3 + t, db3[t]);
@@ -604,7 +633,7 @@ cudaError_t mlp_train_grads(const uint16_t* d_x, const uint8_t* d_y, int rows, c
     if (e != cudaSuccess) return e;
     const int tiles = (rows + 127) / 128;
     const int grid = tiles < num_sms ? tiles : num_sms;
-    mlp_train_kernel<<<grid, 128, kTrainSmem, st>>>(d_x, d_y, rows, reinterpret_cast<const uint4*>(d_images), d_params,
+    mlp_train_kernel<<<grid, kTrainThreads, kTrainSmem, st>>>(d_x, d_y, rows, reinterpret_cast<const uint4*>(d_images), d_params,
                                                     d_grads, d_loss, d_err);
     return cudaGetLastError();
 }

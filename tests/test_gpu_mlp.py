@@ -76,3 +76,25 @@ def test_mlp_training_reduces_loss(checker):
     yb = torch.from_numpy(y).cuda()
     losses = [checker.mlp_train_step_device(xb.data_ptr(), yb.data_ptr(), rows, 3e-3) / rows for _ in range(60)]
     assert losses[-1] < 0.5 * losses[0], (losses[0], losses[-1])
+
+
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 148 * 128 + 1, 40000])
+def test_mlp_gradients_at_tile_edges(checker, rows):
+    """One row, the edges of a 128-row tile, one tile more than the CTAs a launch
+    has, several tiles a CTA: the FP64 oracle's gradients and loss (3e-2: BF16
+    operands, as above)."""
+    import torch
+    from oracle import mlp_oracle
+    rng = np.random.default_rng(rows)
+    p = mlp.init_params(8)
+    checker.mlp_set_params(p)
+    x = rng.normal(0, 1, (rows, 48)).astype(np.float32)
+    x[:, 39:] = 0
+    y = (rng.uniform(0, 1, rows) < 0.4).astype(np.uint8)
+    xb = torch.from_numpy(mlp.to_bf16_bits(x).view(np.int16)).cuda()
+    yb = torch.from_numpy(y).cuda()
+    torch.cuda.synchronize()
+    g, loss = checker.mlp_gradients_device(xb.data_ptr(), yb.data_ptr(), rows)
+    want_loss, want = mlp_oracle.loss_and_grads(p, x, y)
+    assert abs(loss - want_loss) < 1e-2 * want_loss + 1e-3
+    assert np.linalg.norm(g - want) < 3e-2 * np.linalg.norm(want)
