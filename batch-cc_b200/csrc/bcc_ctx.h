@@ -36,7 +36,11 @@ struct DevBuf {
 struct MlpState {
     bool ready = false;      // weights uploaded
     DevBuf params;           // FP32 master parameters (kMlpParams floats)
-    DevBuf grads;            // FP32 gradients
+    DevBuf grads;            // FP32 gradients, then the loss and an error flag
+    float* host = nullptr;   // pinned, kMlpGradBytes: what training and queries read back
+    ~MlpState() {
+        if (host) cudaFreeHost(host);
+    }
     DevBuf adam_m, adam_v;   // Adam moments
     DevBuf images;           // BF16 core-matrix images of W1^T, W2^T, W3^T
     DevBuf acts;             // training activations

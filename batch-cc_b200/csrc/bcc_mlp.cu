@@ -607,26 +607,46 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     if (warp == 0) tc::tmem_free(tmem, 512);
 }
 
-// Adam on the FP32 masters (bias-corrected), then the BF16 images are re-packed.
+// Byte offset of parameter i's BF16 copy in the images, or -1 (b4, and W1's row of
+// the bias feature, have none).  The inverse of mlp_pack_kernel's map.
+__device__ __forceinline__ int image_offset(int i) {
+    if (i < kOffB1) {
+        const int in = i / kMlpHidden, out = i - in * kMlpHidden;
+        return in == kBiasCol ? -1 : (int)tc::cm_offset(out, in, kMlpIn);
+    }
+    if (i < kOffW2) return (int)tc::cm_offset(i - kOffB1, kBiasCol, kMlpIn);
+    if (i < kOffW4) {  // W2 b2 W3 b3
+        const int layer = i >= kOffW3, j = i - (layer ? kOffW3 : kOffW2);
+        const int in = j / kMlpHidden, out = j - in * kMlpHidden;
+        return in < kMlpHidden ? (int)(kImgW1 + layer * kImgW + tc::cm_offset(out, in, kMlpHidden))
+                               : (int)(kImagesW + (1 + layer) * kImgSmall + tc::cm_offset(out, 0, 16));
+    }
+    return i < kOffB4 ? (int)(kImagesW + tc::cm_offset(0, i - kOffW4, kMlpHidden)) : -1;
+}
+
+// Adam on the FP32 masters (bias-corrected) and each parameter's BF16 copy, in
+// one pass; does nothing once the gradient kernel has flagged an error.
 __global__ void mlp_adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                                float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float c1,
-                                float c2) {
+                                float* __restrict__ v, uint8_t* __restrict__ images, const int* __restrict__ err, int n,
+                                float lr, float b1, float b2, float eps, float c1, float c2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || *err) return;
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    const float w = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] = w;
+    const int at = image_offset(i);
+    if (at >= 0) *reinterpret_cast<__nv_bfloat16*>(images + at) = __float2bfloat16_rn(w);
 }
 
 cudaError_t mlp_train_grads(const uint16_t* d_x, const uint8_t* d_y, int rows, const uint8_t* d_images,
-                            const float* d_params, float* d_grads, float* d_loss, int* d_err, int num_sms,
-                            cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(d_grads, 0, sizeof(float) * kMlpParams, st);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(d_loss, 0, sizeof(float), st);
+                            const float* d_params, float* d_grads, int num_sms, cudaStream_t st) {
+    float* d_loss = d_grads + kMlpParams;
+    int* d_err = reinterpret_cast<int*>(d_loss + 1);
+    cudaError_t e = cudaMemsetAsync(d_grads, 0, kMlpGradBytes, st);
     if (e != cudaSuccess) return e;
     if (rows <= 0) return cudaSuccess;
     e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem);
@@ -638,12 +658,13 @@ cudaError_t mlp_train_grads(const uint16_t* d_x, const uint8_t* d_y, int rows, c
     return cudaGetLastError();
 }
 
-cudaError_t mlp_adam(float* d_params, const float* d_grads, float* d_m, float* d_v, long long step, float lr,
-                     cudaStream_t st) {
+cudaError_t mlp_adam(float* d_params, const float* d_grads, float* d_m, float* d_v, uint8_t* d_images, long long step,
+                     float lr, cudaStream_t st) {
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
-    mlp_adam_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(d_params, d_grads, d_m, d_v, kMlpParams, lr, b1, b2,
-                                                              1e-8f, c1, c2);
+    mlp_adam_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(d_params, d_grads, d_m, d_v, d_images,
+                                                              reinterpret_cast<const int*>(d_grads + kMlpParams + 1),
+                                                              kMlpParams, lr, b1, b2, 1e-8f, c1, c2);
     return cudaGetLastError();
 }
 
@@ -683,6 +704,14 @@ int sm_count(int dev) {
     return n > 0 ? n : 1;
 }
 
+// Up to kMlpGradBytes of device memory into the context's pinned buffer
+// (mlp.host), after everything queued on st.
+bool to_host(bcc_ctx* ctx, const void* src, size_t bytes, cudaStream_t st) {
+    if (!ctx->mlp.host && cudaMallocHost(&ctx->mlp.host, bcc::kMlpGradBytes) != cudaSuccess) return false;
+    return cudaMemcpyAsync(ctx->mlp.host, src, bytes, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+           cudaStreamSynchronize(st) == cudaSuccess;
+}
+
 }  // namespace
 
 extern "C" {
@@ -694,7 +723,7 @@ bcc_status bcc_mlp_set_params(bcc_ctx* ctx, const float* params, int32_t n) {
     if (cudaSetDevice(ctx->device) != cudaSuccess) return BCC_ERR_CUDA;
     bcc::MlpState& m = ctx->mlp;
     const size_t pb = sizeof(float) * bcc::kMlpParams;
-    if (m.params.ensure(pb) != cudaSuccess || m.grads.ensure(pb) != cudaSuccess || m.adam_m.ensure(pb) != cudaSuccess ||
+    if (m.params.ensure(pb) != cudaSuccess || m.grads.ensure(bcc::kMlpGradBytes) != cudaSuccess || m.adam_m.ensure(pb) != cudaSuccess ||
         m.adam_v.ensure(pb) != cudaSuccess || m.images.ensure(bcc::kImagesBytes) != cudaSuccess)
         return mlp_fail(ctx, BCC_ERR_CUDA, "MLP allocation failed");
     if (cudaMemcpy(m.params.p, params, pb, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -711,8 +740,9 @@ bcc_status bcc_mlp_set_params(bcc_ctx* ctx, const float* params, int32_t n) {
 bcc_status bcc_mlp_get_params(bcc_ctx* ctx, float* params, int32_t n) {
     if (!ctx || !params || n != bcc::kMlpParams || !ctx->mlp.ready) return BCC_ERR_INVALID_ARGUMENT;
     if (cudaSetDevice(ctx->device) != cudaSuccess ||
-        cudaMemcpy(params, ctx->mlp.params.p, sizeof(float) * n, cudaMemcpyDeviceToHost) != cudaSuccess)
+        !to_host(ctx, ctx->mlp.params.p, sizeof(float) * n, ctx->stream))
         return BCC_ERR_CUDA;
+    std::memcpy(params, ctx->mlp.host, sizeof(float) * n);
     return BCC_OK;
 }
 
@@ -738,38 +768,43 @@ bcc_status bcc_mlp_gradients(bcc_ctx* ctx, const void* d_x_bf16, const uint8_t* 
     if (rows < 0 || (rows > 0 && (!d_x_bf16 || !d_labels))) return BCC_ERR_INVALID_ARGUMENT;
     if (cudaSetDevice(ctx->device) != cudaSuccess) return BCC_ERR_CUDA;
     bcc::MlpState& m = ctx->mlp;
-    if (ctx->error_flag.ensure(sizeof(int)) != cudaSuccess || m.logits.ensure(sizeof(float) * 4) != cudaSuccess)
-        return BCC_ERR_CUDA;
     cudaStream_t st = ctx->stream;
-    if (cudaMemsetAsync(ctx->error_flag.p, 0, sizeof(int), st) != cudaSuccess) return BCC_ERR_CUDA;
     if (bcc::mlp_train_grads(static_cast<const uint16_t*>(d_x_bf16), d_labels, rows, m.images.as<uint8_t>(),
-                             m.params.as<float>(), m.grads.as<float>(), m.logits.as<float>(), ctx->error_flag.as<int>(),
-                             sm_count(ctx->device), st) != cudaSuccess)
+                             m.params.as<float>(), m.grads.as<float>(), sm_count(ctx->device), st) != cudaSuccess)
         return mlp_fail(ctx, BCC_ERR_CUDA, "MLP training kernel launch failed");
+    // loss and error behind the gradients: one copy, one wait
+    const size_t first = h_grads ? 0 : bcc::kMlpParams;
+    if (!to_host(ctx, m.grads.as<float>() + first, bcc::kMlpGradBytes - sizeof(float) * first, st)) return BCC_ERR_CUDA;
+    const float* tail = m.host + (bcc::kMlpParams - first);
     int flag = 0;
-    if (cudaMemcpyAsync(&flag, ctx->error_flag.p, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return BCC_ERR_CUDA;
+    std::memcpy(&flag, tail + 1, sizeof(int));
     if (flag) return mlp_fail(ctx, BCC_ERR_TIMEOUT, "MLP training kernel wait timed out");
-    if (h_grads && cudaMemcpy(h_grads, m.grads.p, sizeof(float) * bcc::kMlpParams, cudaMemcpyDeviceToHost) != cudaSuccess)
-        return BCC_ERR_CUDA;
-    if (h_loss && cudaMemcpy(h_loss, m.logits.p, sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)
-        return BCC_ERR_CUDA;
+    if (h_grads) std::memcpy(h_grads, m.host, sizeof(float) * bcc::kMlpParams);
+    if (h_loss) *h_loss = *tail;
     return BCC_OK;
 }
 
-// One optimisation step: gradients of the batch, Adam update (lr), re-pack.
+// One optimisation step: gradients of the batch, Adam update (lr) and the BF16
+// copies, queued together; the host waits once, for the loss.
 bcc_status bcc_mlp_train_step(bcc_ctx* ctx, const void* d_x_bf16, const uint8_t* d_labels, int32_t rows, float lr,
                               float* h_loss) {
-    bcc_status s = bcc_mlp_gradients(ctx, d_x_bf16, d_labels, rows, nullptr, h_loss);
-    if (s != BCC_OK) return s;
+    if (!ctx || !ctx->mlp.ready) return mlp_fail(ctx, BCC_ERR_INVALID_ARGUMENT, "MLP parameters not set");
+    if (rows < 0 || (rows > 0 && (!d_x_bf16 || !d_labels))) return BCC_ERR_INVALID_ARGUMENT;
+    if (cudaSetDevice(ctx->device) != cudaSuccess) return BCC_ERR_CUDA;
     bcc::MlpState& m = ctx->mlp;
-    m.step += 1;
-    if (bcc::mlp_adam(m.params.as<float>(), m.grads.as<float>(), m.adam_m.as<float>(), m.adam_v.as<float>(), m.step, lr,
-                      ctx->stream) != cudaSuccess ||
-        bcc::mlp_pack(m.params.as<float>(), m.images.as<uint8_t>(), ctx->stream) != cudaSuccess ||
-        cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+    cudaStream_t st = ctx->stream;
+    if (bcc::mlp_train_grads(static_cast<const uint16_t*>(d_x_bf16), d_labels, rows, m.images.as<uint8_t>(),
+                             m.params.as<float>(), m.grads.as<float>(), sm_count(ctx->device), st) != cudaSuccess)
+        return mlp_fail(ctx, BCC_ERR_CUDA, "MLP training kernel launch failed");
+    if (bcc::mlp_adam(m.params.as<float>(), m.grads.as<float>(), m.adam_m.as<float>(), m.adam_v.as<float>(),
+                      m.images.as<uint8_t>(), m.step + 1, lr, st) != cudaSuccess ||
+        !to_host(ctx, m.grads.as<float>() + bcc::kMlpParams, 2 * sizeof(float), st))
         return mlp_fail(ctx, BCC_ERR_CUDA, "MLP update failed");
+    int flag = 0;
+    std::memcpy(&flag, m.host + 1, sizeof(int));
+    if (flag) return mlp_fail(ctx, BCC_ERR_TIMEOUT, "MLP training kernel wait timed out");
+    m.step += 1;
+    if (h_loss) *h_loss = m.host[0];
     return BCC_OK;
 }
 
