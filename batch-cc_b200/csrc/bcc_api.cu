@@ -284,14 +284,11 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     if (total < 0 || total > (1 << 27))
         return fail(ctx, BCC_ERR_LIMIT, "too many samples in one call (edges too long or non-finite)");
     const int NS = ops->num_spheres;
-    const size_t tiles = ((size_t)std::max(total, 1) + bcc::kMaxTableTile - 1) / bcc::kMaxTableTile;
-    BCC_CUDA(ctx, ctx->table.ensure(sizeof(float4) * (size_t)NS * tiles * bcc::kMaxTableTile));
-    BCC_CUDA(ctx, ctx->row_edge.ensure(sizeof(int) * (size_t)std::max(total, 1)));
+    BCC_CUDA(ctx, ctx->table.ensure(sizeof(float4) * (size_t)NS * std::max(total, 1)));
     a.total_rows = total;
     BCC_CUDA(ctx, ctx->seg.ensure(sizeof(float2) * (size_t)G * (std::max(total, bcc::kSegment) / bcc::kSegment)));
     a.seg = ctx->seg.as<float2>();
     a.table = ctx->table.as<float4>();
-    a.row_edge = ctx->row_edge.as<int>();
     a.blobs = ctx->blobs.as<float4>();
     a.env_hdr = ctx->env_hdr.as<float4>();
     a.num_envs = ctx->num_envs;
@@ -508,7 +505,7 @@ bool same_tune(const bcc::Tune& x, const bcc::Tune& y) {
 // A captured graph holds the addresses of the context's buffers: calls of other
 // sizes, orders or robots in between may have replaced some.
 bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
-    return x.steps == y.steps && x.offs == y.offs && x.table == y.table && x.row_edge == y.row_edge && x.seg == y.seg &&
+    return x.steps == y.steps && x.offs == y.offs && x.table == y.table && x.seg == y.seg &&
            x.edge_self == y.edge_self && x.swept == y.swept && x.edge_tri == y.edge_tri &&
            x.grid_bounds == y.grid_bounds && x.blobs == y.blobs && x.env_hdr == y.env_hdr && x.mid == y.mid &&
            x.probe.vox == y.probe.vox && x.queue.entries == y.queue.entries && x.queue.items == y.queue.items &&

@@ -95,7 +95,7 @@ struct bcc_ctx {
     bcc::DevBuf blobs, env_hdr;
     bcc::DevBuf records;     // the upload's records as packed, source of the blobs
     // per-call buffers
-    bcc::DevBuf edges, steps, offs, table, row_edge, edge_self, swept, results, error_flag;
+    bcc::DevBuf edges, steps, offs, table, edge_self, swept, results, error_flag;
     int* h_total = nullptr;  // pinned readback of the sample-row total
     bool profiling = false;
     bool counting = false;

@@ -118,8 +118,6 @@ __device__ __forceinline__ int reference_rank_to_sample(int r, int n) {
 // robots whose reference FK is float code (Panda) and double where the
 // reference evaluates its FK in double (Fetch, Baxter); centres are rounded to
 // float either way, as the reference does when it passes them to the tests.
-// Each sphere is emitted right after its frame is known, so a frame stays
-// live only while later joints or spheres still need it.
 // ---------------------------------------------------------------------------
 template <class M, class T>
 struct Frames {
@@ -127,46 +125,10 @@ struct Frames {
     T p[M::dof + 1][3];
 };
 
-template <class M, int S, class T>
-__device__ __forceinline__ float4 fk_sphere(const Frames<M, T>& F) {
-    constexpr int f = M::sphere_frame[S];
-    constexpr T lx = (T)M::sphere_local[S][0];
-    constexpr T ly = (T)M::sphere_local[S][1];
-    constexpr T lz = (T)M::sphere_local[S][2];
-    float4 c;
-    c.x = (float)(F.R[f][0] * lx + F.R[f][1] * ly + F.R[f][2] * lz + F.p[f][0]);
-    c.y = (float)(F.R[f][3] * lx + F.R[f][4] * ly + F.R[f][5] * lz + F.p[f][1]);
-    c.z = (float)(F.R[f][6] * lx + F.R[f][7] * ly + F.R[f][8] * lz + F.p[f][2]);
-    c.w = M::sphere_radius[S];
-    return c;
-}
-
-// Sample table layout: rows in tiles of M::table_tile rows, sphere-major inside
-// a tile (a tile of 1 is plain row-major).  With tiles of 32, 32 consecutive
-// rows of one sphere are 512 contiguous bytes and the FK kernel's warp (32
-// consecutive rows) writes each sphere with one coalesced store; row-major keeps
-// a row's bounds and leaves together for the check kernel's reads.
-constexpr int kMaxTableTile = 32;  // hosts round row counts up to this
-
+// Sample table: row-major, one row of num_spheres float4 per (edge, sample).
 template <class M>
 __host__ __device__ __forceinline__ size_t table_index(size_t row, int s) {
-    constexpr int TT = M::table_tile;
-    return ((row / TT) * M::num_spheres + s) * TT + (row % TT);
-}
-
-// Write every sphere attached to frame FR into its sample-table position; `out`
-// points at the row's first sphere, spheres M::table_tile float4 apart.
-template <class M, int FR, int S, class T>
-__device__ __forceinline__ void emit_one(const Frames<M, T>& F, float4* __restrict__ out) {
-    if constexpr (M::sphere_frame[S] == FR) {
-        constexpr int pos = M::table_pos[S];
-        out[pos * M::table_tile] = fk_sphere<M, S, T>(F);
-    }
-}
-template <class M, int FR, class T, int... S>
-__device__ __forceinline__ void emit_frame(const Frames<M, T>& F, float4* __restrict__ out,
-                                           std::integer_sequence<int, S...>) {
-    (emit_one<M, FR, S, T>(F, out), ...);
+    return row * M::num_spheres + s;
 }
 
 __device__ __forceinline__ void sin_cos(float q, float* s, float* c) { sincosf(q, s, c); }
@@ -215,32 +177,6 @@ __device__ __forceinline__ void fk_base(Frames<M, T>& F) {
 #pragma unroll
     for (int i = 0; i < 9; ++i) F.R[0][i] = (i % 4 == 0) ? T(1) : T(0);
     F.p[0][0] = F.p[0][1] = F.p[0][2] = T(0);
-}
-
-template <class M, int K, class T>
-struct FkJoint {
-    __device__ __forceinline__ static void run(const float* q, Frames<M, T>& F, float4* __restrict__ out) {
-        T sq = T(0), cq = T(1);
-        if constexpr (M::joint_type[K] == 0) sin_cos((T)q[K], &sq, &cq);
-        fk_advance<M, K, T>((T)q[K], sq, cq, F);
-        emit_frame<M, K + 1, T>(F, out, std::make_integer_sequence<int, M::num_spheres>{});
-        FkJoint<M, K + 1, T>::run(q, F, out);
-    }
-};
-
-template <class M, class T>
-struct FkJoint<M, M::dof, T> {
-    __device__ __forceinline__ static void run(const float*, Frames<M, T>&, float4* __restrict__) {}
-};
-
-// All sphere centres of configuration q into out[table_pos[s] * table_tile].
-template <class M>
-__device__ __forceinline__ void fk_spheres(const float* q, float4* __restrict__ out) {
-    using T = typename std::conditional<M::fk_precision == 64, double, float>::type;
-    Frames<M, T> F;
-    fk_base<M, T>(F);
-    emit_frame<M, 0, T>(F, out, std::make_integer_sequence<int, M::num_spheres>{});
-    FkJoint<M, 0, T>::run(q, F, out);
 }
 
 // Bounded mbarrier wait: gives up after `limit` polls and reports false.

@@ -110,7 +110,6 @@ struct PipelineArgs {
     int* offs;               // [E + 1]
     int total_rows;          // offs[E], read back after the scan
     float4* table;           // [total_rows][num_spheres]
-    int* row_edge;           // [total_rows]
     float2* seg;             // [total_rows / kSegment][groups] segment spheres, null = not needed
     int* edge_self;          // [E]
     float4* swept;           // [E][groups][2]

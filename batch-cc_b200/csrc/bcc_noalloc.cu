@@ -44,9 +44,7 @@ static __device__ __align__(256) int g_steps[kMaxEdges];
 static __device__ __align__(256) int g_offs[kMaxEdges + 1];
 static __device__ __align__(256) int g_edge_self[kMaxEdges];
 static __device__ __align__(256) float4 g_swept[kMaxEdges * kGroupsMax * 2];
-static_assert(kMaxRows % bcc::kMaxTableTile == 0, "the sample table holds whole tiles of rows");
 static __device__ __align__(256) float4 g_table[kMaxRows * kNumSpheresMax];
-static __device__ __align__(256) int g_row_edge[kMaxRows];
 static __device__ __align__(256) int g_error[1];
 
 struct Scratch {
@@ -55,7 +53,6 @@ struct Scratch {
     int* edge_self = nullptr;
     float4* swept = nullptr;
     float4* table = nullptr;
-    int* row_edge = nullptr;
     int* error = nullptr;
     bool ready = false;
     bool tables[3] = {false, false, false};  // robot tables uploaded to this device
@@ -76,7 +73,6 @@ cudaError_t setup_device(int dev, const bcc::RobotOps* ops, Scratch*& out) {
         if ((e = cudaGetSymbolAddress((void**)&s.edge_self, g_edge_self)) != cudaSuccess) return e;
         if ((e = cudaGetSymbolAddress((void**)&s.swept, g_swept)) != cudaSuccess) return e;
         if ((e = cudaGetSymbolAddress((void**)&s.table, g_table)) != cudaSuccess) return e;
-        if ((e = cudaGetSymbolAddress((void**)&s.row_edge, g_row_edge)) != cudaSuccess) return e;
         if ((e = cudaGetSymbolAddress((void**)&s.error, g_error)) != cudaSuccess) return e;
         s.ready = true;
     }
@@ -128,7 +124,6 @@ extern "C" bcc_status bcc_check_noalloc(bcc_robot robot, const float* d_records,
     a.edge_self = s->edge_self;
     a.swept = s->swept;
     a.table = s->table;
-    a.row_edge = s->row_edge;
     if (ops->steps(a, st) != cudaSuccess) return BCC_ERR_CUDA;
     int total = 0;
     if (cudaMemcpyAsync(&total, s->offs + num_edges, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -9,11 +9,12 @@
 // Pipeline of one check (all on one stream):
 //   1. edge_steps_kernel   n per edge (reference discretisation, src/batch_cc.cu:103-107)
 //   2. scan_kernel         exclusive prefix sum of 32 n -> per-edge sample offsets
-//   3. fk_kernel           one thread per (edge, sample): FK of every robot sphere
-//                          into the sample table, env-independent, computed once
-//                          instead of once per environment as in the reference
-//   4. self_kernel         self-collision of every sample (src/utils.cuh:1192-5440
-//                          for Panda), OR-reduced per edge; env-independent
+//   3. fk_staged_kernel    FK of every (edge, sample) into the sample table,
+//                          env-independent, computed once instead of once per
+//                          environment as in the reference
+//   4.                     and, while the rows are in shared memory, their
+//                          self-collision (src/utils.cuh:1192-5440 for Panda),
+//                          OR-reduced per edge, and the segments' spheres
 //   5. swept_kernel        per (edge, link) AABB of the link's cull sphere over
 //                          all the edge's samples
 //   6. probe_kernel        one lane per (environment, edge) pair: decides most pairs
@@ -58,8 +59,13 @@
 namespace bcc {
 
 constexpr unsigned kFull = 0xffffffffu;
+constexpr float kSegMargin = 1e-4f;  // FP32 rounding of centres and distances (~1e-6 m), generously
 
 // ------------------------------------------------------------------ tables
+// Scalar type of a robot's forward kinematics.
+template <class M>
+using FkReal = typename std::conditional<M::fk_precision == 64, double, float>::type;
+
 template <class M>
 struct DevTables {
     int env_bound[M::num_env_groups];
@@ -69,6 +75,7 @@ struct DevTables {
     // Certain-hit radius of env group g (0: none): a primitive whose core lies
     // within rho + cert_r[g] of the bound's centre is hit by a leaf of g.
     float cert_r[M::num_env_groups];
+    float seg_pad[M::num_env_groups];  // radius + inflation + overhang + margin
     // Groups by descending certain-hit radius (the probe's order).
     int probe_group[M::num_env_groups];
     int self_bound[M::num_self_groups][2];
@@ -90,8 +97,11 @@ struct DevTables {
     // to fk_x_end[f] with their x product rounded first, see fk_x_first): offset in the
     // frame and radius, row position.
     int fk_begin[M::dof + 2], fk_x_end[M::dof + 1];
-    float4 fk_local[M::num_spheres];
-    int fk_pos[M::num_spheres];
+    struct alignas(16) FkSphere {  // read as whole 16-byte words
+        FkReal<M> x, y, z;
+        float r;
+        int pos;
+    } fk[M::num_spheres];
     float sphere_radius[M::num_spheres];  // by sample-table position
     float s_m[M::dof], s_a[M::dof];       // joint-limit scale q = u * s_m + s_a
 };
@@ -206,7 +216,6 @@ DevTables<M> host_tables() {
     static_assert(M::num_env_groups <= kMaxEnvGroups, "one cull lane per link group");
     static_assert(M::num_spheres <= kMaxTableSpheres, "sample-table row width");
     static_assert(M::num_spheres <= 256, "self pairs hold 8-bit row positions");
-    static_assert(M::table_tile >= 1 && kMaxTableTile % M::table_tile == 0, "table tiles divide the row padding");
     DevTables<M> t;
     for (int g = 0; g < M::num_env_groups; ++g) {
         t.env_bound[g] = M::env_bound[g];
@@ -239,14 +248,15 @@ DevTables<M> host_tables() {
         for (int y_first = 0; y_first < 2; ++y_first) {
             for (int s = 0; s < M::num_spheres; ++s)
                 if (M::sphere_frame[s] == f && fk_x_first<M>(M::table_pos[s]) == !y_first) {
-                    t.fk_local[at] = make_float4((float)M::sphere_local[s][0], (float)M::sphere_local[s][1],
-                                                 (float)M::sphere_local[s][2], M::sphere_radius[s]);
-                    t.fk_pos[at++] = M::table_pos[s];
+                    t.fk[at++] = {(FkReal<M>)M::sphere_local[s][0], (FkReal<M>)M::sphere_local[s][1],
+                                  (FkReal<M>)M::sphere_local[s][2], M::sphere_radius[s], M::table_pos[s]};
                 }
             if (!y_first) t.fk_x_end[f] = at;
         }
     }
     t.fk_begin[M::dof + 1] = at;
+    for (int g = 0; g < M::num_env_groups; ++g)
+        t.seg_pad[g] = t.sphere_radius[g] + kEnvInflate + t.cull_pad[g] + kSegMargin;
     for (int j = 0; j < M::dof; ++j) {
         t.s_m[j] = M::s_m[j];
         t.s_a[j] = M::s_a[j];
@@ -350,36 +360,7 @@ __global__ void edge_steps_kernel(const float* __restrict__ edges, int E, int re
 // ------------------------------------------------------------------ 3. FK
 // Sample table row: num_spheres float4 (centre xyz, radius) in table_pos order
 // (env-group bounds, then env leaves, then the rest), one row per (edge,
-// sample) in edge order then sample index order; stored in tiles of
-// M::table_tile rows (table_index).
-template <class M>
-__global__ void __launch_bounds__(128) fk_kernel(const float* __restrict__ edges, int E,
-                                                 const int* __restrict__ steps,
-                                                 const int* __restrict__ offs,
-                                                 float4* __restrict__ table,
-                                                 int* __restrict__ row_edge) {
-    const int total = offs[E];
-    const int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= total) return;
-    // edge of this row: binary search over offs
-    int lo = 0, hi = E - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (offs[mid] <= row) lo = mid; else hi = mid - 1;
-    }
-    const int e = lo;
-    const int k = row - offs[e];
-    float s[M::dof], t[M::dof], q[M::dof];
-#pragma unroll
-    for (int j = 0; j < M::dof; ++j) {
-        s[j] = edges[(size_t)e * 2 * M::dof + j];
-        t[j] = edges[(size_t)e * 2 * M::dof + M::dof + j];
-    }
-    edge_sample<M::dof>(s, t, steps[e], k, q);
-    fk_spheres<M>(q, table + table_index<M>(row, 0));
-    row_edge[row] = e;
-}
-
+// sample) in edge order then sample index order.
 __device__ __forceinline__ bool self_hit(float4 a, float4 b) {
     const float dx = a.x - b.x, dy = a.y - b.y, dz = a.z - b.z;
     const float rs = a.w + b.w;
@@ -401,22 +382,8 @@ __device__ __forceinline__ float dist2(float4 a, float4 b) {
 // its middle sample, row kSegMid.  Group g's entry (R, rho) of segment s: the
 // sphere of radius R around the bound's centre there holds all that group g can
 // hit with at any of the samples (bound, overhang, inflation, margin); a leaf's
-// centre stays within rho of where it is at the middle sample.
-constexpr int kSegMid = kSegment / 2;
-constexpr float kSegMargin = 1e-4f;  // FP32 rounding of centres and distances (~1e-6 m), generously
-
-// Shared state of a staged block of 32 rows: how far any sphere of a frame moves
-// from its place at its segment's middle row (squared, as bits: they order like
-// the values), and the (self group, segment) items still in question.
-constexpr int kBlockSegs = 32 / kSegment;
-template <class M>
-struct BlockState {
-    int move2[M::dof + 1][kBlockSegs];
-    int num_items;
-    unsigned short items[M::num_self_groups * kBlockSegs];
-};
-
-// Is every group's leaf in its bound's frame?
+// centre stays within rho of where it is at the middle sample (robots whose groups
+// are rigid, see groups_are_rigid).
 template <class M>
 constexpr bool groups_are_rigid() {
     for (int g = 0; g < M::num_env_groups; ++g)
@@ -424,44 +391,68 @@ constexpr bool groups_are_rigid() {
             if (M::sphere_frame[M::env_leaves[k]] != M::sphere_frame[M::env_bound[g]]) return false;
     return true;
 }
+constexpr int kSegMid = kSegment / 2;
 
-// The four segments of the CTA's 32 staged rows (row base + l at srow + l *
-// num_spheres): every lane measures its row against its segment's middle one,
-// eight lanes reduce.  The warps share out the groups (a group's leaves one
-// after another), then the spheres outside any.
+// Shared state of a staged block of 32 rows: how far any sphere of a frame moves
+// from its place at its segment's middle row, and how far each group's bound does
+// (squared, as bits: they order like the values), and the (self group, segment)
+// items still in question.
+constexpr int kBlockSegs = 32 / kSegment;
 template <class M>
-__device__ __forceinline__ void segment_spheres(const float4* srow, int base, int warp, int warps, BlockState<M>& B,
-                                                float2* __restrict__ seg) {
-    constexpr int G = M::num_env_groups;
-    constexpr int NS = M::num_spheres;
-    static_assert(groups_are_rigid<M>(), "a group's movement is its frame's");
+struct BlockState {
+    int move2[M::dof + 1][kBlockSegs];
+    float bound2[M::num_env_groups][kBlockSegs];
+    int num_items;
+    unsigned short items[M::num_self_groups * kBlockSegs];
+};
+
+// The block's movements: every lane measures its row (row l at srow + l * STRIDE)
+// against its segment's middle one, eight lanes reduce.  The warps share out every
+// frame's spheres and the groups' bounds.
+template <class M, int STRIDE>
+__device__ __forceinline__ void block_movements(const float4* srow, int warp, int warps, BlockState<M>& B) {
     const DevTables<M>& T = tab<M>();
     const int lane = threadIdx.x & 31, sg = lane / kSegment;
-    const float4* mine = srow + lane * NS;
-    const float4* mid = srow + ((lane & ~(kSegment - 1)) + kSegMid) * NS;
-    for (int g = warp; g < G; g += warps) {
-        float b = dist2(mine[g], mid[g]), l = 0.0f;
-        const int end = T.leaf_begin[g + 1];
+    const float4* mine = srow + lane * STRIDE;
+    const float4* mid = srow + ((lane & ~(kSegment - 1)) + kSegMid) * STRIDE;
+    auto reduce = [&](float v) {
+#pragma unroll
+        for (int o = 1; o < kSegment; o <<= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
+        return v;
+    };
+    const bool lead = (lane & (kSegment - 1)) == 0;
+    if constexpr (groups_are_rigid<M>()) {  // a group's spheres are one frame's and contiguous in the row
+        constexpr int G = M::num_env_groups;
+        for (int g = warp; g < G; g += warps) {
+            const float b = reduce(dist2(mine[g], mid[g]));
+            float l = 0.0f;
+            const int end = T.leaf_begin[g + 1];
 #pragma unroll 4
-        for (int i = T.leaf_begin[g]; i < end; ++i) l = fmaxf(l, dist2(mine[G + i], mid[G + i]));
-#pragma unroll
-        for (int o = 1; o < kSegment; o <<= 1) {
-            b = fmaxf(b, __shfl_xor_sync(kFull, b, o));
-            l = fmaxf(l, __shfl_xor_sync(kFull, l, o));
+            for (int i = T.leaf_begin[g]; i < end; ++i) l = fmaxf(l, dist2(mine[G + i], mid[G + i]));
+            l = reduce(l);
+            if (lead) {
+                B.bound2[g][sg] = b;
+                atomicMax(&B.move2[T.frame_at[g]][sg], __float_as_int(fmaxf(b, l)));
+            }
         }
-        if ((lane & (kSegment - 1)) == 0) {
-            if (seg)
-                seg[((size_t)base / kSegment + sg) * G + g] =
-                    make_float2(sqrtf(b) * 1.00001f + T.sphere_radius[g] + kEnvInflate + T.cull_pad[g] + kSegMargin,
-                                sqrtf(l) * 1.00001f + kSegMargin);
-            atomicMax(&B.move2[T.frame_at[g]][sg], __float_as_int(fmaxf(b, l)));
+        for (int p = G + M::num_env_leaves + warp; p < M::num_spheres; p += warps) {
+            const float d = reduce(dist2(mine[p], mid[p]));
+            if (lead) atomicMax(&B.move2[T.frame_at[p]][sg], __float_as_int(d));
         }
-    }
-    for (int p = G + M::num_env_leaves + warp; p < NS; p += warps) {
-        float d = dist2(mine[p], mid[p]);
-#pragma unroll
-        for (int o = 1; o < kSegment; o <<= 1) d = fmaxf(d, __shfl_xor_sync(kFull, d, o));
-        if ((lane & (kSegment - 1)) == 0) atomicMax(&B.move2[T.frame_at[p]][sg], __float_as_int(d));
+    } else {
+        for (int f = 0; f <= M::dof; ++f) {
+            const int begin = T.fk_begin[f] + warp, end = T.fk_begin[f + 1];
+            if (begin >= end) continue;
+            float d = 0.0f;
+#pragma unroll 4
+            for (int i = begin; i < end; i += warps) d = fmaxf(d, dist2(mine[T.fk[i].pos], mid[T.fk[i].pos]));
+            d = reduce(d);
+            if (lead) atomicMax(&B.move2[f][sg], __float_as_int(d));
+        }
+        for (int g = warp; g < M::num_env_groups; g += warps) {
+            const float b = reduce(dist2(mine[g], mid[g]));
+            if (lead) B.bound2[g][sg] = b;
+        }
     }
 }
 
@@ -471,35 +462,55 @@ __device__ __forceinline__ void segment_spheres(const float4* srow, int base, in
 // middle sample, the leaves of either side that stay clear of the other side's
 // bound over the whole segment (that bound grown by its containment pad and by
 // what both frames move), then the pairs that stay clear of each other; the
-// surviving pairs are tested at the segment's eight samples.  Other groups test
-// their whole pair list at each sample.
-template <class M>
+// surviving pairs are tested at the segment's eight samples.  Other groups drop
+// pairs only.
+template <class M, int STRIDE>
 __device__ __forceinline__ bool self_item_hit(const float4* srow, int item, const BlockState<M>& B, uint8_t (*list)[32],
                                               uint8_t (*pair)[2]) {
-    constexpr int NS = M::num_spheres;
     const DevTables<M>& T = tab<M>();
     const DevTables<M>& L = lane_tab<M>();
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int g = item / kBlockSegs, sg = item - g * kBlockSegs;
-    const float4* rows = srow + sg * kSegment * NS;
-    const float4* mid = rows + kSegMid * NS;
+    const float4* rows = srow + sg * kSegment * STRIDE;
+    const float4* mid = rows + kSegMid * STRIDE;
     const int b0 = T.self_bound[g][0], b1 = T.self_bound[g][1];
     // leaf pair (x, y) at sample k of the segment, counted where the bounds overlap
     auto hit_at = [&](int k, int x, int y) {
-        const float4* r = rows + k * NS;
+        const float4* r = rows + k * STRIDE;
         return self_hit(r[x], r[y]) && self_hit(r[b0], r[b1]);
     };
+    auto move_of = [&](int frame) { return sqrtf(__int_as_float(B.move2[frame][sg])) * 1.00001f; };
+    // 32 leaf pairs (x, y), `near` marking those within reach of each other over the
+    // segment: all of its samples.
+    auto expand = [&](bool near, int x, int y) {
+        const unsigned nm = __ballot_sync(kFull, near);
+        if (near) {
+            uint8_t* d = pair[__popc(nm & lt)];
+            d[0] = (uint8_t)x;
+            d[1] = (uint8_t)y;
+        }
+        __syncwarp();
+        const int n = __popc(nm) * kSegment;
+        bool hit = false;
+        for (int q = lane; q - lane < n && !hit; q += 32) {
+            const uint8_t* d = pair[min(q, n - 1) / kSegment];
+            hit = __any_sync(kFull, q < n && hit_at(q & (kSegment - 1), d[0], d[1]));
+        }
+        __syncwarp();
+        return hit;
+    };
     if (!T.self_prod[g]) {
-        const int k0 = T.self_pair_begin[g], m = (T.self_pair_begin[g + 1] - k0) * kSegment;
-        for (int t = lane; t - lane < m; t += 32) {
-            const int k = k0 + min(t, m - 1) / kSegment;
-            if (__any_sync(kFull, t < m && hit_at(t & (kSegment - 1), L.self_pairs[k][0], L.self_pairs[k][1]))) return true;
+        const int k0 = T.self_pair_begin[g], m = T.self_pair_begin[g + 1] - k0;
+        for (int t0 = 0; t0 < m; t0 += 32) {
+            const int k = k0 + min(t0 + lane, m - 1);
+            const int x = L.self_pairs[k][0], y = L.self_pairs[k][1];
+            const float move = move_of(L.frame_at[x]) + move_of(L.frame_at[y]);
+            if (expand(t0 + lane < m && self_hit_pad(mid[x], mid[y], move + kSegMargin), x, y)) return true;
         }
         return false;
     }
-    const float move = sqrtf(__int_as_float(B.move2[T.self_frame[g][0]][sg])) * 1.00001f +
-                       sqrtf(__int_as_float(B.move2[T.self_frame[g][1]][sg])) * 1.00001f;
+    const float move = move_of(T.self_frame[g][0]) + move_of(T.self_frame[g][1]);
     const int a0 = T.self_la_begin[g], na = T.self_la_begin[g + 1] - a0;
     const int c0 = T.self_lb_begin[g], nb = T.self_lb_begin[g + 1] - c0;
     const float4 ba = mid[b0], bb = mid[b1];
@@ -513,27 +524,13 @@ __device__ __forceinline__ bool self_item_hit(const float4* srow, int item, cons
     __syncwarp();
     const int cb = __popc(mb), m = __popc(ma) * cb;
     const float inv = __frcp_rn((float)cb);
-    bool hit = false;
-    for (int t0 = 0; t0 < m && !hit; t0 += 32) {
+    for (int t0 = 0; t0 < m; t0 += 32) {
         const int t = min(t0 + lane, m - 1);
         const int i = (int)(((float)t + 0.5f) * inv);  // t / cb, exact: t < 1024, cb <= 32
         const int x = list[0][i], y = list[1][t - i * cb];
-        const bool near = t0 + lane < m && self_hit_pad(mid[x], mid[y], move + kSegMargin);
-        const unsigned nm = __ballot_sync(kFull, near);
-        if (near) {
-            uint8_t* d = pair[__popc(nm & lt)];
-            d[0] = (uint8_t)x;
-            d[1] = (uint8_t)y;
-        }
-        __syncwarp();
-        const int n = __popc(nm) * kSegment;
-        for (int q = lane; q - lane < n && !hit; q += 32) {
-            const uint8_t* d = pair[min(q, n - 1) / kSegment];
-            hit = __any_sync(kFull, q < n && hit_at(q & (kSegment - 1), d[0], d[1]));
-        }
-        __syncwarp();
+        if (expand(t0 + lane < m && self_hit_pad(mid[x], mid[y], move + kSegMargin), x, y)) return true;
     }
-    return hit;
+    return false;
 }
 
 // Edge of table row `row` (the last e with offs[e] <= row), whole warp: each
@@ -551,12 +548,13 @@ __device__ __forceinline__ int edge_of_row(const int* __restrict__ offs, int E, 
     return lo;
 }
 
-// Row-major tables (tile 1): a CTA of four warps computes 32 consecutive rows
+// FK: a CTA of four (or eight) warps computes 32 consecutive rows
 // (one edge's: every edge has 32 n rows and starts on a multiple of 32) into
-// shared memory, lane l row l.  Each warp evaluates the joints it needs and a
-// quarter of the spheres; the 32 rows leave as one bulk copy, the shared layout
-// being the table's.  While it runs the warps share out the segments' spheres
-// and the self-collision check: one thread per (self group, segment) tests the
+// shared memory, lane l row l.  The warps share out the joints' sines and cosines,
+// then each evaluates the frames and its share of every frame's spheres; the rows
+// leave as one bulk copy (a row length that is odd makes the shared layout the
+// table's; else a copy a row).  While it runs the warps share out the segments'
+// spheres and the self-collision check: one thread per (self group, segment) tests the
 // bounds at the segment's middle sample, grown by what their frames move within
 // it, and the warps take the items that leaves (self_item_hit).  The CTA strides
 // over 32-row blocks.  Shared memory (39 KB for Panda) holds five CTAs an SM, and
@@ -566,97 +564,134 @@ __device__ __forceinline__ int edge_of_row(const int* __restrict__ offs, int E, 
 // alone gave 0.352 (the code, several times the instruction cache, was read once
 // per warp), sphere and joint tables read in loops and the self check by segments
 // 0.194 ms: 9 650 instructions a block, half of the issue slots.
-constexpr int kFkWarps = 4;
+// Robots with wide rows fit three CTAs an SM: eight warps each (Fetch 0.225 ms at
+// four, 0.182 at eight; Baxter 0.297, 0.270), against Panda's four (0.194; eight
+// 0.217).  One coordinate of half of the frames per warp, a sixth of the FP64
+// multiply-adds, was slower (Fetch 0.239, Baxter 0.398): its scalar stores conflict.
+template <class M>
+constexpr int fk_warps() {
+    return M::fk_precision == 64 ? 8 : 4;
+}
+// CTAs an SM the rows leave room for: the register budget the kernel is compiled to.
+template <class M>
+constexpr int fk_ctas() {
+    return 200 * 1024 / (32 * (M::num_spheres | 1) * 16);
+}
 
-// Frame FR's spheres, every kFkWarps-th from `warp`, into the row at out (fk_x_first).
+// Frame FR's spheres, every fk_warps-th from `warp`, into the row at out (fk_x_first).
 template <class M, int FR>
-__device__ __forceinline__ void emit_listed(const Frames<M, float>& F, int warp, float4* out) {
+__device__ __forceinline__ void emit_listed(const Frames<M, FkReal<M>>& F, int warp, float4* out) {
     const DevTables<M>& T = tab<M>();
-    const float* R = F.R[FR];
-    const float* p = F.p[FR];
+    const FkReal<M>* R = F.R[FR];
+    const FkReal<M>* p = F.p[FR];
     const int begin = T.fk_begin[FR], mid = T.fk_x_end[FR], end = T.fk_begin[FR + 1];
+    if constexpr (M::fk_precision == 32) {
 #pragma unroll 2
-    for (int i = begin + warp; i < mid; i += kFkWarps) {
-        const float4 l = T.fk_local[i];
-        float4 c;
-        c.x = __fadd_rn(__fmaf_rn(R[2], l.z, __fmaf_rn(R[1], l.y, __fmul_rn(R[0], l.x))), p[0]);
-        c.y = __fadd_rn(__fmaf_rn(R[5], l.z, __fmaf_rn(R[4], l.y, __fmul_rn(R[3], l.x))), p[1]);
-        c.z = __fadd_rn(__fmaf_rn(R[8], l.z, __fmaf_rn(R[7], l.y, __fmul_rn(R[6], l.x))), p[2]);
-        c.w = l.w;
-        out[T.fk_pos[i]] = c;
-    }
+        for (int i = begin + warp; i < mid; i += fk_warps<M>()) {
+            const auto l = T.fk[i];
+            float4 c;
+            c.x = __fadd_rn(__fmaf_rn(R[2], l.z, __fmaf_rn(R[1], l.y, __fmul_rn(R[0], l.x))), p[0]);
+            c.y = __fadd_rn(__fmaf_rn(R[5], l.z, __fmaf_rn(R[4], l.y, __fmul_rn(R[3], l.x))), p[1]);
+            c.z = __fadd_rn(__fmaf_rn(R[8], l.z, __fmaf_rn(R[7], l.y, __fmul_rn(R[6], l.x))), p[2]);
+            c.w = l.r;
+            out[l.pos] = c;
+        }
 #pragma unroll 2
-    for (int i = mid + warp; i < end; i += kFkWarps) {
-        const float4 l = T.fk_local[i];
-        float4 c;
-        c.x = __fadd_rn(__fmaf_rn(R[2], l.z, __fmaf_rn(R[0], l.x, __fmul_rn(R[1], l.y))), p[0]);
-        c.y = __fadd_rn(__fmaf_rn(R[5], l.z, __fmaf_rn(R[3], l.x, __fmul_rn(R[4], l.y))), p[1]);
-        c.z = __fadd_rn(__fmaf_rn(R[8], l.z, __fmaf_rn(R[6], l.x, __fmul_rn(R[7], l.y))), p[2]);
-        c.w = l.w;
-        out[T.fk_pos[i]] = c;
+        for (int i = mid + warp; i < end; i += fk_warps<M>()) {
+            const auto l = T.fk[i];
+            float4 c;
+            c.x = __fadd_rn(__fmaf_rn(R[2], l.z, __fmaf_rn(R[0], l.x, __fmul_rn(R[1], l.y))), p[0]);
+            c.y = __fadd_rn(__fmaf_rn(R[5], l.z, __fmaf_rn(R[3], l.x, __fmul_rn(R[4], l.y))), p[1]);
+            c.z = __fadd_rn(__fmaf_rn(R[8], l.z, __fmaf_rn(R[6], l.x, __fmul_rn(R[7], l.y))), p[2]);
+            c.w = l.r;
+            out[l.pos] = c;
+        }
+    } else {  // FP64: the order is far below the rounding to float
+#pragma unroll 2
+        for (int i = begin + warp; i < end; i += fk_warps<M>()) {
+            const auto l = T.fk[i];
+            float4 c;
+            c.x = (float)(R[0] * l.x + R[1] * l.y + R[2] * l.z + p[0]);
+            c.y = (float)(R[3] * l.x + R[4] * l.y + R[5] * l.z + p[1]);
+            c.z = (float)(R[6] * l.x + R[7] * l.y + R[8] * l.z + p[2]);
+            c.w = l.r;
+            out[l.pos] = c;
+        }
     }
 }
 
-// Joints K, K + 1, ... of one row from their values and sines and cosines (sc[k]
-// at [k * 32]), the warp's share of every frame's spheres.
+// Joints K, K + 1, ... of one row from their values (q[k * 32]) and sines and
+// cosines, the warp's share of every frame's spheres.
 template <class M, int K>
-__device__ __forceinline__ void fk_rows(const float* q, const float2* sc, Frames<M, float>& F, int warp, float4* out) {
+__device__ __forceinline__ void fk_rows(const float* q, const FkReal<M>* sn, const FkReal<M>* cs,
+                                        Frames<M, FkReal<M>>& F, int warp, float4* out) {
     if constexpr (K == 0) {
-        fk_base<M, float>(F);
+        fk_base<M, FkReal<M>>(F);
         emit_listed<M, 0>(F, warp, out);
     }
     if constexpr (K < M::dof) {
-        fk_advance<M, K, float>(q[K * 32], sc[K * 32].x, sc[K * 32].y, F);
+        fk_advance<M, K, FkReal<M>>((FkReal<M>)q[K * 32], sn[K * 32], cs[K * 32], F);
         emit_listed<M, K + 1>(F, warp, out);
-        fk_rows<M, K + 1>(q, sc, F, warp, out);
+        fk_rows<M, K + 1>(q, sn, cs, F, warp, out);
     }
 }
 
 template <class M>
-__global__ void __launch_bounds__(32 * kFkWarps) fk_staged_kernel(const float* __restrict__ edges, int E,
+__global__ void __launch_bounds__(32 * fk_warps<M>(), fk_ctas<M>()) fk_staged_kernel(const float* __restrict__ edges, int E,
                                                                   const int* __restrict__ steps,
                                                                   const int* __restrict__ offs,
                                                                   float4* __restrict__ table,
                                                                   int* __restrict__ edge_self,
                                                                   float2* __restrict__ seg) {
-    static_assert(M::table_tile == 1 && M::num_spheres % 2 == 1,
-                  "row-major table whose odd row length is a conflict-free stride");
-    constexpr int NS = M::num_spheres;
-    extern __shared__ __align__(128) float4 srow[];  // [32][NS]
+    constexpr int NS = M::num_spheres, STRIDE = NS | 1;  // conflict-free
+    constexpr int G = M::num_env_groups;
+    extern __shared__ __align__(128) float4 srow[];  // [32][STRIDE]
     __shared__ BlockState<M> B;
-    __shared__ uint8_t s_list[kFkWarps][2][32], s_pair[kFkWarps][32][2];
+    __shared__ uint8_t s_list[fk_warps<M>()][2][32], s_pair[fk_warps<M>()][32][2];
     __shared__ float s_q[M::dof][32];
-    __shared__ float2 s_sc[M::dof][32];
+    __shared__ FkReal<M> s_sin[M::dof][32], s_cos[M::dof][32];
     const DevTables<M>& L = lane_tab<M>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int total = offs[E];
     for (int base = blockIdx.x * 32; base < total; base += gridDim.x * 32) {
         const int e = edge_of_row(offs, E, base);
-        {
-            const int n = steps[e], k = base + lane - offs[e];
-            const float* ends = edges + (size_t)e * 2 * M::dof;
+        const int n = steps[e], k = base + lane - offs[e];
+        const float* ends = edges + (size_t)e * 2 * M::dof;
 #pragma unroll 1
-            for (int j = warp; j < M::dof; j += kFkWarps) {
-                const float v = edge_sample_joint(ends[j], ends[M::dof + j], n, k);
-                s_q[j][lane] = v;
-                sin_cos(v, &s_sc[j][lane].x, &s_sc[j][lane].y);
-            }
-            __syncthreads();
-            Frames<M, float> F;
-            fk_rows<M, 0>(&s_q[0][lane], &s_sc[0][lane], F, warp, srow + lane * NS);
+        for (int j = warp; j < M::dof; j += fk_warps<M>()) {
+            const float v = edge_sample_joint(ends[j], ends[M::dof + j], n, k);
+            s_q[j][lane] = v;
+            sin_cos((FkReal<M>)v, &s_sin[j][lane], &s_cos[j][lane]);
+        }
+        __syncthreads();
+        {
+            Frames<M, FkReal<M>> F;
+            fk_rows<M, 0>(&s_q[0][lane], &s_sin[0][lane], &s_cos[0][lane], F, warp, srow + lane * STRIDE);
         }
         if (threadIdx.x < (M::dof + 1) * kBlockSegs) (&B.move2[0][0])[threadIdx.x] = 0;
         if (threadIdx.x == 0) B.num_items = 0;
         fence_async_shared();
         __syncthreads();
-        if (threadIdx.x == 0) bulk_copy_s2g(table + (size_t)base * NS, srow, 32 * NS * sizeof(float4));
-        segment_spheres<M>(srow, base, warp, kFkWarps, B, seg);
+        const bool copies = STRIDE == NS ? threadIdx.x == 0 : threadIdx.x < 32;
+        if (STRIDE == NS) {
+            if (copies) bulk_copy_s2g(table + (size_t)base * NS, srow, 32 * NS * sizeof(float4));
+        } else if (copies) {
+            bulk_copy_s2g(table + (size_t)(base + lane) * NS, srow + lane * STRIDE, NS * sizeof(float4));
+        }
+        block_movements<M, STRIDE>(srow, warp, fk_warps<M>(), B);
         __syncthreads();
+        if (seg)
+            for (int i = threadIdx.x; i < G * kBlockSegs; i += 32 * fk_warps<M>()) {
+                const int sg = i / G, g = i - sg * G;  // consecutive threads write consecutive entries
+                const float r = sqrtf(B.bound2[g][sg]) * 1.00001f + L.seg_pad[g];
+                const float move = sqrtf(__int_as_float(B.move2[L.frame_at[g]][sg])) * 1.00001f + kSegMargin;
+                seg[(size_t)base / kSegment * G + i] = make_float2(r, move);
+            }
         // any hit marks the edge; skipped when another block or warp already has
         if (*(volatile const int*)(edge_self + e) == 0) {
-            for (int i = threadIdx.x; i < M::num_self_groups * kBlockSegs; i += 32 * kFkWarps) {
+            for (int i = threadIdx.x; i < M::num_self_groups * kBlockSegs; i += 32 * fk_warps<M>()) {
                 const int g = i / kBlockSegs, sg = i - g * kBlockSegs;
-                const float4* mid = srow + (sg * kSegment + kSegMid) * NS;
+                const float4* mid = srow + (sg * kSegment + kSegMid) * STRIDE;
                 const float move = sqrtf(__int_as_float(B.move2[L.self_frame[g][0]][sg])) +
                                    sqrtf(__int_as_float(B.move2[L.self_frame[g][1]][sg]));
                 if (self_hit_pad(mid[L.self_bound[g][0]], mid[L.self_bound[g][1]], move * 1.00001f + kSegMargin))
@@ -664,84 +699,15 @@ __global__ void __launch_bounds__(32 * kFkWarps) fk_staged_kernel(const float* _
             }
         }
         __syncthreads();
-        for (int i = warp; i < B.num_items; i += kFkWarps)
-            if (self_item_hit<M>(srow, B.items[i], B, s_list[warp], s_pair[warp])) {
+        for (int i = warp; i < B.num_items; i += fk_warps<M>())
+            if (self_item_hit<M, STRIDE>(srow, B.items[i], B, s_list[warp], s_pair[warp])) {
                 if (lane == 0) atomicOr(edge_self + e, 1);
                 break;
             }
-        if (threadIdx.x == 0) bulk_wait_read();
+        if (copies) bulk_wait_read();
         __syncthreads();  // the next block overwrites srow
     }
-    if (threadIdx.x == 0) bulk_wait();
-}
-
-// ------------------------------------------------------------------ 4. self
-
-// Self-collision of one sample row, by one warp (sphere s at sp[s * stride]).
-// Lanes test the self groups' bound pairs 32 at a time; the leaf pairs of
-// every group whose bound pair hit are then tested 32 at a time (the
-// reference's gate-then-leaves, any hit = self-collision).  The tables are in
-// shared memory: lanes read different entries, which constant memory would
-// serialise.  Warp-uniform result.
-template <class M>
-__device__ __forceinline__ bool self_row_hits(const float4* sp, const short (*bound)[2], const short* begin,
-                                              const unsigned char (*pairs)[2], int stride) {
-    constexpr int NG = M::num_self_groups;
-    const int lane = threadIdx.x & 31;
-    bool hit = false;
-    for (int g0 = 0; g0 < NG && !hit; g0 += 32) {
-        const int g = g0 + lane;
-        const bool gate = g < NG && self_hit(sp[bound[g][0] * stride], sp[bound[g][1] * stride]);
-        uint32_t gm = __ballot_sync(kFull, gate);
-        while (gm && !hit) {
-            const int gg = g0 + __ffs(gm) - 1;
-            gm &= gm - 1u;
-            const int end = begin[gg + 1];
-            for (int k0 = begin[gg]; k0 < end && !hit; k0 += 32) {  // warp-uniform trip count
-                const int k = k0 + lane;
-                const bool h = k < end && self_hit(sp[pairs[k][0] * stride], sp[pairs[k][1] * stride]);
-                hit = __any_sync(kFull, h);
-            }
-        }
-    }
-    return hit;
-}
-
-// One warp per sample row (robots with tiled tables; row-major tables are
-// checked inside fk_staged_kernel), rows strided over the grid, each row by
-// self_row_hits.  Rows of an edge already known to self-collide are skipped.
-constexpr int kSelfThreads = 256;
-
-template <class M>
-__global__ void __launch_bounds__(kSelfThreads) self_kernel(const float4* __restrict__ table, int total,
-                                                             const int* __restrict__ row_edge,
-                                                             int* __restrict__ edge_self) {
-    constexpr int NG = M::num_self_groups;
-    constexpr int NP = M::num_self_pairs;
-    __shared__ short s_bound[NG][2];
-    __shared__ short s_begin[NG + 1];
-    __shared__ unsigned char s_pairs[NP][2];
-    const DevTables<M>& T = tab<M>();
-    for (int i = threadIdx.x; i < NG; i += blockDim.x) {
-        s_bound[i][0] = (short)T.self_bound[i][0];
-        s_bound[i][1] = (short)T.self_bound[i][1];
-    }
-    for (int i = threadIdx.x; i <= NG; i += blockDim.x) s_begin[i] = (short)T.self_pair_begin[i];
-    for (int i = threadIdx.x; i < NP; i += blockDim.x) {
-        s_pairs[i][0] = T.self_pairs[i][0];
-        s_pairs[i][1] = T.self_pairs[i][1];
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < total; row += warps) {
-        const int e = row_edge[row];
-        int decided = lane == 0 ? *(volatile const int*)(edge_self + e) : 0;
-        if (__shfl_sync(kFull, decided, 0)) continue;  // another row already found a self-collision
-        const float4* sp = table + table_index<M>(row, 0);  // sphere s at sp[s * M::table_tile]
-        const bool hit = self_row_hits<M>(sp, s_bound, s_begin, s_pairs, M::table_tile);
-        if (hit && lane == 0) atomicOr(edge_self + e, 1);
-    }
+    if (threadIdx.x < 32) bulk_wait();
 }
 
 // ------------------------------------------------------------------ 5. swept
@@ -769,14 +735,12 @@ __device__ __forceinline__ int slab_tri(float lo, float hi, const float* __restr
 // and (mid non-null) the bound's centre at the edge's middle sample with the
 // radius, inflated likewise, of the sphere around it that holds them all; and
 // (seg non-null, tiled tables) the segments' spheres (see segment_spheres).
-// Lane g ends up holding group g's box.  Row-major tables: lane g scans group
-// g's bound down the rows (a row's bounds are contiguous).  Tiled tables: the
-// lanes scan 32 rows of one group at a time (contiguous in a tile) and a
-// butterfly reduction hands the box to lane g.
+// Lane g ends up holding group g's box: it scans group g's bound down the rows (a
+// row's bounds are contiguous), 32 / G rows at a time.
 template <class M>
 __global__ void swept_kernel(const float4* __restrict__ table, const int* __restrict__ offs, int E,
                              float4* __restrict__ swept, int* __restrict__ edge_tri,
-                             const float* __restrict__ bounds, float4* __restrict__ mid, float2* __restrict__ seg) {
+                             const float* __restrict__ bounds, float4* __restrict__ mid) {
     constexpr int G = M::num_env_groups;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -786,73 +750,28 @@ __global__ void swept_kernel(const float4* __restrict__ table, const int* __rest
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     float far2 = 0.0f;  // largest squared distance of the bound's centre from its middle one
     const int rm = r0 + ((r1 - r0) >> 1);
-    if constexpr (M::table_tile == 1) {
-        // 32 / G row streams: lane s G + g scans group g's bound on rows
-        // r0 + s, r0 + s + 32 / G, ... (bounds lead every table row); lane g then
-        // folds in the other streams' boxes.
-        constexpr int RS = kLanes / G;
-        const int rs = lane / G, gl = lane - rs * G;
-        if (rs < RS) {
-            const float4 m = table[table_index<M>(rm, gl)];
-            for (int r = r0 + rs; r < r1; r += RS) {
-                const float4 c = table[table_index<M>(r, gl)];
-                far2 = fmaxf(far2, dist2(c, m));
-                lo[0] = fminf(lo[0], c.x); lo[1] = fminf(lo[1], c.y); lo[2] = fminf(lo[2], c.z);
-                hi[0] = fmaxf(hi[0], c.x); hi[1] = fmaxf(hi[1], c.y); hi[2] = fmaxf(hi[2], c.z);
-            }
+    // 32 / G row streams: lane s G + g scans group g's bound on rows
+    // r0 + s, r0 + s + 32 / G, ... (bounds lead every table row); lane g then
+    // folds in the other streams' boxes.
+    constexpr int RS = kLanes / G;
+    const int rs = lane / G, gl = lane - rs * G;
+    if (rs < RS) {
+        const float4 m = table[table_index<M>(rm, gl)];
+        for (int r = r0 + rs; r < r1; r += RS) {
+            const float4 c = table[table_index<M>(r, gl)];
+            far2 = fmaxf(far2, dist2(c, m));
+            lo[0] = fminf(lo[0], c.x); lo[1] = fminf(lo[1], c.y); lo[2] = fminf(lo[2], c.z);
+            hi[0] = fmaxf(hi[0], c.x); hi[1] = fmaxf(hi[1], c.y); hi[2] = fmaxf(hi[2], c.z);
         }
+    }
 #pragma unroll
-        for (int t = 1; t < RS; ++t) {
-            const int src = min(lane + t * G, kLanes - 1);  // lanes >= G read a valid lane and discard it
-            far2 = fmaxf(far2, __shfl_sync(kFull, far2, src));
+    for (int t = 1; t < RS; ++t) {
+        const int src = min(lane + t * G, kLanes - 1);  // lanes >= G read a valid lane and discard it
+        far2 = fmaxf(far2, __shfl_sync(kFull, far2, src));
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = fminf(lo[a], __shfl_sync(kFull, lo[a], src));
-                hi[a] = fmaxf(hi[a], __shfl_sync(kFull, hi[a], src));
-            }
-        }
-    } else {
-        for (int g = 0; g < G; ++g) {
-            float l3[3] = {INFINITY, INFINITY, INFINITY}, h3[3] = {-INFINITY, -INFINITY, -INFINITY};
-            const float4 m = table[table_index<M>(rm, g)];
-            float f2 = 0.0f;
-            for (int r = r0 + lane; r < r1; r += 32) {
-                const float4 c = table[table_index<M>(r, g)];
-                f2 = fmaxf(f2, dist2(c, m));
-                if (seg) {  // rows r0 + 32 i: eight lanes hold a segment
-                    const int src = (lane & ~(kSegment - 1)) + kSegMid;
-                    float4 s;
-                    s.x = __shfl_sync(kFull, c.x, src);
-                    s.y = __shfl_sync(kFull, c.y, src);
-                    s.z = __shfl_sync(kFull, c.z, src);
-                    float d = dist2(c, s);
-#pragma unroll
-                    for (int o = 1; o < kSegment; o <<= 1) d = fmaxf(d, __shfl_xor_sync(kFull, d, o));
-                    if ((lane & (kSegment - 1)) == 0)
-                        seg[(size_t)(r / kSegment) * G + g] =
-                            make_float2(sqrtf(d) * 1.00001f + T.sphere_radius[g] + kEnvInflate + T.cull_pad[g] +
-                                            kSegMargin, 0.0f);
-                }
-                l3[0] = fminf(l3[0], c.x); l3[1] = fminf(l3[1], c.y); l3[2] = fminf(l3[2], c.z);
-                h3[0] = fmaxf(h3[0], c.x); h3[1] = fmaxf(h3[1], c.y); h3[2] = fmaxf(h3[2], c.z);
-            }
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                f2 = fmaxf(f2, __shfl_xor_sync(kFull, f2, o));
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    l3[a] = fminf(l3[a], __shfl_xor_sync(kFull, l3[a], o));
-                    h3[a] = fmaxf(h3[a], __shfl_xor_sync(kFull, h3[a], o));
-                }
-            }
-            if (lane == g) {
-                far2 = f2;
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    lo[a] = l3[a];
-                    hi[a] = h3[a];
-                }
-            }
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(lo[a], __shfl_sync(kFull, lo[a], src));
+            hi[a] = fmaxf(hi[a], __shfl_sync(kFull, hi[a], src));
         }
     }
     if (lane >= G) return;
@@ -1177,10 +1096,11 @@ __device__ __forceinline__ bool walk_segments(const CheckParams& P, size_t row0,
     constexpr int GB = group_bits<M>();
     constexpr bool kOver = has_overhang<M>();
     static_assert(kSegment == 8, "segments are expanded eight lanes an item");
+    static_assert(kOver || groups_are_rigid<M>(), "a leaf moves no further than its group's frame");
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int S = kLanes / kSegment * n;
-    const float4* __restrict__ rows = P.table + table_index<M>(row0, 0);  // row0 starts a tile
+    const float4* __restrict__ rows = P.table + table_index<M>(row0, 0);
     const float2* __restrict__ segs = P.seg + row0 / kSegment * G;
     // a / C in FP32, exact (walk_pairs)
     const float inv_c = __frcp_rn((float)C);
@@ -2235,8 +2155,7 @@ __global__ void queue_features_kernel(CheckParams P, const float* __restrict__ e
 // code of environment cluster c.  One thread per row.
 template <class M>
 __global__ void cluster_features_kernel(CheckParams P, const float* __restrict__ edges,
-                                        const float* __restrict__ centroids, int K, const int* __restrict__ row_edge,
-                                        uint16_t* __restrict__ x) {
+                                        const float* __restrict__ centroids, int K, uint16_t* __restrict__ x) {
     const long long S = P.total_segs;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= S * K) return;
@@ -2251,7 +2170,6 @@ __global__ void cluster_features_kernel(CheckParams P, const float* __restrict__
         if (P.offs[mid] <= row) lo = mid; else hi = mid - 1;
     }
     const int e = lo;
-    (void)row_edge;
     const int j = sg - P.offs[e] / kSegment;
     float s[M::dof], t[M::dof], q[M::dof];
 #pragma unroll
@@ -2303,16 +2221,16 @@ __device__ __forceinline__ bool sample_hits_env(const CheckParams& P, int env, s
     const float4 hd0 = P.env_hdr[2 * env], hd1 = P.env_hdr[2 * env + 1];
     const float4* rec = P.blobs + __float_as_uint(hd0.w);
     const int np = (int)(__float_as_uint(hd1.w) & 0xffffu);
-    const float4* r = P.table + table_index<M>(row, 0);  // sphere s at r[s * M::table_tile]
+    const float4* r = P.table + table_index<M>(row, 0);
     const DevTables<M>& T = tab<M>();
     for (int g = 0; g < G; ++g) {
-        float4 b = r[g * M::table_tile];
+        float4 b = r[g];
         b.w += kEnvInflate;
         bool gate = false;
         for (int p = 0; p < np && !gate; ++p) gate = sphere_hits_prim(b, rec + p * kPrimF4);
         if (!gate) continue;
         for (int li = T.leaf_begin[g]; li < T.leaf_begin[g + 1]; ++li) {
-            float4 l = r[(G + li) * M::table_tile];
+            float4 l = r[G + li];
             l.w += kEnvInflate;
             for (int p = 0; p < np; ++p)
                 if (sphere_hits_prim(l, rec + p * kPrimF4)) return true;
@@ -2567,41 +2485,24 @@ cudaError_t run_prep(const PipelineArgs& a, cudaStream_t st) {
     cudaError_t err = cudaMemsetAsync(a.edge_self, 0, sizeof(int) * E, st);
     if (err != cudaSuccess) return err;
     if (R > 0) {
-        if constexpr (M::table_tile == 1) {
-            // FK and self-collision in one kernel; a grid of the resident CTAs
-            // strides over the 32-row blocks
-            const size_t smem = 32 * (size_t)M::num_spheres * sizeof(float4);
-            err = cudaFuncSetAttribute(fk_staged_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (err != cudaSuccess) return err;
-            int dev = 0, sms = 0, per_sm = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk_staged_kernel<M>, 32 * kFkWarps, smem);
-            if (err != cudaSuccess) return err;
-            const int blocks = (R + 31) / 32;
-            const int grid = std::min(blocks, std::max(per_sm, 1) * std::max(sms, 1));
-            fk_staged_kernel<M><<<grid, 32 * kFkWarps, smem, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.edge_self,
-                                                                   a.seg);
-        } else {
-            fk_kernel<M><<<(R + 127) / 128, 128, 0, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.row_edge);
-        }
+        // FK and self-collision in one kernel; a grid of the resident CTAs strides
+        // over the 32-row blocks
+        const size_t smem = 32 * (size_t)(M::num_spheres | 1) * sizeof(float4);
+        err = cudaFuncSetAttribute(fk_staged_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (err != cudaSuccess) return err;
+        int dev = 0, sms = 0, per_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fk_staged_kernel<M>, 32 * fk_warps<M>(), smem);
+        if (err != cudaSuccess) return err;
+        const int blocks = (R + 31) / 32;
+        const int grid = std::min(blocks, std::max(per_sm, 1) * std::max(sms, 1));
+        fk_staged_kernel<M><<<grid, 32 * fk_warps<M>(), smem, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.edge_self, a.seg);
     }
     if (ev) cudaEventRecord(ev[2], st);
-    if constexpr (M::table_tile != 1) {  // row-major tables: checked by fk_staged_kernel
-        if (R > 0) {
-            // one warp per row; a grid of at most 16 CTAs per SM strides over the rows
-            int dev = 0, sms = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            const long long want = ((long long)R * 32 + kSelfThreads - 1) / kSelfThreads;
-            const int grid = (int)std::min<long long>(want, 16ll * std::max(sms, 1));
-            self_kernel<M><<<grid, kSelfThreads, 0, st>>>(a.table, R, a.row_edge, a.edge_self);
-        }
-    }
     if (ev) cudaEventRecord(ev[3], st);
     swept_kernel<M><<<(E * 32 + 255) / 256, 256, 0, st>>>(a.table, a.offs, E, a.swept,
-                                                           a.grid_bounds ? a.edge_tri : nullptr, a.grid_bounds, a.mid,
-                                                           M::table_tile == 1 ? nullptr : a.seg);
+                                                           a.grid_bounds ? a.edge_tri : nullptr, a.grid_bounds, a.mid);
     if (ev) cudaEventRecord(ev[4], st);
     return cudaGetLastError();
 }
@@ -2635,7 +2536,7 @@ cudaError_t run_cluster_order_inputs(const PipelineArgs& a, const float* centroi
     const long long rows = (long long)K * a.total_segs;
     if (rows <= 0) return cudaSuccess;
     cluster_features_kernel<M><<<(unsigned)((rows + 127) / 128), 128, 0, st>>>(params_of(a), a.d_edges, centroids, K,
-                                                                               a.row_edge, x);
+                                                                               x);
     return cudaGetLastError();
 }
 

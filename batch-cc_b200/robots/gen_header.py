@@ -33,13 +33,6 @@ LIMITS = {
 # algorithmic FLOP count.
 FK_FLOPS = {"panda": 1150, "fetch": 983, "baxter": 1792}
 
-# Rows per tile of the sample table (sphere-major inside a tile): 32 makes the FK
-# kernel's stores coalesced, 1 keeps each row contiguous for the check kernel's
-# bound and leaf reads.  Measured on B200: tiling speeds up the Fetch and Baxter
-# checks (126 / 107 spheres per row, FP64 FK) by 5-6 % and slowed Panda's (70
-# spheres at the time, a check dominated by its walk) by 6 %.
-TABLE_TILE = {"panda": 1, "fetch": 32, "baxter": 32}
-
 # Resident warps per SM the check kernel is compiled for (its register budget
 # is 65536 / (32 x this)).  Swept on B200 (uneven / multi workloads, autotuned
 # launch shapes): Panda 48 (40 registers) beats 40 and 56; Fetch's
@@ -95,8 +88,6 @@ def main():
     w("    // (32: float expressions; 64: double expressions, centres rounded to float).")
     w("    static constexpr int fk_precision = %d;" % m.get("fk_precision", 32))
     w("    static constexpr int fk_flops = %d;" % FK_FLOPS[name])
-    w("    // Sample-table rows per tile (sphere-major inside a tile; 1 = row-major).")
-    w("    static constexpr int table_tile = %d;" % TABLE_TILE[name])
     w("    // Resident warps per SM the check kernel is compiled for (register budget).")
     w("    static constexpr int check_warps_per_sm = %d;" % CHECK_WARPS_PER_SM[name])
     w("")
