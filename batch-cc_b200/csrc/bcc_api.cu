@@ -203,9 +203,15 @@ constexpr long long kProbeMinPairs = 1 << 14;
 bcc::Tune launch_shape(const bcc_ctx* ctx, int E) {
     bcc::Tune t = ctx->tune;
     if (t.tuned) return t;
-    t.persistent = (long long)ctx->num_envs * E >= kProbeMinPairs ? 1 : 0;
+    const long long pairs = (long long)ctx->num_envs * E;
+    t.persistent = pairs >= kProbeMinPairs ? 1 : 0;
+    if (!t.persistent) {  // spread few pairs over the SMs: a pass of 12 edges fills a CTA's four warps
+        t.warps = 4;
+        t.edges_per_cta = (int)std::max<long long>(12, std::min<long long>(128, pairs / (148 * 4)));
+        return t;
+    }
     // Large records leave room for fewer CTAs an SM: eight warps share one copy.
-    t.warps = t.persistent && ctx->blob_smem <= 8192 ? 4 : 8;
+    t.warps = ctx->blob_smem <= 8192 ? 4 : 8;
     return t;
 }
 
@@ -236,8 +242,8 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     BCC_CUDA(ctx, ctx->error_flag.ensure(sizeof(int)));
     // Probed checks: grids, middle spheres and the queue, all or none.
     const bcc::Tune tune = launch_shape(ctx, E);
-    if (d_results && tune.persistent && (long long)E <= bcc::kQueuePairs &&
-        ctx->blob_smem + bcc::kProbeBatch * sizeof(uint2) + 2 * bcc::kMaxVoxels <= 200 * 1024) {
+    if (d_results && tune.persistent && E <= 65535 * bcc::kProbeBatch &&
+        ctx->blob_smem + bcc::kProbeBatch * bcc::kProbeEntryBytes + 2 * bcc::kMaxVoxels <= 200 * 1024) {
         const long long cap = std::min<long long>((long long)ctx->num_envs * E, bcc::kQueuePairs);
         const long long slab = cap / E;
         // Pairs per work item: few where there are few pairs, so that the undecided
@@ -245,8 +251,14 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
         // ms, Fetch 0.43 against 0.54, Baxter 0.30 against 0.45), many where an item's
         // barriers and staging count (uneven Panda 1.39 ms at 96 against 1.64 at 12).
         const int chunk = (int)std::max<long long>(12, std::min<long long>(96, (long long)ctx->num_envs * E / 100000 / 12 * 12));
+        // Edges per probe CTA: fewer where that leaves SMs idle (plain 100 x 1000: 0.13
+        // ms at 128, 0.14 at 512, 0.18 at 1024; uneven 1000 x 10000: 1.50 at 128, 1.19
+        // at 512 and 1024; Fetch 0.40 at 512, 0.46 at 1024).
+        const long long even = (long long)ctx->num_envs * E / 740 / 32 * 32;
+        const int batch = std::max((int)std::max<long long>(128, std::min<long long>(bcc::kProbeBatch, even)),
+                                   (E + 65534) / 65535);
         // items: every full chunk, and one part chunk per probe CTA
-        const size_t items = (size_t)(cap / chunk + slab * ((E + bcc::kProbeBatch - 1) / bcc::kProbeBatch));
+        const size_t items = (size_t)(cap / chunk + slab * ((E + batch - 1) / batch));
         a.probe = probe_grid(ctx, ops, st);
         if (a.probe.vox && ctx->mid.ensure(sizeof(float4) * (size_t)G * E) == cudaSuccess &&
             ctx->pq_entries.ensure(sizeof(uint2) * (size_t)cap) == cudaSuccess &&
@@ -254,7 +266,7 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
             ctx->pq_head.ensure(16 * (size_t)((ctx->num_envs + slab - 1) / slab)) == cudaSuccess) {
             a.mid = ctx->mid.as<float4>();
             a.queue = bcc::ProbeQueue{ctx->pq_entries.as<uint2>(), ctx->pq_items.as<int4>(), ctx->pq_head.as<int>(),
-                                      cap, chunk};
+                                      cap, chunk, batch};
         } else {
             cudaGetLastError();  // no memory for it: one pass over all pairs
             a.probe = bcc::ProbeGrid{};
@@ -509,7 +521,7 @@ bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
            x.edge_self == y.edge_self && x.swept == y.swept && x.edge_tri == y.edge_tri &&
            x.grid_bounds == y.grid_bounds && x.blobs == y.blobs && x.env_hdr == y.env_hdr && x.mid == y.mid &&
            x.probe.vox == y.probe.vox && x.queue.entries == y.queue.entries && x.queue.items == y.queue.items &&
-           x.queue.head == y.queue.head && x.queue.chunk == y.queue.chunk && x.warps == y.warps &&
+           x.queue.head == y.queue.head && x.queue.chunk == y.queue.chunk && x.queue.batch == y.queue.batch && x.warps == y.warps &&
            x.edges_per_cta == y.edges_per_cta && x.q_head == y.q_head && x.q_pairs == y.q_pairs &&
            x.q_rows == y.q_rows && x.logits == y.logits && x.perms == y.perms && x.env_cluster == y.env_cluster &&
            x.features == y.features && x.work_counter == y.work_counter && x.error_flag == y.error_flag;
@@ -896,10 +908,11 @@ bcc_status bcc_check(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32_t 
     bcc_status s = run_check(ctx, robot, ctx->edges.as<float>(), num_edges, resolution,
                              ctx->results.as<uint8_t>(), opts, st);
     if (s != BCC_OK) return s;
+    // (the sample total was read before the check was launched: its word is free)
+    BCC_CUDA(ctx, cudaMemcpyAsync(ctx->h_total, ctx->error_flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     BCC_CUDA(ctx, cudaMemcpyAsync(results, ctx->results.p, rb, cudaMemcpyDeviceToHost, st));
     BCC_CUDA(ctx, cudaStreamSynchronize(st));
-    int flag = 0;
-    BCC_CUDA(ctx, cudaMemcpy(&flag, ctx->error_flag.p, sizeof(int), cudaMemcpyDeviceToHost));
+    const int flag = *ctx->h_total;
     if (flag & 4) return fail(ctx, BCC_ERR_TIMEOUT, "a walk exceeded its step bound");
     if (flag) return fail(ctx, BCC_ERR_TIMEOUT, "a bounded device wait gave up (bulk copy did not complete)");
     return BCC_OK;

@@ -179,6 +179,30 @@ __device__ __forceinline__ void fk_base(Frames<M, T>& F) {
     F.p[0][0] = F.p[0][1] = F.p[0][2] = T(0);
 }
 
+// Exclusive prefix sum of v over a CTA of 1024 threads; `total` gets the sum.
+// sums: 32 entries of shared memory, free again when the call returns.
+__device__ __forceinline__ long long block_scan_exclusive(long long v, long long* sums, long long& total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) sums[warp] = x;
+    __syncthreads();
+    long long w = sums[lane];  // every warp scans the 32 warp sums
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+    }
+    total = __shfl_sync(0xffffffffu, w, 31);
+    const long long before = __shfl_sync(0xffffffffu, w, (warp + 31) & 31);
+    __syncthreads();
+    return (warp ? before : 0) + x - v;
+}
+
 // Bounded mbarrier wait: gives up after `limit` polls and reports false.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint32_t limit) {
     const uint32_t addr = (uint32_t)__cvta_generic_to_shared(bar);

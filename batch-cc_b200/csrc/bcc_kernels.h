@@ -50,6 +50,7 @@ struct ProbeQueue {
     int* head;               // per slab: entries used, items, next item, -
     long long cap;
     int chunk;               // entries per work item
+    int batch;               // edges per probe CTA (at most kProbeBatch)
 };
 
 struct CheckParams {
@@ -161,6 +162,7 @@ struct RecordsParams {
     const int* offs;
     const float4* table;
     const float4* swept;
+    const float2* seg;
     const int* edge_self;
     uint8_t* results;
     int* error_flag;
@@ -175,8 +177,9 @@ constexpr int kRecordsWarps = 4;  // warps per CTA of the records check kernel
 // Entries of a warp's (primitive, link) pair list in shared memory; a pair with
 // more candidates is walked in segments of this many.
 constexpr int kPairCap = 1024;
-// Edges a probe CTA takes (their undecided ones are listed in shared memory).
-constexpr int kProbeBatch = 1024;
+// Most edges a probe CTA takes (their undecided ones are listed in shared memory).
+constexpr int kProbeBatch = 512;
+constexpr size_t kProbeEntryBytes = sizeof(uint2) + sizeof(unsigned);
 // Pairs a probed check takes at a time: bounds the queue (8 bytes a pair) to
 // 512 MB however many environments and edges a call has.
 constexpr long long kQueuePairs = 64ll << 20;

@@ -45,6 +45,7 @@ static __device__ __align__(256) int g_offs[kMaxEdges + 1];
 static __device__ __align__(256) int g_edge_self[kMaxEdges];
 static __device__ __align__(256) float4 g_swept[kMaxEdges * kGroupsMax * 2];
 static __device__ __align__(256) float4 g_table[kMaxRows * kNumSpheresMax];
+static __device__ __align__(256) float2 g_seg[kMaxRows / bcc::kSegment * kGroupsMax];
 static __device__ __align__(256) int g_error[1];
 
 struct Scratch {
@@ -53,6 +54,7 @@ struct Scratch {
     int* edge_self = nullptr;
     float4* swept = nullptr;
     float4* table = nullptr;
+    float2* seg = nullptr;
     int* error = nullptr;
     bool ready = false;
     bool tables[3] = {false, false, false};  // robot tables uploaded to this device
@@ -73,6 +75,7 @@ cudaError_t setup_device(int dev, const bcc::RobotOps* ops, Scratch*& out) {
         if ((e = cudaGetSymbolAddress((void**)&s.edge_self, g_edge_self)) != cudaSuccess) return e;
         if ((e = cudaGetSymbolAddress((void**)&s.swept, g_swept)) != cudaSuccess) return e;
         if ((e = cudaGetSymbolAddress((void**)&s.table, g_table)) != cudaSuccess) return e;
+        if ((e = cudaGetSymbolAddress((void**)&s.seg, g_seg)) != cudaSuccess) return e;
         if ((e = cudaGetSymbolAddress((void**)&s.error, g_error)) != cudaSuccess) return e;
         s.ready = true;
     }
@@ -124,6 +127,7 @@ extern "C" bcc_status bcc_check_noalloc(bcc_robot robot, const float* d_records,
     a.edge_self = s->edge_self;
     a.swept = s->swept;
     a.table = s->table;
+    a.seg = s->seg;
     if (ops->steps(a, st) != cudaSuccess) return BCC_ERR_CUDA;
     int total = 0;
     if (cudaMemcpyAsync(&total, s->offs + num_edges, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -139,11 +143,14 @@ extern "C" bcc_status bcc_check_noalloc(bcc_robot robot, const float* d_records,
     P.num_envs = num_envs;
     P.num_edges = num_edges;
     P.max_prims = max_prims_per_env > 0 ? max_prims_per_env : 1;
-    P.edges_per_cta = 64;
+    // a warp takes an edge at a time: four edges a CTA until the SMs are full
+    const long long pairs = (long long)num_envs * num_edges;
+    P.edges_per_cta = pairs >= 148 * 4 * 64 ? 64 : pairs <= 148 * 4 * 4 ? 4 : (int)(pairs / (148 * 4));
     P.steps = s->steps;
     P.offs = s->offs;
     P.table = s->table;
     P.swept = s->swept;
+    P.seg = s->seg;
     P.edge_self = s->edge_self;
     P.results = d_results;
     P.error_flag = s->error;

@@ -70,11 +70,13 @@ template <class M>
 struct DevTables {
     int env_bound[M::num_env_groups];
     int leaf_begin[M::num_env_groups + 1];
+    unsigned char leaf_group[M::num_env_leaves], leaf_over[M::num_env_leaves];  // group, overhangs its bound
     int over_count[M::num_env_groups];
     float cull_pad[M::num_env_groups];
     // Certain-hit radius of env group g (0: none): a primitive whose core lies
     // within rho + cert_r[g] of the bound's centre is hit by a leaf of g.
     float cert_r[M::num_env_groups];
+    float gate_r[M::num_env_groups];   // the bound's radius, inflated
     float seg_pad[M::num_env_groups];  // radius + inflation + overhang + margin
     // Groups by descending certain-hit radius (the probe's order).
     int probe_group[M::num_env_groups];
@@ -227,6 +229,11 @@ DevTables<M> host_tables() {
     std::stable_sort(t.probe_group, t.probe_group + M::num_env_groups,
                      [&](int a, int b) { return t.cert_r[a] > t.cert_r[b]; });
     for (int g = 0; g <= M::num_env_groups; ++g) t.leaf_begin[g] = M::env_leaf_begin[g];
+    for (int g = 0; g < M::num_env_groups; ++g)
+        for (int l = t.leaf_begin[g]; l < t.leaf_begin[g + 1]; ++l) {
+            t.leaf_group[l] = (unsigned char)g;
+            t.leaf_over[l] = l < t.leaf_begin[g] + M::env_over_count[g];
+        }
     // Self tables hold sample-table row positions, not sphere indices.
     for (int g = 0; g < M::num_self_groups; ++g) {
         t.self_bound[g][0] = M::table_pos[M::self_bound[g][0]];
@@ -255,6 +262,7 @@ DevTables<M> host_tables() {
         }
     }
     t.fk_begin[M::dof + 1] = at;
+    for (int g = 0; g < M::num_env_groups; ++g) t.gate_r[g] = t.sphere_radius[g] + kEnvInflate;
     for (int g = 0; g < M::num_env_groups; ++g)
         t.seg_pad[g] = t.sphere_radius[g] + kEnvInflate + t.cull_pad[g] + kSegMargin;
     for (int j = 0; j < M::dof; ++j) {
@@ -340,21 +348,47 @@ constexpr bool has_overhang() {
 }
 
 // ------------------------------------------------------------------ 1. steps
+// Step count of edge e.  Non-finite endpoints would give an unbounded one: clamped,
+// and the host rejects the resulting sample total (BCC_ERR_LIMIT).
 template <class M>
-__global__ void edge_steps_kernel(const float* __restrict__ edges, int E, int resolution,
-                                  int* __restrict__ steps) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
+__device__ __forceinline__ int clamped_steps(const float* __restrict__ edges, int e, int resolution) {
     float s[M::dof], t[M::dof];
 #pragma unroll
     for (int j = 0; j < M::dof; ++j) {
         s[j] = edges[(size_t)e * 2 * M::dof + j];
         t[j] = edges[(size_t)e * 2 * M::dof + M::dof + j];
     }
-    // Non-finite endpoints would give an unbounded step count: clamp, and let the
-    // host reject the resulting sample total (BCC_ERR_LIMIT).
     const int n = edge_steps<M::dof>(s, t, resolution);
-    steps[e] = (n < 1 || n > (1 << 20)) ? (1 << 20) : n;
+    return (n < 1 || n > (1 << 20)) ? (1 << 20) : n;
+}
+
+template <class M>
+__global__ void edge_steps_kernel(const float* __restrict__ edges, int E, int resolution,
+                                  int* __restrict__ steps) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < E) steps[e] = clamped_steps<M>(edges, e, resolution);
+}
+
+// Steps and sample offsets of at most 1024 edges in one launch of one CTA (see
+// scan_kernel): small calls are a chain of launches.
+constexpr int kFusedSteps = 1024;
+
+template <class M>
+__global__ void __launch_bounds__(kFusedSteps) edge_offsets_kernel(const float* __restrict__ edges, int E,
+                                                                   int resolution, int* __restrict__ steps,
+                                                                   int* __restrict__ offs) {
+    __shared__ long long sums[32];
+    const int e = threadIdx.x;
+    long long v = 0;
+    if (e < E) {
+        const int n = clamped_steps<M>(edges, e, resolution);
+        steps[e] = n;
+        v = (long long)kLanes * n;
+    }
+    long long total;
+    const long long at = block_scan_exclusive(v, sums, total);
+    if (e < E) offs[e] = (int)min(at, 2147483647ll);
+    if (e == 0) offs[E] = (int)min(total, 2147483647ll);
 }
 
 // ------------------------------------------------------------------ 3. FK
@@ -1089,9 +1123,10 @@ __device__ __forceinline__ bool walk_pairs(const float4* __restrict__ table, siz
 // one per sample: the walk is bound by instruction issue, and on the uneven
 // Panda workload most of it went to pairs that never collide.
 template <class M>
-__device__ __forceinline__ bool walk_segments(const CheckParams& P, size_t row0, int n, int C, const uint16_t* pairs,
-                                              const float4* prim, int np, const uint8_t* order, const GroupLanes& GL,
-                                              uint2* scratch, WalkStats& st) {
+__device__ __forceinline__ bool walk_segments(const float4* __restrict__ table, const float2* __restrict__ seg,
+                                              size_t row0, int n, int C, const uint16_t* pairs, const float4* prim, int np,
+                                              const uint8_t* order, const GroupLanes& GL, uint2* scratch,
+                                              WalkStats& st) {
     constexpr int G = M::num_env_groups;
     constexpr int GB = group_bits<M>();
     constexpr bool kOver = has_overhang<M>();
@@ -1100,8 +1135,8 @@ __device__ __forceinline__ bool walk_segments(const CheckParams& P, size_t row0,
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int S = kLanes / kSegment * n;
-    const float4* __restrict__ rows = P.table + table_index<M>(row0, 0);
-    const float2* __restrict__ segs = P.seg + row0 / kSegment * G;
+    const float4* __restrict__ rows = table + table_index<M>(row0, 0);
+    const float2* __restrict__ segs = seg + row0 / kSegment * G;
     // a / C in FP32, exact (walk_pairs)
     const float inv_c = __frcp_rn((float)C);
     const int dr = (int)(32.5f * inv_c), dc = 32 - dr * C;
@@ -1194,7 +1229,7 @@ __device__ __forceinline__ bool walk_segments(const CheckParams& P, size_t row0,
                 const int m = __popc(nm) * kSegment;
                 for (int q = lane; q - lane < m; q += 32) {
                     const uint2 x = scratch[min(q, m - 1) / kSegment];
-                    if (walk_items<M>(P.table, row0, (int)x.x + (q & (kSegment - 1)), x.y, q < m, prim, np,
+                    if (walk_items<M>(table, row0, (int)x.x + (q & (kSegment - 1)), x.y, q < m, prim, np,
                                       GL, st))
                         return true;
                 }
@@ -1381,7 +1416,7 @@ __device__ __forceinline__ void check_pair(const CheckParams& P, int env, int e,
                                            queue);
             }
         } else if constexpr (MODE == 0 || MODE == 4) {
-            collide = walk_segments<M>(P, row0, n, Cs, pairs, prim, np, MODE == 4 ? inline_perm(P, env, e, n) : nullptr,
+            collide = walk_segments<M>(P.table, P.seg, row0, n, Cs, pairs, prim, np, MODE == 4 ? inline_perm(P, env, e, n) : nullptr,
                                        GL, warp_scratch(), st);
         } else {
             collide = walk_pairs<M, MODE>(P.table, row0, n, Cs, pairs, prim, np, learned ? perm_buf : nullptr,
@@ -1492,7 +1527,7 @@ __device__ __forceinline__ void walk_listed_pair(const CheckParams& P, int env, 
             collide = walk_pairs<M, 0>(P.table, row0, n, C, pairs, prim, np, nullptr, 0, GL, undecided, st, queue);
         }
     } else if constexpr (MODE == 0 || MODE == 4) {
-        collide = walk_segments<M>(P, row0, n, C, pairs, prim, np, MODE == 4 ? inline_perm(P, env, e, n) : nullptr, GL,
+        collide = walk_segments<M>(P.table, P.seg, row0, n, C, pairs, prim, np, MODE == 4 ? inline_perm(P, env, e, n) : nullptr, GL,
                                    warp_scratch(), st);
     } else {
         collide = walk_pairs<M, MODE>(P.table, row0, n, C, pairs, prim, np, nullptr, P.queue_min_items, GL, undecided,
@@ -1636,65 +1671,136 @@ constexpr int check_min_ctas() {
     return M::check_warps_per_sm / WARPS < 32 ? M::check_warps_per_sm / WARPS : 32;
 }
 
+// Voxel lookup: the word of the voxel nearest to c and the squared distance r2 (m^2,
+// rounded up) of c from its centre; c's signed distance to the nearest primitive
+// then lies in [lo - sqrt(r2), lo + kVoxStep + 2 kVoxSlack + sqrt(r2)), lo =
+// voxel_low(word).
+struct VoxelGrid {
+    const uint16_t* vox;
+    float inv_h, bx, by, bz, mx, my, mz, sy, sz, h2;
+    __device__ __forceinline__ VoxelGrid(const ProbeGrid& V, const uint16_t* words)
+        : vox(words), inv_h(V.inv_h), bx(-V.ox * V.inv_h), by(-V.oy * V.inv_h), bz(-V.oz * V.inv_h),
+          mx((float)(V.nx - 1)), my((float)(V.ny - 1)), mz((float)(V.nz - 1)), sy((float)V.nx),
+          sz((float)(V.nx * V.ny)), h2(V.h * V.h * 1.0002f) {}
+    __device__ __forceinline__ unsigned at(float4 c, float& r2) const {
+        constexpr float kRound = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
+        // position in voxels from the centre of voxel 0, the nearest voxel, the offset from it
+        const float fx = fmaf(c.x, inv_h, bx), fy = fmaf(c.y, inv_h, by), fz = fmaf(c.z, inv_h, bz);
+        const float ix = (fminf(fmaxf(fx, 0.0f), mx) + kRound) - kRound;
+        const float iy = (fminf(fmaxf(fy, 0.0f), my) + kRound) - kRound;
+        const float iz = (fminf(fmaxf(fz, 0.0f), mz) + kRound) - kRound;
+        const float rx = fx - ix, ry = fy - iy, rz = fz - iz;
+        r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz)) * h2;
+        return vox[(int)fmaf(iz, sz, fmaf(iy, sy, ix))];
+    }
+    // ... the voxel's primitive alone.
+    __device__ __forceinline__ unsigned nearest(float4 c) const {
+        float r2;
+        return at(c, r2) >> 8;
+    }
+};
+__device__ __forceinline__ float voxel_low(unsigned word) {
+    return fmaf((float)(word & 255u), kVoxStep, kVoxMin - kVoxSlack);
+}
+
+// Is c, looked up as (word, r2), certainly within `reach` of some primitive
+// (signed distance below it)?  By the voxel's distance where that decides, else by
+// the exact test on the voxel's nearest primitive (a non-finite centre is left to
+// the walk).
+__device__ __forceinline__ bool voxel_hit(float4 c, unsigned word, float r2, float lo, float reach, const float4* prim) {
+    const float up = reach - (lo + kVoxStep + 2.0f * kVoxSlack), dn = lo - reach;
+    if (up > 0.0f && up * up > r2) return true;
+    if ((dn > 0.0f && dn * dn > r2) || !(r2 < 1e30f) || (word >> 8) == kVoxUnknown) return false;
+    float rho;
+    const float d2 = prim_core_d2(c, prim + (word >> 8) * kPrimF4, &rho);
+    const float rc = rho + reach;
+    return d2 - rc * rc < 0.0f;
+}
+
 // Probe of pair (env, e), one lane per pair (decided: the lane has none).  Per
 // group P.mid holds the bound's centre at the edge's middle sample and the
 // radius R of the sphere around it that holds the group's leaves, inflated,
-// over all of the edge's samples.  The voxel of the centre gives the signed
-// distance to the nearest primitive, good to the offset from the voxel's
-// centre.  Well inside the certain-hit radius (cert_radius) it proves a leaf
-// hit at the middle sample; above R it proves the group free along the whole
-// edge; between the two the exact certain-hit test on the voxel's nearest
-// primitive finds most of the other hits.  Returns 1 for a hit, else 0; `alive`
-// gets the groups not proved free (none: the pair is free).  Groups in
-// descending certain-hit radius; the warp leaves once all its lanes are decided.
+// over all of the edge's samples.  A centre within the certain-hit radius
+// (cert_radius) of a primitive proves a leaf hit at the middle sample; a distance
+// above R proves the group free along the whole edge.  Returns whether a hit is
+// proved; `alive` gets the groups not proved free (none: the pair is free), `near`
+// those whose bound may touch a primitive at the middle sample.
+// Groups in descending certain-hit radius; the warp leaves once all its lanes are
+// decided.
 template <class M>
-__device__ __forceinline__ bool probe_pair(const CheckParams& P, int e, bool decided, const uint16_t* vox,
-                                           const float4* prim, unsigned& alive) {
+__device__ __forceinline__ bool probe_pair(const CheckParams& P, int e, bool decided, const VoxelGrid& V,
+                                           const float4* prim, unsigned& alive, unsigned& near) {
     const DevTables<M>& T = tab<M>();
-    const ProbeGrid& V = P.probe;
-    const float bx = -V.ox * V.inv_h, by = -V.oy * V.inv_h, bz = -V.oz * V.inv_h;
-    const float mx = (float)(V.nx - 1), my = (float)(V.ny - 1), mz = (float)(V.nz - 1);
-    const float sy = (float)V.nx, sz = (float)(V.nx * V.ny);
-    const float h2 = V.h * V.h * 1.0002f;
-    constexpr float kRound = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
     bool hit = false;
-    alive = 0u;
+    alive = near = 0u;
     for (int i = 0; i < M::num_env_groups; ++i) {
         if (__all_sync(kFull, decided)) break;
         const int g = T.probe_group[i];
         if (!decided) {
             const float4 c = P.mid[(size_t)g * P.num_edges + e];
             const float kappa = T.cert_r[g];
-            // position in voxels from the centre of voxel 0, the nearest voxel, the offset from it
-            const float fx = fmaf(c.x, V.inv_h, bx), fy = fmaf(c.y, V.inv_h, by), fz = fmaf(c.z, V.inv_h, bz);
-            const float ix = (fminf(fmaxf(fx, 0.0f), mx) + kRound) - kRound;
-            const float iy = (fminf(fmaxf(fy, 0.0f), my) + kRound) - kRound;
-            const float iz = (fminf(fmaxf(fz, 0.0f), mz) + kRound) - kRound;
-            const float rx = fx - ix, ry = fy - iy, rz = fz - iz;
-            const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz)) * h2;  // squared offset (m^2)
-            const unsigned w = vox[(int)fmaf(iz, sz, fmaf(iy, sy, ix))];
-            // the voxel's distance lies in [lo, lo + step + 2 slack)
-            const float lo = fmaf((float)(w & 255u), kVoxStep, kVoxMin - kVoxSlack);
-            const float miss = lo - c.w, up = kappa - (lo + kVoxStep + 2.0f * kVoxSlack), dn = lo - kappa;
+            float r2;
+            const unsigned w = V.at(c, r2);
+            const float lo = voxel_low(w), miss = lo - c.w;
             if (miss > 0.0f && miss * miss > r2) continue;
             alive |= 1u << g;
-            if (kappa > 0.0f) {
-                if (up > 0.0f && up * up > r2) {
-                    hit = decided = true;
-                } else if (!(dn > 0.0f && dn * dn > r2) && r2 < 1e30f && (w >> 8) != kVoxUnknown) {
-                    // the voxel leaves it open (a non-finite centre is left to the walk)
-                    float rho;
-                    const float d2 = prim_core_d2(c, prim + (w >> 8) * kPrimF4, &rho);
-                    const float rc = rho + kappa;
-                    hit = decided = d2 - rc * rc < 0.0f;
-                }
-            }
+            const float clear = lo - T.gate_r[g];
+            if (!(clear > 0.0f && clear * clear > r2)) near |= 1u << g;
+            if (kappa > 0.0f) hit = decided = voxel_hit(c, w, r2, lo, kappa, prim);
         }
     }
     return hit;
 }
 
-// First pass of a check with probe grids: CTA = one environment x kProbeBatch
+// Second probe of an undecided pair, whole warp, lanes over the leaves (a row's are
+// contiguous): those of its `near` groups at the middle sample against the nearest
+// primitive of the voxel they lie in.  A hit is a leaf hit the walk would find:
+// exactly its test for robots whose leaves lie inside their bounds; for the others
+// only leaves inside their bounds count, by kCertMargin (a hit then implies the
+// bound's).  Most pairs that collide in contact shallower than the groups'
+// certain-hit radii end here.  bits[k]: the group bit of this lane's leaf 32 k +
+// lane, 0 where none counts.
+template <class M>
+constexpr int kLeafSteps = (M::num_env_leaves + 31) / 32;
+
+template <class M>
+__device__ __forceinline__ void leaf_bits(unsigned (&bits)[kLeafSteps<M>]) {
+    const DevTables<M>& L = lane_tab<M>();
+#pragma unroll
+    for (int k = 0; k < kLeafSteps<M>; ++k) {
+        const int l = 32 * k + (threadIdx.x & 31);
+        bits[k] = l < M::num_env_leaves && !L.leaf_over[l] ? 1u << L.leaf_group[l] : 0u;
+    }
+}
+
+template <class M>
+__device__ __forceinline__ bool probe_leaves(const CheckParams& P, int e, unsigned near, const VoxelGrid& V,
+                                             const float4* prim, const unsigned (&bits)[kLeafSteps<M>]) {
+    constexpr float kInflate = has_overhang<M>() ? kEnvInflate - (float)kCertMargin : kEnvInflate;
+    const float4* row = P.table + table_index<M>((size_t)P.offs[e] + 16 * (size_t)P.steps[e], M::num_env_groups) +
+                        (threadIdx.x & 31);
+#pragma unroll
+    for (int k = 0; k < kLeafSteps<M>; ++k) {
+        const bool mine = (near & bits[k]) != 0u;
+        if (!__any_sync(kFull, mine)) continue;
+        bool hit = false;
+        if (mine) {
+            const float4 c = row[32 * k];
+            const unsigned id = V.nearest(c);
+            // (a non-finite centre is left to the walk)
+            if (id != kVoxUnknown && fabsf(c.x + c.y + c.z) < 1e30f) {
+                float rho;
+                const float d2 = prim_core_d2(c, prim + id * kPrimF4, &rho);
+                const float rr = c.w + kInflate + rho;
+                hit = d2 - rr * rr < 0.0f;
+            }
+        }
+        if (__any_sync(kFull, hit)) return true;
+    }
+    return false;
+}
+
+// First pass of a check with probe grids: CTA = one environment x Q.batch
 // edges, one lane per pair.  Decided pairs get their verdict; the others go to
 // the queue (Q) as (edge, alive groups), contiguous per CTA, with one work item
 // per Q.chunk of them.  On the uneven Panda workload (1000 x 10000) it decides
@@ -1704,12 +1810,15 @@ __device__ __forceinline__ bool probe_pair(const CheckParams& P, int e, bool dec
 constexpr int kProbeThreads = 256;
 
 template <class M>
-__global__ void __launch_bounds__(kProbeThreads, 6) probe_kernel(CheckParams P, ProbeQueue Q, int env0) {
+#ifndef PMIN
+#define PMIN 5
+#endif
+__global__ void __launch_bounds__(kProbeThreads, PMIN) probe_kernel(CheckParams P, ProbeQueue Q, int env0) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
-    __shared__ int s_cnt, s_base, s_item;
-    const int env = env0 + blockIdx.x, e0 = blockIdx.y * kProbeBatch;
-    const int nb = min(kProbeBatch, P.num_edges - e0);
+    __shared__ int s_cnt, s_open, s_base, s_item;
+    const int env = env0 + blockIdx.x, e0 = blockIdx.y * Q.batch;
+    const int nb = min(Q.batch, P.num_edges - e0);
     const int lane = threadIdx.x & 31;
     const float4 h0 = P.env_hdr[2 * env + 0];
     const float4 h1 = P.env_hdr[2 * env + 1];
@@ -1717,10 +1826,10 @@ __global__ void __launch_bounds__(kProbeThreads, 6) probe_kernel(CheckParams P, 
     const int np = (int)(__float_as_uint(h1.w) & 0xffffu);
     const bool probe = np > 0 && !(__float_as_uint(h1.z) & kEnvIrregular);
     const float4* prim = reinterpret_cast<const float4*>(smem);
-    const uint16_t* vox = reinterpret_cast<const uint16_t*>(smem + P.blob_smem);
     uint2* list = reinterpret_cast<uint2*>(smem + P.blob_smem + P.probe.stride);
+    unsigned* list_near = reinterpret_cast<unsigned*>(list + Q.batch);
     if (threadIdx.x == 0) {
-        s_cnt = 0;
+        s_cnt = s_open = 0;
         mbar_init(&bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1739,37 +1848,76 @@ __global__ void __launch_bounds__(kProbeThreads, 6) probe_kernel(CheckParams P, 
             return;
         }
     }
-    for (int i0 = threadIdx.x & ~31; i0 < nb; i0 += kProbeThreads) {
-        const int i = i0 + lane, e = e0 + min(i, nb - 1);
-        const int self = i < nb ? P.edge_self[e] : 1;
-        unsigned alive = np > 0 ? kFull : 0u;
-        bool hit = self != 0;
-        if (probe) hit = probe_pair<M>(P, e, hit, vox, prim, alive) || hit;
-        const bool open = !hit && alive != 0u;
-        if (i < nb && !open) P.results[(size_t)e * P.num_envs + env] = hit ? 1 : 0;
+    const VoxelGrid V(P.probe, reinterpret_cast<const uint16_t*>(smem + P.blob_smem));
+    // Undecided pairs to list[from s_cnt on]; verdicts of the decided ones.
+    auto settle = [&](bool live, bool hit, bool open, int e, unsigned alive, unsigned near) {
+        if (live && !open) P.results[(size_t)e * P.num_envs + env] = hit ? 1 : 0;
         const unsigned m = __ballot_sync(kFull, open);
         int at = 0;
         if (lane == 0 && m) at = atomicAdd(&s_cnt, __popc(m));
         at = __shfl_sync(kFull, at, 0);
-        if (open) list[at + __popc(m & ((1u << lane) - 1u))] = make_uint2((unsigned)e, alive);
-        if (P.counters && np > 0) {
-            const unsigned dec = __ballot_sync(kFull, !open && !self), col = __ballot_sync(kFull, hit && !self);
+        if (open) {
+            at += __popc(m & ((1u << lane) - 1u));
+            list[at] = make_uint2((unsigned)e, alive);
+            list_near[at] = near;
+        }
+    };
+    auto count = [&](bool decided, bool hit) {  // pairs settled here (self-colliding ones are not counted)
+        const unsigned dec = __ballot_sync(kFull, decided), col = __ballot_sync(kFull, hit);
+        if (lane == 0) {
+            atomicAdd(P.counters + 0, (unsigned long long)__popc(dec));
+            atomicAdd(P.counters + 5, (unsigned long long)__popc(col));
+        }
+    };
+    for (int i0 = threadIdx.x & ~31; i0 < nb; i0 += kProbeThreads) {
+        const int i = i0 + lane, e = e0 + min(i, nb - 1);
+        const int self = i < nb ? P.edge_self[e] : 1;
+        unsigned alive = np > 0 ? kFull : 0u, near = 0u;
+        bool hit = self != 0;
+        if (probe) hit = probe_pair<M>(P, e, hit, V, prim, alive, near) || hit;
+        const bool open = !hit && alive != 0u;
+        settle(i < nb, hit, open, e, alive, near);
+        if (P.counters && np > 0) count(!open && !self, hit && !self);
+    }
+    __syncthreads();
+    const int n = s_cnt;
+    unsigned bits[kLeafSteps<M>];
+    leaf_bits<M>(bits);
+    for (int i = threadIdx.x >> 5; i < n; i += kProbeThreads / 32) {
+        const unsigned near = list_near[i];  // none without a probe
+        if (near == 0u) continue;
+        const int e = (int)list[i].x;
+        if (probe_leaves<M>(P, e, near, V, prim, bits)) {
             if (lane == 0) {
-                atomicAdd(P.counters + 0, (unsigned long long)__popc(dec));
-                atomicAdd(P.counters + 5, (unsigned long long)__popc(col));
+                P.results[(size_t)e * P.num_envs + env] = 1;
+                list[i].y = 0u;  // settled
             }
+            if (P.counters) count(lane == 0, lane == 0);
         }
     }
     __syncthreads();
-    const int u = s_cnt;
+    for (int i0 = threadIdx.x & ~31; i0 < n; i0 += kProbeThreads) {
+        const unsigned m = __ballot_sync(kFull, i0 + lane < n && list[i0 + lane].y != 0u);
+        if (lane == 0 && m) atomicAdd(&s_open, __popc(m));
+    }
+    __syncthreads();
+    const int u = s_open;
     if (u == 0) return;
     const int items = (u + Q.chunk - 1) / Q.chunk;
     if (threadIdx.x == 0) {
         s_base = atomicAdd(Q.head + 0, u);
         s_item = atomicAdd(Q.head + 1, items);
+        s_cnt = 0;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < u; i += kProbeThreads) Q.entries[s_base + i] = list[i];
+    for (int i0 = threadIdx.x & ~31; i0 < n; i0 += kProbeThreads) {
+        const uint2 x = i0 + lane < n ? list[i0 + lane] : make_uint2(0u, 0u);
+        const unsigned m = __ballot_sync(kFull, x.y != 0u);
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(&s_cnt, __popc(m));
+        at = s_base + __shfl_sync(kFull, at, 0);
+        if (x.y) Q.entries[at + __popc(m & ((1u << lane) - 1u))] = x;
+    }
     for (int i = threadIdx.x; i < items; i += kProbeThreads)
         Q.items[s_item + i] = make_int4(env, s_base + i * Q.chunk, min(Q.chunk, u - i * Q.chunk), 0);
 }
@@ -2369,11 +2517,11 @@ __global__ void __launch_bounds__(WARPS * 32) check_records_kernel(RecordsParams
         }
         __syncwarp();
 
-        bool collide = false, undecided = false;
+        bool collide = false;
         WalkStats st;
         if (C > 0)
-            collide = walk_pairs<M, 0>(P.table, (size_t)P.offs[e], P.steps[e], C, pairs, prim, np, nullptr, 0,
-                                       GL, undecided, st, [] { return false; });
+            collide = walk_segments<M>(P.table, P.seg, (size_t)P.offs[e], P.steps[e], C, pairs, prim, np, nullptr, GL,
+                                       warp_scratch(), st);
         __syncwarp();
         if (lane == 0) *out = collide ? 1 : 0;
     }
@@ -2384,6 +2532,10 @@ template <class M>
 cudaError_t run_steps(const PipelineArgs& a, cudaStream_t st) {
     const int E = a.num_edges;
     if (a.stage_events) cudaEventRecord(a.stage_events[0], st);
+    if (E <= kFusedSteps) {
+        edge_offsets_kernel<M><<<1, kFusedSteps, 0, st>>>(a.d_edges, E, a.resolution, a.steps, a.offs);
+        return cudaGetLastError();
+    }
     edge_steps_kernel<M><<<(E + 255) / 256, 256, 0, st>>>(a.d_edges, E, a.resolution, a.steps);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
@@ -2393,7 +2545,7 @@ cudaError_t run_steps(const PipelineArgs& a, cudaStream_t st) {
 // Probe and walk, in slabs of environments whose pairs fit the queue.
 template <class M, int W, int MODE>
 cudaError_t launch_probed(const CheckParams& P, int E, cudaStream_t st) {
-    const size_t smem = P.blob_smem + P.probe.stride + kProbeBatch * sizeof(uint2);
+    const size_t smem = P.blob_smem + P.probe.stride + P.queue.batch * kProbeEntryBytes;
     const size_t walk_smem = check_smem_bytes(P.max_prims, M::num_env_groups, P.blob_smem, W);
     cudaError_t err = cudaFuncSetAttribute(probe_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
@@ -2411,7 +2563,7 @@ cudaError_t launch_probed(const CheckParams& P, int E, cudaStream_t st) {
     if (err != cudaSuccess) return err;
     for (int env0 = 0; env0 < P.num_envs; env0 += slab, Q.head += 4) {
         const int n = std::min(slab, P.num_envs - env0);
-        probe_kernel<M><<<dim3(n, (E + kProbeBatch - 1) / kProbeBatch), kProbeThreads, smem, st>>>(P, Q, env0);
+        probe_kernel<M><<<dim3(n, (E + Q.batch - 1) / Q.batch), kProbeThreads, smem, st>>>(P, Q, env0);
         const long long most = (long long)n * E;  // every pair undecided
         const int grid = (int)std::min<long long>(slots, (most + Q.chunk - 1) / Q.chunk);
         walk_kernel<M, W, MODE><<<grid, W * 32, walk_smem, st>>>(P, Q);

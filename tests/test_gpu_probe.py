@@ -25,11 +25,12 @@ def both(checker, envs, edges, robot, resolution=32):
     return out[1]
 
 
-# 1023 .. 1025 edges: a probe CTA's batch; 255 .. 257 primitives: the ids a voxel
+# 511 .. 513 edges: a probe CTA's batch; 1023 .. 1025, 4097: the offset scan's
+# launches and rounds; 255 .. 257 primitives: the ids a voxel
 # holds; resolution 1 / 200: one sample block and long edges.
 @pytest.mark.parametrize("name,nenv,nedge,resolution", [
     ("uneven", 1, 1, 32), ("uneven", 33, 31, 32), ("uneven", 20, 1023, 32), ("stress", 20, 1024, 32),
-    ("stress", 9, 1025, 200), ("plain", 40, 333, 32), ("uneven", 40, 500, 1), ("multi_fetch", 60, 1025, 32),
+    ("stress", 9, 1025, 200), ("uneven", 300, 511, 32), ("stress", 300, 513, 32), ("uneven", 5, 4097, 32), ("plain", 40, 333, 32), ("uneven", 40, 500, 1), ("multi_fetch", 60, 1025, 32),
     ("multi_baxter", 40, 400, 32)])
 def test_probed_check_is_the_one_pass_check(checker, name, nenv, nedge, resolution):
     robot = workload.robot_of(name)
