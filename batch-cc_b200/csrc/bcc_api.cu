@@ -156,6 +156,20 @@ bool regular_rec(const Rec& r) {
 
 int clamp_tile(int v, int lo, int hi) { return std::max(lo, std::min(hi, v)); }
 
+// Sample rows of a call at most (the sample table's limit).
+constexpr int kMaxSampleRows = 1 << 27;
+
+// The sample total of the call whose offsets were launched last: waits for its
+// offset kernel only.  offs[] is int32 and the scan saturates at INT32_MAX instead
+// of wrapping, so an oversized total shows up here.
+bcc_status await_total(bcc_ctx* ctx, int& total) {
+    BCC_CUDA(ctx, cudaEventSynchronize(ctx->ev_total));
+    total = *(volatile const int*)ctx->h_total;
+    if (total < 0 || total > kMaxSampleRows)
+        return fail(ctx, BCC_ERR_LIMIT, "too many samples in one call (edges too long or non-finite)");
+    return BCC_OK;
+}
+
 // Probe grids of the uploaded set for a robot's reach, built on the first check
 // that uses them after an upload (or after a check of another robot): cubic
 // voxels, as many as kMaxVoxels allow.  Stream-ordered on st; the caller
@@ -217,8 +231,11 @@ bcc::Tune launch_shape(const bcc_ctx* ctx, int E) {
 
 // Discretisation, sample offsets and every per-call buffer of a check; fills
 // `a` up to (not including) the FK / self / swept / check launches.
+// With `ahead` the sample total is not waited for when the tables of an earlier
+// call exist: a.total_rows stays -1, the kernels work within a.cap_rows, and the
+// caller settles the total afterwards (await_total).
 bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution, uint8_t* d_results,
-                   const bcc_opts* opts, cudaStream_t st, bcc::PipelineArgs& a) {
+                   const bcc_opts* opts, cudaStream_t st, bcc::PipelineArgs& a, bool ahead = false) {
     const int r = (int)robot;
     const bcc::RobotOps* ops = bcc::robot_ops(r);
     if (!ops) return fail(ctx, BCC_ERR_NOT_SUPPORTED, "robot not built into this library");
@@ -287,18 +304,22 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
         BCC_CUDA(ctx, cudaMemsetAsync(a.counters, 0, sizeof(unsigned long long) * bcc::kNumCounters, st));
     }
     BCC_CUDA(ctx, cudaMemsetAsync(a.error_flag, 0, sizeof(int), st));
+    a.host_total = ctx->h_total;
     BCC_CUDA(ctx, ops->steps(a, st));
-    BCC_CUDA(ctx, cudaMemcpyAsync(ctx->h_total, a.offs + E, sizeof(int), cudaMemcpyDeviceToHost, st));
-    BCC_CUDA(ctx, cudaStreamSynchronize(st));
-    const int total = *ctx->h_total;
-    // offs[] is int32 and the scan saturates at INT32_MAX instead of wrapping, so
-    // an oversized total shows up here; cap the sample table at 2^27 rows.
-    if (total < 0 || total > (1 << 27))
-        return fail(ctx, BCC_ERR_LIMIT, "too many samples in one call (edges too long or non-finite)");
+    BCC_CUDA(ctx, cudaEventRecord(ctx->ev_total, st));
     const int NS = ops->num_spheres;
-    BCC_CUDA(ctx, ctx->table.ensure(sizeof(float4) * (size_t)NS * std::max(total, 1)));
-    a.total_rows = total;
-    BCC_CUDA(ctx, ctx->seg.ensure(sizeof(float2) * (size_t)G * (std::max(total, bcc::kSegment) / bcc::kSegment)));
+    const size_t held = std::min(ctx->table.cap / (sizeof(float4) * NS), ctx->seg.cap / (sizeof(float2) * G) * bcc::kSegment);
+    if (ahead && held >= bcc::kLanes) {
+        a.total_rows = -1;
+        a.cap_rows = (int)std::min<size_t>(held, kMaxSampleRows);
+    } else {
+        bcc_status s = await_total(ctx, a.total_rows);
+        if (s != BCC_OK) return s;
+        a.cap_rows = a.total_rows;
+        BCC_CUDA(ctx, ctx->table.ensure(sizeof(float4) * (size_t)NS * std::max(a.total_rows, 1)));
+        BCC_CUDA(ctx, ctx->seg.ensure(sizeof(float2) * (size_t)G *
+                                      (std::max(a.total_rows, bcc::kSegment) / bcc::kSegment)));
+    }
     a.seg = ctx->seg.as<float2>();
     a.table = ctx->table.as<float4>();
     a.blobs = ctx->blobs.as<float4>();
@@ -527,10 +548,14 @@ bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
            x.features == y.features && x.work_counter == y.work_counter && x.error_flag == y.error_flag;
 }
 
-bcc_status run_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution,
-                     uint8_t* d_results, const bcc_opts* opts, cudaStream_t st) {
-    bcc::PipelineArgs a;
-    bcc_status s = prepare(ctx, robot, d_edges, E, resolution, d_results, opts, st, a);
+// Launches a check.  A plain one that finds the tables of an earlier call is queued
+// whole before the host looks at its sample total, so the GPU does not wait for the
+// host in the middle of it; should the tables turn out too small, its kernels have
+// done nothing and it is launched again.  (Learned checks size their MLP rows by
+// the total, profiled ones bracket their stages.)
+bcc_status launch_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution,
+                        uint8_t* d_results, const bcc_opts* opts, cudaStream_t st, bool ahead, bcc::PipelineArgs& a) {
+    bcc_status s = prepare(ctx, robot, d_edges, E, resolution, d_results, opts, st, a, ahead);
     if (s != BCC_OK) return s;
     const bool learned = opts && opts->order == BCC_ORDER_LEARNED;
     if (learned) {
@@ -549,7 +574,7 @@ bcc_status run_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E,
     // the launches): replayed while the inputs and configuration are unchanged.
     bcc::GraphCache& G = ctx->graph[learned ? 1 : 0];
     const bool hit = G.exec && G.edges == d_edges && G.results == d_results && G.num_edges == E &&
-                     G.resolution == resolution && G.total_rows == a.total_rows && G.robot == (int)robot &&
+                     G.resolution == resolution && G.total_rows == a.total_rows && G.args.cap_rows == a.cap_rows && G.robot == (int)robot &&
                      G.row_cap == a.row_cap &&
                      G.env_version == ctx->env_version && same_tune(G.tune, ctx->tune) && same_buffers(G.args, a);
     if (!hit) {
@@ -595,6 +620,18 @@ bcc_status run_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E,
     return BCC_OK;
 }
 
+bcc_status run_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution,
+                     uint8_t* d_results, const bcc_opts* opts, cudaStream_t st) {
+    const bool ahead = !(opts && opts->order == BCC_ORDER_LEARNED) && !ctx->profiling && !ctx->counting;
+    bcc::PipelineArgs a;
+    bcc_status s = launch_check(ctx, robot, d_edges, E, resolution, d_results, opts, st, ahead, a);
+    if (s != BCC_OK || a.total_rows >= 0) return s;
+    int total = 0;
+    s = await_total(ctx, total);
+    if (s != BCC_OK || total <= a.cap_rows) return s;
+    return launch_check(ctx, robot, d_edges, E, resolution, d_results, opts, st, false, a);
+}
+
 }  // namespace
 
 extern "C" {
@@ -608,6 +645,7 @@ bcc_status bcc_create(bcc_ctx** out, int device) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->capture_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_total, sizeof(int));
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_total, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         delete c;
         return BCC_ERR_CUDA;
@@ -622,6 +660,7 @@ void bcc_destroy(bcc_ctx* ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (auto& e : ctx->ev)
         if (e) cudaEventDestroy(e);
+    if (ctx->ev_total) cudaEventDestroy(ctx->ev_total);
     if (ctx->h_total) cudaFreeHost(ctx->h_total);
     for (auto& g : ctx->graph)
         if (g.exec) {

@@ -96,7 +96,8 @@ struct bcc_ctx {
     bcc::DevBuf records;     // the upload's records as packed, source of the blobs
     // per-call buffers
     bcc::DevBuf edges, steps, offs, table, edge_self, swept, results, error_flag;
-    int* h_total = nullptr;  // pinned readback of the sample-row total
+    int* h_total = nullptr;  // pinned: the sample-row total, written by the offset kernel
+    cudaEvent_t ev_total = nullptr;  // ... once this has passed
     bool profiling = false;
     bool counting = false;
     bcc::DevBuf counters;

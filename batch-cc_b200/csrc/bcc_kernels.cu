@@ -32,7 +32,8 @@ const RobotOps* robot_ops(int robot) {
 // instead of 49).  Sums run in 64 bits and every offset saturates at INT32_MAX, so
 // a total too large for the sample table can never wrap into a small,
 // valid-looking one; the host rejects any total above its limit.
-__global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ steps, int E, int* __restrict__ offs) {
+__global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ steps, int E, int* __restrict__ offs,
+                                                    int* __restrict__ host_total) {
     __shared__ long long warp_sums[32];
     long long carry = 0;
     for (int base = 0; base < E; base += 4096) {
@@ -50,11 +51,14 @@ __global__ void __launch_bounds__(1024) scan_kernel(const int* __restrict__ step
         }
         carry += all;
     }
-    if (threadIdx.x == 0) offs[E] = (int)min(carry, 2147483647ll);
+    if (threadIdx.x == 0) {
+        offs[E] = (int)min(carry, 2147483647ll);
+        if (host_total) *host_total = (int)min(carry, 2147483647ll);
+    }
 }
 
-cudaError_t launch_scan(const int* steps, int E, int* offs, cudaStream_t st) {
-    scan_kernel<<<1, 1024, 0, st>>>(steps, E, offs);
+cudaError_t launch_scan(const int* steps, int E, int* offs, int* host_total, cudaStream_t st) {
+    scan_kernel<<<1, 1024, 0, st>>>(steps, E, offs, host_total);
     return cudaGetLastError();
 }
 

@@ -65,6 +65,7 @@ struct CheckParams {
     int edges_per_cta;
     const int* steps;        // [E] n per edge
     const int* offs;         // [E + 1] first sample row of each edge
+    int cap_rows;            // nothing is checked when offs[E] exceeds it (the tables do not hold them)
     const float4* table;     // [rows][num_spheres] sphere centres + radius
     const float4* swept;     // [E][groups][2] cull AABB centre / half-size
     const float2* seg;       // [rows / kSegment][groups] segment spheres (plain and inline learned walks)
@@ -109,7 +110,9 @@ struct PipelineArgs {
     int resolution;
     int* steps;              // [E]
     int* offs;               // [E + 1]
-    int total_rows;          // offs[E], read back after the scan
+    int total_rows;          // offs[E], or -1: not known to the host yet
+    int cap_rows;            // sample rows the buffers hold; kernels leave untouched what needs more
+    int* host_total;         // null, or pinned: offs[E] for the host
     float4* table;           // [total_rows][num_spheres]
     float2* seg;             // [total_rows / kSegment][groups] segment spheres, null = not needed
     int* edge_self;          // [E]
@@ -160,6 +163,7 @@ struct RecordsParams {
     int edges_per_cta;
     const int* steps;
     const int* offs;
+    int cap_rows;
     const float4* table;
     const float4* swept;
     const float2* seg;
@@ -222,7 +226,7 @@ struct RobotOps {
 const RobotOps* robot_ops(int robot);
 
 // Robot-independent kernels (bcc_kernels.cu).
-cudaError_t launch_scan(const int* steps, int E, int* offs, cudaStream_t st);
+cudaError_t launch_scan(const int* steps, int E, int* offs, int* host_total, cudaStream_t st);
 cudaError_t launch_env_encode(const float4* blobs, const float4* env_hdr, int num_envs, float* code, cudaStream_t st);
 // Row gather for training: x2[i] = x[perm[i]] (kMlpIn BF16 values), y2[i] = y[perm[i]].
 cudaError_t launch_gather_rows(const uint16_t* x, const uint8_t* y, const int* perm, int rows, uint16_t* x2,
@@ -248,6 +252,7 @@ inline CheckParams params_of(const PipelineArgs& a) {
     P.edges_per_cta = a.edges_per_cta;
     P.steps = a.steps;
     P.offs = a.offs;
+    P.cap_rows = a.cap_rows;
     P.table = a.table;
     P.swept = a.swept;
     P.seg = a.seg;

@@ -128,14 +128,11 @@ extern "C" bcc_status bcc_check_noalloc(bcc_robot robot, const float* d_records,
     a.swept = s->swept;
     a.table = s->table;
     a.seg = s->seg;
-    if (ops->steps(a, st) != cudaSuccess) return BCC_ERR_CUDA;
-    int total = 0;
-    if (cudaMemcpyAsync(&total, s->offs + num_edges, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return BCC_ERR_CUDA;
-    if (total < 0 || total > kMaxRows) return BCC_ERR_LIMIT;  // the edges need more samples than the arrays hold
-    a.total_rows = total;
-    if (ops->prep(a, st) != cudaSuccess) return BCC_ERR_CUDA;
+    // The working arrays are as large as they get, so nothing waits for the sample
+    // total: the kernels read it and do nothing beyond kMaxRows.
+    a.total_rows = -1;
+    a.cap_rows = kMaxRows;
+    if (ops->steps(a, st) != cudaSuccess || ops->prep(a, st) != cudaSuccess) return BCC_ERR_CUDA;
 
     bcc::RecordsParams P{};
     P.records = reinterpret_cast<const float4*>(d_records);
@@ -148,6 +145,7 @@ extern "C" bcc_status bcc_check_noalloc(bcc_robot robot, const float* d_records,
     P.edges_per_cta = pairs >= 148 * 4 * 64 ? 64 : pairs <= 148 * 4 * 4 ? 4 : (int)(pairs / (148 * 4));
     P.steps = s->steps;
     P.offs = s->offs;
+    P.cap_rows = kMaxRows;
     P.table = s->table;
     P.swept = s->swept;
     P.seg = s->seg;
@@ -155,10 +153,12 @@ extern "C" bcc_status bcc_check_noalloc(bcc_robot robot, const float* d_records,
     P.results = d_results;
     P.error_flag = s->error;
     if (ops->check_records(P, st) != cudaSuccess) return BCC_ERR_CUDA;
-    int flag = 0;
+    int flag = 0, total = 0;
     if (cudaMemcpyAsync(&flag, s->error, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaMemcpyAsync(&total, s->offs + num_edges, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return BCC_ERR_CUDA;
+    if (total < 0 || total > kMaxRows) return BCC_ERR_LIMIT;  // the edges need more samples than the arrays hold
     if (flag & 2) return BCC_ERR_INVALID_ARGUMENT;  // an environment exceeds max_prims_per_env
     return flag ? BCC_ERR_TIMEOUT : BCC_OK;
 }

@@ -376,7 +376,8 @@ constexpr int kFusedSteps = 1024;
 template <class M>
 __global__ void __launch_bounds__(kFusedSteps) edge_offsets_kernel(const float* __restrict__ edges, int E,
                                                                    int resolution, int* __restrict__ steps,
-                                                                   int* __restrict__ offs) {
+                                                                   int* __restrict__ offs,
+                                                                   int* __restrict__ host_total) {
     __shared__ long long sums[32];
     const int e = threadIdx.x;
     long long v = 0;
@@ -388,7 +389,10 @@ __global__ void __launch_bounds__(kFusedSteps) edge_offsets_kernel(const float* 
     long long total;
     const long long at = block_scan_exclusive(v, sums, total);
     if (e < E) offs[e] = (int)min(at, 2147483647ll);
-    if (e == 0) offs[E] = (int)min(total, 2147483647ll);
+    if (e == 0) {
+        offs[E] = (int)min(total, 2147483647ll);
+        if (host_total) *host_total = (int)min(total, 2147483647ll);
+    }
 }
 
 // ------------------------------------------------------------------ 3. FK
@@ -673,7 +677,7 @@ __device__ __forceinline__ void fk_rows(const float* q, const FkReal<M>* sn, con
 template <class M>
 __global__ void __launch_bounds__(32 * fk_warps<M>(), fk_ctas<M>()) fk_staged_kernel(const float* __restrict__ edges, int E,
                                                                   const int* __restrict__ steps,
-                                                                  const int* __restrict__ offs,
+                                                                  const int* __restrict__ offs, int cap,
                                                                   float4* __restrict__ table,
                                                                   int* __restrict__ edge_self,
                                                                   float2* __restrict__ seg) {
@@ -687,6 +691,7 @@ __global__ void __launch_bounds__(32 * fk_warps<M>(), fk_ctas<M>()) fk_staged_ke
     const DevTables<M>& L = lane_tab<M>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int total = offs[E];
+    if (total > cap) return;
     for (int base = blockIdx.x * 32; base < total; base += gridDim.x * 32) {
         const int e = edge_of_row(offs, E, base);
         const int n = steps[e], k = base + lane - offs[e];
@@ -772,13 +777,13 @@ __device__ __forceinline__ int slab_tri(float lo, float hi, const float* __restr
 // Lane g ends up holding group g's box: it scans group g's bound down the rows (a
 // row's bounds are contiguous), 32 / G rows at a time.
 template <class M>
-__global__ void swept_kernel(const float4* __restrict__ table, const int* __restrict__ offs, int E,
+__global__ void swept_kernel(const float4* __restrict__ table, const int* __restrict__ offs, int E, int cap,
                              float4* __restrict__ swept, int* __restrict__ edge_tri,
                              const float* __restrict__ bounds, float4* __restrict__ mid) {
     constexpr int G = M::num_env_groups;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (warp >= E) return;
+    if (warp >= E || offs[E] > cap) return;
     const int r0 = offs[warp], r1 = offs[warp + 1];
     const DevTables<M>& T = tab<M>();
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -1817,6 +1822,7 @@ __global__ void __launch_bounds__(kProbeThreads, PMIN) probe_kernel(CheckParams 
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
     __shared__ int s_cnt, s_open, s_base, s_item;
+    if (P.offs[P.num_edges] > P.cap_rows) return;
     const int env = env0 + blockIdx.x, e0 = blockIdx.y * Q.batch;
     const int nb = min(Q.batch, P.num_edges - e0);
     const int lane = threadIdx.x & 31;
@@ -2050,7 +2056,7 @@ __global__ void __launch_bounds__(WARPS * 32, check_min_ctas<M, WARPS>()) check_
     __shared__ int s_next;
     const int env = blockIdx.x, tile = blockIdx.y;
     const int n_slots = tile_slots(P, tile);
-    if (n_slots <= 0) return;
+    if (n_slots <= 0 || P.offs[P.num_edges] > P.cap_rows) return;
     const float4 h0 = P.env_hdr[2 * env + 0];
     const float4 h1 = P.env_hdr[2 * env + 1];
     const uint32_t bytes = record_bytes_of(h1);
@@ -2446,6 +2452,7 @@ __global__ void __launch_bounds__(WARPS * 32) check_records_kernel(RecordsParams
     __shared__ uint64_t bar;
     __shared__ float4 boxes[WARPS][G][2];
 
+    if (P.offs[P.num_edges] > P.cap_rows) return;
     const int env = blockIdx.x;
     const int e_begin = blockIdx.y * P.edges_per_cta;
     const int e_end = min(e_begin + P.edges_per_cta, P.num_edges);
@@ -2533,13 +2540,14 @@ cudaError_t run_steps(const PipelineArgs& a, cudaStream_t st) {
     const int E = a.num_edges;
     if (a.stage_events) cudaEventRecord(a.stage_events[0], st);
     if (E <= kFusedSteps) {
-        edge_offsets_kernel<M><<<1, kFusedSteps, 0, st>>>(a.d_edges, E, a.resolution, a.steps, a.offs);
+        edge_offsets_kernel<M><<<1, kFusedSteps, 0, st>>>(a.d_edges, E, a.resolution, a.steps, a.offs,
+                                                                a.host_total);
         return cudaGetLastError();
     }
     edge_steps_kernel<M><<<(E + 255) / 256, 256, 0, st>>>(a.d_edges, E, a.resolution, a.steps);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
-    return launch_scan(a.steps, E, a.offs, st);
+    return launch_scan(a.steps, E, a.offs, a.host_total, st);
 }
 
 // Probe and walk, in slabs of environments whose pairs fit the queue.
@@ -2631,7 +2639,7 @@ cudaError_t check_by_warps(const CheckParams& P, int E, int warps, int mode, cud
 template <class M>
 cudaError_t run_prep(const PipelineArgs& a, cudaStream_t st) {
     const int E = a.num_edges;
-    const int R = a.total_rows;
+    const int R = a.total_rows >= 0 ? a.total_rows : a.cap_rows;  // at most: the kernels read the total
     cudaEvent_t* ev = a.stage_events;
     if (ev) cudaEventRecord(ev[1], st);
     cudaError_t err = cudaMemsetAsync(a.edge_self, 0, sizeof(int) * E, st);
@@ -2649,11 +2657,12 @@ cudaError_t run_prep(const PipelineArgs& a, cudaStream_t st) {
         if (err != cudaSuccess) return err;
         const int blocks = (R + 31) / 32;
         const int grid = std::min(blocks, std::max(per_sm, 1) * std::max(sms, 1));
-        fk_staged_kernel<M><<<grid, 32 * fk_warps<M>(), smem, st>>>(a.d_edges, E, a.steps, a.offs, a.table, a.edge_self, a.seg);
+        fk_staged_kernel<M><<<grid, 32 * fk_warps<M>(), smem, st>>>(a.d_edges, E, a.steps, a.offs, a.cap_rows, a.table,
+                                                                    a.edge_self, a.seg);
     }
     if (ev) cudaEventRecord(ev[2], st);
     if (ev) cudaEventRecord(ev[3], st);
-    swept_kernel<M><<<(E * 32 + 255) / 256, 256, 0, st>>>(a.table, a.offs, E, a.swept,
+    swept_kernel<M><<<(E * 32 + 255) / 256, 256, 0, st>>>(a.table, a.offs, E, a.cap_rows, a.swept,
                                                            a.grid_bounds ? a.edge_tri : nullptr, a.grid_bounds, a.mid);
     if (ev) cudaEventRecord(ev[4], st);
     return cudaGetLastError();

@@ -116,3 +116,37 @@ def test_self_collision_by_segments(checker, name, nedge, resolution):
     want = orc.check(envs, edges, resolution=resolution)
     assert 0 < int(got.sum()) < nedge
     assert len(orc.adjudicate(envs, edges, got, want, resolution=resolution)[2]) == 0
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_tables_of_an_earlier_call_too_small(graph):
+    """A check is queued before its sample total is known to the host, within the
+    tables the calls before it left: growing calls, another robot's wider rows, too
+    many samples (nothing is written) and a small call after them."""
+    import torch
+    from bcc.lib import BccError, Checker
+    chk = Checker(0)
+    envs = workload.gen_envs("uneven", 40, seed=5)
+    chk.upload(envs)
+    for name, n, resolution in (("uneven", 20, 32), ("uneven", 700, 32), ("plain", 300, 64), ("multi_fetch", 400, 32),
+                                ("uneven", 20, 32), ("plain", 600, 200)):
+        robot, edges = workload.robot_of(name), workload.gen_edges(name, n, seed=5)
+        other = Checker(0)
+        other.upload(envs)
+        want = other.check(edges, robot=robot, resolution=resolution)
+        other.close()
+        for _ in range(2):
+            assert np.array_equal(chk.check(edges, robot=robot, resolution=resolution, graph=graph), want)
+    bad = workload.gen_edges("uneven", 50, seed=6)
+    bad[3:8, 1, 2] = np.inf  # 2^20 steps each: beyond the 2^27 samples of a call
+    d_edges = torch.from_numpy(bad).cuda()
+    out = torch.full((50, 40), 7, dtype=torch.uint8, device="cuda")
+    with pytest.raises(BccError):
+        chk.check_device(d_edges.data_ptr(), 50, out.data_ptr(), graph=graph)
+    torch.cuda.synchronize()
+    assert int((out != 7).sum()) == 0
+    edges = workload.gen_edges("uneven", 33, seed=7)
+    a, b = chk.check(edges, graph=graph), chk.check(edges, graph=graph, order="plain")
+    assert np.array_equal(a, b)
+    assert len(orc.adjudicate(envs, edges, a, orc.check(envs, edges))[2]) == 0
+    chk.close()
