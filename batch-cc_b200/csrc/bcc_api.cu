@@ -154,6 +154,8 @@ bool regular_rec(const Rec& r) {
     return true;
 }
 
+size_t aligned(size_t n, size_t to) { return (n + to - 1) / to * to; }
+
 int clamp_tile(int v, int lo, int hi) { return std::max(lo, std::min(hi, v)); }
 
 // Sample rows of a call at most (the sample table's limit).
@@ -250,12 +252,14 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     a.d_edges = d_edges;
     a.num_edges = E;
     a.resolution = resolution;
-    BCC_CUDA(ctx, ctx->steps.ensure(sizeof(int) * (size_t)E));
-    BCC_CUDA(ctx, ctx->offs.ensure(sizeof(int) * ((size_t)E + 1)));
-    BCC_CUDA(ctx, ctx->edge_self.ensure(sizeof(int) * (size_t)E));
+    // Per-edge buffers, one allocation (a first call on new buffers pays for each).
     const int G = ops->num_env_groups;
-    BCC_CUDA(ctx, ctx->swept.ensure(sizeof(float4) * 2 * (size_t)G * E));
-    BCC_CUDA(ctx, ctx->edge_tri.ensure(sizeof(int) * (size_t)G * E));
+    const size_t word = sizeof(int) * aligned((size_t)E + 1, 64);
+    BCC_CUDA(ctx, ctx->per_edge.ensure((3 + (size_t)G) * word));
+    a.steps = ctx->per_edge.as<int>();
+    a.offs = a.steps + word / sizeof(int);
+    a.edge_self = a.offs + word / sizeof(int);
+    a.edge_tri = a.edge_self + word / sizeof(int);
     BCC_CUDA(ctx, ctx->error_flag.ensure(sizeof(int)));
     // Probed checks: grids, middle spheres and the queue, all or none.
     const bcc::Tune tune = launch_shape(ctx, E);
@@ -277,23 +281,22 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
         // items: every full chunk, and one part chunk per probe CTA
         const size_t items = (size_t)(cap / chunk + slab * ((E + batch - 1) / batch));
         a.probe = probe_grid(ctx, ops, st);
-        if (a.probe.vox && ctx->mid.ensure(sizeof(float4) * (size_t)G * E) == cudaSuccess &&
-            ctx->pq_entries.ensure(sizeof(uint2) * (size_t)cap) == cudaSuccess &&
-            ctx->pq_items.ensure(sizeof(int4) * items) == cudaSuccess &&
-            ctx->pq_head.ensure(16 * (size_t)((ctx->num_envs + slab - 1) / slab)) == cudaSuccess) {
-            a.mid = ctx->mid.as<float4>();
-            a.queue = bcc::ProbeQueue{ctx->pq_entries.as<uint2>(), ctx->pq_items.as<int4>(), ctx->pq_head.as<int>(),
-                                      cap, chunk, batch};
+        const size_t mid_bytes = sizeof(float4) * (size_t)G * E, item_bytes = sizeof(int4) * items;
+        const size_t head_bytes = 16 * (size_t)((ctx->num_envs + slab - 1) / slab);
+        if (a.probe.vox &&
+            ctx->queue.ensure(mid_bytes + item_bytes + head_bytes + sizeof(uint2) * (size_t)cap) == cudaSuccess) {
+            a.mid = ctx->queue.as<float4>();
+            a.queue.items = reinterpret_cast<int4*>(ctx->queue.as<char>() + mid_bytes);
+            a.queue.head = reinterpret_cast<int*>(ctx->queue.as<char>() + mid_bytes + item_bytes);
+            a.queue.entries = reinterpret_cast<uint2*>(ctx->queue.as<char>() + mid_bytes + item_bytes + head_bytes);
+            a.queue.cap = cap;
+            a.queue.chunk = chunk;
+            a.queue.batch = batch;
         } else {
             cudaGetLastError();  // no memory for it: one pass over all pairs
             a.probe = bcc::ProbeGrid{};
         }
     }
-    a.steps = ctx->steps.as<int>();
-    a.offs = ctx->offs.as<int>();
-    a.edge_self = ctx->edge_self.as<int>();
-    a.swept = ctx->swept.as<float4>();
-    a.edge_tri = ctx->edge_tri.as<int>();
     a.grid_bounds = ctx->grid_bounds.as<float>();
     a.error_flag = ctx->error_flag.as<int>();
     a.stage_events = ctx->profiling ? ctx->ev : nullptr;
@@ -539,7 +542,7 @@ bool same_tune(const bcc::Tune& x, const bcc::Tune& y) {
 // sizes, orders or robots in between may have replaced some.
 bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
     return x.steps == y.steps && x.offs == y.offs && x.table == y.table && x.seg == y.seg &&
-           x.edge_self == y.edge_self && x.swept == y.swept && x.edge_tri == y.edge_tri &&
+           x.edge_self == y.edge_self && x.edge_tri == y.edge_tri &&
            x.grid_bounds == y.grid_bounds && x.blobs == y.blobs && x.env_hdr == y.env_hdr && x.mid == y.mid &&
            x.probe.vox == y.probe.vox && x.queue.entries == y.queue.entries && x.queue.items == y.queue.items &&
            x.queue.head == y.queue.head && x.queue.chunk == y.queue.chunk && x.queue.batch == y.queue.batch && x.warps == y.warps &&

@@ -95,7 +95,7 @@ struct bcc_ctx {
     bcc::DevBuf blobs, env_hdr;
     bcc::DevBuf records;     // the upload's records as packed, source of the blobs
     // per-call buffers
-    bcc::DevBuf edges, steps, offs, table, edge_self, swept, results, error_flag;
+    bcc::DevBuf edges, per_edge, table, results, error_flag;  // per_edge: steps, offs, edge_self, edge_tri
     int* h_total = nullptr;  // pinned: the sample-row total, written by the offset kernel
     cudaEvent_t ev_total = nullptr;  // ... once this has passed
     bool profiling = false;
@@ -104,10 +104,8 @@ struct bcc_ctx {
     cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     // learned proposal
     bcc::MlpState mlp;
-    bcc::DevBuf edge_tri;    // [E][groups] packed slab ranges of each group's swept box
     bcc::DevBuf grid_bounds; // [3][kGridSlabs + 1] slab boundaries of the uploaded set's cull grid
-    bcc::DevBuf mid;         // [groups][E] probe spheres around the edges' middle samples
-    bcc::DevBuf pq_entries, pq_items, pq_head;  // queue of the pairs a probe leaves undecided
+    bcc::DevBuf queue;       // probe spheres of the edges' middle samples, and the queue of undecided pairs
     bcc::DevBuf vox;         // probe grids of the uploaded set
     bcc::ProbeGrid probe{};  // ... their shape (vox null: none)
     int probe_robot = -1;    // ... the robot and upload they were built for

@@ -67,7 +67,6 @@ struct CheckParams {
     const int* offs;         // [E + 1] first sample row of each edge
     int cap_rows;            // nothing is checked when offs[E] exceeds it (the tables do not hold them)
     const float4* table;     // [rows][num_spheres] sphere centres + radius
-    const float4* swept;     // [E][groups][2] cull AABB centre / half-size
     const float2* seg;       // [rows / kSegment][groups] segment spheres (plain and inline learned walks)
     const int* edge_tri;     // [E][groups] slab ranges on the set's grid (tx | ty << 10 | tz << 20), -1 = none
     const int* edge_self;    // [E] 1 when some sample self-collides
@@ -116,7 +115,7 @@ struct PipelineArgs {
     float4* table;           // [total_rows][num_spheres]
     float2* seg;             // [total_rows / kSegment][groups] segment spheres, null = not needed
     int* edge_self;          // [E]
-    float4* swept;           // [E][groups][2]
+    float4* swept;           // [E][groups][2], null = not needed
     int* edge_tri;           // [E][groups], null = not needed (records check)
     ProbeGrid probe;
     ProbeQueue queue;
@@ -254,7 +253,6 @@ inline CheckParams params_of(const PipelineArgs& a) {
     P.offs = a.offs;
     P.cap_rows = a.cap_rows;
     P.table = a.table;
-    P.swept = a.swept;
     P.seg = a.seg;
     P.edge_tri = a.edge_tri;
     P.edge_self = a.edge_self;

@@ -769,7 +769,7 @@ __device__ __forceinline__ int slab_tri(float lo, float hi, const float* __restr
 
 // One warp per edge: AABB (lo, hi) of every link group's bounding sphere over
 // the edge's samples, inflated by radius + 0.005 + the group's leaf overhang +
-// cull margin; and (edge_tri non-null) its slab ranges on the set's cull grid,
+// cull margin, written where swept is given (the records check); and (edge_tri non-null) its slab ranges on the set's cull grid,
 // packed tx | ty << 10 | tz << 20 (-1 when some axis misses every primitive);
 // and (mid non-null) the bound's centre at the edge's middle sample with the
 // radius, inflated likewise, of the sphere around it that holds them all; and
@@ -823,8 +823,10 @@ __global__ void swept_kernel(const float4* __restrict__ table, const int* __rest
     }
     const float4 l = make_float4(lo[0] - pad, lo[1] - pad, lo[2] - pad, 0.0f);
     const float4 h = make_float4(hi[0] + pad, hi[1] + pad, hi[2] + pad, 0.0f);
-    swept[((size_t)warp * G + g) * 2 + 0] = l;
-    swept[((size_t)warp * G + g) * 2 + 1] = h;
+    if (swept) {
+        swept[((size_t)warp * G + g) * 2 + 0] = l;
+        swept[((size_t)warp * G + g) * 2 + 1] = h;
+    }
     if (edge_tri) {
         const int tx = slab_tri(l.x, h.x, bounds);
         const int ty = slab_tri(l.y, h.y, bounds + (kGridSlabs + 1));
