@@ -50,9 +50,8 @@ constexpr uint32_t kImagesBytes = kImagesW + 3 * kImgSmall;  // ... | W4 | B2 | 
 constexpr int kBiasCol = kMlpIn - 1;                        // feature 47: reserved, read as 1 by the forward kernel
 
 // Shared-memory map of the forward kernel (bytes): the images, the ones image
-// (A operand of the bias MMAs), then per row group one buffer for its X tile
-// (128 x 48) and, once the first MMA has consumed X, its H tile (128 x 128),
-// b4, the groups' mbarriers and the TMEM address slot.
+// (A operand of the bias MMAs), then per row group its X tile (128 x 48), b4, the
+// groups' mbarriers and the TMEM address slot.
 constexpr uint32_t kSmW1 = 0;
 constexpr uint32_t kSmW2 = kSmW1 + kImgW1;
 constexpr uint32_t kSmW3 = kSmW2 + kImgW;
@@ -60,12 +59,15 @@ constexpr uint32_t kSmW4 = kSmW3 + kImgW;
 constexpr uint32_t kSmB2 = kSmW4 + kImgSmall;
 constexpr uint32_t kSmB3 = kSmB2 + kImgSmall;
 constexpr uint32_t kSmOnes = kSmB3 + kImgSmall;
-constexpr int kFwdGroups = 4;                              // independent 128-row tile streams per CTA
-constexpr uint32_t kFwdTmemCols = 512;                     // power of two >= 128 x groups
-// Group g's buffer at kSmGroup0 + g * stride holds its X tile (128 x 48) until
-// the first layer's MMA has read it, then its H tile (128 x 128).
+constexpr int kFwdGroups = 2;                              // independent 128-row tile streams per CTA
+constexpr int kFwdGroupThreads = 256;                      // two threads a row
+// Tensor memory of group g, columns 256 g ..: the accumulator (128), H as the next
+// layer's A operand (64, two BF16 values a column), the logits' accumulator (16).
+constexpr uint32_t kFwdTmemCols = 512;
+constexpr uint32_t kFwdH = kMlpHidden;
+constexpr uint32_t kFwdC = kFwdH + kMlpHidden / 2;
 constexpr uint32_t kSmGroup0 = kSmOnes + kImgSmall;
-constexpr uint32_t kSmGroupStride = kImgW;
+constexpr uint32_t kSmGroupStride = kImgW1;
 constexpr uint32_t kSmVec = kSmGroup0 + kFwdGroups * kSmGroupStride;  // b4
 constexpr uint32_t kSmBar = kSmVec + 16;
 constexpr uint32_t kSmTmem = kSmBar + 8 * kFwdGroups;
@@ -119,55 +121,52 @@ __device__ __forceinline__ uint32_t relu_bf16x2(float lo, float hi) {
 }
 
 // Forward epilogue of a hidden layer whose bias the MMAs already added: this
-// thread's accumulator row, ReLU, BF16 into the H image (one conversion per
-// two values).  Two 16-column loads are in flight before each wait.
-__device__ __forceinline__ void epilogue_relu_only(uint32_t taddr, uint8_t* himg, int row) {
-#pragma unroll 1
-    for (int c0 = 0; c0 < kMlpHidden; c0 += 32) {
-        float v[32];
-        tc::tmem_ld16(taddr + c0, v);
-        tc::tmem_ld16(taddr + c0 + 16, v + 16);
-        tc::wait_ld();
+// thread's half (64 columns) of its accumulator row, ReLU, BF16 into the H columns
+// (one conversion per two values).
+__device__ __forceinline__ void epilogue_relu_only(uint32_t acc, uint32_t h) {
+    float v[64];
+    uint32_t w[32];
+    tc::tmem_ld64(acc, v);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            uint4 w;
-            w.x = relu_bf16x2(v[8 * q + 0], v[8 * q + 1]);
-            w.y = relu_bf16x2(v[8 * q + 2], v[8 * q + 3]);
-            w.z = relu_bf16x2(v[8 * q + 4], v[8 * q + 5]);
-            w.w = relu_bf16x2(v[8 * q + 6], v[8 * q + 7]);
-            *reinterpret_cast<uint4*>(himg + tc::cm_offset(row, c0 + 8 * q, kMlpHidden)) = w;
-        }
-    }
+    for (int i = 0; i < 32; ++i) w[i] = relu_bf16x2(v[2 * i], v[2 * i + 1]);
+    tc::tmem_st32(h, w);
+    tc::wait_st();
 }
 
-// Barrier of one 128-thread warp group (named barrier 1 + group).
-__device__ __forceinline__ void group_sync(int grp) {
-    asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-}
-
-// Barrier of one warp group that also ORs a predicate over its threads.
+// Barrier of one warp group (named barrier 1 + group) that also ORs a predicate
+// over its threads.
 __device__ __forceinline__ bool group_sync_or(bool pred, int grp) {
     uint32_t r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, %2, 128, p;\n\t"
+        "bar.red.or.pred q, %2, %3, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"((uint32_t)pred), "r"(1 + grp)
+        : "r"((uint32_t)pred), "r"(1 + grp), "n"(kFwdGroupThreads)
         : "memory");
     return r != 0;
 }
 
-// Persistent: each CTA loads the weights once; its four warp groups (4 warps,
-// one row per thread each) run independent streams of 128-row tiles, each with
-// its own X/H buffer, TMEM accumulator (columns 128 g ..) and mbarrier, so one
-// group's MMAs overlap the others' epilogues (all 512 TMEM columns in use).  The biases ride in the MMAs (b1
-// as column 47 of W1^T against feature 47 read as 1; b2, b3 by a K = 16 MMA of
-// a ones column against B2 / B3) and the output layer is an N = 16 MMA against
-// W4, so each hidden epilogue is only ReLU + BF16 conversion + store.  x: BF16
+// Persistent: each CTA loads the weights once; its two warp groups (8 warps, two
+// threads a row) run independent streams of 128-row tiles, each with its own X
+// buffer, TMEM columns and mbarrier, so one group's MMAs overlap the other's
+// epilogues.  The biases ride in the MMAs (b1 as column 47 of W1^T against feature
+// 47 read as 1; b2, b3 by a K = 16 MMA of a ones column against B2 / B3) and the
+// output layer is an N = 16 MMA against W4, issued together with the next tile's
+// first layer, so a tile is three rounds of MMAs and epilogues.  x: BF16
 // [rows][48] row-major (feature 47 zero); logits: FP32 [rows].
-__global__ void __launch_bounds__(128 * kFwdGroups, 1)
+//
+// H lives in tensor memory as the A operand of layers 2 to 4.  With H in shared
+// memory a 128 x 128 x 16 MMA read 8 KB of operands, and with the epilogue's
+// stores a tile took 2500 cycles of the shared memory's 128 B a cycle: 109 us for
+// 1 000 003 rows.  Without, it takes 960 of a stream's 3 x 1800, and 89 us; the
+// MMAs alone would take 1400 a tile.  A stage's chain bounds it: 440 cycles around
+// its MMAs, 160 of epilogue, 130 of barrier, and the other stream's MMAs.  So the
+// logits and the next X are written behind the second layer's MMAs (98 us before
+// them).  Four streams of 128 columns, layers in two halves of 64 outputs, spilled
+// and took 113 us.
+__global__ void __launch_bounds__(kFwdGroupThreads * kFwdGroups, 1)
     mlp_forward_kernel(const uint16_t* __restrict__ x, int rows, const int* __restrict__ rows_dev,
                        const uint4* __restrict__ images, const float* __restrict__ params, float* __restrict__ logits,
                        int* __restrict__ err) {
@@ -177,12 +176,12 @@ __global__ void __launch_bounds__(128 * kFwdGroups, 1)
     // device count leave before loading the weights.
     if ((long long)blockIdx.x * kFwdGroups * 128 >= (long long)rows) return;
     extern __shared__ __align__(1024) uint8_t sm[];
-    const int t = threadIdx.x, warp = t >> 5, grp = t >> 7, gt = t & 127;
+    const int t = threadIdx.x, warp = t >> 5, grp = t / kFwdGroupThreads, gt = t % kFwdGroupThreads;
+    const int r = gt & 127, half = gt >> 7;
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kSmBar) + grp;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + kSmTmem);
     float* vec = reinterpret_cast<float*>(sm + kSmVec);
     uint8_t* xs = sm + kSmGroup0 + grp * kSmGroupStride;
-    uint8_t* hs = xs;  // H overwrites X once the first layer's MMA has read it
 
     for (uint32_t i = t; i < kImagesBytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(sm)[i] = images[i];
     if (t < 128) {  // ones image [128][16]: column 0 = 1 (BF16 0x3f80), the rest 0
@@ -195,10 +194,11 @@ __global__ void __launch_bounds__(128 * kFwdGroups, 1)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tc::tmem_alloc(tmem_slot, kFwdTmemCols);
+    tc::fence_async_smem();
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t tmem = *tmem_slot + 128u * grp;
+    const uint32_t tmem = *tmem_slot + 256u * grp;
     const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     const uint32_t idesc = tc::make_idesc_bf16(128, kMlpHidden, 0, 0);
     const uint32_t idesc16 = tc::make_idesc_bf16(128, 16, 0, 0);
@@ -210,71 +210,106 @@ __global__ void __launch_bounds__(128 * kFwdGroups, 1)
     const int tiles = (rows + 127) / 128;
     const int tile_step = gridDim.x * kFwdGroups;
     // X rows are loaded one tile ahead into registers, so their latency overlaps
-    // the current tile's layers.
-    uint4 xv[kMlpIn / 8];
+    // the current tile's layers: half a row a thread, three 16-byte chunks.
+    constexpr int kChunks = kMlpIn / 16;
+    static_assert(kMlpIn % 16 == 0 && kBiasCol == kMlpIn - 1, "the bias feature is the last of the row's last chunk");
+    uint4 xv[kChunks];
     auto load_x = [&](int tile) {
-        const int row = tile * 128 + gt;
-        const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * kMlpIn);
+        const int row = tile * 128 + r;
+        const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * kMlpIn) + kChunks * half;
 #pragma unroll
-        for (int j = 0; j < kMlpIn / 8; ++j) xv[j] = (tile < tiles && row < rows) ? src[j] : make_uint4(0, 0, 0, 0);
+        for (int j = 0; j < kChunks; ++j) xv[j] = (tile < tiles && row < rows) ? src[j] : make_uint4(0, 0, 0, 0);
     };
-    static_assert(kBiasCol == kMlpIn - 1, "the bias feature is the last of the row's last 16-byte chunk");
-    load_x(blockIdx.x * kFwdGroups + grp);
-    for (int tile = blockIdx.x * kFwdGroups + grp; tile < tiles && !bad; tile += tile_step) {
-        const int row = tile * 128 + gt;
-        // X tile: this thread's row, six 16-byte chunks of 8 features; feature 47
-        // (zero in the input) is read as 1 to pick up b1 from W1^T's column 47.
-        xv[kMlpIn / 8 - 1].w = (xv[kMlpIn / 8 - 1].w & 0xffffu) | 0x3f800000u;
+    // ... into the X buffer; feature 47 (zero in the input) is read as 1 to pick up
+    // b1 from W1^T's column 47.
+    auto store_x = [&] {
+        if (half) xv[kChunks - 1].w = (xv[kChunks - 1].w & 0xffffu) | 0x3f800000u;
 #pragma unroll
-        for (int j = 0; j < kMlpIn / 8; ++j) *reinterpret_cast<uint4*>(xs + tc::cm_offset(gt, 8 * j, kMlpIn)) = xv[j];
+        for (int j = 0; j < kChunks; ++j)
+            *reinterpret_cast<uint4*>(xs + tc::cm_offset(r, 8 * (kChunks * half + j), kMlpIn)) = xv[j];
+        tc::fence_async_smem();
+    };
+    // MMAs of a stage, by the group's first thread.
+    auto first_layer = [&] {
+        const uint32_t a0 = tc::smem_addr(xs), b0 = sbase + kSmW1;
+        constexpr uint32_t sbo = (uint32_t)(kMlpIn / 8) * 128u;
+        for (int s = 0; s < kMlpIn / 16; ++s)
+            tc::mma_bf16(tmem, tc::make_desc(a0 + 256u * s, 128u, sbo), tc::make_desc(b0 + 256u * s, 128u, sbo), idesc,
+                         s > 0 ? 1u : 0u);
+    };
+    auto h_layer = [&](uint32_t d, uint32_t b0, uint32_t id) {
+        constexpr uint32_t sbo = (uint32_t)(kMlpHidden / 8) * 128u;
+        for (int s = 0; s < kMlpHidden / 16; ++s)
+            tc::mma_bf16_ts(d, tmem + kFwdH + 8u * s, tc::make_desc(b0 + 256u * s, 128u, sbo), id, s > 0 ? 1u : 0u);
+    };
+    // Waits for the stage in flight (once a wait has run out, for none).
+    auto await = [&] {
+        if (!bad) bad = !mbar_wait_bounded(bar, phase, 1u << 22);
+        if (!bad) phase ^= 1u;
+        tc::fence_after();
+    };
+    auto write_logits = [&](int tile) {
+        if (half) return;  // whole warps
+        const float z = tc::tmem_ld1(taddr + kFwdC);
+        tc::wait_ld();
+        const int row = tile * 128 + r;
+        if (!bad && row < rows) logits[row] = z + b4;
+    };
+
+    int tile = blockIdx.x * kFwdGroups + grp, done = -1;  // done: the tile whose logits are in flight
+    bool stop = tile >= tiles;
+    if (!stop) {
+        load_x(tile);
+        store_x();
         load_x(tile + tile_step);
-        // Four MMA stages (three hidden layers, the output layer): MMAs from the
-        // group's first thread, epilogue from all.
+        tc::fence_before();
+        group_sync_or(false, grp);
+        if (gt == 0) {
+            tc::fence_after();
+            first_layer();
+            tc::commit(bar);
+        }
+    }
+    for (; !stop && tile < tiles; tile += tile_step) {
+        const int next = tile + tile_step;
 #pragma unroll 1
-        for (int layer = 0; layer < 4; ++layer) {
-            tc::fence_async_smem();
+        for (int layer = 1; layer < 4; ++layer) {
+            await();
+            epilogue_relu_only(taddr + 64u * half, taddr + kFwdH + 32u * half);
             tc::fence_before();
-            group_sync(grp);
+            if (group_sync_or(bad, grp)) {  // group-uniform decision
+                bad = stop = true;
+                break;
+            }
             if (gt == 0) {
                 tc::fence_after();
-                if (layer == 0) {
-                    const uint32_t a0 = tc::smem_addr(xs), b0 = sbase + kSmW1;
-                    constexpr uint32_t sbo = (uint32_t)(kMlpIn / 8) * 128u;
-                    for (int s = 0; s < kMlpIn / 16; ++s)
-                        tc::mma_bf16(tmem, tc::make_desc(a0 + 256u * s, 128u, sbo),
-                                     tc::make_desc(b0 + 256u * s, 128u, sbo), idesc, s > 0 ? 1u : 0u);
+                if (layer < 3) {
+                    h_layer(tmem, sbase + (layer == 1 ? kSmW2 : kSmW3), idesc);
+                    // + bias: ones [128][16] x B [128][16]^T
+                    tc::mma_bf16(tmem, tc::make_desc(sbase + kSmOnes, 128u, 256u),
+                                 tc::make_desc(sbase + (layer == 1 ? kSmB2 : kSmB3), 128u, 256u), idesc, 1u);
                 } else {
-                    const uint32_t a0 = tc::smem_addr(hs);
-                    const uint32_t b0 = sbase + (layer == 1 ? kSmW2 : layer == 2 ? kSmW3 : kSmW4);
-                    constexpr uint32_t sbo = (uint32_t)(kMlpHidden / 8) * 128u;
-                    for (int s = 0; s < kMlpHidden / 16; ++s)
-                        tc::mma_bf16(tmem, tc::make_desc(a0 + 256u * s, 128u, sbo),
-                                     tc::make_desc(b0 + 256u * s, 128u, sbo), layer == 3 ? idesc16 : idesc,
-                                     s > 0 ? 1u : 0u);
-                    if (layer < 3)  // + bias: ones [128][16] x B [128][16]^T
-                        tc::mma_bf16(tmem, tc::make_desc(sbase + kSmOnes, 128u, 256u),
-                                     tc::make_desc(sbase + (layer == 1 ? kSmB2 : kSmB3), 128u, 256u), idesc, 1u);
+                    h_layer(tmem + kFwdC, sbase + kSmW4, idesc16);
+                    if (next < tiles) first_layer();
                 }
                 tc::commit(bar);
             }
-            const bool ok = mbar_wait_bounded(bar, phase, 1u << 22);
-            if (group_sync_or(!ok, grp)) {  // group-uniform decision
-                bad = true;
-                break;
-            }
-            phase ^= 1u;
-            tc::fence_after();
-            if (layer < 3) {
-                epilogue_relu_only(taddr, hs, gt);
-            } else {
-                const float z = tc::tmem_ld1(taddr);
-                tc::wait_ld();
-                if (row < rows) logits[row] = z + b4;
+            if (layer == 1) {  // behind these MMAs: the last tile's logits, the next tile's X
+                if (done >= 0) write_logits(done);
+                store_x();
+                load_x(next + tile_step);
             }
         }
+        done = tile;
     }
-    if (bad && gt == 0) atomicOr(err, 1);
-    if (bad) mbar_wait_bounded(bar, phase, 1u << 22);  // let in-flight MMAs finish before freeing TMEM
+    if (done >= 0 && !stop) {
+        await();
+        write_logits(done);
+    }
+    if (bad) {
+        atomicOr(err, 1);
+        mbar_wait_bounded(bar, phase, 1u << 22);  // let in-flight MMAs finish before freeing TMEM
+    }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
@@ -682,7 +717,7 @@ cudaError_t mlp_forward(const uint16_t* d_x, int rows, const uint8_t* d_images, 
     const int tiles = (rows + 127) / 128;
     const int ctas = (tiles + kFwdGroups - 1) / kFwdGroups;
     const int grid = ctas < num_sms ? ctas : num_sms;
-    mlp_forward_kernel<<<grid, 128 * kFwdGroups, kFwdSmem, st>>>(d_x, rows, d_rows,
+    mlp_forward_kernel<<<grid, kFwdGroupThreads * kFwdGroups, kFwdSmem, st>>>(d_x, rows, d_rows,
                                                                  reinterpret_cast<const uint4*>(d_images), d_params,
                                                                  d_logits, d_err);
     return cudaGetLastError();

@@ -34,6 +34,33 @@ def test_mlp_forward_matches_reference(checker):
     assert np.allclose(checker.mlp_get_params(), p)
 
 
+@pytest.mark.parametrize("rows", [1, 127, 129, 256, 257, 2 * 148 * 128, 2 * 148 * 128 + 1, 5 * 148 * 128 + 77])
+def test_mlp_forward_at_tile_edges(checker, rows):
+    """One row, the edges of a 128-row tile, one and two tiles of a CTA's two
+    streams, one tile a stream over all CTAs and one more, streams of two and three
+    tiles: every logit against the reference (2e-2: BF16 operands, as above), its
+    neighbour past the end untouched."""
+    import torch
+    rng = np.random.default_rng(rows)
+    p = mlp.init_params(3)
+    P = mlp.unflatten(p)
+    for b in ("b1", "b2", "b3"):
+        P[b][:] = rng.normal(0, 0.1, 128)
+    P["b4"][:] = -0.2
+    checker.mlp_set_params(p)
+    x = rng.normal(0, 1, (rows, 48)).astype(np.float32)
+    x[:, 39:] = 0
+    xb = torch.from_numpy(mlp.to_bf16_bits(x).view(np.int16)).cuda()
+    out = torch.full((rows + 1,), 7.5, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    checker.mlp_forward_device(xb.data_ptr(), rows, out.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    want = mlp.forward_reference(p, x)
+    assert got[rows] == 7.5
+    assert np.abs(got[:rows] - want).max() < 2e-2 * (np.abs(want).max() + 1.0)
+
+
 def test_mlp_gradients_match_cpu_oracle(checker):
     """Tensor-core training kernel gradients vs the FP64 CPU oracle."""
     import torch
