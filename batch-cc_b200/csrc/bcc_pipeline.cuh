@@ -1808,19 +1808,19 @@ __device__ __forceinline__ bool probe_leaves(const CheckParams& P, int e, unsign
 }
 
 // First pass of a check with probe grids: CTA = one environment x Q.batch
-// edges, one lane per pair.  Decided pairs get their verdict; the others go to
-// the queue (Q) as (edge, alive groups), contiguous per CTA, with one work item
-// per Q.chunk of them.  On the uneven Panda workload (1000 x 10000) it decides
-// 84 % of the pairs in 0.33 ms, 29 warp instructions a pair, bound by issue;
-// walking every pair took 390 instructions a pair and 4.2 ms, probe and walk
-// take 1.4 ms.
+// edges, one lane per pair (probe_pair), then one warp per undecided pair
+// (probe_leaves).  Decided pairs get their verdict; the others go to the queue (Q)
+// as (edge, alive groups), contiguous per CTA, with one work item per Q.chunk of
+// them.  Bound by instruction issue.  On the uneven Panda workload (1000 x 10000)
+// walking every pair took 390 warp instructions a pair and 4.2 ms.  The bounds
+// alone decide 84 % of the pairs in 0.33 ms (29 instructions a pair), probe and walk
+// 1.38 ms; the leaves settle two thirds of the colliding rest: 0.70 ms (58 a pair),
+// probe and walk 1.19 ms.  Five CTAs an SM against four: 1.19 and 1.23 ms.
 constexpr int kProbeThreads = 256;
+constexpr int kProbeCtas = 5;
 
 template <class M>
-#ifndef PMIN
-#define PMIN 5
-#endif
-__global__ void __launch_bounds__(kProbeThreads, PMIN) probe_kernel(CheckParams P, ProbeQueue Q, int env0) {
+__global__ void __launch_bounds__(kProbeThreads, kProbeCtas) probe_kernel(CheckParams P, ProbeQueue Q, int env0) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t bar;
     __shared__ int s_cnt, s_open, s_base, s_item;
@@ -1932,7 +1932,8 @@ __global__ void __launch_bounds__(kProbeThreads, PMIN) probe_kernel(CheckParams 
 
 // Resident warps per SM the walk is compiled for: 48 registers a thread.  Swept
 // on 1000 x 20000 stress pairs: 5.97 ms at 48 warps, 5.16 at 40, 5.73 at 32,
-// 6.34 at 24 (probe 0.77 ms included).
+// 6.34 at 24 (with a probe of 0.77 ms by the bounds alone; 4.78 since the probe
+// tests leaves too).
 constexpr int kWalkWarps = 40;
 
 template <class M, int WARPS>
