@@ -157,58 +157,97 @@ cudaError_t launch_build_arena(const float4* records, const float4* env_hdr, con
 }
 
 // ------------------------------------------------------------------ probe grid
-// One thread per voxel: the signed distance of the voxel's centre to every
-// primitive (outside: to the rounded box; inside: minus the depth), the nearest
-// one and its quantised distance.
-// Bound by FP32 issue: ~35 instructions a (voxel, primitive), the record read
-// as a shared-memory broadcast.
+// Per voxel the signed distance of its centre to every primitive (outside: to the
+// rounded box; inside: minus the depth), the nearest one and its quantised distance.
+// One warp per brick of 4 x 4 x 2 voxels.  Distances are 1-Lipschitz (where they are
+// not, kEnvIrregular, the grid is not read): lanes over the primitives, those within
+// twice the brick's radius of the nearest one to its centre can be nearest to a
+// voxel, and only they are tested by the lanes as voxels.
+// Bound by FP32 issue, ~35 instructions a test, the record read as a shared-memory
+// broadcast: 0.37 ms for 1000 environments of 8 .. 64 primitives, 0.53 for 500 of 16 .. 256,
+// against 0.76 and 1.48 for every voxel against every primitive.
 constexpr int kGridThreads = 256;
 constexpr int kGridChunk = 128;  // records staged at a time
+constexpr int kBrickX = 4, kBrickY = 4, kBrickZ = 2;
+static_assert(kBrickX * kBrickY * kBrickZ == 32, "a lane a voxel");
+
+__device__ __forceinline__ float prim_signed_dist(const float4* rec, float x, float y, float z) {
+    const float4 w0 = rec[0], w1 = rec[1], w2 = rec[2], w3 = rec[3];
+    const float dx = x - w0.x, dy = y - w0.y, dz = z - w0.z;
+    const float p1 = fabsf(fmaf(w1.x, dx, fmaf(w1.y, dy, w1.z * dz))) - w1.w;
+    const float p2 = fabsf(fmaf(w2.x, dx, fmaf(w2.y, dy, w2.z * dz))) - w2.w;
+    const float p3 = fabsf(fmaf(w3.x, dx, fmaf(w3.y, dy, w3.z * dz))) - w3.w;
+    const float e1 = fmaxf(p1, 0.0f), e2 = fmaxf(p2, 0.0f), e3 = fmaxf(p3, 0.0f);
+    const float in = fminf(fmaxf(p1, fmaxf(p2, p3)), 0.0f);
+    return sqrtf(fmaf(e1, e1, fmaf(e2, e2, e3 * e3))) + in - w0.w;
+}
+
+__device__ __host__ __forceinline__ int grid_bricks(const ProbeGrid& p) {
+    return (p.nx + kBrickX - 1) / kBrickX * ((p.ny + kBrickY - 1) / kBrickY) * ((p.nz + kBrickZ - 1) / kBrickZ);
+}
 
 __global__ void __launch_bounds__(kGridThreads) probe_grid_kernel(const float4* __restrict__ blobs,
                                                                   const float4* __restrict__ hdr, ProbeGrid p,
                                                                   uint16_t* __restrict__ vox) {
     __shared__ float4 rec[kGridChunk * 4];
-    const int env = blockIdx.x, nv = p.nx * p.ny * p.nz;
-    const int v = blockIdx.y * kGridThreads + threadIdx.x;
+    constexpr int kSteps = kGridChunk / 32;
+    const int env = blockIdx.x, lane = threadIdx.x & 31;
+    const int brick = blockIdx.y * (kGridThreads / 32) + (threadIdx.x >> 5);
     const float4 h0 = hdr[2 * env], h1 = hdr[2 * env + 1];
     const float4* src = blobs + __float_as_uint(h0.w);
     const int np = (int)(__float_as_uint(h1.w) & 0xffffu);
-    uint16_t* dst = vox + (size_t)env * (p.stride / 2);
-    const int ix = v % p.nx, iy = (v / p.nx) % p.ny, iz = v / (p.nx * p.ny);
+    const int bx = (p.nx + kBrickX - 1) / kBrickX, by = (p.ny + kBrickY - 1) / kBrickY;
+    const int x0 = brick % bx * kBrickX, y0 = brick / bx % by * kBrickY, z0 = brick / (bx * by) * kBrickZ;
+    const int ix = x0 + lane % kBrickX, iy = y0 + lane / kBrickX % kBrickY, iz = z0 + lane / (kBrickX * kBrickY);
     const float x = fmaf((float)ix, p.h, p.ox), y = fmaf((float)iy, p.h, p.oy), z = fmaf((float)iz, p.h, p.oz);
-    float best = INFINITY;
+    const float cx = fmaf((float)x0 + 0.5f * (kBrickX - 1), p.h, p.ox);
+    const float cy = fmaf((float)y0 + 0.5f * (kBrickY - 1), p.h, p.oy);
+    const float cz = fmaf((float)z0 + 0.5f * (kBrickZ - 1), p.h, p.oz);
+    // twice half a brick's diagonal, from voxel centre to voxel centre
+    const float span = p.h * sqrtf((kBrickX - 1) * (kBrickX - 1) + (kBrickY - 1) * (kBrickY - 1) +
+                                   (kBrickZ - 1) * (kBrickZ - 1));
+    float best = INFINITY, near = INFINITY;
     unsigned id = 0u;
     for (int p0 = 0; p0 < np; p0 += kGridChunk) {
         const int m = min(kGridChunk, np - p0);
         __syncthreads();
         for (int i = threadIdx.x; i < m * 4; i += kGridThreads) rec[i] = src[(size_t)(p0 + i / 4) * kPrimF4 + (i & 3)];
         __syncthreads();
-        for (int k = 0; k < m; ++k) {
-            const float4 w0 = rec[4 * k], w1 = rec[4 * k + 1], w2 = rec[4 * k + 2], w3 = rec[4 * k + 3];
-            const float dx = x - w0.x, dy = y - w0.y, dz = z - w0.z;
-            const float p1 = fabsf(fmaf(w1.x, dx, fmaf(w1.y, dy, w1.z * dz))) - w1.w;
-            const float p2 = fabsf(fmaf(w2.x, dx, fmaf(w2.y, dy, w2.z * dz))) - w2.w;
-            const float p3 = fabsf(fmaf(w3.x, dx, fmaf(w3.y, dy, w3.z * dz))) - w3.w;
-            const float e1 = fmaxf(p1, 0.0f), e2 = fmaxf(p2, 0.0f), e3 = fmaxf(p3, 0.0f);
-            const float in = fminf(fmaxf(p1, fmaxf(p2, p3)), 0.0f);
-            const float d = sqrtf(fmaf(e1, e1, fmaf(e2, e2, e3 * e3))) + in - w0.w;
-            if (d < best) {
-                best = d;
-                id = (unsigned)(p0 + k);
+        float d[kSteps];
+#pragma unroll
+        for (int s = 0; s < kSteps; ++s) {
+            d[s] = INFINITY;
+            if (32 * s + lane < m) d[s] = prim_signed_dist(rec + 4 * (32 * s + lane), cx, cy, cz);
+            near = fminf(near, d[s]);
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) near = fminf(near, __shfl_xor_sync(0xffffffffu, near, o));
+        // (a margin over FP32 rounding of the distances)
+        const float reach = near + span + 1e-4f + 1e-5f * fabsf(near);
+#pragma unroll
+        for (int s = 0; s < kSteps; ++s) {
+            unsigned todo = __ballot_sync(0xffffffffu, 32 * s + lane < m && d[s] <= reach);
+            for (; todo; todo &= todo - 1u) {
+                const int k = 32 * s + __ffs(todo) - 1;
+                const float v = prim_signed_dist(rec + 4 * k, x, y, z);
+                if (v < best) {
+                    best = v;
+                    id = (unsigned)(p0 + k);
+                }
             }
         }
     }
-    if (v >= nv) return;
+    if (ix >= p.nx || iy >= p.ny || iz >= p.nz) return;
     const float q = (best - kVoxMin) * (1.0f / kVoxStep);
     const unsigned code = (unsigned)(int)fminf(fmaxf(floorf(q), 0.0f), 255.0f);
-    dst[v] = (uint16_t)(min(id, kVoxUnknown) << 8 | code);
+    vox[(size_t)env * (p.stride / 2) + ((size_t)iz * p.ny + iy) * p.nx + ix] =
+        (uint16_t)(min(id, kVoxUnknown) << 8 | code);
 }
 
 cudaError_t launch_probe_grid(const float4* blobs, const float4* env_hdr, int num_envs, const ProbeGrid& p,
                               uint16_t* vox, cudaStream_t st) {
     if (num_envs <= 0) return cudaSuccess;
-    const dim3 grid((unsigned)num_envs, (unsigned)((p.nx * p.ny * p.nz + kGridThreads - 1) / kGridThreads));
+    const dim3 grid((unsigned)num_envs, (unsigned)((grid_bricks(p) + kGridThreads / 32 - 1) / (kGridThreads / 32)));
     probe_grid_kernel<<<grid, kGridThreads, 0, st>>>(blobs, env_hdr, p, vox);
     return cudaGetLastError();
 }
