@@ -37,10 +37,10 @@ COUNTS_FILE = os.path.join("profiles", "check_kernel_counts.md")
 
 
 def committed_counts(workload_name_):
-    """Per-pair counts of the plain-order check kernel on a workload, from the
-    committed ncu summary: warp instructions executed, FP32 FFMA / FADD / FMUL
-    thread instructions and DRAM bytes, each divided by the pairs of the
-    captured launch (None when the workload has no capture)."""
+    """Per-pair counts of the plain-order check's two kernels (probe and walk) on a
+    workload, from the committed ncu summary: warp instructions executed, FP32 FFMA
+    / FADD / FMUL thread instructions and DRAM bytes, each divided by the pairs of
+    the captured launches (None when the workload has no capture)."""
     import re
     path = os.path.join(ROOT, COUNTS_FILE)
     if not os.path.exists(path):
@@ -331,9 +331,9 @@ def tune_edges(E, N):
 
 
 def plain_launches(robot):
-    """Kernel launches of one plain-order check: Panda's row-major sample table
-    has its self-collision check fused into the FK kernel."""
-    return 5 if robot == "panda" else 6
+    """Kernel launches of one plain-order check of more than 1024 edges: steps,
+    offsets, FK with self-collision, swept boxes, probe, walk."""
+    return 6
 
 
 TRAIN_QUEUE_MIN_ITEMS = 128  # the lowest queue threshold the tuner tries: its population holds every higher one's
@@ -641,15 +641,14 @@ def run_ours(args, world, rank, local, dist):
             "verdict_mismatches_learned_vs_plain": mismatch,
             "proposal": dict(proposal, scored_segments_per_step=learned_rows, queued_pairs_per_step=learned_pairs,
                              queued_fraction=learned_pairs / float(N * E), ranking=ranking),
-            # plain: steps, scan, FK (+ self-collision for row-major tables), [self,]
-            # swept, check; learned adds features, MLP and ranking; its ablation
-            # launches the same
+            # plain: steps, scan, FK (+ self-collision), swept, probe, walk; learned
+            # adds features, MLP and ranking; its ablation launches the same
             "gpu_launches": (3 * plain_launches(robot) + 2 * 3) * args.steps,
             "clocks": clk.summary()}
     line["e2e"] = {"value": world * N * E / e2e_s, "unit": UNIT, "h2d_bytes_per_step": int(edges.nbytes),
                    "d2h_bytes_per_step": int(N * E),
                    "path": "bcc_check (host edges in, host verdicts out; bcc_opts.use_graph = 1)"}
-    # Roofline of the dominant kernel (environment check, plain order).  It is
+    # Roofline of the environment check's two kernels (plain order).  They are
     # bound by instruction issue (integer/logic and FP32 SIMT work on L2- and
     # shared-memory-resident inputs, DRAM a few per cent busy), so the roofline
     # is issue slots: achieved = warp instructions per launch (the committed ncu
@@ -671,7 +670,7 @@ def run_ours(args, world, rank, local, dist):
     roof = {"bound": "issue", "unit": "G warp-instructions/s", "peak": issue_peak,
             "peak_source": "%d SMs x 4 warp-instruction issue slots per cycle x %.0f MHz (median SM clock sampled "
                            "during the timed region)" % (sms, sm_mhz),
-            "kernel": "check_kernel (plain order)", "kernel_ms": chk_ms,
+            "kernel": "probe_kernel + walk_kernel (plain order)", "kernel_ms": chk_ms,
             "work_avoided": {"reference_plain_order_flops_per_launch": ref_flops,
                              "flop_estimate_rel_stderr": rel_err,
                              "note": "FP32 FLOPs the reference's literal plain order spends on these pairs (oracle "
@@ -684,8 +683,8 @@ def run_ours(args, world, rank, local, dist):
                      "traffic": counts["dram_bytes_per_pair"] * pairs,
                      "executed_warp_instructions_per_launch": inst,
                      "counts_source": "ncu sm__inst_executed.sum, smsp__sass_thread_inst_executed_op_{ffma,fadd,"
-                                      "fmul}_pred_on.sum, dram__bytes_{read,write}.sum of one plain check_kernel "
-                                      "launch, per pair, scaled by this launch's pairs (%s)" % COUNTS_FILE,
+                                      "fmul}_pred_on.sum, dram__bytes_{read,write}.sum of one plain check's probe_kernel "
+                                      "and walk_kernel, per pair, scaled by this launch's pairs (%s)" % COUNTS_FILE,
                      "fp32": {"achieved_tflops": flop / (chk_ms * 1e-3) / 1e12, "peak": fp32_peak,
                               "frac": flop / (chk_ms * 1e-3) / 1e12 / fp32_peak,
                               "peak_source": "FP32 FMA probe kernel measured in this run (bcc_measure_fp32_peak)"}})
