@@ -154,6 +154,14 @@ bool regular_rec(const Rec& r) {
     return true;
 }
 
+// Host to device, complete on return.  A copy from pageable memory may return with its
+// last DMA in flight on the legacy stream, which a context's (non-blocking) streams are
+// not ordered after.
+cudaError_t copy_in(void* dst, const void* src, size_t bytes) {
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 size_t aligned(size_t n, size_t to) { return (n + to - 1) / to * to; }
 
 int clamp_tile(int v, int lo, int hi) { return std::max(lo, std::min(hi, v)); }
@@ -417,9 +425,8 @@ bcc_status ensure_env_clusters(bcc_ctx* ctx, cudaStream_t st) {
     }
     BCC_CUDA(ctx, ctx->env_cluster.ensure(sizeof(int) * (size_t)std::max(N, 1)));
     BCC_CUDA(ctx, ctx->centroids.ensure(sizeof(float) * cen.size()));
-    BCC_CUDA(ctx, cudaMemcpy(ctx->env_cluster.p, id.data(), sizeof(int) * (size_t)N, cudaMemcpyHostToDevice));
-    BCC_CUDA(ctx, cudaMemcpy(ctx->centroids.p, cen.data(), sizeof(float) * cen.size(), cudaMemcpyHostToDevice));
-    BCC_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));  // (see bcc_upload_envs)
+    BCC_CUDA(ctx, copy_in(ctx->env_cluster.p, id.data(), sizeof(int) * (size_t)N));
+    BCC_CUDA(ctx, copy_in(ctx->centroids.p, cen.data(), sizeof(float) * cen.size()));
     ctx->cluster_k = K;
     return BCC_OK;
 }
@@ -975,7 +982,7 @@ bcc_status bcc_mlp_train(bcc_ctx* ctx, bcc_robot robot, const float* edges, int3
     if (dof < 0) return fail(ctx, BCC_ERR_INVALID_ARGUMENT, "unknown robot");
     cudaStream_t st = ctx->stream;
     BCC_CUDA(ctx, ctx->edges.ensure(sizeof(float) * 2 * (size_t)dof * num_edges));
-    BCC_CUDA(ctx, cudaMemcpy(ctx->edges.p, edges, sizeof(float) * 2 * (size_t)dof * num_edges, cudaMemcpyHostToDevice));
+    BCC_CUDA(ctx, copy_in(ctx->edges.p, edges, sizeof(float) * 2 * (size_t)dof * num_edges));
     bcc::PipelineArgs a;
     bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), num_edges, resolution, nullptr, nullptr, st, a);
     if (s != BCC_OK) return s;
@@ -1022,7 +1029,7 @@ bcc_status bcc_mlp_evaluate(bcc_ctx* ctx, bcc_robot robot, const float* edges, i
     const int dof = bcc_robot_dof(robot);
     cudaStream_t st = ctx->stream;
     BCC_CUDA(ctx, ctx->edges.ensure(sizeof(float) * 2 * (size_t)dof * num_edges));
-    BCC_CUDA(ctx, cudaMemcpy(ctx->edges.p, edges, sizeof(float) * 2 * (size_t)dof * num_edges, cudaMemcpyHostToDevice));
+    BCC_CUDA(ctx, copy_in(ctx->edges.p, edges, sizeof(float) * 2 * (size_t)dof * num_edges));
     bcc::PipelineArgs a;
     bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), num_edges, resolution, nullptr, nullptr, st, a);
     if (s != BCC_OK) return s;
@@ -1088,7 +1095,7 @@ bcc_status queue_population(bcc_ctx* ctx, bcc_robot robot, const float* edges, i
     cudaStream_t st = ctx->stream;
     const size_t eb = sizeof(float) * 2 * (size_t)dof * E;
     BCC_CUDA(ctx, ctx->edges.ensure(eb));
-    BCC_CUDA(ctx, cudaMemcpy(ctx->edges.p, edges, eb, cudaMemcpyHostToDevice));
+    BCC_CUDA(ctx, copy_in(ctx->edges.p, edges, eb));
     BCC_CUDA(ctx, ctx->results.ensure((size_t)E * ctx->num_envs));
     bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), E, resolution, ctx->results.as<uint8_t>(), nullptr, st, a);
     if (s != BCC_OK) return s;
@@ -1151,7 +1158,7 @@ bcc_status bcc_mlp_train_queued(bcc_ctx* ctx, bcc_robot robot, const float* edge
     BCC_CUDA(ctx, m.perm.ensure(sizeof(int) * (size_t)used));
     BCC_CUDA(ctx, m.x2.ensure(sizeof(uint16_t) * bcc::kMlpIn * (size_t)used));
     BCC_CUDA(ctx, m.y2.ensure((size_t)used));
-    BCC_CUDA(ctx, cudaMemcpy(m.perm.p, idx.data(), sizeof(int) * (size_t)used, cudaMemcpyHostToDevice));
+    BCC_CUDA(ctx, copy_in(m.perm.p, idx.data(), sizeof(int) * (size_t)used));
     BCC_CUDA(ctx, bcc::launch_gather_rows(m.x.as<uint16_t>(), m.y.as<uint8_t>(), m.perm.as<int>(), used,
                                           m.x2.as<uint16_t>(), m.y2.as<uint8_t>(), ctx->stream));
     const long long nb = used / batch;
@@ -1362,7 +1369,7 @@ bcc_status bcc_autotune(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32
     const size_t eb = sizeof(float) * 2 * (size_t)dof * num_edges;
     BCC_CUDA(ctx, ctx->edges.ensure(eb));
     BCC_CUDA(ctx, ctx->results.ensure((size_t)num_edges * ctx->num_envs));
-    BCC_CUDA(ctx, cudaMemcpy(ctx->edges.p, edges, eb, cudaMemcpyHostToDevice));
+    BCC_CUDA(ctx, copy_in(ctx->edges.p, edges, eb));
     // One full check captures the configuration's graph (everything after the
     // discretisation, which depends only on the edges); then the median of
     // kTuneReps timed replays of that graph, each after L2 was overwritten

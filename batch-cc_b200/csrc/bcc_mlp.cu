@@ -762,7 +762,8 @@ bcc_status bcc_mlp_set_params(bcc_ctx* ctx, const float* params, int32_t n) {
         m.adam_v.ensure(pb) != cudaSuccess || m.images.ensure(bcc::kImagesBytes) != cudaSuccess)
         return mlp_fail(ctx, BCC_ERR_CUDA, "MLP allocation failed");
     if (cudaMemcpy(m.params.p, params, pb, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemset(m.adam_m.p, 0, pb) != cudaSuccess || cudaMemset(m.adam_v.p, 0, pb) != cudaSuccess)
+        cudaMemset(m.adam_m.p, 0, pb) != cudaSuccess || cudaMemset(m.adam_v.p, 0, pb) != cudaSuccess ||
+        cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)  // (see copy_in, bcc_api.cu)
         return mlp_fail(ctx, BCC_ERR_CUDA, "MLP upload failed");
     if (bcc::mlp_pack(m.params.as<float>(), m.images.as<uint8_t>(), ctx->stream) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess)
