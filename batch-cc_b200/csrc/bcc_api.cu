@@ -85,11 +85,19 @@ Rec make_rec(const double c[3], const double A[3][3], const double h[3], double 
     return r;
 }
 
+// A sphere or capsule whose centre line is not finite is hit by nothing (the
+// reference's comparison is then false): the record's radius says so.
+double radius_of(float r, const double* p, const double* v) {
+    for (int i = 0; i < 3; ++i)
+        if (!std::isfinite(p[i]) || !std::isfinite(v[i])) return NAN;
+    return r;
+}
+
 Rec rec_sphere(const float* s) {
     double c[3] = {s[0], s[1], s[2]};
     double A[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}};
     double h[3] = {0, 0, 0};
-    return make_rec(c, A, h, s[3]);
+    return make_rec(c, A, h, radius_of(s[3], c, h));
 }
 
 // Capsule x1 y1 z1 xv yv zv r rdv: segment p1 -> p1 + v with radius r
@@ -113,7 +121,7 @@ Rec rec_capsule(const float* k, bool z_aligned) {
         A[1][i] = w[i];
         A[2][i] = a[i];
     }
-    return make_rec(c, A, h, k[6]);
+    return make_rec(c, A, h, radius_of(k[6], p1, v));
 }
 
 // Cuboid x y z a1 a2 a3 h1 h2 h3 (src/utils.cuh:159-178); the z-aligned variant
@@ -134,10 +142,10 @@ Rec rec_cuboid(const float* b, bool z_aligned) {
     return make_rec(c, A, h, 0.0);
 }
 
-// Does the record's distance function bound how distances change (1-Lipschitz,
-// all values finite, no negative radius)?  The caller's axes are taken as given;
-// only near-orthonormal ones, or shorter, do.  By Gershgorin the largest
-// eigenvalue of A A^T is at most the largest absolute row sum.
+// Is the record a rounded box: orthonormal axes, all values finite, no negative
+// radius?  The caller's axes are taken as given.  Others' distances change by more
+// or less than the metres moved, and their extents are not the cull box's (see
+// kEnvIrregular).
 bool regular_rec(const Rec& r) {
     for (int k = 0; k < 16; ++k)
         if (!std::isfinite(r.v[k])) return false;
@@ -145,11 +153,11 @@ bool regular_rec(const Rec& r) {
     for (int i = 0; i < 3; ++i) {
         double row = 0.0;
         for (int j = 0; j < 3; ++j) {
-            double d = 0.0;
+            double d = i == j ? -1.0 : 0.0;
             for (int k = 0; k < 3; ++k) d += (double)r.v[4 + 4 * i + k] * r.v[4 + 4 * j + k];
             row += std::fabs(d);
         }
-        if (!(row <= 1.0001)) return false;
+        if (!(row <= (double)bcc::kAxesTol)) return false;
     }
     return true;
 }
@@ -335,6 +343,8 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     a.table = ctx->table.as<float4>();
     a.blobs = ctx->blobs.as<float4>();
     a.env_hdr = ctx->env_hdr.as<float4>();
+    a.irregular = ctx->irregular.as<int>();
+    a.num_irregular = ctx->num_irregular;
     a.num_envs = ctx->num_envs;
     a.max_prims = std::max(ctx->max_prims, 1);
     a.blob_smem = ctx->blob_smem;
@@ -796,6 +806,7 @@ bcc_status pack(bcc_ctx* ctx, const bcc_env_soa* envs, std::vector<Rec>& recs, s
 // interval-mask tables -- are laid out by launch_build_arena.
 struct Arena {
     std::vector<float> hdr;      // [N][8]
+    std::vector<int> irregular;  // environments flagged kEnvIrregular
     size_t float4s = 0;          // of all blobs
     size_t max_record_bytes = 0;
     // Cull grid shared by every environment of the set: slab s of axis a is
@@ -858,6 +869,7 @@ void describe_arena(const std::vector<Rec>& recs, const std::vector<int>& off, A
         uint32_t flags = 0;
         for (int p = 0; p < np; ++p)
             if (!regular_rec(recs[p0 + p])) flags = bcc::kEnvIrregular;
+        if (flags) A.irregular.push_back(i);
         float* h = &A.hdr[(size_t)i * 8];
         std::memcpy(&h[3], &off16, 4);
         std::memcpy(&h[4], &first, 4);
@@ -905,9 +917,13 @@ bcc_status bcc_upload_envs(bcc_ctx* ctx, const bcc_env_soa* envs) {
     BCC_CUDA(ctx, ctx->blobs.ensure(std::max<size_t>(1, A.float4s) * sizeof(float4)));
     BCC_CUDA(ctx, ctx->env_hdr.ensure(std::max<size_t>(1, A.hdr.size()) * sizeof(float)));
     BCC_CUDA(ctx, ctx->grid_bounds.ensure(sizeof(A.bnd)));
+    BCC_CUDA(ctx, ctx->irregular.ensure(sizeof(int) * A.irregular.size()));
     BCC_CUDA(ctx, ctx->records.ensure(std::max<size_t>(16, rec_bytes)));
     BCC_CUDA(ctx, cudaMemcpy(ctx->grid_bounds.p, A.bnd, sizeof(A.bnd), cudaMemcpyHostToDevice));
     if (rec_bytes) BCC_CUDA(ctx, cudaMemcpy(ctx->records.p, recs.data(), rec_bytes, cudaMemcpyHostToDevice));
+    if (!A.irregular.empty())
+        BCC_CUDA(ctx, cudaMemcpy(ctx->irregular.p, A.irregular.data(), sizeof(int) * A.irregular.size(),
+                                 cudaMemcpyHostToDevice));
     if (N > 0) {
         BCC_CUDA(ctx, cudaMemcpy(ctx->env_hdr.p, A.hdr.data(), A.hdr.size() * sizeof(float), cudaMemcpyHostToDevice));
         BCC_CUDA(ctx, bcc::launch_build_arena(ctx->records.as<float4>(), ctx->env_hdr.as<float4>(),
@@ -920,6 +936,7 @@ bcc_status bcc_upload_envs(bcc_ctx* ctx, const bcc_env_soa* envs) {
     ctx->num_envs = N;
     ctx->max_prims = max_prims;
     ctx->blob_smem = blob_smem;
+    ctx->num_irregular = (int)A.irregular.size();
     ctx->env_code_ready = false;
     ctx->cluster_k = 0;
     ctx->env_version += 1;

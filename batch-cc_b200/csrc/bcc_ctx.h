@@ -93,6 +93,8 @@ struct bcc_ctx {
     size_t blob_smem = 0;
 
     bcc::DevBuf blobs, env_hdr;
+    bcc::DevBuf irregular;   // environments flagged kEnvIrregular
+    int num_irregular = 0;
     bcc::DevBuf records;     // the upload's records as packed, source of the blobs
     // per-call buffers
     bcc::DevBuf edges, per_edge, table, results, error_flag;  // per_edge: steps, offs, edge_self, edge_tri

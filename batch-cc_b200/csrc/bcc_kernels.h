@@ -30,10 +30,15 @@ constexpr float kVoxMin = -0.128f;
 constexpr float kVoxStep = 0.003f;     // codes reach 0.637 m
 constexpr float kVoxSlack = 1e-4f;     // FP32 rounding of distances and positions (~1e-6 m), generously
 constexpr unsigned kVoxUnknown = 255u;
-// Environment header flag (second float4, z): some record's axes stretch
-// distances or hold non-finite values, so no distance bound holds and the
-// check makes every test on the primitives themselves.
+// Environment header flag (second float4, z): some record is not a box (its axes
+// are not orthonormal), or holds non-finite values or a negative radius.  Neither
+// the bounds on distances nor the cull boxes hold there, nor does a leaf's hit imply
+// its bound's: exact_kernel decides all pairs of such an environment by the
+// reference's own tests, the other check kernels leave them alone.
 constexpr unsigned kEnvIrregular = 1u;
+// How far the axes' products may be from the identity (row sums): what the margins of
+// the cull and the distance bounds (1e-4 m) absorb for boxes of metres.
+constexpr float kAxesTol = 5e-5f;
 
 struct ProbeGrid {
     const uint16_t* vox;     // [num_envs][stride / 2] voxel words, null = no grid
@@ -57,6 +62,8 @@ struct CheckParams {
     const float4* blobs;     // per env: [np][5] rounded-box records, then 3 x kGridTri x W masks
     const float4* env_hdr;   // [num_envs][2]: (0, 0, 0, blob offset in float4s),
                              //                 (first record, 0, flags, np | W << 16)
+    const int* irregular;    // [num_irregular] environments flagged kEnvIrregular
+    int num_irregular;
     int num_envs;
     int num_edges;
     int max_prims;           // max primitives of one env (pair-list sizing)
@@ -123,6 +130,8 @@ struct PipelineArgs {
     const float* grid_bounds;  // [3][kGridSlabs + 1] cull-grid slab boundaries of the environment set
     const float4* blobs;
     const float4* env_hdr;
+    const int* irregular;
+    int num_irregular;
     int num_envs;
     int max_prims;
     size_t blob_smem;
@@ -244,6 +253,8 @@ inline CheckParams params_of(const PipelineArgs& a) {
     CheckParams P{};
     P.blobs = a.blobs;
     P.env_hdr = a.env_hdr;
+    P.irregular = a.irregular;
+    P.num_irregular = a.num_irregular;
     P.num_envs = a.num_envs;
     P.num_edges = a.num_edges;
     P.max_prims = a.max_prims;

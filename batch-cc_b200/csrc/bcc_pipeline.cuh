@@ -105,6 +105,10 @@ struct DevTables {
         int pos;
     } fk[M::num_spheres];
     float sphere_radius[M::num_spheres];  // by sample-table position
+    // The reference's own groups, as row positions (walk_exact).
+    unsigned char ref_bound[M::num_ref_env_groups];
+    int ref_leaf_begin[M::num_ref_env_groups + 1];
+    unsigned char ref_leaf[sizeof(M::ref_env_leaves) / sizeof(int)];
     float s_m[M::dof], s_a[M::dof];       // joint-limit scale q = u * s_m + s_a
 };
 
@@ -262,6 +266,11 @@ DevTables<M> host_tables() {
         }
     }
     t.fk_begin[M::dof + 1] = at;
+    for (int g = 0; g < M::num_ref_env_groups; ++g)
+        t.ref_bound[g] = (unsigned char)M::table_pos[M::ref_env_bound[g]];
+    for (int g = 0; g <= M::num_ref_env_groups; ++g) t.ref_leaf_begin[g] = M::ref_env_leaf_begin[g];
+    for (int l = 0; l < t.ref_leaf_begin[M::num_ref_env_groups]; ++l)
+        t.ref_leaf[l] = (unsigned char)M::table_pos[M::ref_env_leaves[l]];
     for (int g = 0; g < M::num_env_groups; ++g) t.gate_r[g] = t.sphere_radius[g] + kEnvInflate;
     for (int g = 0; g < M::num_env_groups; ++g)
         t.seg_pad[g] = t.sphere_radius[g] + kEnvInflate + t.cull_pad[g] + kSegMargin;
@@ -1257,6 +1266,60 @@ __device__ __forceinline__ bool walk_segments(const float4* __restrict__ table, 
     return false;
 }
 
+// ------------------------------------------------------------------ irregular environments
+// Whole warp, one row of the sample table against np records: the reference's
+// environment test as it stands (fkcc, src/utils.cuh:806-1190) -- each of its groups'
+// bounds against every primitive, then the leaves of the groups whose bound hit one
+// against every primitive -- with nothing ruled out by distance.
+template <class M>
+__device__ __forceinline__ bool exact_hit(const float4* row, const float4* prim, int np) {
+    const DevTables<M>& L = lane_tab<M>();
+    const int lane = threadIdx.x & 31;
+    // items [0, spheres x np), primitives innermost
+    const int ds = 32 / np, dp = 32 - ds * np;
+    auto any_of = [&](const unsigned char* pos, int spheres, auto&& found) {
+        int s = lane / np, p = lane - s * np;
+        for (int i0 = 0; i0 < spheres * np; i0 += 32) {
+            bool hit = false;
+            if (s < spheres) {
+                float4 c = row[pos[s]];
+                c.w += kEnvInflate;
+                hit = sphere_hits_prim(c, prim + p * kPrimF4);
+            }
+            if (found(hit, s)) return true;
+            s += ds;
+            p += dp;
+            if (p >= np) {
+                p -= np;
+                ++s;
+            }
+        }
+        return false;
+    };
+    unsigned gates = 0u;
+    any_of(L.ref_bound, M::num_ref_env_groups, [&](bool hit, int g) {
+        gates |= hit ? 1u << g : 0u;
+        return false;
+    });
+    gates = __reduce_or_sync(kFull, gates);
+    for (; gates; gates &= gates - 1u) {
+        const int g = __ffs((int)gates) - 1;
+        const int l0 = L.ref_leaf_begin[g], l1 = L.ref_leaf_begin[g + 1];
+        if (any_of(L.ref_leaf + l0, l1 - l0, [](bool hit, int) { return __any_sync(kFull, hit) != 0; })) return true;
+    }
+    return false;
+}
+
+// ... over an edge's samples in the reference's order.
+template <class M>
+__device__ __noinline__ bool walk_exact(const float4* __restrict__ table, size_t row0, int n, const float4* prim, int np) {
+    static_assert(M::num_ref_env_groups <= 32, "a bit per group");
+    for (int r = 0; r < kLanes * n; ++r)
+        if (exact_hit<M>(table + table_index<M>(row0 + (size_t)reference_rank_to_sample(r, n), 0), prim, np))
+            return true;
+    return false;
+}
+
 // Learned order, whole warp: perm_buf[rank] = segment, the edge's nseg <= 64
 // segments in descending MLP score (scores[0 .. nseg)), ties by index, NaN
 // last, with first_ahead segment 0 before all others; returns segment 0's rank.
@@ -1836,7 +1899,8 @@ __global__ void __launch_bounds__(kProbeThreads, kProbeCtas) probe_kernel(CheckP
     const float4 h1 = P.env_hdr[2 * env + 1];
     const uint32_t bytes = record_bytes_of(h1);
     const int np = (int)(__float_as_uint(h1.w) & 0xffffu);
-    const bool probe = np > 0 && !(__float_as_uint(h1.z) & kEnvIrregular);
+    if (__float_as_uint(h1.z) & kEnvIrregular) return;  // exact_kernel's
+    const bool probe = np > 0;
     const float4* prim = reinterpret_cast<const float4*>(smem);
     uint2* list = reinterpret_cast<uint2*>(smem + P.blob_smem + P.probe.stride);
     unsigned* list_near = reinterpret_cast<unsigned*>(list + Q.batch);
@@ -2066,6 +2130,7 @@ __global__ void __launch_bounds__(WARPS * 32, check_min_ctas<M, WARPS>()) check_
     if (n_slots <= 0 || P.offs[P.num_edges] > P.cap_rows) return;
     const float4 h0 = P.env_hdr[2 * env + 0];
     const float4 h1 = P.env_hdr[2 * env + 1];
+    if (__float_as_uint(h1.z) & kEnvIrregular) return;  // exact_kernel's
     const uint32_t bytes = record_bytes_of(h1);
     if (threadIdx.x == 0) s_next = 0;
     if (bytes) {
@@ -2087,6 +2152,33 @@ __global__ void __launch_bounds__(WARPS * 32, check_min_ctas<M, WARPS>()) check_
         __syncthreads();  // s_next is set before any warp takes a pass
     }
     check_tile<M, WARPS, MODE>(P, env, tile, n_slots, smem, h0, h1, &s_next);
+}
+
+// The pairs of the irregular environments, one warp a pair, environments outermost;
+// records are read through L1.  Every sample takes every test, some ten times the
+// instructions of the walk: such environments are the exception.
+constexpr int kExactWarps = 4;
+
+template <class M>
+__global__ void __launch_bounds__(32 * kExactWarps) exact_kernel(CheckParams P) {
+    const int lane = threadIdx.x & 31, E = P.num_edges;
+    if (P.offs[E] > P.cap_rows) return;
+    const long long pairs = (long long)P.num_irregular * E, step = (long long)gridDim.x * kExactWarps;
+    for (long long i = (long long)blockIdx.x * kExactWarps + (threadIdx.x >> 5); i < pairs; i += step) {
+        const int env = P.irregular[i / E], e = (int)(i % E);
+        const float4 h0 = P.env_hdr[2 * env], h1 = P.env_hdr[2 * env + 1];
+        const int np = (int)(__float_as_uint(h1.w) & 0xffffu);  // at least one
+        const bool self = P.edge_self[e] != 0;
+        const bool hit = self || walk_exact<M>(P.table, (size_t)P.offs[e], P.steps[e],
+                                               P.blobs + (size_t)__float_as_uint(h0.w), np);
+        if (lane == 0) {
+            P.results[(size_t)e * P.num_envs + env] = hit ? 1 : 0;
+            if (P.counters && !self) {
+                atomicAdd(P.counters + 0, 1ull);
+                atomicAdd(P.counters + 5, hit ? 1ull : 0ull);
+            }
+        }
+    }
 }
 
 // Learned order, phase 3: each CTA pulls queued pairs from finish_counter, one
@@ -2447,6 +2539,17 @@ __global__ void training_rows_kernel(CheckParams P, const float* __restrict__ ed
 }
 
 // ------------------------------------------------------------------ records variant
+// regular_rec (bcc_api.cu) of a record on the device.
+__device__ __forceinline__ bool regular_prim(const float4* rec) {
+    const float4 c = rec[0], a1 = rec[1], a2 = rec[2], a3 = rec[3];
+    auto zero = [](float4 v) { return 0.0f * v.x + 0.0f * v.y + (0.0f * v.z + 0.0f * v.w); };  // unless not finite
+    auto dot = [](float4 u, float4 v) { return fmaf(u.x, v.x, fmaf(u.y, v.y, u.z * v.z)); };
+    const float xy = fabsf(dot(a1, a2)), xz = fabsf(dot(a1, a3)), yz = fabsf(dot(a2, a3));
+    return zero(c) + zero(a1) + (zero(a2) + zero(a3)) == 0.0f && c.w >= 0.0f &&
+           fabsf(dot(a1, a1) - 1.0f) + xy + xz <= kAxesTol && fabsf(dot(a2, a2) - 1.0f) + xy + yz <= kAxesTol &&
+           fabsf(dot(a3, a3) - 1.0f) + xz + yz <= kAxesTol;
+}
+
 // Environment check from the host-packed rounded-box records of bcc_pack_envs
 // (no interval-mask tables), used by the allocation-free entry point: culls
 // (primitive, link) pairs with an exact AABB overlap test, one primitive per
@@ -2490,6 +2593,10 @@ __global__ void __launch_bounds__(WARPS * 32) check_records_kernel(RecordsParams
             return;
         }
     }
+    // Whether the environment is irregular is not in the records: found here.
+    bool odd = false;
+    for (int p = threadIdx.x; p < np; p += WARPS * 32) odd |= !regular_prim(prim + p * kPrimF4);
+    const bool exact = __syncthreads_or(odd) != 0;
     const uint32_t lt = (1u << lane) - 1u;
     const GroupLanes GL = group_lanes<M>();
 
@@ -2498,6 +2605,11 @@ __global__ void __launch_bounds__(WARPS * 32) check_records_kernel(RecordsParams
         const int self = P.edge_self[e];
         if (np == 0 || self) {
             if (lane == 0) *out = self ? 1 : 0;
+            continue;
+        }
+        if (exact) {
+            const bool hit = walk_exact<M>(P.table, (size_t)P.offs[e], P.steps[e], prim, np);
+            if (lane == 0) *out = hit ? 1 : 0;
             continue;
         }
         if (lane < G) {
@@ -2678,7 +2790,17 @@ cudaError_t run_prep(const PipelineArgs& a, cudaStream_t st) {
 // Environment check only (the FK/self/swept stages already ran), in a.mode.
 template <class M>
 cudaError_t run_check_mode(const PipelineArgs& a, cudaStream_t st) {
-    return check_by_warps<M>(params_of(a), a.num_edges, a.warps, a.mode, st);
+    const CheckParams P = params_of(a);
+    if (P.num_irregular > 0 && a.mode != 2) {  // (the finish pass has none of their pairs)
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const long long ctas = ((long long)P.num_irregular * P.num_edges + kExactWarps - 1) / kExactWarps;
+        exact_kernel<M><<<(unsigned)std::min<long long>(ctas, 16 * std::max(sms, 1)), 32 * kExactWarps, 0, st>>>(P);
+        const cudaError_t err = cudaGetLastError();
+        if (err != cudaSuccess) return err;
+    }
+    return check_by_warps<M>(P, a.num_edges, a.warps, a.mode, st);
 }
 
 template <class M>
