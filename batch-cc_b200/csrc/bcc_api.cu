@@ -261,7 +261,6 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
         return fail(ctx, BCC_ERR_LIMIT, "an environment has more primitives than this robot's checker supports");
     if (!ctx->tables[r]) {
         BCC_CUDA(ctx, ops->upload_tables());
-        BCC_CUDA(ctx, cudaStreamSynchronize(cudaStreamLegacy));  // (see bcc_upload_envs)
         ctx->tables[r] = true;
     }
     a = bcc::PipelineArgs{};

@@ -206,7 +206,7 @@ struct RobotOps {
     int max_prims;           // primitives per environment the pair packing allows
     // Box around the group bounds' centres over the joint limits (probe grid domain).
     void (*reach)(float lo[3], float hi[3]);
-    cudaError_t (*upload_tables)();  // robot tables -> __constant__ of the current device
+    cudaError_t (*upload_tables)();  // robot tables -> the current device, complete on return
     // Stage 1: steps + sample offsets (total rows land in offs[E]).
     cudaError_t (*steps)(const PipelineArgs& a, cudaStream_t st);
     // Stage 2: FK table, self-collision, swept volumes, environment check.

@@ -281,6 +281,17 @@ DevTables<M> host_tables() {
     return t;
 }
 
+// The robot's tables into both of its symbols, complete on return: the copies, from
+// pageable memory, may return with their last DMA in flight on the legacy stream,
+// which a non-blocking stream's kernels are not ordered after.
+template <class M>
+cudaError_t upload_to(const DevTables<M>& global, const DevTables<M>& constant) {
+    const DevTables<M> t = host_tables<M>();
+    cudaError_t err = cudaMemcpyToSymbol(global, &t, sizeof(t));
+    if (err == cudaSuccess) err = cudaMemcpyToSymbol(constant, &t, sizeof(t));
+    return err == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : err;
+}
+
 // Box around the group bounds' centres over the joint limits: the domain of the
 // probe grid.  Sampled (a seeded sequence of 2048 configurations, 2 cm added):
 // a centre outside it costs the probe precision there, never correctness.

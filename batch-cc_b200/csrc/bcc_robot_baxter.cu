@@ -19,9 +19,7 @@ __device__ __forceinline__ const DevTables<BaxterModel>& lane_tab<BaxterModel>()
 }
 
 static cudaError_t upload_baxter_tables() {
-    const DevTables<BaxterModel> t = host_tables<BaxterModel>();
-    const cudaError_t err = cudaMemcpyToSymbol(g_tab_baxter, &t, sizeof(t));
-    return err != cudaSuccess ? err : cudaMemcpyToSymbol(c_tab_baxter, &t, sizeof(t));
+    return upload_to<BaxterModel>(g_tab_baxter, c_tab_baxter);
 }
 
 extern const RobotOps kBaxterOps = robot_ops_of<BaxterModel>(BCC_ROBOT_BAXTER, upload_baxter_tables);

@@ -19,9 +19,7 @@ __device__ __forceinline__ const DevTables<FetchModel>& lane_tab<FetchModel>() {
 }
 
 static cudaError_t upload_fetch_tables() {
-    const DevTables<FetchModel> t = host_tables<FetchModel>();
-    const cudaError_t err = cudaMemcpyToSymbol(g_tab_fetch, &t, sizeof(t));
-    return err != cudaSuccess ? err : cudaMemcpyToSymbol(c_tab_fetch, &t, sizeof(t));
+    return upload_to<FetchModel>(g_tab_fetch, c_tab_fetch);
 }
 
 extern const RobotOps kFetchOps = robot_ops_of<FetchModel>(BCC_ROBOT_FETCH, upload_fetch_tables);

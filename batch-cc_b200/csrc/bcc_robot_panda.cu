@@ -25,9 +25,7 @@ constexpr bool fk_x_first<PandaModel>(int pos) {
 }
 
 static cudaError_t upload_panda_tables() {
-    const DevTables<PandaModel> t = host_tables<PandaModel>();
-    const cudaError_t err = cudaMemcpyToSymbol(g_tab_panda, &t, sizeof(t));
-    return err != cudaSuccess ? err : cudaMemcpyToSymbol(c_tab_panda, &t, sizeof(t));
+    return upload_to<PandaModel>(g_tab_panda, c_tab_panda);
 }
 
 extern const RobotOps kPandaOps = robot_ops_of<PandaModel>(BCC_ROBOT_PANDA, upload_panda_tables);

@@ -9,6 +9,9 @@ contact), on two calls in a row with different edges -- the second call runs
 on arrays the first one left behind.  The file is named to be collected last.
 """
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -103,3 +106,37 @@ def test_noalloc_rejects_sizes_beyond_its_limit():
     assert fn(0, d_rec.data_ptr() + 4, d_off.data_ptr(), 2, max_prims, d_edges.data_ptr(), 8, 32,
               d_res.data_ptr(), stream) == 1  # BCC_ERR_INVALID_ARGUMENT
     torch.cuda.synchronize()
+
+
+FIRST_CALL = '''
+import sys
+import numpy as np, torch
+sys.path.insert(0, %r)
+import test_zz_no_alloc as t
+from bcc import workload
+from oracle import oracle as orc
+for name in %r:
+    robot = workload.robot_of(name)
+    envs, edges = workload.gen_envs(name, 6, seed=46), workload.gen_edges(name, 20, seed=46)
+    rec, off, most = t._pack(envs)
+    d = [torch.from_numpy(a).cuda() for a in (rec, off, edges)]
+    out = torch.full((len(edges), 6), 7, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()  # not ordered after the legacy stream
+    s = t._noalloc_fn()(t.bcclib.ROBOTS[robot], d[0].data_ptr(), d[1].data_ptr(), 6, most, d[2].data_ptr(),
+                        len(edges), 32, out.data_ptr(), t.ctypes.c_void_p(st.cuda_stream))
+    assert s == 0, s
+    got, want = out.cpu().numpy(), orc.check(envs, edges, robot=robot)
+    assert len(orc.adjudicate(envs, edges, got, want, robot=robot)[2]) == 0, name
+'''
+
+
+@pytest.mark.parametrize("first", ["uneven", "multi_fetch", "multi_baxter"])
+def test_first_call_of_a_process_on_a_stream_of_its_own(first):
+    """The first call uploads the robot's tables; its kernels, on a stream that is not
+    ordered after the default one, read them complete."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    root = os.path.dirname(here)
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "batch-cc_b200")]))
+    names = [first] + [n for n in ("uneven", "multi_fetch", "multi_baxter") if n != first]
+    subprocess.run([sys.executable, "-c", FIRST_CALL % (here, names)], check=True, env=env, timeout=300)
