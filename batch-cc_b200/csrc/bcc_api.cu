@@ -498,8 +498,8 @@ bcc_status run_learned(bcc_ctx* ctx, const bcc::RobotOps* ops, bcc::PipelineArgs
 
 // Inline learned order: buffers for K x segments MLP rows and the
 // per-(cluster, edge) segment orders, sized outside any stream capture.
-bcc_status prepare_inline(bcc_ctx* ctx, bcc::PipelineArgs& a) {
-    bcc_status s = ensure_env_clusters(ctx, ctx->stream);
+bcc_status prepare_inline(bcc_ctx* ctx, bcc::PipelineArgs& a, cudaStream_t st) {
+    bcc_status s = ensure_env_clusters(ctx, st);
     if (s != BCC_OK) return s;
     const int K = ctx->cluster_k;
     a.total_segs = a.total_rows / bcc::kSegment;
@@ -584,7 +584,7 @@ bcc_status launch_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int
         if (s != BCC_OK) return s;
         if (opts->learned_row_cap < 0)
             return fail(ctx, BCC_ERR_INVALID_ARGUMENT, "learned_row_cap must be >= 0");
-        s = ctx->tune.learned_mode == 0 ? prepare_inline(ctx, a) : prepare_learned(ctx, a, opts->learned_row_cap);
+        s = ctx->tune.learned_mode == 0 ? prepare_inline(ctx, a, st) : prepare_learned(ctx, a, opts->learned_row_cap);
         if (s != BCC_OK) return s;
     }
     const bool graph = opts && opts->use_graph && !ctx->counting && !(opts->tile_override > 0);

@@ -260,3 +260,49 @@ def test_learned_order_overhang_robots(checker, name, mode, split):
         assert np.array_equal(plain, learned)
     finally:
         checker.set_launch_config(**cfg)
+
+
+def test_clusters_of_the_first_learned_check_on_a_busy_stream():
+    """The environment codes are made on the caller's stream; the clusters of the inline
+    order come from them, not from what the buffer held: the walk takes the same steps
+    as in a context whose calls are synchronous."""
+    import threading
+    import time
+
+    import torch
+    from bcc.lib import Checker
+    sets = [workload.gen_envs("uneven", 64, seed=s) for s in (81, 82)]
+    edges = workload.gen_edges("uneven", 400, seed=81)
+    steps = []
+    for busy in (False, True):
+        chk = Checker(0)
+        chk.mlp_set_params(mlp.init_params(4))
+        chk.set_launch_config(edges_per_cta=64, warps=4, persistent=0, clusters=8)
+        d_edges = torch.from_numpy(edges).cuda()
+        out = torch.empty((400, 64), dtype=torch.uint8, device="cuda")
+        st = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        for envs in sets:
+            chk.upload(envs)
+            chk.set_profiling(True, counters=True)
+            stop = threading.Event()
+
+            def load():  # keeps work ahead of the call's own launches in the stream
+                while not stop.is_set():
+                    with torch.cuda.stream(st):
+                        torch.cuda._sleep(200000)
+                    time.sleep(1e-4)
+            t = threading.Thread(target=load)
+            if busy:
+                t.start()
+            try:
+                chk.check_device(d_edges.data_ptr(), 400, out.data_ptr(), order="learned", stream=st.cuda_stream)
+            finally:
+                stop.set()
+                if busy:
+                    t.join()
+            torch.cuda.synchronize()
+            steps.append(chk.work_counters()["chunks"])
+            chk.set_profiling(False)
+        chk.close()
+    assert steps[:2] == steps[2:]
