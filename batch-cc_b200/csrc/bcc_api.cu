@@ -512,6 +512,7 @@ bcc_status prepare_inline(bcc_ctx* ctx, bcc::PipelineArgs& a, cudaStream_t st) {
     a.logits = ctx->mlp.logits.as<float>();
     a.features = ctx->mlp.x.p;
     a.env_cluster = ctx->env_cluster.as<int>();
+    a.centroids = ctx->centroids.as<float>();
     a.perms = ctx->perms.as<uint8_t>();
     a.row_cap = (int)rows;
     ctx->last_inline_rows = (long long)rows;
@@ -528,7 +529,7 @@ bcc_status run_learned_inline(bcc_ctx* ctx, const bcc::RobotOps* ops, bcc::Pipel
     const int K = ctx->cluster_k;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    BCC_CUDA(ctx, ops->cluster_features(a, ctx->centroids.as<float>(), K, ctx->mlp.x.as<uint16_t>(), st));
+    BCC_CUDA(ctx, ops->cluster_features(a, a.centroids, K, ctx->mlp.x.as<uint16_t>(), st));
     BCC_CUDA(ctx, bcc::mlp_forward(ctx->mlp.x.as<uint16_t>(), a.row_cap, ctx->mlp.images.as<uint8_t>(),
                                    ctx->mlp.params.as<float>(), ctx->mlp.logits.as<float>(), a.error_flag,
                                    std::max(sms, 1), st));
@@ -564,6 +565,7 @@ bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
            x.queue.head == y.queue.head && x.queue.chunk == y.queue.chunk && x.queue.batch == y.queue.batch && x.warps == y.warps &&
            x.edges_per_cta == y.edges_per_cta && x.q_head == y.q_head && x.q_pairs == y.q_pairs &&
            x.q_rows == y.q_rows && x.logits == y.logits && x.perms == y.perms && x.env_cluster == y.env_cluster &&
+           x.centroids == y.centroids &&
            x.features == y.features && x.work_counter == y.work_counter && x.error_flag == y.error_flag;
 }
 

@@ -154,6 +154,7 @@ struct PipelineArgs {
     int finish_split;
     int* work_counter;
     const int* env_cluster;
+    const float* centroids;  // [K][32] cluster codes, inline learned order
     const uint8_t* perms;
     const void* features;    // the MLP feature rows of a learned check
     int total_segs;

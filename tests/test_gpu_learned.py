@@ -306,3 +306,18 @@ def test_clusters_of_the_first_learned_check_on_a_busy_stream():
             chk.set_profiling(False)
         chk.close()
     assert steps[:2] == steps[2:]
+
+
+def test_graph_after_the_centroids_moved():
+    """A captured check of one cluster, a direct one of eight (whose centroids take a
+    larger buffer), one cluster again: the graph reads the buffer of now."""
+    from bcc.lib import Checker
+    envs, edges = workload.gen_envs("uneven", 30, seed=83), workload.gen_edges("uneven", 300, seed=83)
+    chk = Checker(0)
+    chk.upload(envs)
+    chk.mlp_set_params(mlp.init_params(4))
+    want = chk.check(edges)
+    for clusters, graph in ((1, True), (8, False), (1, True), (8, True), (1, False), (8, True)):
+        chk.set_launch_config(clusters=clusters)
+        assert np.array_equal(chk.check(edges, order="learned", graph=graph), want), (clusters, graph)
+    chk.close()
