@@ -1369,7 +1369,7 @@ bcc_status bcc_set_launch_config(bcc_ctx* ctx, const int32_t* cfg) {
     ctx->tune.learned_mode = cfg[5];
     ctx->tune.clusters = cfg[6];
     ctx->tune.lanes = cfg[7];
-    ctx->tune.tuned = true;
+    ctx->tune.tuned = !ctx->tune.initial_shape();
     return BCC_OK;
 }
 
@@ -1464,7 +1464,7 @@ bcc_status bcc_autotune(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32
                     t.edges_per_cta = tiles[ti];
                     t.warps = warps[wi];
                     t.persistent = pe;
-                    keep(t);
+                    if (!t.initial_shape()) keep(t);
                 }
     };
     bcc::Tune start = base;
@@ -1496,7 +1496,7 @@ bcc_status bcc_autotune(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32
     cudaEventDestroy(e1);
     ctx->profiling = saved_prof;
     best.tuned = true;
-    ctx->tune = best;
+    ctx->tune = s == BCC_OK ? best : base;
     if (s != BCC_OK) return s;
     if (chosen) bcc_get_launch_config(ctx, chosen);
     return BCC_OK;

@@ -50,10 +50,12 @@ struct MlpState {
     long long step = 0;      // Adam step count
 };
 
-// Launch configuration of the environment check (set by bcc_autotune).
+// Launch configuration of the environment check (set by bcc_autotune).  The shape
+// (first three values) it starts with stands for one chosen by the call's size
+// (launch_shape), also when it is set again: get and set restore it.
 struct Tune {
     int edges_per_cta = 128;
-    int warps = 4;
+    int warps = 8;
     int persistent = 1;
     int queue_min_items = 128;
     int finish_split = 0;    // learned order, queued: 1 = split each queued pair over a CTA's warps
@@ -61,6 +63,11 @@ struct Tune {
     int clusters = 1;        // learned order, inline: environment clusters scored per edge
     int lanes = 32;          // accepted and reported; every walk takes a whole warp
     bool tuned = false;      // set or tuned: taken as it is, else the shape is chosen by size
+
+    bool initial_shape() const {
+        const Tune t;
+        return edges_per_cta == t.edges_per_cta && warps == t.warps && persistent == t.persistent;
+    }
 };
 
 // A captured launch sequence (everything after the discretisation) and the

@@ -292,6 +292,9 @@ bcc_status bcc_measure_fp32_peak(int32_t device, double* tflops);
  * environment codes; the MLP scores each edge's segments once per cluster),
  * cfg[7] lanes per walking pair: 32, or 16 for builds with a half-warp walk (this
  * one has none: 32 are used).
+ * A context's initial cfg[0..2], 128 8 1, stand for a shape chosen by the size of
+ * each call (one pass for few pairs); setting them again, as when a saved
+ * configuration is restored, returns to that.
  */
 #define BCC_LAUNCH_CONFIG_LEN 8
 bcc_status bcc_get_launch_config(const bcc_ctx* ctx, int32_t* cfg);

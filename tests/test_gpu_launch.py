@@ -98,3 +98,57 @@ def test_autotune_picks_a_valid_config(checker, case):
     if cfg["learned_mode"] == 1:
         assert cfg["queue_min_items"] in (64, 128, 256, 512, 1024, 2048, 4096)
     assert np.array_equal(checker.check(edges, order="learned"), base)
+
+
+@pytest.mark.parametrize("name,nenv,nedge", [
+    ("uneven", 40, 408), ("stress", 1, 64), ("multi_fetch", 40, 400),  # below 2^14 pairs: one pass
+    ("uneven", 400, 10000), ("multi_fetch", 500, 5000)])               # records of up to, and above, 8192 bytes: probed
+def test_shape_chosen_by_size_survives_a_saved_configuration(name, nenv, nedge):
+    """A fresh context's launch shapes: the oracle's verdicts, and the same work (which
+    tells the one-pass check from the probed one) after its configuration was saved,
+    changed and restored, or set in other values only."""
+    from bcc.lib import Checker
+    from oracle import oracle as orc
+    robot = workload.robot_of(name)
+    envs, edges = workload.gen_envs(name, nenv, seed=53), workload.gen_edges(name, nedge, seed=53)
+    work = {}
+    for how in ("fresh", "restored", "threshold"):
+        chk = Checker(0)
+        chk.upload(envs)
+        chk.set_profiling(True, counters=True)
+        cfg = chk.launch_config()
+        assert (cfg["edges_per_cta"], cfg["warps"], cfg["persistent"]) == (128, 8, 1)
+        if how == "restored":
+            for persistent in (0, 1):
+                chk.set_launch_config(edges_per_cta=64, warps=4, persistent=persistent)
+                work[persistent] = (chk.check(edges, robot=robot), chk.work_counters())
+            chk.set_launch_config(**cfg)
+        elif how == "threshold":
+            chk.set_launch_config(queue_min_items=64)
+        got = [chk.check(edges, robot=robot) for _ in range(2)]
+        work[how] = (got[1], chk.work_counters())
+        assert np.array_equal(got[0], got[1])
+        chk.close()
+    assert work[0][1]["candidates"] != work[1][1]["candidates"]
+    for how in ("fresh", "restored", "threshold"):
+        assert work[how][1] == work[1 if nenv * nedge >= 1 << 14 else 0][1], how
+        assert np.array_equal(work[how][0], work[1][0])
+    part = edges[:80]
+    want = orc.check(envs, part, robot=robot)
+    assert len(orc.adjudicate(envs, part, work["fresh"][0][:80], want, robot=robot)[2]) == 0
+
+
+def test_failed_autotune_leaves_the_configuration():
+    """No network for the learned order: an error, and the shapes as before it."""
+    from bcc.lib import BccError, Checker
+    envs, edges = workload.gen_envs("uneven", 30, seed=54), workload.gen_edges("uneven", 300, seed=54)
+    chk = Checker(0)
+    chk.upload(envs)
+    chk.set_profiling(True, counters=True)
+    want = chk.check(edges), chk.work_counters()
+    with pytest.raises(BccError):
+        chk.autotune(edges, order="learned")
+    chk.set_profiling(True, counters=True)
+    got = chk.check(edges), chk.work_counters()
+    assert np.array_equal(got[0], want[0]) and got[1] == want[1]
+    chk.close()
