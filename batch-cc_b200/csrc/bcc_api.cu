@@ -188,14 +188,16 @@ bcc_status await_total(bcc_ctx* ctx, int& total) {
     return BCC_OK;
 }
 
-// Probe grids of the uploaded set for a robot's reach, built on the first check
-// that uses them after an upload (or after a check of another robot): cubic
+// Probe grids of the uploaded set for a robot's reach, built on the robot's first
+// check that uses them after an upload (each robot keeps its own: a context that
+// alternates robots would build them at every change): cubic
 // voxels, as many as kMaxVoxels allow.  Stream-ordered on st; the caller
 // synchronises st before any other stream can use the grids.  Without the
 // memory for them checks run unprobed.
 bcc::ProbeGrid probe_grid(bcc_ctx* ctx, const bcc::RobotOps* ops, cudaStream_t st) {
-    bcc::ProbeGrid& g = ctx->probe;
-    if (ctx->probe_robot == ops->robot && ctx->probe_version == ctx->env_version) return g;
+    bcc::ProbeSet& set = ctx->probe[ops->robot];
+    bcc::ProbeGrid& g = set.grid;
+    if (set.version == ctx->env_version) return g;
     float lo[3], hi[3];
     ops->reach(lo, hi);
     double ext[3], h = 0.0;
@@ -215,15 +217,14 @@ bcc::ProbeGrid probe_grid(bcc_ctx* ctx, const bcc::RobotOps* ops, cudaStream_t s
     g.oy = (float)(0.5 * (lo[1] + hi[1]) - 0.5 * (n[1] - 1) * h);
     g.oz = (float)(0.5 * (lo[2] + hi[2]) - 0.5 * (n[2] - 1) * h);
     g.stride = (uint32_t)((n[0] * n[1] * n[2] * 2 + 15) & ~15);
-    ctx->probe_robot = ops->robot;
-    ctx->probe_version = ctx->env_version;
-    if (ctx->vox.ensure((size_t)g.stride * ctx->num_envs) != cudaSuccess ||
+    set.version = ctx->env_version;
+    if (set.vox.ensure((size_t)g.stride * ctx->num_envs) != cudaSuccess ||
         bcc::launch_probe_grid(ctx->blobs.as<float4>(), ctx->env_hdr.as<float4>(), ctx->num_envs, g,
-                               ctx->vox.as<uint16_t>(), st) != cudaSuccess) {
+                               set.vox.as<uint16_t>(), st) != cudaSuccess) {
         cudaGetLastError();  // not an error of the check
         return g;            // vox stays null
     }
-    g.vox = ctx->vox.as<uint16_t>();
+    g.vox = set.vox.as<uint16_t>();
     return g;
 }
 

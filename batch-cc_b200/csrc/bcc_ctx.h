@@ -70,6 +70,13 @@ struct Tune {
     }
 };
 
+// Probe grids of the uploaded set for one robot's reach.
+struct ProbeSet {
+    DevBuf vox;
+    ProbeGrid grid{};        // their shape (vox null: none)
+    long long version = -1;  // the upload they were built for
+};
+
 // A captured launch sequence (everything after the discretisation) and the
 // inputs it was captured for.
 struct GraphCache {
@@ -115,10 +122,7 @@ struct bcc_ctx {
     bcc::MlpState mlp;
     bcc::DevBuf grid_bounds; // [3][kGridSlabs + 1] slab boundaries of the uploaded set's cull grid
     bcc::DevBuf queue;       // probe spheres of the edges' middle samples, and the queue of undecided pairs
-    bcc::DevBuf vox;         // probe grids of the uploaded set
-    bcc::ProbeGrid probe{};  // ... their shape (vox null: none)
-    int probe_robot = -1;    // ... the robot and upload they were built for
-    long long probe_version = -1;
+    bcc::ProbeSet probe[3];  // by robot
     bcc::DevBuf env_code;    // [num_envs][32] environment encodings
     bool env_code_ready = false;
     // inline learned order: environment clusters (k-means over the codes)

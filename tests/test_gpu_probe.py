@@ -150,3 +150,30 @@ def test_tables_of_an_earlier_call_too_small(graph):
     assert np.array_equal(a, b)
     assert len(orc.adjudicate(envs, edges, a, orc.check(envs, edges))[2]) == 0
     chk.close()
+
+
+def test_grids_are_built_once_a_robot_and_upload(checker):
+    """A context that alternates robots builds each one's grids once an upload."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    envs = workload.gen_envs("multi_fetch", 40, seed=91)
+    calls = [(r, workload.gen_edges(n, 300, seed=91)) for r, n in (("panda", "uneven"), ("fetch", "multi_fetch"),
+                                                                   ("baxter", "multi_baxter"))]
+    checker.upload(envs)
+    cfg = checker.launch_config()
+    checker.set_launch_config(edges_per_cta=64, warps=4, persistent=1)
+    try:
+        with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
+            torch.zeros(1, device="cuda")
+            got = [checker.check(edges, robot=robot) for _ in range(3) for robot, edges in calls]
+            torch.cuda.synchronize()
+    finally:
+        checker.set_launch_config(**cfg)
+    for k, (robot, edges) in enumerate(calls):
+        assert np.array_equal(got[k], got[k + 3]) and np.array_equal(got[k], got[k + 6])
+        want = orc.check(envs, edges[:60], robot=robot)
+        assert len(orc.adjudicate(envs, edges[:60], got[k][:60], want, robot=robot)[2]) == 0
+    names = [e.name for e in prof.events()]
+    if not any("walk_kernel" in n for n in names):
+        pytest.skip("this profiler does not see the library's kernels")
+    assert sum("probe_grid_kernel" in n for n in names) == 3
