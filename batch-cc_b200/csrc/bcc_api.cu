@@ -189,7 +189,7 @@ bcc_status await_total(bcc_ctx* ctx, int& total) {
 }
 
 // Probe grids of the uploaded set for a robot's reach, built on the robot's first
-// check that uses them after an upload (each robot keeps its own: a context that
+// probed check after an upload (each robot keeps its own: a context that
 // alternates robots would build them at every change): cubic
 // voxels, as many as kMaxVoxels allow.  Stream-ordered on st; the caller
 // synchronises st before any other stream can use the grids.  Without the
@@ -228,16 +228,36 @@ bcc::ProbeGrid probe_grid(bcc_ctx* ctx, const bcc::RobotOps* ops, cudaStream_t s
     return g;
 }
 
+// Whether a check of a new set should be the one that builds its grids: once the
+// unprobed checks of the set, this one among them, have missed as much as that costs
+// (so calls on sets that are checked once or twice never pay for it).  In us, measured
+// on 16 .. 1000 environments x 20 .. 10 000 edges of all three robots: a probed check
+// saves 20 and 0.2 to 2 ns a pair, less 30 ns an environment (its grid is staged); the
+// grids take 0.4 to 1 an environment, a new device allocation 330 of any size.
+// 100 x 1000 pairs: a first call of 1.89 ms with the grids, 1.25 without; then 0.33
+// against 0.41.
+bool grids_pay(bcc_ctx* ctx, bcc::ProbeSet& set, long long pairs) {
+    if (set.version == ctx->env_version) return true;  // built
+    if (set.counted != ctx->env_version) {
+        set.counted = ctx->env_version;
+        set.saving = 0.0;
+    }
+    set.saving += std::max(0.0, 20.0 + 5e-4 * (double)pairs - 0.03 * ctx->num_envs);
+    const bool vox = set.vox.cap < (size_t)ctx->num_envs * 2 * bcc::kMaxVoxels;
+    const bool queue = ctx->queue.cap < sizeof(uint2) * (size_t)std::min(pairs, bcc::kQueuePairs);
+    return set.saving >= 1.0 * ctx->num_envs + 330.0 * (vox + queue);
+}
+
 // The launch shape of a check of E edges: the context's once it was set or
 // tuned, else by size.  Below kProbeMinPairs pairs the probe's extra kernels cost
 // as much as the walks they save.
 constexpr long long kProbeMinPairs = 1 << 14;
 
-bcc::Tune launch_shape(const bcc_ctx* ctx, int E) {
+bcc::Tune launch_shape(bcc_ctx* ctx, const bcc::RobotOps* ops, int E) {
     bcc::Tune t = ctx->tune;
     if (t.tuned) return t;
     const long long pairs = (long long)ctx->num_envs * E;
-    t.persistent = pairs >= kProbeMinPairs ? 1 : 0;
+    t.persistent = pairs >= kProbeMinPairs && grids_pay(ctx, ctx->probe[ops->robot], pairs) ? 1 : 0;
     if (!t.persistent) {  // spread few pairs over the SMs: a pass of 12 edges fills a CTA's four warps
         t.warps = 4;
         t.edges_per_cta = (int)std::max<long long>(12, std::min<long long>(128, pairs / (148 * 4)));
@@ -278,7 +298,7 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     a.edge_tri = a.edge_self + word / sizeof(int);
     BCC_CUDA(ctx, ctx->error_flag.ensure(sizeof(int)));
     // Probed checks: grids, middle spheres and the queue, all or none.
-    const bcc::Tune tune = launch_shape(ctx, E);
+    const bcc::Tune tune = launch_shape(ctx, ops, E);
     if (d_results && tune.persistent && E <= 65535 * bcc::kProbeBatch &&
         ctx->blob_smem + bcc::kProbeBatch * bcc::kProbeEntryBytes + 2 * bcc::kMaxVoxels <= 200 * 1024) {
         const long long cap = std::min<long long>((long long)ctx->num_envs * E, bcc::kQueuePairs);

@@ -75,6 +75,8 @@ struct ProbeSet {
     DevBuf vox;
     ProbeGrid grid{};        // their shape (vox null: none)
     long long version = -1;  // the upload they were built for
+    long long counted = -1;  // the upload whose unprobed checks `saving` counts
+    double saving = 0.0;     // us that grids would have saved them
 };
 
 // A captured launch sequence (everything after the discretisation) and the

@@ -177,3 +177,45 @@ def test_grids_are_built_once_a_robot_and_upload(checker):
     if not any("walk_kernel" in n for n in names):
         pytest.skip("this profiler does not see the library's kernels")
     assert sum("probe_grid_kernel" in n for n in names) == 3
+
+
+def _kernels(call):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
+        torch.zeros(1, device="cuda")
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    if not any("fk_staged_kernel" in n for n in names):
+        pytest.skip("this profiler does not see the library's kernels")
+    return sum("probe_grid_kernel" in n for n in names), sum("walk_kernel" in n for n in names)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_first_check_of_a_small_set_builds_no_grids(graph):
+    """A set's grids cost more than they save its first few checks of a middle size:
+    those take one pass; a set that goes on being checked is probed, with one build, and
+    a new set starts over.  A large first check is probed at once."""
+    from bcc.lib import Checker
+    chk = Checker(0)
+    sets = [workload.gen_envs("uneven", 60, seed=s) for s in (92, 93)]
+    edges = workload.gen_edges("uneven", 800, seed=92)
+    for envs in sets:
+        want = orc.check(envs, edges[:60])
+        chk.upload(envs)
+        seen = []
+        for _ in range(40):
+            got = []
+            seen.append(_kernels(lambda: got.append(chk.check(edges, graph=graph))))
+            if len(seen) in (1, 2, 40):
+                assert len(orc.adjudicate(envs, edges[:60], got[0][:60], want)[2]) == 0
+        assert seen[0] == (0, 0) and seen[-1] == (0, 1)
+        assert sum(g for g, _ in seen) == 1  # then every check is probed
+        assert [w for _, w in seen] == sorted(w for _, w in seen)
+    chk.close()
+    big = Checker(0)
+    big.upload(workload.gen_envs("uneven", 600, seed=94))
+    edges = workload.gen_edges("uneven", 8000, seed=94)
+    assert _kernels(lambda: big.check(edges)) == (1, 1)
+    big.close()
