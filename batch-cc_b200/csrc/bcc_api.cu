@@ -346,21 +346,22 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     a.host_total = ctx->h_total;
     BCC_CUDA(ctx, ops->steps(a, st));
     BCC_CUDA(ctx, cudaEventRecord(ctx->ev_total, st));
+    // The rows and their segments' spheres, one allocation (330 us each to a first call),
+    // for a whole number of the 32-row blocks that every edge has.
     const int NS = ops->num_spheres;
-    const size_t held = std::min(ctx->table.cap / (sizeof(float4) * NS), ctx->seg.cap / (sizeof(float2) * G) * bcc::kSegment);
-    if (ahead && held >= bcc::kLanes) {
+    const size_t row_bytes = sizeof(float4) * NS + sizeof(float2) * G / bcc::kSegment;
+    auto held = [&] { return ctx->table.cap / row_bytes / bcc::kLanes * bcc::kLanes; };
+    if (ahead && held() > 0) {
         a.total_rows = -1;
-        a.cap_rows = (int)std::min<size_t>(held, kMaxSampleRows);
+        a.cap_rows = (int)std::min<size_t>(held(), kMaxSampleRows);
     } else {
         bcc_status s = await_total(ctx, a.total_rows);
         if (s != BCC_OK) return s;
         a.cap_rows = a.total_rows;
-        BCC_CUDA(ctx, ctx->table.ensure(sizeof(float4) * (size_t)NS * std::max(a.total_rows, 1)));
-        BCC_CUDA(ctx, ctx->seg.ensure(sizeof(float2) * (size_t)G *
-                                      (std::max(a.total_rows, bcc::kSegment) / bcc::kSegment)));
+        BCC_CUDA(ctx, ctx->table.ensure(row_bytes * (size_t)std::max(a.total_rows, bcc::kLanes)));
     }
-    a.seg = ctx->seg.as<float2>();
     a.table = ctx->table.as<float4>();
+    a.seg = reinterpret_cast<float2*>(a.table + (size_t)NS * held());
     a.blobs = ctx->blobs.as<float4>();
     a.env_hdr = ctx->env_hdr.as<float4>();
     a.irregular = ctx->irregular.as<int>();

@@ -113,7 +113,8 @@ struct bcc_ctx {
     int num_irregular = 0;
     bcc::DevBuf records;     // the upload's records as packed, source of the blobs
     // per-call buffers
-    bcc::DevBuf edges, per_edge, table, results, error_flag;  // per_edge: steps, offs, edge_self, edge_tri
+    bcc::DevBuf edges, per_edge, table, results, error_flag;  // per_edge: steps, offs, edge_self, edge_tri;
+                                                              // table: the rows, then their segments' spheres
     int* h_total = nullptr;  // pinned: the sample-row total, written by the offset kernel
     cudaEvent_t ev_total = nullptr;  // ... once this has passed
     bool profiling = false;
@@ -132,7 +133,6 @@ struct bcc_ctx {
     bcc::DevBuf centroids;   // [K][32] cluster centroid codes
     int cluster_k = 0;       // K of the current clustering, 0 = none
     bcc::DevBuf perms;       // [K][edges][kMaxSegments] per-check segment orders
-    bcc::DevBuf seg;         // [rows / kSegment][groups] segment spheres
     bcc::DevBuf q_head, q_pairs, q_rows;   // learned-order queue of undecided pairs
     const int* learned_rows_dev = nullptr; // queue head of the last learned check (entries << 32 | rows)
     int learned_row_cap = 0;

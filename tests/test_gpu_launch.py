@@ -152,3 +152,24 @@ def test_failed_autotune_leaves_the_configuration():
     got = chk.check(edges), chk.work_counters()
     assert np.array_equal(got[0], want[0]) and got[1] == want[1]
     chk.close()
+
+
+def test_first_check_allocates_its_tables_at_once():
+    """A first check's device allocations: a fixed few, each a cost of its own; the rows
+    and their segments' spheres share one, whatever their sizes."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from bcc.lib import Checker
+    envs, edges = workload.gen_envs("multi_baxter", 4, seed=55), workload.gen_edges("multi_baxter", 3000, seed=55)
+    torch.zeros(1, device="cuda")  # the profiled region's own
+    chk = Checker(0)
+    chk.upload(envs)
+    chk.check(edges[:1], robot="baxter")  # the buffers of fixed sizes
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as prof:
+        chk.check(edges, robot="baxter")
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    chk.close()
+    if not any("cudaLaunchKernel" in x for x in names):
+        pytest.skip("this profiler does not see the library's calls")
+    assert sum(x == "cudaMalloc" for x in names) == 4  # edges, verdicts, the edges' values, the table
