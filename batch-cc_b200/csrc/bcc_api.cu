@@ -198,8 +198,7 @@ bcc::ProbeGrid probe_grid(bcc_ctx* ctx, const bcc::RobotOps* ops, cudaStream_t s
     bcc::ProbeSet& set = ctx->probe[ops->robot];
     bcc::ProbeGrid& g = set.grid;
     if (set.version == ctx->env_version) return g;
-    float lo[3], hi[3];
-    ops->reach(lo, hi);
+    const float *lo = ops->reach_lo, *hi = ops->reach_hi;
     double ext[3], h = 0.0;
     for (int a = 0; a < 3; ++a) ext[a] = std::max(1e-3, (double)hi[a] - lo[a]);
     int n[3];

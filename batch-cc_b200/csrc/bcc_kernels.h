@@ -206,7 +206,8 @@ struct RobotOps {
     int num_env_groups;
     int max_prims;           // primitives per environment the pair packing allows
     // Box around the group bounds' centres over the joint limits (probe grid domain).
-    void (*reach)(float lo[3], float hi[3]);
+    const float* reach_lo;
+    const float* reach_hi;
     cudaError_t (*upload_tables)();  // robot tables -> the current device, complete on return
     // Stage 1: steps + sample offsets (total rows land in offs[E]).
     cudaError_t (*steps)(const PipelineArgs& a, cudaStream_t st);

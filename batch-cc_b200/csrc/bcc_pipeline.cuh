@@ -292,62 +292,6 @@ cudaError_t upload_to(const DevTables<M>& global, const DevTables<M>& constant) 
     return err == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : err;
 }
 
-// Box around the group bounds' centres over the joint limits: the domain of the
-// probe grid.  Sampled (a seeded sequence of 2048 configurations, 2 cm added):
-// a centre outside it costs the probe precision there, never correctness.
-template <class M>
-void sample_reach(float lo[3], float hi[3]) {
-    double l[3] = {1e30, 1e30, 1e30}, h[3] = {-1e30, -1e30, -1e30};
-    uint64_t rng = 0x9E3779B97F4A7C15ull;
-    for (int it = 0; it < 2048; ++it) {
-        double R[M::dof + 1][9] = {{1, 0, 0, 0, 1, 0, 0, 0, 1}}, p[M::dof + 1][3] = {};
-        for (int k = 0; k < M::dof; ++k) {
-            rng = rng * 6364136223846793005ull + 1442695040888963407ull;
-            const double q = (double)(rng >> 11) / 9007199254740992.0 * (double)M::s_m[k] + (double)M::s_a[k];
-            const double* f = M::joint_tf[k];
-            const double* P = R[M::joint_parent[k]];
-            double A[9];
-            for (int a = 0; a < 3; ++a) {
-                for (int b = 0; b < 3; ++b)
-                    A[a * 3 + b] = P[a * 3] * f[b] + P[a * 3 + 1] * f[4 + b] + P[a * 3 + 2] * f[8 + b];
-                p[k + 1][a] = P[a * 3] * f[3] + P[a * 3 + 1] * f[7] + P[a * 3 + 2] * f[11] + p[M::joint_parent[k]][a];
-            }
-            const bool rev = M::joint_type[k] == 0;
-            const double s = rev ? std::sin(q) : 0.0, c = rev ? std::cos(q) : 1.0;
-            for (int a = 0; a < 3; ++a) {
-                R[k + 1][a * 3 + 0] = A[a * 3] * c + A[a * 3 + 1] * s;
-                R[k + 1][a * 3 + 1] = A[a * 3 + 1] * c - A[a * 3] * s;
-                R[k + 1][a * 3 + 2] = A[a * 3 + 2];
-                if (!rev) p[k + 1][a] += A[a * 3 + 2] * q;
-            }
-        }
-        for (int g = 0; g < M::num_env_groups; ++g) {
-            const int b = M::env_bound[g], fr = M::sphere_frame[b];
-            const double* o = M::sphere_local[b];
-            for (int a = 0; a < 3; ++a) {
-                const double c = R[fr][a * 3] * o[0] + R[fr][a * 3 + 1] * o[1] + R[fr][a * 3 + 2] * o[2] + p[fr][a];
-                l[a] = std::min(l[a], c);
-                h[a] = std::max(h[a], c);
-            }
-        }
-    }
-    for (int a = 0; a < 3; ++a) {
-        lo[a] = (float)(l[a] - 0.02);
-        hi[a] = (float)(h[a] + 0.02);
-    }
-}
-
-template <class M>
-void reach_box(float lo[3], float hi[3]) {
-    struct Box {
-        float lo[3], hi[3];
-        Box() { sample_reach<M>(lo, hi); }
-    };
-    static const Box box;  // once per process
-    std::copy(box.lo, box.lo + 3, lo);
-    std::copy(box.hi, box.hi + 3, hi);
-}
-
 // Bits of the link-group index in a packed (primitive, group) pair.
 template <class M>
 constexpr int group_bits() {
@@ -2888,7 +2832,8 @@ RobotOps robot_ops_of(int robot, cudaError_t (*upload)()) {
     o.num_spheres = M::num_spheres;
     o.num_env_groups = M::num_env_groups;
     o.max_prims = max_prims_of<M>();
-    o.reach = reach_box<M>;
+    o.reach_lo = M::reach_lo;
+    o.reach_hi = M::reach_hi;
     o.upload_tables = upload;
     o.steps = run_steps<M>;
     o.check = run_check<M>;

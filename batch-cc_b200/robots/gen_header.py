@@ -56,6 +56,32 @@ def fmt(v):
     return repr(float(v))
 
 
+def reach_box(tfs, parents, types, bounds, s_m, s_a):
+    """Box around the group bounds' centres over the joint limits: 2048 seeded
+    configurations, 2 cm added.  A centre outside it costs the checker's probe
+    precision there, never correctness."""
+    dof = len(tfs)
+    rng, u = 0x9E3779B97F4A7C15, np.empty((2048, dof))
+    for i in range(u.size):
+        rng = (rng * 6364136223846793005 + 1442695040888963407) % (1 << 64)
+        u.flat[i] = (rng >> 11) / 9007199254740992.0
+    q = u * np.float32(s_m).astype(np.float64) + np.float32(s_a).astype(np.float64)
+    R, p = [np.broadcast_to(np.eye(3), (2048, 3, 3))], [np.zeros((2048, 3))]
+    for k in range(dof):
+        tf = np.asarray(tfs[k], np.float64).reshape(3, 4)
+        A = R[parents[k]] @ tf[:, :3]
+        at = R[parents[k]] @ tf[:, 3] + p[parents[k]]
+        if types[k]:
+            R.append(A)
+            p.append(at + A[:, :, 2] * q[:, k, None])
+        else:
+            c, s = np.cos(q[:, k, None]), np.sin(q[:, k, None])
+            R.append(np.stack([A[:, :, 0] * c + A[:, :, 1] * s, A[:, :, 1] * c - A[:, :, 0] * s, A[:, :, 2]], -1))
+            p.append(at)
+    c = np.concatenate([R[b["frame"]] @ np.asarray(b["local"], np.float64) + p[b["frame"]] for b in bounds])
+    return c.min(0) - 0.02, c.max(0) + 0.02
+
+
 def main():
     src, out = sys.argv[1], sys.argv[2]
     m = json.load(open(src))
@@ -95,7 +121,7 @@ def main():
     w("    // frame k+1 = frame joint_parent[k] * F_k * J_k(q_k), J = Rz(q) for a revolute")
     w("    // joint (type 0), Tz(q) for a prismatic one (type 1); frame 0 is the base.")
     w("    static constexpr double joint_tf[%d][12] = {" % dof)
-    parents, types = [], []
+    tfs, parents, types = [], [], []
     for k, j in enumerate(m["joints"]):
         if "tf" in j:
             vals = j["tf"]
@@ -104,6 +130,7 @@ def main():
             t = j["xyz"]
             vals = [R[0, 0], R[0, 1], R[0, 2], t[0], R[1, 0], R[1, 1], R[1, 2], t[1],
                     R[2, 0], R[2, 1], R[2, 2], t[2]]
+        tfs.append(vals)
         parents.append(j.get("parent_frame", k))
         types.append(1 if j.get("type") == "prismatic" else 0)
         w("        {%s}," % ", ".join(fmt(v) for v in vals))
@@ -180,6 +207,9 @@ def main():
     w("    // Joint-limit scale of the robot description: q = u * s_m + s_a.")
     w("    static constexpr float s_m[%d] = {%s};" % (dof, ", ".join(repr(float(np.float32(v))) + "f" for v in s_m)))
     w("    static constexpr float s_a[%d] = {%s};" % (dof, ", ".join(repr(float(np.float32(v))) + "f" for v in s_a)))
+    w("    // Box (m) around the env-group bounds' centres over the joint limits, sampled.")
+    for side, v in zip(("lo", "hi"), reach_box(tfs, parents, types, [sph[g["bound"]] for g in env], s_m, s_a)):
+        w("    static constexpr float reach_%s[3] = {%s};" % (side, ", ".join(repr(float(np.float32(x))) + "f" for x in v)))
     w("};")
     w("")
     w("}  // namespace bcc")

@@ -166,3 +166,22 @@ def test_regroup_encloses_leaves_and_rejects_bad_partitions():
         X.regroup(base, X.PANDA_CHECK_GROUPS[:-1])               # a leaf missing
     with pytest.raises(SystemExit):
         X.regroup(base, [X.PANDA_CHECK_GROUPS[0] + X.PANDA_CHECK_GROUPS[1]] + X.PANDA_CHECK_GROUPS[2:])  # two frames
+
+
+@pytest.mark.parametrize("robot", ["panda", "fetch", "baxter"])
+def test_header_carries_the_reach_of_the_bounds(robot):
+    """The probe grid's box is a constant of the header: it holds the oracle's bound
+    centres of fresh configurations (2 cm past 2048 sampled ones, so all but a few in
+    a thousand) and is no wider than they need."""
+    from bcc import workload
+    from oracle import oracle as orc
+    text = open(os.path.join(HEADERS, "robot_%s.h" % robot)).read()
+    lo, hi = (np.array([float(v.rstrip("f")) for v in re.search(
+        r"reach_%s\[3\] = \{([^}]*)\};" % side, text).group(1).split(", ")]) for side in ("lo", "hi"))
+    s_m, s_a = workload.LIMITS[robot]
+    rng = np.random.default_rng(5)
+    bounds = [g["bound"] for g in cases.robot_model(robot)["env_groups"]]
+    c = np.stack([orc.fk((rng.uniform(0, 1, len(s_m)) * s_m + s_a).astype(np.float32), robot)[bounds]
+                  for _ in range(2000)])
+    assert ((c < lo) | (c > hi)).any((1, 2)).mean() < 0.01
+    assert (c.min((0, 1)) - lo < 0.1).all() and (hi - c.max((0, 1)) < 0.1).all()
