@@ -1477,7 +1477,10 @@ bcc_status bcc_autotune(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32
     // Launch shape first (for the learned order at a middle threshold with
     // one-warp finishes), then the learned order's threshold x finish mode at
     // that shape, then the shape once more at the chosen threshold and mode.
+    // The probed check takes no edge tile (queue.batch and queue.chunk are its), the
+    // queued order no probe: one timing each where a value changes nothing.
     auto sweep_shape = [&](const bcc::Tune& from) {
+        const bool queued = learned && from.learned_mode == 1;
         for (int ti = 0; ti < 4 && s == BCC_OK; ++ti)
             for (int wi = 0; wi < 2 && s == BCC_OK; ++wi)
                 for (int pe = 0; pe < 2 && s == BCC_OK; ++pe) {
@@ -1485,6 +1488,7 @@ bcc_status bcc_autotune(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32
                     t.edges_per_cta = tiles[ti];
                     t.warps = warps[wi];
                     t.persistent = pe;
+                    if (queued ? pe != from.persistent : pe == 1 && ti != 3) continue;
                     if (!t.initial_shape()) keep(t);
                 }
     };

@@ -173,3 +173,25 @@ def test_first_check_allocates_its_tables_at_once():
     if not any("cudaLaunchKernel" in x for x in names):
         pytest.skip("this profiler does not see the library's calls")
     assert sum(x == "cudaMalloc" for x in names) == 4  # edges, verdicts, the edges' values, the table
+
+
+def test_autotune_times_a_probed_shape_once():
+    """The probed check has no edge tile: its two warp counts are timed, a check and five
+    replays each, not once a tile."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from bcc.lib import Checker
+    envs, edges = workload.gen_envs("uneven", 30, seed=56), workload.gen_edges("uneven", 300, seed=56)
+    chk = Checker(0)
+    chk.upload(envs)
+    want = chk.check(edges)
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
+        torch.zeros(1, device="cuda")
+        chk.autotune(edges, order="plain")
+        torch.cuda.synchronize()
+    assert np.array_equal(chk.check(edges), want)
+    chk.close()
+    names = [e.name for e in prof.events()]
+    if not any("check_kernel" in n for n in names):
+        pytest.skip("this profiler does not see the library's kernels")
+    assert sum("probe_kernel" in n for n in names) == 2 * 6
