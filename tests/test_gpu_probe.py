@@ -219,3 +219,45 @@ def test_first_check_of_a_small_set_builds_no_grids(graph):
     edges = workload.gen_edges("uneven", 8000, seed=94)
     assert _kernels(lambda: big.check(edges)) == (1, 1)
     big.close()
+
+
+def _oracles(envs, edges, got, robot="panda"):
+    want = orc.check(envs, edges, robot=robot)
+    assert 0 < int(want.sum()) < want.size
+    assert len(orc.adjudicate(envs, edges, got, want, robot=robot)[2]) == 0
+
+
+@pytest.mark.parametrize("prims", [255, 256, 257, 600])
+def test_primitives_beyond_voxel_ids_are_the_oracles(checker, prims):
+    rng = np.random.default_rng(prims)
+    c = rng.uniform(-1.0, 1.0, (prims, 3))
+    r = rng.uniform(0.01, 0.03, prims)
+    # the nearest primitives are the last ones
+    far = {"spheres": make_spheres(np.concatenate([c[:-40] * 0.2 + np.sign(c[:-40]) * 0.9, c[-40:]]), r)}
+    envs = EnvSet.from_lists([far, {"spheres": make_spheres(c, r)}, {}])
+    edges = workload.gen_edges("uneven", 300, seed=5)
+    _oracles(envs, edges, both(checker, envs, edges, "panda"))
+
+
+def test_pairs_on_both_sides_of_the_queues_slabs_are_the_oracles(checker):
+    """70 000 environments x 1000 edges: the first slab ends at environment 67 108."""
+    n = 70000
+    rng = np.random.default_rng(8)
+    r = make_spheres(rng.uniform(-0.8, 0.8, (n, 3)) + [0, 0, 0.5], rng.uniform(0.05, 0.15, n))
+    envs = EnvSet({"spheres": np.ones(n, np.uint32)}, {"spheres": r})
+    edges = workload.gen_edges("uneven", 1000, seed=9)
+    got = both(checker, envs, edges, "panda")
+    for lo, hi in ((0, 10), (67098, 67118), (69990, 70000)):
+        _oracles(EnvSet({"spheres": np.ones(hi - lo, np.uint32)}, {"spheres": r[lo:hi]}), edges[::5], got[::5, lo:hi])
+
+
+@pytest.mark.parametrize("name,nenv,nedge", [("uneven", 24, 700), ("stress", 16, 1030), ("multi_fetch", 17, 600),
+                                             ("multi_baxter", 11, 520)])
+def test_probed_check_is_the_oracles(checker, name, nenv, nedge):
+    """Every edge of batches that end within a probe CTA's, not the first ones only
+    (three primitives of each kind for the larger robots: with all few edges are free)."""
+    robot = workload.robot_of(name)
+    envs, edges = workload.gen_envs(name, nenv, seed=73), workload.gen_edges(name, nedge, seed=73)
+    if robot != "panda":
+        envs = EnvSet.from_lists([{k: r[:3] for k, r in envs.env(i).items()} for i in range(nenv)])
+    _oracles(envs, edges, both(checker, envs, edges, robot), robot)
