@@ -1239,7 +1239,8 @@ __device__ __forceinline__ bool exact_hit(const float4* row, const float4* prim,
             if (s < spheres) {
                 float4 c = row[pos[s]];
                 c.w += kEnvInflate;
-                hit = sphere_hits_prim(c, prim + p * kPrimF4);
+                // (a centre that is not finite is nowhere, as in the culls of the other walks)
+                hit = isfinite(c.x + c.y + c.z) && sphere_hits_prim(c, prim + p * kPrimF4);
             }
             if (found(hit, s)) return true;
             s += ds;

@@ -130,3 +130,12 @@ def test_packed_irregular_records_are_the_oracles(robot):
     assert f(bcclib.ROBOTS[robot], d_rec.data_ptr(), d_off.data_ptr(), envs.num_envs, most.value, d_edges.data_ptr(),
              len(edges), 32, out.data_ptr(), None) == 0
     _is_the_oracles(envs, edges, out.cpu().numpy(), robot, orc.check(envs, edges, robot=robot))
+
+
+def test_edges_that_are_not_numbers_hit_nothing(checker):
+    """As in environments of boxes: a link whose place is not a number is nowhere."""
+    envs, edges = _case("panda", 40)
+    edges[::2, 1, 0] = np.nan  # the first joint: every link
+    checker.upload(envs)
+    got = checker.check(edges)
+    assert not got[::2].any() and got[1::2].any()
