@@ -382,8 +382,8 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     a.queue_min_items = ctx->tune.queue_min_items;
     a.finish_split = ctx->tune.finish_split;
     a.mode = 0;
-    BCC_CUDA(ctx, ctx->work_counter.ensure(64));
-    a.work_counter = ctx->work_counter.as<int>();
+    BCC_CUDA(ctx, ctx->finish_counter.ensure(sizeof(int)));
+    a.finish_counter = ctx->finish_counter.as<int>();
     return BCC_OK;
 }
 
@@ -488,7 +488,6 @@ bcc_status prepare_learned(bcc_ctx* ctx, bcc::PipelineArgs& a, int row_cap) {
     a.logits = ctx->mlp.logits.as<float>();
     a.features = ctx->mlp.x.p;
     a.queue_min_items = ctx->tune.queue_min_items;
-    a.finish_counter = a.work_counter + 1;
     ctx->learned_rows_dev = reinterpret_cast<int*>(a.q_head);  // the low word counts rows
     ctx->last_learned_inline = false;
     ctx->learned_row_cap = cap;
@@ -587,7 +586,7 @@ bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
            x.edges_per_cta == y.edges_per_cta && x.q_head == y.q_head && x.q_pairs == y.q_pairs &&
            x.q_rows == y.q_rows && x.logits == y.logits && x.perms == y.perms && x.env_cluster == y.env_cluster &&
            x.centroids == y.centroids &&
-           x.features == y.features && x.work_counter == y.work_counter && x.error_flag == y.error_flag;
+           x.features == y.features && x.finish_counter == y.finish_counter && x.error_flag == y.error_flag;
 }
 
 // Launches a check.  A plain one that finds the tables of an earlier call is queued
@@ -996,12 +995,11 @@ bcc_status bcc_check(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32_t 
     bcc_status s = run_check(ctx, robot, ctx->edges.as<float>(), num_edges, resolution,
                              ctx->results.as<uint8_t>(), opts, st);
     if (s != BCC_OK) return s;
-    // (the sample total was read before the check was launched: its word is free)
+    // (run_check has read the sample total: its word is free)
     BCC_CUDA(ctx, cudaMemcpyAsync(ctx->h_total, ctx->error_flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     BCC_CUDA(ctx, cudaMemcpyAsync(results, ctx->results.p, rb, cudaMemcpyDeviceToHost, st));
     BCC_CUDA(ctx, cudaStreamSynchronize(st));
     const int flag = *ctx->h_total;
-    if (flag & 4) return fail(ctx, BCC_ERR_TIMEOUT, "a walk exceeded its step bound");
     if (flag) return fail(ctx, BCC_ERR_TIMEOUT, "a bounded device wait gave up (bulk copy did not complete)");
     return BCC_OK;
 }
@@ -1358,11 +1356,11 @@ int64_t bcc_last_learned_pairs(const bcc_ctx* ctx) {
 }
 
 // Launch configuration (BCC_LAUNCH_CONFIG_LEN values): [0] edges per CTA,
-// [1] warps per CTA, [2] persistent kernel (0/1), [3] learned-order queue
+// [1] warps per CTA, [2] probed (1) or one pass (0), [3] learned-order queue
 // threshold (items), [4] learned-order finish: 1 = each queued pair split over
 // a CTA's warps, 0 = one warp per pair, [5] learned order: 0 = inline, 1 =
-// queued, [6] inline learned order: environment clusters (1..64), [7] lanes
-// per walking pair in the plain-order walk (32, or 16: half-warps).
+// queued, [6] inline learned order: environment clusters (1..64), [7] 32 or 16,
+// without an effect (every walk takes a whole warp).
 bcc_status bcc_get_launch_config(const bcc_ctx* ctx, int32_t* cfg) {
     if (!ctx || !cfg) return BCC_ERR_INVALID_ARGUMENT;
     cfg[0] = ctx->tune.edges_per_cta;

@@ -43,7 +43,6 @@ struct MlpState {
     }
     DevBuf adam_m, adam_v;   // Adam moments
     DevBuf images;           // BF16 core-matrix images of W1^T, W2^T, W3^T
-    DevBuf acts;             // training activations
     DevBuf x, y, logits;     // per-call inputs / outputs
     DevBuf lab;              // learned-order population: per-sample verdicts (8 per row)
     DevBuf x2, y2, perm;     // shuffled training rows and their permutation
@@ -86,7 +85,7 @@ struct GraphCache {
     const void* edges = nullptr;
     void* results = nullptr;
     cudaStream_t stream = nullptr;
-    int num_edges = -1, resolution = -1, total_rows = -1, order = -1, robot = -1, row_cap = -1;
+    int num_edges = -1, resolution = -1, total_rows = -1, robot = -1, row_cap = -1;
     long long env_version = -1;
     Tune tune;
     PipelineArgs args{};     // the buffers it was captured with
@@ -140,7 +139,7 @@ struct bcc_ctx {
     long long last_inline_rows = 0;        // its (cluster, segment) rows
     int learned_q_cap = 0;
     bcc::Tune tune;                        // launch configuration (autotuned or default)
-    bcc::DevBuf work_counter;              // persistent-kernel work queue head
+    bcc::DevBuf finish_counter;            // learned order, queued: next entry to finish
     long long env_version = 0;             // bumped by every upload (graph cache key)
     bcc::GraphCache graph[2];              // per order (plain, learned)
 };

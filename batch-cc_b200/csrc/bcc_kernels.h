@@ -152,7 +152,6 @@ struct PipelineArgs {
     int queue_min_items;
     int* finish_counter;
     int finish_split;
-    int* work_counter;
     const int* env_cluster;
     const float* centroids;  // [K][32] cluster codes, inline learned order
     const uint8_t* perms;

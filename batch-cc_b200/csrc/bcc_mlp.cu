@@ -1,11 +1,14 @@
 // bcc_mlp.cu -- the collision-likelihood MLP on 5th-generation tensor cores.
 //
 // Network (per sample configuration in one environment):
-//     x (48 = 7 normalised joints + 32 environment code + 9 zero) -> 128 -> 128 -> 128 -> 1
-// ReLU between layers, logit output.  Weights and activations are BF16 in
-// shared memory (core-matrix images, see bcc_tc.cuh), products accumulate in
-// FP32 tensor memory via tcgen05.mma (M = 128 rows per tile, N = 128), the
-// epilogues (bias, ReLU, final 128-wide dot product) run in FP32 registers.
+//     x (48: normalised joints, 32 environment code, zeros, position along the edge,
+//     bias input) -> 128 -> 128 -> 128 -> 1
+// ReLU between layers, logit output.  Weights are BF16 in shared memory (core-matrix
+// images, see bcc_tc.cuh), products accumulate in FP32 tensor memory via tcgen05.mma
+// (M = 128 rows per tile, N = 128).  Activations are BF16, in tensor memory in the
+// forward kernel (biases and the last layer are MMAs too, the epilogue is a ReLU), in
+// shared memory in the training kernel (bias, ReLU and the last dot product in FP32
+// registers).
 //
 // Parameters (FP32 masters, flat, kMlpParams floats):
 //     W1 [48][128] (in x out), b1 [128], W2 [128][128], b2 [128],

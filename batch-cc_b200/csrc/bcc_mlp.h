@@ -6,7 +6,7 @@
 
 namespace bcc {
 
-constexpr int kMlpIn = 48;       // 7 joints + 32 environment code + 9 zero padding
+constexpr int kMlpIn = 48;       // joints, 32 environment code, zeros, position along the edge, bias input
 constexpr int kMlpJoints = 7;
 constexpr int kEnvCode = 32;
 constexpr int kMlpHidden = 128;

@@ -35,10 +35,12 @@
 //
 // Gate semantics.  The reference tests a link's leaves only after the link's
 // bounding sphere hit SOME primitive (fkcc: `if (bound in collision) { if
-// (leaf in collision) return false; ... }`).  Per (sample, primitive, link)
-// item the checker tests the bound against that primitive and, on a hit, every
-// leaf against it.  That is the same verdict wherever the leaves lie inside
-// the bound.  For the leaves that stick out of their bound (Fetch, Baxter:
+// (leaf in collision) return false; ... }`).  Where the leaves lie inside the
+// bound a leaf's hit implies its bound's, so any order of tests gives the
+// reference's verdict: the walk by segments goes from a segment's sphere to the
+// leaves, the walk by samples tests the bound against a primitive and, on a hit,
+// every leaf against it.  (Environments where a hit does not imply the bound's:
+// kEnvIrregular.)  For the leaves that stick out of their bound (Fetch, Baxter:
 // up to 0.6 mm, the model's env_over_count / env_cull_pad) the checker also
 // tests them against primitives the bound misses but the padded bound reaches,
 // and a hit there counts only after a scan of the whole environment confirms
@@ -733,11 +735,11 @@ __device__ __forceinline__ int slab_tri(float lo, float hi, const float* __restr
 
 // One warp per edge: AABB (lo, hi) of every link group's bounding sphere over
 // the edge's samples, inflated by radius + 0.005 + the group's leaf overhang +
-// cull margin, written where swept is given (the records check); and (edge_tri non-null) its slab ranges on the set's cull grid,
-// packed tx | ty << 10 | tz << 20 (-1 when some axis misses every primitive);
-// and (mid non-null) the bound's centre at the edge's middle sample with the
-// radius, inflated likewise, of the sphere around it that holds them all; and
-// (seg non-null, tiled tables) the segments' spheres (see segment_spheres).
+// cull margin, written where swept is given (the records check); and (edge_tri
+// non-null) its slab ranges on the set's cull grid, packed tx | ty << 10 | tz << 20
+// (-1 when some axis misses every primitive); and (mid non-null) the bound's centre
+// at the edge's middle sample with the radius, inflated likewise, of the sphere
+// around it that holds them all.
 // Lane g ends up holding group g's box: it scans group g's bound down the rows (a
 // row's bounds are contiguous), 32 / G rows at a time.
 template <class M>

@@ -54,6 +54,9 @@ typedef enum bcc_robot {
  * (src/utils.cuh:213-245), never tested: the reference drivers pass
  * cylinders as capsules.
  * A null count array means zero primitives of that kind in every environment.
+ * Records are taken as given.  Where an environment has one that is not a box (axes
+ * further than 5e-5 from orthonormal, a negative radius, a value that is not finite)
+ * all of its pairs take the reference's tests at every sample, several times the work.
  */
 typedef struct bcc_env_soa {
     int32_t num_envs;
@@ -87,7 +90,14 @@ typedef struct bcc_opts {
 
 typedef struct bcc_ctx bcc_ctx;
 
-/* Context lifetime.  A context owns device buffers that persist across calls. */
+/*
+ * Context lifetime.  A context owns device buffers that persist across calls, as
+ * large as its largest call needed: per sample row of the edges 16 bytes a robot
+ * sphere and one a link group, the verdicts of host calls, and for probed checks 28 KB
+ * an environment and robot (voxel grids), 8 bytes a pair up to 64 M pairs (512 MB)
+ * and 16 bytes an edge and link group.  Without the memory for those a check takes
+ * one pass over all pairs.
+ */
 bcc_status bcc_create(bcc_ctx** out, int device);
 void bcc_destroy(bcc_ctx* ctx);
 const char* bcc_last_error(const bcc_ctx* ctx);
@@ -170,8 +180,9 @@ int32_t bcc_work_counters(bcc_ctx* ctx, uint64_t* out, int32_t max_counters);
  * (sum over edges of 32 n); beyond either the call returns BCC_ERR_LIMIT
  * without checking anything.  d_records must be 16-byte aligned (bulk copies
  * stage it); a misaligned pointer returns BCC_ERR_INVALID_ARGUMENT before any
- * launch.  Synchronous on `stream`: every call reads the sample count back and
- * synchronises, so no call can be made inside a stream capture.  The first call
+ * launch.  Synchronous on `stream`: its kernels are queued whole (they do nothing
+ * beyond 4096 samples), then the sample count and an error flag are read back, so no
+ * call can be made inside a stream capture.  The first call
  * on a device sets that device up for the life of the process (resolves the
  * arrays' addresses, uploads the robot tables); a cudaDeviceReset after it is
  * not supported.  Every call reuses the same arrays, so calls that overlap on
