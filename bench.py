@@ -652,7 +652,7 @@ def run_ours(args, world, rank, local, dist):
     # bound by instruction issue (integer/logic and FP32 SIMT work on L2- and
     # shared-memory-resident inputs, DRAM a few per cent busy), so the roofline
     # is issue slots: achieved = warp instructions per launch (the committed ncu
-    # count per pair x this launch's pairs) / the launch's CUDA-event duration,
+    # count of this workload at this size) / the launch's CUDA-event duration,
     # peak = 148 SMs x 4 issue slots per cycle x the SM clock sampled during the
     # timed region.  The executed FP32 arithmetic is reported beside it against
     # the FMA probe's peak, and the reference's plain-order work (oracle count)
@@ -684,7 +684,7 @@ def run_ours(args, world, rank, local, dist):
                      "executed_warp_instructions_per_launch": inst,
                      "counts_source": "ncu sm__inst_executed.sum, smsp__sass_thread_inst_executed_op_{ffma,fadd,"
                                       "fmul}_pred_on.sum, dram__bytes_{read,write}.sum of one plain check's probe_kernel "
-                                      "and walk_kernel, per pair, scaled by this launch's pairs (%s)" % COUNTS_FILE,
+                                      "and walk_kernel on this workload at this size, per pair (%s)" % COUNTS_FILE,
                      "fp32": {"achieved_tflops": flop / (chk_ms * 1e-3) / 1e12, "peak": fp32_peak,
                               "frac": flop / (chk_ms * 1e-3) / 1e12 / fp32_peak,
                               "peak_source": "FP32 FMA probe kernel measured in this run (bcc_measure_fp32_peak)"}})

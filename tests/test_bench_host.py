@@ -42,3 +42,15 @@ def test_tuning_subset_outgrows_l2_like_the_full_workload():
     assert 5000 <= n <= 10000
     assert n * 32 * 1.1 * 77 * 16 > 126e6
     assert bench.tune_edges(300, 10) == 300            # small cases: every edge
+
+
+def test_committed_counts_are_the_workloads_own():
+    """The roofline divides by the full workload's time: its counts come from that size,
+    not from a smaller case whose pairs take more instructions."""
+    import re
+    bench = _bench()
+    text = open(os.path.join(ROOT, bench.COUNTS_FILE)).read()
+    full = text.split("## Instruction counts: full uneven workload (1000 envs x 10 000 edges)")[1].split("\n## ")[0]
+    row = re.search(r"`sm__inst_executed.sum`[^|]*\|([^|]*)\|([^|]*)\|", full)
+    total = sum(int(v.replace(" ", "")) for v in row.groups())
+    assert abs(bench.committed_counts("uneven")["inst_per_pair"] - total / 1e7) < 0.01
