@@ -269,11 +269,14 @@ bcc::Tune launch_shape(bcc_ctx* ctx, const bcc::RobotOps* ops, int E) {
 
 // Discretisation, sample offsets and every per-call buffer of a check; fills
 // `a` up to (not including) the FK / self / swept / check launches.
-// With `ahead` the sample total is not waited for when the tables of an earlier
-// call exist: a.total_rows stays -1, the kernels work within a.cap_rows, and the
-// caller settles the total afterwards (await_total).
+// With `ahead` a.total_rows stays -1 and the kernels work within a.cap_rows, what the
+// table holds; the sample total is waited for, and the table grown, only where there
+// is none from an earlier call or the caller asks for it (`grow`), and the caller
+// settles the total afterwards (await_total).  A captured check is then the same
+// from its first call on.
 bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution, uint8_t* d_results,
-                   const bcc_opts* opts, cudaStream_t st, bcc::PipelineArgs& a, bool ahead = false) {
+                   const bcc_opts* opts, cudaStream_t st, bcc::PipelineArgs& a, bool ahead = false,
+                   bool grow = false) {
     const int r = (int)robot;
     const bcc::RobotOps* ops = bcc::robot_ops(r);
     if (!ops) return fail(ctx, BCC_ERR_NOT_SUPPORTED, "robot not built into this library");
@@ -350,14 +353,15 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     const int NS = ops->num_spheres;
     const size_t row_bytes = sizeof(float4) * NS + sizeof(float2) * G / bcc::kSegment;
     auto held = [&] { return ctx->table.cap / row_bytes / bcc::kLanes * bcc::kLanes; };
-    if (ahead && held() > 0) {
-        a.total_rows = -1;
-        a.cap_rows = (int)std::min<size_t>(held(), kMaxSampleRows);
-    } else {
+    if (!ahead || grow || held() == 0) {
         bcc_status s = await_total(ctx, a.total_rows);
         if (s != BCC_OK) return s;
         a.cap_rows = a.total_rows;
         BCC_CUDA(ctx, ctx->table.ensure(row_bytes * (size_t)std::max(a.total_rows, bcc::kLanes)));
+    }
+    if (ahead) {
+        a.total_rows = -1;
+        a.cap_rows = (int)std::min<size_t>(held(), kMaxSampleRows);
     }
     a.table = ctx->table.as<float4>();
     a.seg = reinterpret_cast<float2*>(a.table + (size_t)NS * held());
@@ -595,8 +599,9 @@ bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
 // done nothing and it is launched again.  (Learned checks size their MLP rows by
 // the total, profiled ones bracket their stages.)
 bcc_status launch_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution,
-                        uint8_t* d_results, const bcc_opts* opts, cudaStream_t st, bool ahead, bcc::PipelineArgs& a) {
-    bcc_status s = prepare(ctx, robot, d_edges, E, resolution, d_results, opts, st, a, ahead);
+                        uint8_t* d_results, const bcc_opts* opts, cudaStream_t st, bool ahead, bool grow,
+                        bcc::PipelineArgs& a) {
+    bcc_status s = prepare(ctx, robot, d_edges, E, resolution, d_results, opts, st, a, ahead, grow);
     if (s != BCC_OK) return s;
     const bool learned = opts && opts->order == BCC_ORDER_LEARNED;
     if (learned) {
@@ -665,12 +670,12 @@ bcc_status run_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E,
                      uint8_t* d_results, const bcc_opts* opts, cudaStream_t st) {
     const bool ahead = !(opts && opts->order == BCC_ORDER_LEARNED) && !ctx->profiling && !ctx->counting;
     bcc::PipelineArgs a;
-    bcc_status s = launch_check(ctx, robot, d_edges, E, resolution, d_results, opts, st, ahead, a);
+    bcc_status s = launch_check(ctx, robot, d_edges, E, resolution, d_results, opts, st, ahead, false, a);
     if (s != BCC_OK || a.total_rows >= 0) return s;
     int total = 0;
     s = await_total(ctx, total);
     if (s != BCC_OK || total <= a.cap_rows) return s;
-    return launch_check(ctx, robot, d_edges, E, resolution, d_results, opts, st, false, a);
+    return launch_check(ctx, robot, d_edges, E, resolution, d_results, opts, st, true, true, a);
 }
 
 }  // namespace

@@ -195,3 +195,32 @@ def test_autotune_times_a_probed_shape_once():
     if not any("check_kernel" in n for n in names):
         pytest.skip("this profiler does not see the library's kernels")
     assert sum("probe_kernel" in n for n in names) == 2 * 6
+
+
+def test_graph_is_captured_once():
+    """Equal captured calls of a new context share one graph from the first on; one whose
+    edges need a larger table takes another."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from bcc.lib import Checker
+    envs = workload.gen_envs("uneven", 10, seed=57)
+    small, large = workload.gen_edges("uneven", 200, seed=57), workload.gen_edges("plain", 200, seed=57)
+    chk, other = Checker(0), Checker(0)
+    chk.upload(envs)
+    other.upload(envs)
+    counts = []
+    for edges, n in ((small, 3), (large, 3), (small, 2)):
+        want = other.check(edges)
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA], acc_events=True) as prof:
+            torch.zeros(1, device="cuda")
+            for _ in range(n):
+                assert np.array_equal(chk.check(edges, graph=True), want)
+            torch.cuda.synchronize()
+        names = [e.name for e in prof.events()]
+        if not any(n.startswith("cudaGraphLaunch") for n in names):
+            pytest.skip("this profiler does not see the library's calls")
+        counts.append(sum(x.startswith("cudaGraphInstantiate") for x in names))
+    chk.close()
+    other.close()
+    # the larger call queues the graph at hand, finds the table too small, and captures again
+    assert counts == [1, 1, 0], counts
