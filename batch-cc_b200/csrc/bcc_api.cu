@@ -252,12 +252,14 @@ bool grids_pay(bcc_ctx* ctx, bcc::ProbeSet& set, long long pairs) {
 // as much as the walks they save.
 constexpr long long kProbeMinPairs = 1 << 14;
 
-bcc::Tune launch_shape(bcc_ctx* ctx, const bcc::RobotOps* ops, int E) {
+bcc::Tune launch_shape(bcc_ctx* ctx, const bcc::RobotOps* ops, int E, bool probes) {
     bcc::Tune t = ctx->tune;
+    if (!probes) t.persistent = 0;
     if (t.tuned) return t;
     const long long pairs = (long long)ctx->num_envs * E;
-    t.persistent = pairs >= kProbeMinPairs && grids_pay(ctx, ctx->probe[ops->robot], pairs) ? 1 : 0;
-    if (!t.persistent) {  // spread few pairs over the SMs: a pass of 12 edges fills a CTA's four warps
+    const bool many = pairs >= kProbeMinPairs;
+    t.persistent = many && probes && grids_pay(ctx, ctx->probe[ops->robot], pairs) ? 1 : 0;
+    if (!t.persistent && !(many && !probes)) {  // spread few pairs over the SMs: a pass of 12 edges fills a CTA's four warps
         t.warps = 4;
         t.edges_per_cta = (int)std::max<long long>(12, std::min<long long>(128, pairs / (148 * 4)));
         return t;
@@ -269,13 +271,15 @@ bcc::Tune launch_shape(bcc_ctx* ctx, const bcc::RobotOps* ops, int E) {
 
 // Discretisation, sample offsets and every per-call buffer of a check; fills
 // `a` up to (not including) the FK / self / swept / check launches.
+// `queued`: for the queued learned order, whose probe is the walk of first samples
+// (no grids).
 // With `ahead` a.total_rows stays -1 and the kernels work within a.cap_rows, what the
 // table holds; the sample total is waited for, and the table grown, only where there
 // is none from an earlier call or the caller asks for it (`grow`), and the caller
 // settles the total afterwards (await_total).  A captured check is then the same
 // from its first call on.
 bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution, uint8_t* d_results,
-                   const bcc_opts* opts, cudaStream_t st, bcc::PipelineArgs& a, bool ahead = false,
+                   const bcc_opts* opts, cudaStream_t st, bcc::PipelineArgs& a, bool queued, bool ahead = false,
                    bool grow = false) {
     const int r = (int)robot;
     const bcc::RobotOps* ops = bcc::robot_ops(r);
@@ -300,8 +304,9 @@ bcc_status prepare(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, i
     a.edge_tri = a.edge_self + word / sizeof(int);
     BCC_CUDA(ctx, ctx->error_flag.ensure(sizeof(int)));
     // Probed checks: grids, middle spheres and the queue, all or none.
-    const bcc::Tune tune = launch_shape(ctx, ops, E);
-    if (d_results && tune.persistent && E <= 65535 * bcc::kProbeBatch &&
+    const bool probes = d_results && !queued;
+    const bcc::Tune tune = launch_shape(ctx, ops, E, probes);
+    if (tune.persistent && E <= 65535 * bcc::kProbeBatch &&
         ctx->blob_smem + bcc::kProbeBatch * bcc::kProbeEntryBytes + 2 * bcc::kMaxVoxels <= 200 * 1024) {
         const long long cap = std::min<long long>((long long)ctx->num_envs * E, bcc::kQueuePairs);
         const long long slab = cap / E;
@@ -601,9 +606,10 @@ bool same_buffers(const bcc::PipelineArgs& x, const bcc::PipelineArgs& y) {
 bcc_status launch_check(bcc_ctx* ctx, bcc_robot robot, const float* d_edges, int E, int resolution,
                         uint8_t* d_results, const bcc_opts* opts, cudaStream_t st, bool ahead, bool grow,
                         bcc::PipelineArgs& a) {
-    bcc_status s = prepare(ctx, robot, d_edges, E, resolution, d_results, opts, st, a, ahead, grow);
-    if (s != BCC_OK) return s;
     const bool learned = opts && opts->order == BCC_ORDER_LEARNED;
+    bcc_status s = prepare(ctx, robot, d_edges, E, resolution, d_results, opts, st, a,
+                           learned && ctx->tune.learned_mode == 1, ahead, grow);
+    if (s != BCC_OK) return s;
     if (learned) {
         if (!ctx->mlp.ready)
             return fail(ctx, BCC_ERR_INVALID_ARGUMENT, "learned order needs MLP parameters (bcc_mlp_train or bcc_mlp_set_params)");
@@ -1026,7 +1032,7 @@ bcc_status bcc_mlp_train(bcc_ctx* ctx, bcc_robot robot, const float* edges, int3
     BCC_CUDA(ctx, ctx->edges.ensure(sizeof(float) * 2 * (size_t)dof * num_edges));
     BCC_CUDA(ctx, copy_in(ctx->edges.p, edges, sizeof(float) * 2 * (size_t)dof * num_edges));
     bcc::PipelineArgs a;
-    bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), num_edges, resolution, nullptr, nullptr, st, a);
+    bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), num_edges, resolution, nullptr, nullptr, st, a, false);
     if (s != BCC_OK) return s;
     BCC_CUDA(ctx, bcc::robot_ops((int)robot)->prep(a, st));
     s = ensure_env_code(ctx, st);
@@ -1073,7 +1079,7 @@ bcc_status bcc_mlp_evaluate(bcc_ctx* ctx, bcc_robot robot, const float* edges, i
     BCC_CUDA(ctx, ctx->edges.ensure(sizeof(float) * 2 * (size_t)dof * num_edges));
     BCC_CUDA(ctx, copy_in(ctx->edges.p, edges, sizeof(float) * 2 * (size_t)dof * num_edges));
     bcc::PipelineArgs a;
-    bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), num_edges, resolution, nullptr, nullptr, st, a);
+    bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), num_edges, resolution, nullptr, nullptr, st, a, false);
     if (s != BCC_OK) return s;
     BCC_CUDA(ctx, bcc::robot_ops((int)robot)->prep(a, st));
     s = ensure_env_code(ctx, st);
@@ -1139,7 +1145,7 @@ bcc_status queue_population(bcc_ctx* ctx, bcc_robot robot, const float* edges, i
     BCC_CUDA(ctx, ctx->edges.ensure(eb));
     BCC_CUDA(ctx, copy_in(ctx->edges.p, edges, eb));
     BCC_CUDA(ctx, ctx->results.ensure((size_t)E * ctx->num_envs));
-    bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), E, resolution, ctx->results.as<uint8_t>(), nullptr, st, a);
+    bcc_status s = prepare(ctx, robot, ctx->edges.as<float>(), E, resolution, ctx->results.as<uint8_t>(), nullptr, st, a, true);
     if (s != BCC_OK) return s;
     if ((s = ensure_env_code(ctx, st)) != BCC_OK) return s;
     if ((s = prepare_learned(ctx, a, 0)) != BCC_OK) return s;

@@ -321,3 +321,27 @@ def test_graph_after_the_centroids_moved():
         chk.set_launch_config(clusters=clusters)
         assert np.array_equal(chk.check(edges, order="learned", graph=graph), want), (clusters, graph)
     chk.close()
+
+
+def test_queued_order_builds_no_voxel_grids():
+    """Its probe is the walk of first samples: neither its checks nor the training on its
+    population use or build the grids."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    from bcc.lib import Checker
+    envs, edges = workload.gen_envs("uneven", 60, seed=84), workload.gen_edges("uneven", 900, seed=84)
+    chk = Checker(0)
+    chk.upload(envs)
+    chk.mlp_set_params(mlp.init_params(4))
+    chk.set_launch_config(edges_per_cta=64, warps=4, persistent=1, learned_mode=1)
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
+        torch.zeros(1, device="cuda")
+        chk.mlp_train_queued(edges, num_samples=4096, epochs=1, batch=1024)
+        got = chk.check(edges, order="learned")
+        torch.cuda.synchronize()
+    assert np.array_equal(got, chk.check(edges))
+    chk.close()
+    names = [e.name for e in prof.events()]
+    if not any("fk_staged_kernel" in n for n in names):
+        pytest.skip("this profiler does not see the library's kernels")
+    assert not any("probe_grid_kernel" in n for n in names)
