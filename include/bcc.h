@@ -124,7 +124,9 @@ bcc_status bcc_check(bcc_ctx* ctx, bcc_robot robot, const float* edges, int32_t 
 /*
  * Device-resident variant: edges and results are device pointers; the call is
  * stream-ordered on `stream` (a cudaStream_t, 0 = legacy default stream) and
- * returns without synchronising.
+ * returns without synchronising.  A context's calls share its buffers: a caller that
+ * changes streams between them (the other entry points have one of their own) orders
+ * them first.
  */
 bcc_status bcc_check_device(bcc_ctx* ctx, bcc_robot robot, const float* d_edges,
                             int32_t num_edges, int32_t resolution, uint8_t* d_results,
