@@ -147,8 +147,8 @@ bcc_status bcc_pack_envs(const bcc_env_soa* envs, float* records, int32_t* env_o
  * Stage timing.  With profiling on, every check records CUDA events around its
  * stages on the launch stream; bcc_stage_times returns the last check's device
  * milliseconds (after the stream has been synchronised by the caller):
- *   [0] discretisation + sample offsets  [1] forward kinematics table
- *   [2] self-collision                    [3] swept cull volumes
+ *   [0] discretisation + sample offsets  [1] forward kinematics and self-collision
+ *   [2] nothing (self-collision had it)   [3] swept cull volumes
  *   [4] environment check (the dominant kernel)
  * Returns the number of stages written, or -1.
  */
